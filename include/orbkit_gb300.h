@@ -130,6 +130,12 @@ int okg_rho(const okg_basis* basis, const okg_grid* grid, int nmo, const double*
             int ndrv, const int* h_drv, int exact_mixed, double* d_rho, double* d_drho, int64_t ld,
             double* d_mo_norm, okg_stream stream);
 
+/* Whether a device wait of an okg_rho / okg_eval_mo call expired (OKG_ERR_TIMEOUT; the
+ * outputs of that call are then incomplete) since the last query; clears the record.  The
+ * device writes it during the call: query it after waiting for the call's stream.  Large
+ * calls run on the tensor cores with waits between the warps of a block, each bounded. */
+int okg_wait_status(int* status);
+
 /* ------------------------------------------------ operations on given grids
  * FP64 operations on AO / MO values the caller already holds on the device, every
  * array row-major (row, point) with points contiguous and its own leading dimension

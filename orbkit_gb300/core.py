@@ -187,6 +187,7 @@ def _eval(qc_geo, ao_spec, mo_spec, x, y, z, is_vector, what, drv_codes, exact_m
             o = torch.empty((nd, nmo, j - i), dtype=torch.float64, device=dev)
             _lib.check(L.okg_eval_mo(b.handle, gd, nmo, _lib.ptr(C), nd, codes, em, _lib.ptr(o), j - i, st))
             out[:, :, i:j] = o.cpu().numpy()
+        _lib.check(L.okg_wait_status(None))
         return out
     if occ is None:
         occ = numpy.array([m["occ_num"] for m in mo_spec], dtype=numpy.float64)
@@ -205,6 +206,7 @@ def _eval(qc_geo, ao_spec, mo_spec, x, y, z, is_vector, what, drv_codes, exact_m
         rho[i:j] = r.cpu().numpy()
         if nd:
             drho[:, i:j] = dr[:nd].cpu().numpy()
+    _lib.check(L.okg_wait_status(None))
     if mo_norm:
         return rho, drho, norm_d.cpu().numpy()
     return rho, drho

@@ -82,11 +82,15 @@ __global__ void prim_weights_kernel(const double* __restrict__ prim_in, const in
 // tile keeps a prefix of them when screening (the radial sums do not depend on
 // the order).  One thread per shell, insertion sort (a handful of primitives).
 // The FP64 {alpha, w} copy used for the cusp points of the mixed path is sorted
-// along (same permutation).
+// along (same permutation), and the FP64 tensor-core path's tables are filled in the
+// sorted order; *flags is raised by a parameter or position that is not a number.
 __global__ void sort_prim_mx_kernel(const Shell* __restrict__ shells, int nshell, PrimMx* __restrict__ prim_mx,
-                                    double2* __restrict__ prim_cusp)
+                                    double2* __restrict__ prim_cusp, const double* __restrict__ atoms, int natom,
+                                    float4* __restrict__ split_lg, SplitPrim* __restrict__ split_pr, int* __restrict__ flags)
 {
     int s = blockIdx.x * blockDim.x + threadIdx.x;
+    for (int i = s; i < natom; i += gridDim.x * blockDim.x)
+        if (!isfinite(atoms[4 * i]) || !isfinite(atoms[4 * i + 1]) || !isfinite(atoms[4 * i + 2])) atomicOr(flags, 1);
     if (s >= nshell) return;
     const int p0 = shells[s].prim0, np = shells[s].nprim;
     for (int i = 1; i < np; ++i) {
@@ -101,11 +105,14 @@ __global__ void sort_prim_mx_kernel(const Shell* __restrict__ shells, int nshell
         prim_mx[p0 + j + 1] = v;
         prim_cusp[p0 + j + 1] = c;
     }
+    for (int i = 0; i < np; ++i)
+        if (!split_prim(prim_cusp[p0 + i], split_lg[p0 + i], split_pr[p0 + i])) atomicOr(flags, 1);
 }
 
-__global__ void atoms_kernel(const double* __restrict__ geo, int natom, double* __restrict__ atoms)
+__global__ void atoms_kernel(const double* __restrict__ geo, int natom, double* __restrict__ atoms, int* __restrict__ flags)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) *flags = 0;
     if (i >= natom) return;
     atoms[4 * i + 0] = geo[3 * i + 0];
     atoms[4 * i + 1] = geo[3 * i + 1];
@@ -209,6 +216,21 @@ cudaError_t upload_mixed(okg_basis* b, const MixedLayout& m)
     if (e == cudaSuccess)
         e = cudaMemcpy((void*)d.mcol_g, m.mcol_g.data(), sizeof(double) * m.mcol_g.size(), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) d.nmchunk = (int)m.mchunks.size();
+    return e;
+}
+
+// Upload the FP64 tensor-core path's panels (capacity: one panel per shell).
+cudaError_t upload_split(okg_basis* b, const SplitLayout& m)
+{
+    SplitDev& d = b->split;
+    auto put = [](const void* dst, const auto& v) {
+        return cudaMemcpy((void*)dst, v.data(), sizeof(v[0]) * v.size(), cudaMemcpyHostToDevice);
+    };
+    cudaError_t e = put(d.shell, m.shell);
+    if (e == cudaSuccess) e = put(d.panel, m.panel);
+    if (e == cudaSuccess) e = put(d.col_cart, m.col_cart);
+    if (e == cudaSuccess) e = put(d.col_g, m.col_g);
+    if (e == cudaSuccess) d.npanel = (int)m.panel.size() - 1;
     return e;
 }
 }  // namespace
@@ -364,6 +386,14 @@ extern "C" int okg_basis_create(int natom, int nshell, const int* h_shell_atom, 
     const size_t o_mch = lay.take(sizeof(int4) * nshell);
     const size_t o_mcc = lay.take(sizeof(int) * OKG_MKC * nshell);
     const size_t o_mcg = lay.take(sizeof(double) * OKG_MKC * nshell);
+    const size_t o_ssh = lay.take(sizeof(int4) * nshell);
+    const size_t o_spn = lay.take(sizeof(int) * (nshell + 1));
+    const size_t o_scc = lay.take(sizeof(int) * OKG_SPLIT_PK * nshell);
+    const size_t o_scg = lay.take(sizeof(double) * OKG_SPLIT_PK * nshell);
+    const size_t o_slg = lay.take(sizeof(float4) * nprim);
+    const size_t o_spr = lay.take(sizeof(SplitPrim) * nprim);
+    const size_t o_sfl = lay.take(sizeof(int));
+    const size_t o_exp = lay.take(sizeof(uint64_t) * OKG_SPLIT_EXP);
     const size_t bytes = lay.take(0);
     char* blk = nullptr;
     cudaError_t e = cudaMalloc((void**)&blk, bytes);
@@ -405,6 +435,17 @@ extern "C" int okg_basis_create(int natom, int nshell, const int* h_shell_atom, 
     d.mcol_cart = (const int*)(blk + o_mcc);
     d.mcol_g = (const double*)(blk + o_mcg);
     if (e == cudaSuccess) e = upload_mixed(b, mixed);
+    b->split.shell = (const int4*)(blk + o_ssh);
+    b->split.panel = (const int*)(blk + o_spn);
+    b->split.col_cart = (const int*)(blk + o_scc);
+    b->split.col_g = (const double*)(blk + o_scg);
+    b->split.prim_lg = (const float4*)(blk + o_slg);
+    b->split.prim = (const SplitPrim*)(blk + o_spr);
+    b->split.flags = (const int*)(blk + o_sfl);
+    b->split.exp_tab = (const uint64_t*)(blk + o_exp);
+    if (e == cudaSuccess) e = upload_split(b, split_layout(shells, comp_row, comp_g, nullptr));
+    if (e == cudaSuccess)
+        e = cudaMemcpy(blk + o_exp, split_exp_table(), sizeof(uint64_t) * OKG_SPLIT_EXP, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
         cudaFree(blk);
         free(b);
@@ -474,6 +515,7 @@ extern "C" int okg_basis_set_mixed_order(okg_basis* b, const int* h_order)
     if (e == cudaSuccess)
         e = cudaMemcpy(comp_g.data(), b->dev.comp_g, sizeof(double) * b->ncomp, cudaMemcpyDeviceToHost);
     if (e == cudaSuccess) e = upload_mixed(b, mixed_layout(shells, comp_row, comp_g, h_order));
+    if (e == cudaSuccess) e = upload_split(b, split_layout(shells, comp_row, comp_g, h_order));
     return cuda_status(e, "okg_basis_set_mixed_order");
 }
 
@@ -500,12 +542,15 @@ extern "C" int okg_basis_set_params(okg_basis* b, const double* d_geo, const dou
 {
     if (!b || !d_geo || !d_prim) return set_error(OKG_ERR_ARG, "okg_basis_set_params: NULL argument");
     cudaStream_t st = (cudaStream_t)stream;
-    atoms_kernel<<<(b->natom + 127) / 128, 128, 0, st>>>(d_geo, b->natom, (double*)b->dev.atoms);
+    atoms_kernel<<<(b->natom + 127) / 128, 128, 0, st>>>(d_geo, b->natom, (double*)b->dev.atoms,
+                                                          (int*)b->split.flags);
     prim_weights_kernel<<<(b->nprim + 127) / 128, 128, 0, st>>>(d_prim, b->prim_L, b->nprim, b->is_normalized,
                                                                  (double*)b->dev.prim, (float*)b->dev.prim32,
                                                                  (PrimMx*)b->dev.prim_mx, (double*)b->dev.prim_adj,
                                                                  (double2*)b->dev.prim_cusp);
     sort_prim_mx_kernel<<<(b->nshell + 127) / 128, 128, 0, st>>>(b->dev.shells, b->nshell, (PrimMx*)b->dev.prim_mx,
-                                                                 (double2*)b->dev.prim_cusp);
+                                                                 (double2*)b->dev.prim_cusp, b->dev.atoms, b->natom,
+                                                                 (float4*)b->split.prim_lg, (SplitPrim*)b->split.prim,
+                                                                 (int*)b->split.flags);
     return cuda_status(cudaGetLastError(), "okg_basis_set_params");
 }

@@ -257,6 +257,9 @@ extern "C" int okg_eval_mo(const okg_basis* b, const okg_grid* grid, int nmo, co
     A.mixed_ref = !exact_mixed;
     A.out = d_out;
     A.ld = ld;
+    bool done = false;
+    const SplitCall sc{nmo, d_coeff, nullptr, A.drv, mask | 1u, true, d_out, nullptr, nullptr, ld};
+    if ((st = split_run(b, g, sc, (cudaStream_t)stream, done)) || done) return st;
     return dispatch_fused<true>(b, g, A, mask | 1u, (cudaStream_t)stream);
 }
 
@@ -292,6 +295,9 @@ extern "C" int okg_rho(const okg_basis* b, const okg_grid* grid, int nmo, const 
     A.dout = d_drho;
     A.mo_norm = d_mo_norm;
     A.ld = ld;
+    bool done = false;
+    const SplitCall sc{nmo, d_coeff, d_occ, A.drv, need, false, d_rho, d_drho, d_mo_norm, ld};
+    if ((st = split_run(b, g, sc, (cudaStream_t)stream, done)) || done) return st;
     // (the MO-norm sums reduce over warps of one MO group: 64-point CTAs only)
     if (g.npts <= FEW_MAX_POINTS && !A.mo_norm) return dispatch_few(b, g, A, need, (cudaStream_t)stream);
     return dispatch_fused<false>(b, g, A, need, (cudaStream_t)stream);

@@ -14,6 +14,7 @@
 #include <utility>
 
 #include "../../include/orbkit_gb300.h"
+#include "okg_split64.cuh"
 
 #define OKG_MAX_L 4
 #define OKG_MAX_NCART 15  // (L+1)(L+2)/2 at L = 4
@@ -249,6 +250,7 @@ __host__ __device__ inline bool need_r2(unsigned m) { return (m & (CH_HESS_D | C
 // Host-side helpers shared by the translation units (okg_api.cu).
 struct okg_basis {
     okg::BasisDev dev;
+    okg::SplitDev split;  // tables of the FP64 path on the tensor cores
     void* dev_block;  // single device allocation holding every table
     size_t dev_bytes;
     int* h_shell_L;   // unused (kept zero)
@@ -307,4 +309,30 @@ inline int make_drv(int ndrv, const int* h_drv, DrvList& d, unsigned& mask)
     }
     return OKG_OK;
 }
+
+// FP64 path on the tensor cores (okg_split64.cu).
+struct SplitLayout {
+    std::vector<int4> shell;
+    std::vector<int> panel, col_cart;
+    std::vector<double> col_g;
+};
+// Column panels of a shell order (order: nshell shell indices, or null for basis order).
+SplitLayout split_layout(const std::vector<Shell>& shells, const std::vector<int>& comp_row,
+                         const std::vector<double>& comp_g, const int* order);
+const uint64_t* split_exp_table();                   // host, OKG_SPLIT_EXP entries
+
+struct SplitCall {
+    int nmo;
+    const double* C;    // nmo x ncart
+    const double* occ;  // nmo, or null for MO output
+    DrvList drv;
+    unsigned need;      // channels (bit mask of drv codes, values included)
+    bool mo_out;
+    double* out;
+    double* dout;
+    double* mo_norm;
+    long long ld;
+};
+// Runs the call on the tensor cores if it is one for them (done = true), else leaves it.
+int split_run(const okg_basis* b, const Grid& g, const SplitCall& c, cudaStream_t st, bool& done);
 }  // namespace okg

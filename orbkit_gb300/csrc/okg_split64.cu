@@ -1,0 +1,1591 @@
+// FP64-accurate AO -> MO -> density on the tensor cores (the large calls of okg_rho and
+// okg_eval_mo, value / gradient / Laplacian channels).
+//
+// Reference computation: orbkit/c_grid-based.c:9-79 (AOs), orbkit/cy_core.pyx:82-101
+// (MO = C . AO) and orbkit/core.py:266-304 (density and derivatives).
+//
+// Why: the FP64 pipe runs 2 FMAs per clock and SM (6.3e11 FMA/s), so the contraction
+// C . AO, 4 NMO NAO FMAs per point with gradients, bounds a DFMA kernel.  The FP16
+// tensor cores are 1500 times faster, and an FP64 product can be composed of exact
+// small-integer products (K. Ozaki et al., "Error-free transformations of matrix
+// multiplication", Numer. Algorithms 59 (2012)):
+//   * every AO value a (FP64) of a grid point is scaled by a power of two 2^-E above the
+//     largest AO of that point and rounded to a 55-bit integer, cut into 7 balanced
+//     base-256 digits (-128 .. 127); the coefficients likewise per MO;
+//   * digit products are integers below 2^14; sums over up to 160 columns stay below
+//     2^24, so the FP32 accumulators of tcgen05.mma hold them exactly;
+//   * the products d_i(a) d_j(c) with i + j = w have the weight 2^(-14 - 8 w); w = 0..6
+//     are kept, 7 accumulators per MO; what is left out is below 2^-52 of the largest
+//     product, less than the rounding of an FP64 accumulation of the same sum.
+//
+// Screening.  A shell (and the steep primitives of a shell) whose bound over the tile's
+// points lies 2^-62 below a value that the scale 2^E of every point is known to reach
+// cannot change a digit and is left out, and so are panels of 16 columns without a kept
+// shell.  Bounds are taken per channel class (values, first, second derivatives).
+//
+// Tile: 128 operand rows (2 x 128 with second derivatives): 128 points x 1 channel, or
+// 32 points x (value, d/dx, d/dy, d/dz) [+ 32 x (xx, yy, zz, unused)].  Persistent CTAs,
+// one per SM, tiles handed out by a device counter; warps of a CTA:
+//   8 generation warps  FP64 radial sums and polynomials of the kept shells, digits
+//                       written to the panel's operand slot (ring of slots);
+//   4 epilogue warps    accumulators -> FP64 MO values (integer arithmetic) -> outputs;
+//   1 MMA warp, 1 coefficient loader (bulk copies), 1 tile warp (screening, scales).
+// Every wait is bounded and raises the status word instead of hanging (okg_wait_status).
+//
+// What bounds it (20 atoms, 180 AOs, 40 MOs, 160^3 points, density and gradient): 16.6 ms
+// against 234 ms of the DFMA kernel, per 32-point tile and SM 39 K cycles, of which the
+// FP64 pipe needs about 9 K and the tensor cores 4 K; the rest is the latency of the
+// integer code (digits, exponentials, conversion of the accumulators), which is why the
+// kernel runs with 23 warps of 80 registers: 8 generation warps in lock step with 128
+// registers took 21.2 ms.
+#include <cuda_fp16.h>
+#include <math.h>
+
+#include <mutex>
+#include <vector>
+
+#include "okg_internal.cuh"
+#include "okg_split64.cuh"
+#include "okg_tc.cuh"
+
+namespace okg {
+namespace sp {
+
+using namespace mx;
+
+constexpr int ND = 7;                   // digits of an operand
+constexpr int PK = OKG_SPLIT_PK;        // columns of a panel: one MMA K-step
+constexpr int DT = 128 * PK * 2;        // bytes of one digit of one 128-row operand tile
+constexpr int GROUP = 10;               // panels per accumulation (exact FP32 sums: see the header)
+constexpr int MAX_SHELLS = 2048;
+constexpr int MAX_PANELS = 768;
+constexpr int NBUF = 4;                 // tile buffers
+constexpr int NTW = 2;                  // tile warps, each with every second buffer
+constexpr int MAX_BIG = 512;
+constexpr int TABN = OKG_SPLIT_EXP;     // entries of the 2^(j/2048) table
+constexpr int SMEM_MAX = 232448;
+constexpr int ROW_NAN = 30000, ROW_ZERO = 30001;  // row exponents of points without finite AO values
+constexpr int MO_NAN = 200000;                      // exponent of an MO with a non-finite coefficient
+constexpr float KEEP_LOG2 = 62.0f;
+constexpr float ABS_FLOOR = -1000.0f;   // values below 2^-1000 are dropped
+
+template <int NCH>
+struct Cfg {
+    static constexpr int RG = NCH == 7 ? 2 : 1;       // 128-row operand tiles
+    static constexpr int PTS = NCH == 1 ? 128 : 32;   // points of an operand tile
+    static constexpr int SUB = PTS / 32;              // points per lane of an operand tile
+    static constexpr int NCLS = NCH == 1 ? 1 : NCH == 4 ? 2 : 3;
+    // Warps.  Most of the kernel's time is latency (integer digit and exponential code, a
+    // slow FP64 pipe), so values and gradients run with 23 warps of 80 registers; second
+    // derivatives need 128 registers (15 warps).
+    static constexpr int TEAM = 4;                         // generation warps working on one panel
+    static constexpr int NTEAM = NCH == 7 ? 2 : 3;         // panels under generation at a time
+    static constexpr int NGW = TEAM * NTEAM;
+    static constexpr int EPQ = NCH == 7 ? 1 : 2;           // epilogue warps per 32 accumulator rows
+    static constexpr int NEW = 4 * EPQ;
+    static constexpr int NT = 32 * (NGW + NEW + NTW + 1);
+};
+
+struct Args {
+    BasisDev B;
+    SplitDev S;
+    Grid g;
+    int nmo, np, npass;           // MOs, columns per pass (multiple of 16), passes
+    const unsigned char* bpack;   // [npass][npanel][7 np rows x 32 B]
+    const int* fexp;              // [npass np] exponent of each MO's coefficients
+    const double* occ;            // [npass np] occupations, zero padded
+    unsigned long long* counter;  // tile counter, zero at launch
+    double* phi;                  // per CTA [RG][np][128] partial MO values (bases beyond GROUP panels)
+    int* status;                  // raised when a wait expires
+    DrvList drv;
+    double* out;                  // MO output: ndrv x nmo x ld; density: rho
+    double* dout;                 // density: ndrv x ld
+    double* mo_norm;              // density: nmo sums of MO^2, or null
+    long long ld, ntiles;
+    int brick, nby, nbz;
+    int nsub;                     // 32-point runs of a tile: 4 (128 points), or 1 for few points with derivatives
+    int nslot, nacc;              // operand slots, accumulator sets
+    unsigned tm_cols;
+    int norm_smem;                // the MO norms are summed in shared memory
+};
+
+// ------------------------------------------------------------------ tile geometry
+// Point r of a tile: a brick of nsub x 4 x 8 points of a whole regular grid, else 32 nsub
+// consecutive points.
+__device__ __forceinline__ bool tile_point(const Args& A, long long tile, int r, long long& p, double& x, double& y,
+                                           double& z)
+{
+    if (A.brick) {
+        const long long nbyz = (long long)A.nby * A.nbz;
+        int bi, rem;
+        if (A.ntiles < 0x7FFFFFFFll) {
+            bi = (int)tile / (int)nbyz;
+            rem = (int)tile - bi * (int)nbyz;
+        } else {
+            bi = (int)(tile / nbyz);
+            rem = (int)(tile - (long long)bi * nbyz);
+        }
+        const int bj = rem / A.nbz, bk = rem - bj * A.nbz;
+        const int i = bi * A.nsub + (r >> 5), j = bj * 4 + ((r >> 3) & 3), k = bk * 8 + (r & 7);
+        const bool valid = i < A.g.nx && j < A.g.ny && k < A.g.nz;
+        x = __ldg(A.g.x + (i < A.g.nx ? i : A.g.nx - 1));
+        y = __ldg(A.g.y + (j < A.g.ny ? j : A.g.ny - 1));
+        z = __ldg(A.g.z + (k < A.g.nz ? k : A.g.nz - 1));
+        p = valid ? ((long long)i * A.g.ny + j) * A.g.nz + k : 0;
+        return valid;
+    }
+    p = tile * (32 * A.nsub) + r;
+    const bool valid = p < A.g.npts;
+    if (!valid) p = A.g.npts - 1;
+    grid_point(A.g, p, x, y, z);
+    return valid;
+}
+
+// ------------------------------------------------------------------ shared memory
+struct State {
+    unsigned char* slots;   // nslot x (operand digits, coefficient digits)
+    uint32_t slot_bytes, a_bytes;
+    uint64_t* tab;          // 2^(63 - j/2048)
+    long long* tile;        // NBUF
+    int* npan;              // NBUF
+    double* pts;            // value channel: NBUF x 3 x 128 coordinates
+    short* rowexp;          // NBUF x 3 x 128
+    unsigned short* plist;  // NBUF x MAX_PANELS
+    unsigned char* nkeep;   // NBUF x MAX_SHELLS
+    unsigned short* big;    // NTW x MAX_BIG (tile warps)
+    unsigned* pbits;        // NTW x MAX_PANELS / 32 (tile warps)
+    double* norm;           // 8 x npass np, when A.norm_smem
+    double* part;           // 4 x 32: density sums of the second epilogue warp of a row group
+    int* last_use;          // nslot: last phase whose coefficient copy was requested, or -1
+    int* abort_flag;
+    uint32_t full, empty, bfull;          // nslot mbarriers each, 8 B apart
+    uint32_t acc_full, acc_empty;         // 2 each
+    uint32_t screened, kfree;             // NBUF each
+    uint32_t part_full, part_free;        // 4 each
+    uint32_t drain;
+    uint32_t tmem;
+};
+constexpr int MAX_SLOTS = 6;
+constexpr int NBAR = 3 * MAX_SLOTS + 4 + 2 * NBUF + 8 + 1;
+constexpr int AUX_BYTES = TABN * 8 + NBUF * 8 + NBUF * 4 + MAX_SLOTS * 4 + 8 + NBUF * 2 * 3 * 128 + NBUF * MAX_PANELS * 2 +
+                          NBUF * MAX_SHELLS + NTW * MAX_BIG * 2 + NTW * MAX_PANELS / 8 +
+                          NBAR * 8 + 4 * 32 * 8 + 64;
+
+// Bounded wait that also ends when another role gave up.
+__device__ __forceinline__ bool wait(const State& S, uint32_t bar, uint32_t parity, int* status)
+{
+    for (long long it = 0; it < WAIT_LIMIT; ++it) {
+        if (mbar_try(bar, parity)) return true;
+        if ((it & 255) == 255 && *(volatile int*)S.abort_flag) return false;
+    }
+    atomicExch(status, 1);
+    *(volatile int*)S.abort_flag = 1;
+    return false;
+}
+
+// One answer for the warp (collective instructions follow).
+__device__ __forceinline__ bool warp_wait(const State& S, uint32_t bar, uint32_t parity, int* status)
+{
+    return __all_sync(0xffffffffu, wait(S, bar, parity, status));
+}
+
+// ------------------------------------------------------------------ digits
+// v = t 2^(E - 55), t rounded to an integer of 7 balanced base-256 digits; returned
+// biased by 128 per digit (byte b holds digit + 128), rs0 = E + 1030.  Integer
+// instructions only; |v| < 0.99 2^E.
+__device__ __forceinline__ uint64_t digits7(double v, int rs0)
+{
+    const int hi = __double2hiint(v);
+    const unsigned lo = (unsigned)__double2loint(v);
+    const int ex = (hi >> 20) & 0x7FF;
+    const unsigned mh = ((unsigned)hi & 0xFFFFFu) | 0x100000u;
+    const uint64_t m = ((uint64_t)__funnelshift_l(lo, mh, 10) << 32) | (uint64_t)(lo << 10);
+    int s = rs0 - 1 - ex;
+    s = s < 7 ? 7 : s > 63 ? 63 : s;
+    const uint64_t q = ((m >> s) + 1) >> 1;
+    const uint64_t neg = (uint64_t)(long long)(hi >> 31);
+    return ((q ^ neg) - neg) + 0x0080808080808080ull;
+}
+
+// Two biased digit bytes (byte b of two values) -> two FP16 digits.
+__device__ __forceinline__ uint32_t digit_pair(uint32_t w0, uint32_t w1, int b)
+{
+    const uint32_t r = (__byte_perm(w0, w1, (uint32_t)(b | (b << 4) | ((4 + b) << 8) | (b << 12))) & 0x00FF00FFu) | 0x64006400u;
+    const __half2 h = __hsub2(*reinterpret_cast<const __half2*>(&r), __half2(__ushort_as_half(0x6480), __ushort_as_half(0x6480)));
+    return *reinterpret_cast<const uint32_t*>(&h);
+}
+
+// byte offset of (row m, column k) in a 128 x 16 FP16 digit tile: M-major, 128-byte
+// swizzle (64 rows per 128-byte line, lines of 8 columns per atom)
+__device__ __forceinline__ uint32_t a_off(int m, int k)
+{
+    return (uint32_t)((m >> 6) * 1024 + (k >> 3) * 2048 + (k & 7) * 128 + ((((m >> 3) ^ k) & 7) << 4) + ((m & 7) << 1));
+}
+
+// byte offset of (row n, column k) of the coefficient digits: K-major, 32-byte rows,
+// 32-byte swizzle
+__host__ __device__ __forceinline__ uint32_t b_off(int n, int k)
+{
+    return (uint32_t)((n >> 3) * 256 + (n & 7) * 32 + ((((k >> 3) ^ (n >> 2)) & 1) << 4) + ((k & 7) << 1));
+}
+
+__device__ __forceinline__ uint64_t a_desc(uint32_t addr)
+{
+    return (uint64_t)((addr >> 4) & 0x3FFF) | ((uint64_t)(1024 >> 4) << 16) | ((uint64_t)(2048 >> 4) << 32) |
+           ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
+}
+__device__ __forceinline__ uint64_t b_desc(uint32_t addr)
+{
+    return (uint64_t)((addr >> 4) & 0x3FFF) | ((uint64_t)1 << 16) | ((uint64_t)(256 >> 4) << 32) | ((uint64_t)1 << 46) |
+           ((uint64_t)6 << 61);
+}
+// kind::f16, A = B = FP16, D = FP32, M-major A, K-major B, M = 128
+__host__ __device__ constexpr uint32_t idesc(int n) { return (1u << 4) | (1u << 15) | ((uint32_t)(n >> 3) << 17) | (8u << 24); }
+
+__device__ __forceinline__ void mma_f16(uint32_t d, uint64_t a, uint64_t b, uint32_t id, uint32_t acc)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d),
+        "l"(a), "l"(b), "r"(id), "r"(acc));
+}
+
+// ------------------------------------------------------------------ FP64 AO values
+// e^(-alpha rr) as an FP64 value in integer arithmetic (the FP64 pipe is what bounds this
+// kernel: an FP64 exponential took 9 of its operations per primitive and point, this one
+// takes none).  mr 2^er = rr with a 64-bit mantissa; A 2^ea = alpha log2(e) likewise.
+//   u = alpha log2(e) rr from the upper half of mr A, as a fixed-point number with 53
+//   fraction bits: integer part k, 11 bits j, remainder f (42 bits);
+//   e = 2^-k 2^(-j/2048) 2^-f, 2^(-j/2048) from a table of 64-bit fixed-point numbers
+//   (table-driven exponential after P. T. P. Tang, ACM TOMS 15 (1989)) and
+//   2^-f = 1 - f (c1 - f (c2 - f (c3 - f c4))), c_n = (ln 2)^n / n! (f < 2^-11: the first
+//   term left out is below 2^-65), the inner terms in 32 bits.
+// Error before the final rounding: 0.7 2^-53 relative (the truncation of u).
+__device__ __forceinline__ double exp_neg(uint64_t mr, int er, uint64_t A, int ea, const uint64_t* __restrict__ tab)
+{
+    int s = -(er + ea) - 117;
+    const uint64_t Y = __umul64hi(mr, A) >> (s > 63 ? 63 : s < 0 ? 0 : s);
+    const int k = (int)(Y >> 53);
+    const uint64_t T = tab[(unsigned)(Y >> 42) & (TABN - 1)];
+    const uint64_t F = Y << 22;
+    const unsigned fh = (unsigned)(F >> 32);
+    const unsigned r3 = 3814213304u - (__umulhi(fh, 2643811198u) >> 13);
+    const unsigned r2 = 4127059964u - (__umulhi(fh, r3) >> 13);
+    const uint64_t c = 0xB17217F7D1CF79ACull - (((uint64_t)fh * r2) >> 13);
+    const uint64_t E = T - (__umul64hi(T, __umul64hi(F, c)) >> 11);
+    const int lz = __clz((int)(E >> 32));
+    const uint64_t n = E << lz;
+    const uint64_t m = (n >> 11) + ((n >> 10) & 1);
+    const uint64_t bits = m + ((uint64_t)(unsigned)(1022 - lz - k) << 52);
+    return (s < 0 || k > 1000) ? 0.0 : __longlong_as_double((long long)bits);
+}
+
+__device__ __noinline__ double slow_exp(double x) { return exp(x); }
+
+// position of x^a y^b z^c among the monomials of its degree
+__host__ __device__ constexpr int midx(int a, int b, int c) { return (b + c) * (b + c + 1) / 2 + c; }
+
+// s times the monomials of degree D from those of degree D - 1, in place
+template <int D>
+__device__ __forceinline__ void raise(double* T, double X, double Y, double Z)
+{
+    T[midx(0, 0, D)] = Z * T[midx(0, 0, D - 1)];
+#pragma unroll
+    for (int c = D - 1; c >= 0; --c) T[midx(0, D - c, c)] = Y * T[midx(0, D - c - 1, c)];
+#pragma unroll
+    for (int i = 0; i < D * (D + 1) / 2; ++i) T[i] *= X;
+}
+template <int N0, int N1>
+__device__ __forceinline__ void raise_to(double* T, double X, double Y, double Z)
+{
+    if constexpr (N0 < N1) {
+        raise<N0 + 1>(T, X, Y, Z);
+        raise_to<N0 + 1, N1>(T, X, Y, Z);
+    }
+}
+
+// Power of two nearest to the inverse of the angular norm 1/sqrt((2a-1)!!(2b-1)!!(2c-1)!!) of
+// a component: the operand holds 2^-shift chi, the coefficients the rest of the norm, so
+// that no column takes digits from the others.
+__host__ __device__ constexpr int norm_shift(int a, int b, int c)
+{
+    constexpr int s[5] = {0, 0, 1, 2, 3};  // 1, 1, 3, 15, 105
+    if (a == 2 && b == 2 || a == 2 && c == 2 || b == 2 && c == 2) return 2;  // 9
+    return s[a] > s[b] ? (s[a] > s[c] ? s[a] : s[c]) : (s[b] > s[c] ? s[b] : s[c]);
+}
+
+// Values, gradients and pure second derivatives of every canonical component of a shell:
+// with S0 = R0, S1 = -2 R1, S2 = 4 R2,
+//   chi = P S0,  d_x chi = P x S1 + a (P/x) S0,  d_xx chi = P x^2 S2 + (2a + 1) P S1 + a (a-1) (P/x^2) S0,
+// about 1.5 FP64 operations per value (monomials built with the radial sum as a factor).
+template <int L, int NCH, typename Sink>
+__device__ __forceinline__ void shell_values(double X, double Y, double Z, double R0, double S1, double S2, Sink&& sink)
+{
+    constexpr int N = (L + 1) * (L + 2) / 2;
+    double V[N], Vm[L > 0 ? N - L - 1 : 1], Vmm[L > 1 ? N - 2 * L - 1 : 1];
+    double G[NCH >= 4 ? (L + 2) * (L + 3) / 2 : 1], G0[NCH == 7 ? N : 1];
+    double H[NCH == 7 ? (L + 3) * (L + 4) / 2 : 1];
+    V[0] = R0;
+    if constexpr (L >= 2) {
+        raise_to<0, L - 2>(V, X, Y, Z);
+        if constexpr (NCH == 7)
+            for (int i = 0; i < N - 2 * L - 1; ++i) Vmm[i] = V[i];
+        raise<L - 1>(V, X, Y, Z);
+    }
+    if constexpr (L >= 1) {
+        if constexpr (NCH >= 4)
+            for (int i = 0; i < N - L - 1; ++i) Vm[i] = V[i];
+        raise<L>(V, X, Y, Z);
+    }
+    if constexpr (NCH >= 4) {
+        G[0] = S1;
+        raise_to<0, L>(G, X, Y, Z);
+        if constexpr (NCH == 7)
+            for (int i = 0; i < N; ++i) G0[i] = G[i];
+        raise<L + 1>(G, X, Y, Z);
+    }
+    if constexpr (NCH == 7) {
+        H[0] = S2;
+        raise_to<0, L + 2>(H, X, Y, Z);
+    }
+    [&]<int... J>(std::integer_sequence<int, J...>) {
+        (
+            [&] {
+                constexpr int a = canon_l(L, J, 0), b = canon_l(L, J, 1), c = canon_l(L, J, 2);
+                double v[NCH];
+                v[0] = V[midx(a, b, c)];
+                if constexpr (NCH >= 4) {
+                    v[1] = G[midx(a + 1, b, c)];
+                    v[2] = G[midx(a, b + 1, c)];
+                    v[3] = G[midx(a, b, c + 1)];
+                    if constexpr (a > 0) v[1] = fma((double)a, Vm[midx(a - 1, b, c)], v[1]);
+                    if constexpr (b > 0) v[2] = fma((double)b, Vm[midx(a, b - 1, c)], v[2]);
+                    if constexpr (c > 0) v[3] = fma((double)c, Vm[midx(a, b, c - 1)], v[3]);
+                }
+                if constexpr (NCH == 7) {
+                    const double g0 = G0[midx(a, b, c)];
+                    v[4] = fma((double)(2 * a + 1), g0, H[midx(a + 2, b, c)]);
+                    v[5] = fma((double)(2 * b + 1), g0, H[midx(a, b + 2, c)]);
+                    v[6] = fma((double)(2 * c + 1), g0, H[midx(a, b, c + 2)]);
+                    if constexpr (a > 1) v[4] = fma((double)(a * (a - 1)), Vmm[midx(a - 2, b, c)], v[4]);
+                    if constexpr (b > 1) v[5] = fma((double)(b * (b - 1)), Vmm[midx(a, b - 2, c)], v[5]);
+                    if constexpr (c > 1) v[6] = fma((double)(c * (c - 1)), Vmm[midx(a, b, c - 2)], v[6]);
+                }
+                sink(J, norm_shift(a, b, c), v);
+            }(),
+            ...);
+    }(std::make_integer_sequence<int, N>{});
+}
+
+__device__ __forceinline__ void sts16(uint32_t a, unsigned v) { asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "h"((unsigned short)v) : "memory"); }
+__device__ __forceinline__ void sts64(uint32_t a, uint32_t x, uint32_t y) { asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(a), "r"(x), "r"(y) : "memory"); }
+
+// Digits of one column value (value channel alone) into the 7 digit tiles.  A call, like
+// put4: the digit code appears once instead of once per component and angular momentum
+// (inlined, the kernel's hot code was far beyond the instruction cache: 30 % of its
+// instruction requests missed).
+__device__ __noinline__ void put1(double v, int rs, uint32_t a)
+{
+    const uint64_t t = digits7(v, rs);
+    const uint32_t lo = (uint32_t)t, hi = (uint32_t)(t >> 32);
+    // digit 0 is the most significant byte (byte 6)
+    const uint32_t h20 = digit_pair(hi, hi >> 16, 0), h1 = digit_pair(hi, hi, 1);
+    const uint32_t h64 = digit_pair(lo, lo >> 16, 0), h53 = digit_pair(lo, lo >> 16, 1);
+    sts16(a + 0 * DT, h20 >> 16);
+    sts16(a + 1 * DT, h1);
+    sts16(a + 2 * DT, h20);
+    sts16(a + 3 * DT, h53 >> 16);
+    sts16(a + 4 * DT, h64 >> 16);
+    sts16(a + 5 * DT, h53);
+    sts16(a + 6 * DT, h64);
+}
+
+// Digits of four rows (channels of a point) of a column.
+__device__ __noinline__ void put4(double v0, double v1, double v2, double v3, int rs0, int rs1, uint32_t a)
+{
+    const uint64_t t0 = digits7(v0, rs0), t1 = digits7(v1, rs1), t2 = digits7(v2, rs1), t3 = digits7(v3, rs1);
+#pragma unroll
+    for (int i = 0; i < ND; ++i) {
+        const int b = 6 - i;
+        if (b >= 4)
+            sts64(a + i * DT, digit_pair((uint32_t)(t0 >> 32), (uint32_t)(t1 >> 32), b - 4),
+                  digit_pair((uint32_t)(t2 >> 32), (uint32_t)(t3 >> 32), b - 4));
+        else
+            sts64(a + i * DT, digit_pair((uint32_t)t0, (uint32_t)t1, b), digit_pair((uint32_t)t2, (uint32_t)t3, b));
+    }
+}
+
+// Values of one shell at the lane's point into the slot; row: first operand row of the
+// point (4 rows per point with derivatives, else 1).
+template <int L, int NCH>
+__device__ __forceinline__ void put_shell(uint32_t slot, int col, double X, double Y, double Z, double R0, double S1,
+                                          double S2, int row, int e0, int e1, int e2)
+{
+    shell_values<L, NCH>(X, Y, Z, R0, S1, S2, [&](int j, int sh, const double* v) {
+        const uint32_t a = slot + a_off(row, col + j);
+        if constexpr (NCH == 1) {
+            put1(v[0], e0 + sh, a);
+        } else {
+            put4(v[0], v[1], v[2], v[3], e0 + sh, e1 + sh, a);
+            if constexpr (NCH == 7) put4(v[4], v[5], v[6], 0.0, e2 + sh, e2 + sh, a + ND * DT);
+        }
+    });
+}
+
+template <int NCH>
+__device__ __forceinline__ void gen_shell(const Args& A, const State& S, uint32_t slot, int L, int col, int prim0, int nk,
+                                          double X, double Y, double Z, int row, int e0, int e1, int e2)
+{
+    const double rr = X * X + Y * Y + Z * Z;
+    // rr = mr 2^er, mr with its top bit set (rr = 0: a value far below any alpha's range)
+    const unsigned rh = (unsigned)__double2hiint(rr), rl = (unsigned)__double2loint(rr);
+    const int er = (int)(rh >> 20) - 1086;
+    const uint64_t mr = ((uint64_t)__funnelshift_l(rl, (rh & 0xFFFFFu) | 0x100000u, 11) << 32) | (uint64_t)(rl << 11);
+    // radial sums R0 = sum w e, S1 = -2 sum w alpha e, S2 = 4 sum w alpha^2 e
+    double R0 = 0.0, S1 = 0.0, S2 = 0.0;
+#pragma unroll 1
+    for (int q = 0; q < nk; ++q) {
+        const SplitPrim* pr = A.S.prim + prim0 + q;
+        const ulonglong2 ae = __ldg((const ulonglong2*)pr);
+        const double2 w01 = __ldg((const double2*)pr + 1);
+        double e = exp_neg(mr, er, ae.x, (int)(ae.y >> 32), S.tab);
+        if ((int)ae.y) e = slow_exp(__ldg(&pr->neg_alpha) * rr);  // alpha <= 0
+        R0 = fma(w01.x, e, R0);
+        if (NCH >= 4) S1 = fma(w01.y, e, S1);
+        if (NCH == 7) S2 = fma(__ldg(&pr->w2), e, S2);
+    }
+    switch (L) {
+    case 0: put_shell<0, NCH>(slot, col, X, Y, Z, R0, S1, S2, row, e0, e1, e2); break;
+    case 1: put_shell<1, NCH>(slot, col, X, Y, Z, R0, S1, S2, row, e0, e1, e2); break;
+    case 2: put_shell<2, NCH>(slot, col, X, Y, Z, R0, S1, S2, row, e0, e1, e2); break;
+    case 3: put_shell<3, NCH>(slot, col, X, Y, Z, R0, S1, S2, row, e0, e1, e2); break;
+    default: put_shell<4, NCH>(slot, col, X, Y, Z, R0, S1, S2, row, e0, e1, e2); break;
+    }
+}
+
+// Accumulation groups of a tile with n kept panels: nearly equal, at most GROUP panels.
+__device__ __forceinline__ int ngroups(int n) { return (n + GROUP - 1) / GROUP; }
+__device__ __forceinline__ int group_begin(int n, int ng, int g) { return n * g / ng; }
+
+// The tile warps take turns with the buffers (warp w: buffers of ordinal w mod NTW); a tile
+// of -1 ends one tile warp's sequence, the consumers go on with the other's.
+struct TileSeq {
+    unsigned ord = 0, ended = 0;
+    // next buffer, or -1 (all sequences ended, or the wait gave up)
+    template <bool WARP>
+    __device__ __forceinline__ int next(const State& S, int* status, long long& tile)
+    {
+        for (;; ++ord) {
+            if ((ended >> (ord % NTW)) & 1u) continue;
+            const int b = ord % NBUF;
+            const bool ok = WARP ? warp_wait(S, S.screened + 8 * b, (ord / NBUF) & 1, status)
+                                 : wait(S, S.screened + 8 * b, (ord / NBUF) & 1, status);
+            if (!ok) return -1;
+            tile = S.tile[b];
+            if (tile >= 0) {
+                ++ord;
+                return b;
+            }
+            ended |= 1u << (ord % NTW);
+            if (ended == (1u << NTW) - 1u) return -1;
+        }
+    }
+};
+
+// Generation: team t of TEAM warps fills the operand slots of the panels t, t + NTEAM, ...
+// (the shells of a panel are dealt to the team's warps); lane 0 of the team's first warp
+// also requests the panel's coefficient digits (bulk copy).
+template <int NCH>
+__device__ __forceinline__ void gen_role(const Args& A, const State& S)
+{
+    using C = Cfg<NCH>;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, team = warp / C::TEAM, tw = warp % C::TEAM;
+    int* status = A.status;
+    const uint32_t bytes = (uint32_t)(ND * A.np * PK * 2);
+    unsigned seq = 0, turn = 0;
+    TileSeq ts;
+    long long tile;
+    bool ok = true;
+    while (ok) {
+        const int b = ts.next<true>(S, status, tile);
+        if (b < 0) break;
+        const int npan = S.npan[b];
+        const unsigned short* plist = S.plist + b * MAX_PANELS;
+        const unsigned char* nkeep = S.nkeep + b * MAX_SHELLS;
+        const short* rowexp = S.rowexp + b * 3 * 128;
+        for (int sub = 0; ok && sub < A.nsub; sub += C::SUB) {
+            double px = 0.0, py = 0.0, pz = 0.0;
+            int e0 = 0, e1 = 0, e2 = 0;
+            if (NCH >= 4) {
+                long long p;
+                tile_point(A, tile, sub * 32 + lane, p, px, py, pz);
+                e0 = rowexp[sub * 32 + lane] + 1030;
+                e1 = rowexp[128 + sub * 32 + lane] + 1030;
+            }
+            if (NCH == 7) e2 = rowexp[256 + sub * 32 + lane] + 1030;
+            for (int pp = 0, pi = 0, pass = 0; pp < A.npass * npan; ++pp, ++pi, ++seq) {
+                if (pi == npan) {
+                    pi = 0;
+                    ++pass;
+                }
+                if (seq % C::NTEAM != (unsigned)team) continue;
+                const unsigned sl = seq % (unsigned)A.nslot, use = seq / (unsigned)A.nslot;
+                const int pan = plist[pi];
+                const int s0 = __ldg(A.S.panel + pan), cnt = __ldg(A.S.panel + pan + 1) - s0;
+                int4 rec = make_int4(0, 0, 0, 0);
+                int nk = 0;
+                if (lane < cnt) {
+                    rec = __ldg(A.S.shell + s0 + lane);
+                    nk = nkeep[s0 + lane];
+                }
+                const unsigned kept = __ballot_sync(0xffffffffu, nk > 0);
+                if (use > 0 && !warp_wait(S, S.empty + 8 * sl, (use - 1) & 1, status)) {
+                    ok = false;
+                    break;
+                }
+                const uint32_t slot = smem_u32(S.slots) + sl * S.slot_bytes;
+                if (tw == 0 && lane == 0) {
+                    S.last_use[sl] = (int)use;
+                    bulk_load(slot + S.a_bytes, A.bpack + ((size_t)pass * A.S.npanel + pan) * bytes, bytes, S.bfull + 8 * sl);
+                }
+                unsigned m = kept;
+                while (m) {
+                    const int i = __ffs(m) - 1;
+                    m &= m - 1;
+                    if (turn++ % C::TEAM != (unsigned)tw) continue;
+                    const int atom = __shfl_sync(0xffffffffu, rec.x, i), pk = __shfl_sync(0xffffffffu, rec.y, i),
+                              prim0 = __shfl_sync(0xffffffffu, rec.z, i), nkq = __shfl_sync(0xffffffffu, nk, i);
+                    const double ax = __ldg(A.B.atoms + 4 * atom), ay = __ldg(A.B.atoms + 4 * atom + 1),
+                                 az = __ldg(A.B.atoms + 4 * atom + 2);
+#pragma unroll 1
+                    for (int q = 0; q < C::SUB; ++q) {
+                        if (NCH == 1) {
+                            const double* pt = S.pts + b * 3 * 128 + q * 32 + lane;
+                            px = pt[0];
+                            py = pt[128];
+                            pz = pt[256];
+                            e0 = rowexp[q * 32 + lane] + 1030;
+                        }
+                        gen_shell<NCH>(A, S, slot, pk & 0xFF, (pk >> 8) & 0xFF, prim0, nkq, px - ax, py - ay, pz - az,
+                                       NCH == 1 ? q * 32 + lane : 4 * lane, e0, e1, e2);
+                    }
+                }
+                // the columns of screened shells hold an earlier panel's digits: zeros
+                m = (cnt < 32 ? (1u << cnt) - 1u : 0xffffffffu) & ~kept;
+                while (m) {
+                    const int i = __ffs(m) - 1;
+                    m &= m - 1;
+                    if (turn++ % C::TEAM != (unsigned)tw) continue;
+                    const int pk = __shfl_sync(0xffffffffu, rec.y, i);
+                    const int L = pk & 0xFF, col = (pk >> 8) & 0xFF, nc = (L + 1) * (L + 2) / 2;
+                    // per column and digit two 128-byte lines: 16 lanes of 16 bytes
+                    const uint32_t z0 = slot + ((lane >> 3) & 1) * 1024 + (lane & 7) * 16;
+                    for (int k = col; k < col + nc; ++k)
+#pragma unroll 1
+                        for (int dg = lane >> 4; dg < ND * C::RG; dg += 2)
+                            asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(z0 + dg * DT + (k >> 3) * 2048 + (k & 7) * 128), "r"(0) : "memory");
+                }
+                fence_proxy_async();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(S.full + 8 * sl);
+            }
+        }
+        __syncwarp();
+        if (ok && lane == 0) mbar_arrive(S.kfree + 8 * b);
+    }
+    __syncwarp();
+}
+
+template <int NCH>
+__device__ __forceinline__ void mma_role(const Args& A, const State& S)
+{
+    if ((threadIdx.x & 31) != 0) return;
+    using C = Cfg<NCH>;
+    int* status = A.status;
+    const int np = A.np, dmax = 256 / np;  // digits per instruction (N <= 256)
+    unsigned seq = 0, job = 0;
+    bool ok = true, issued = false;
+    TileSeq ts;
+    long long tile;
+    while (ok) {
+        const int b = ts.next<false>(S, status, tile);
+        if (b < 0) break;
+        const int npan = S.npan[b], ng = ngroups(npan);
+        for (int pg = 0; ok && pg < A.nsub / C::SUB * A.npass * ng; ++pg, ++job) {
+            const int gr = pg % ng;
+            const unsigned ab = job % (unsigned)A.nacc, ause = job / (unsigned)A.nacc;
+            if (ause > 0 && !wait(S, S.acc_empty + 8 * ab, (ause - 1) & 1, status)) {
+                ok = false;
+                break;
+            }
+            tc_fence_after();
+            const uint32_t acc = S.tmem + ab * (uint32_t)(C::RG * ND * np);
+            const int p0 = group_begin(npan, ng, gr), p1 = group_begin(npan, ng, gr + 1);
+            for (int pi = p0; pi < p1; ++pi, ++seq) {
+                const unsigned sl = seq % (unsigned)A.nslot, ph = (seq / (unsigned)A.nslot) & 1;
+                if (!wait(S, S.bfull + 8 * sl, ph, status) ||
+                    !wait(S, S.full + 8 * sl, ph, status)) {
+                    ok = false;
+                    break;
+                }
+                tc_fence_after();
+                const uint32_t sa = smem_u32(S.slots + sl * S.slot_bytes), sb = sa + S.a_bytes;
+#pragma unroll 1
+                for (int rg = 0; rg < C::RG; ++rg)
+#pragma unroll 1
+                    for (int i = 0; i < ND; ++i) {
+                        // digit i of the AOs times digits 0 .. 6 - i of the coefficients:
+                        // neighbouring accumulators, one instruction per dmax digits
+                        const uint64_t ad = a_desc(sa + (uint32_t)(rg * ND + i) * DT);
+#pragma unroll 1
+                        for (int j = 0; j < ND - i; j += dmax) {
+                            const int nd = ND - i - j < dmax ? ND - i - j : dmax;
+                            mma_f16(acc + (uint32_t)((rg * ND + i + j) * np), ad, b_desc(sb + (uint32_t)(j * np * PK * 2)),
+                                    idesc(nd * np), (pi > p0 || i > 0) ? 1u : 0u);
+                        }
+                    }
+                mma_commit(S.empty + 8 * sl);
+                issued = true;
+            }
+            if (ok) mma_commit(S.acc_full + 8 * ab);
+        }
+        if (ok) mbar_arrive(S.kfree + 8 * b);
+    }
+    if (issued) {
+        mma_commit(S.drain);
+        mbar_drain(S.drain, 0);
+    }
+}
+
+// ------------------------------------------------------------------ epilogue
+// Seven accumulators of four MOs (columns n0 .. n0 + 3) of this lane's row.
+struct Acc4 {
+    uint32_t r[7][4];
+};
+__device__ __forceinline__ void acc_load(Acc4& a, uint32_t taddr, int np)
+{
+#pragma unroll
+    for (int w = 0; w < 7; ++w)
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                     : "=r"(a.r[w][0]), "=r"(a.r[w][1]), "=r"(a.r[w][2]), "=r"(a.r[w][3])
+                     : "r"(taddr + (uint32_t)(w * np)));
+}
+// (the loaded registers are operands: no use of them moves before the wait)
+__device__ __forceinline__ void acc_wait(Acc4& a)
+{
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(a.r[0][0]), "+r"(a.r[0][1]), "+r"(a.r[0][2]), "+r"(a.r[0][3]), "+r"(a.r[1][0]), "+r"(a.r[1][1]), "+r"(a.r[1][2]), "+r"(a.r[1][3]), "+r"(a.r[2][0]), "+r"(a.r[2][1]), "+r"(a.r[2][2]), "+r"(a.r[2][3]), "+r"(a.r[3][0]), "+r"(a.r[3][1]), "+r"(a.r[3][2]), "+r"(a.r[3][3]), "+r"(a.r[4][0]), "+r"(a.r[4][1]), "+r"(a.r[4][2]), "+r"(a.r[4][3]), "+r"(a.r[5][0]), "+r"(a.r[5][1]), "+r"(a.r[5][2]), "+r"(a.r[5][3]), "+r"(a.r[6][0]), "+r"(a.r[6][1]), "+r"(a.r[6][2]), "+r"(a.r[6][3]));
+}
+
+__device__ __forceinline__ int f2i(uint32_t r) { return __float2int_rn(__uint_as_float(r)); }
+
+// sum_w acc_w 2^(-8 w) 2^x as an FP64 value, rounded once, in integer arithmetic (a
+// conversion on the FP64 pipe would cost its bound): t = sum acc_w 2^(40 - 8 w) in 64
+// bits, x = scale - 40 included by the caller.
+__device__ __forceinline__ double combine7(const int (&a)[7], int x)
+{
+    const long long lo = (long long)a[4] * 256 + a[5] + ((a[6] + 128) >> 8);
+    const long long t = (((long long)(a[0] * 256 + a[1])) << 32) + ((long long)(a[2] * 256 + a[3]) << 16) + lo;
+    const unsigned long long neg = (unsigned long long)(t >> 63);
+    const unsigned long long u = ((unsigned long long)t ^ neg) - neg;
+    const int lz = __clzll((long long)u);
+    const unsigned long long n = u << (lz & 63);
+    const unsigned long long m = (n >> 11) + ((n >> 10) & 1);  // 53 bits, rounded
+    const int e = 1023 + 63 - lz + x;                          // biased exponent of the leading bit
+    if (u == 0 || e <= 0) return 0.0;
+    if (e >= 0x7FF) return __hiloint2double((int)(0x7FF00000u | (unsigned)(neg & 0x80000000u)), 0);
+    const unsigned long long bits = ((unsigned long long)(unsigned)(e - 1) << 52) + m;
+    return __longlong_as_double((long long)(bits | (neg & 0x8000000000000000ull)));
+}
+
+// Accumulators of four MOs -> FP64 values of this lane's row.
+__device__ __forceinline__ void acc_values(const Acc4& a, int rowx, const int4& f4, double (&v)[4])
+{
+    const int f[4] = {f4.x, f4.y, f4.z, f4.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int t[7] = {f2i(a.r[0][i]), f2i(a.r[1][i]), f2i(a.r[2][i]), f2i(a.r[3][i]), f2i(a.r[4][i]), f2i(a.r[5][i]), f2i(a.r[6][i])};
+        // a = t 2^(E - 55), c = s 2^(F - 55); leading digits weigh 2^48: products 2^(E + F - 14)
+        v[i] = combine7(t, rowx + f[i] - 54);
+        if (rowx >= ROW_NAN || f[i] == MO_NAN) v[i] = (rowx == ROW_ZERO && f[i] != MO_NAN) ? 0.0 : __longlong_as_double(0x7FF8000000000000ll);
+    }
+}
+
+__device__ __forceinline__ double shfl_d(double v, int src)
+{
+    return __hiloint2double(__shfl_sync(0xffffffffu, __double2hiint(v), src),
+                            __shfl_sync(0xffffffffu, __double2loint(v), src));
+}
+
+// o 2^x v: through the exponent field where the occupation o is a power of two (2, 1, ...;
+// the FP64 pipe is the bound), the same value as the product.
+__device__ __forceinline__ double times_occ(double v, double o, int x)
+{
+    const int ho = __double2hiint(o), eo = (ho >> 20) & 0x7FF;
+    if ((ho & 0xFFFFF) == 0 && __double2loint(o) == 0 && eo > 0 && eo < 0x7FF) {
+        const int hv = __double2hiint(v), ev = (hv >> 20) & 0x7FF, e = ev + eo - 1023 + x;
+        if (ev > 0 && ev < 0x7FF && e > 0 && e < 0x7FF)
+            return __hiloint2double((hv & 0x800FFFFF) ^ (int)((unsigned)ho & 0x80000000u) | (e << 20), __double2loint(v));
+    }
+    return (x ? 2.0 * o : o) * v;
+}
+
+template <int NCH, bool MO_OUT>
+__device__ __forceinline__ void epi_role(const Args& A, const State& S)
+{
+    using C = Cfg<NCH>;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, quad = warp & 3;
+    const int half = (warp - C::NGW) >> 2;            // of a row group's EPQ warps: MOs 4 half, 4 half + 4 EPQ, ...
+    const int row = quad * 32 + lane;                 // accumulator row
+    const int pt = NCH == 1 ? row : row >> 2;         // point of the tile
+    const int ch = NCH == 1 ? 0 : lane & 3;           // channel (of the first row tile)
+    const int lane0 = NCH == 1 ? lane : lane & ~3;    // lane of the point's value
+    int* status = A.status;
+    const int np = A.np;
+    double* phi = A.phi ? A.phi + (size_t)blockIdx.x * C::RG * np * 128 + row : nullptr;
+    unsigned job = 0, round = 0;
+    TileSeq ts;
+    long long tile;
+    for (;;) {
+        const int b = ts.next<true>(S, status, tile);
+        if (b < 0) return;
+        const int npan = S.npan[b], ng = ngroups(npan);
+        const short* rowexp = S.rowexp + b * 3 * 128;
+        for (int sub = 0; sub < A.nsub; sub += C::SUB) {
+            const int rx0 = rowexp[(ch == 0 ? 0 : 128) + sub * 32 + pt], rx1 = NCH == 7 ? rowexp[256 + sub * 32 + pt] : 0;
+            long long p;
+            double px, py, pz;
+            const bool valid = tile_point(A, tile, sub * 32 + pt, p, px, py, pz);
+            double accs[2] = {0.0, 0.0}, acc1 = 0.0;
+            for (int pass = 0; pass < A.npass; ++pass) {
+                const int* fexp = A.fexp + pass * np;
+                for (int gr = 0; gr < (ng ? ng : 1); ++gr) {
+                    const unsigned ab = job % (unsigned)A.nacc, ause = job / (unsigned)A.nacc;
+                    const bool last = gr + 1 >= ng;
+                    uint32_t taddr = S.tmem + ab * (uint32_t)(C::RG * ND * np) + ((uint32_t)(quad * 32) << 16);
+                    if (ng) {
+                        if (!warp_wait(S, S.acc_full + 8 * ab, ause & 1, status)) return;
+                        tc_fence_after();
+                    }
+                    const int nmo = A.nmo - pass * np < np ? A.nmo - pass * np : np;  // MOs of this pass
+                    Acc4 va, ua;
+#pragma unroll 1
+                    for (int n0 = 4 * half; n0 < nmo; n0 += 4 * C::EPQ) {
+                        double v[4], u[4];
+                        const int4 f4 = __ldg((const int4*)(fexp + n0));
+                        if (ng) {
+                            acc_load(va, taddr + (uint32_t)n0, np);
+                            if (NCH == 7) acc_load(ua, taddr + (uint32_t)(ND * np + n0), np);
+                            acc_wait(va);
+                            if (NCH == 7) acc_wait(ua);
+                            acc_values(va, rx0, f4, v);
+                            if (NCH == 7) acc_values(ua, rx1, f4, u);
+                            if (ng > 1) {
+#pragma unroll
+                                for (int i = 0; i < 4; ++i) {
+                                    double* q = phi + (size_t)(n0 + i) * 128;
+                                    if (gr > 0) v[i] += *q;
+                                    if (!last) *q = v[i];
+                                    if (NCH == 7) {
+                                        q += (size_t)np * 128;
+                                        if (gr > 0) u[i] += *q;
+                                        if (!last) *q = u[i];
+                                    }
+                                }
+                            }
+                        } else {
+                            // no shell reaches this tile: zeros (or NaN where the input has it)
+                            const int f[4] = {f4.x, f4.y, f4.z, f4.w};
+#pragma unroll
+                            for (int i = 0; i < 4; ++i)
+                                v[i] = u[i] = (rx0 == ROW_NAN || f[i] == MO_NAN) ? __longlong_as_double(0x7FF8000000000000ll) : 0.0;
+                        }
+                        if (!last) continue;
+                        if (MO_OUT) {
+                            for (int d = 0; d < A.drv.n; ++d) {
+                                const int code = A.drv.code[d];
+                                const bool first = code < 4;
+                                if (!valid || (first ? ch != code : (NCH != 7 || ch != code - 4))) continue;
+                                double* out = A.out + ((long long)d * A.nmo + pass * np + n0) * A.ld + p;
+#pragma unroll
+                                for (int i = 0; i < 4; ++i)
+                                    if (n0 + i < nmo) out[i * A.ld] = first ? v[i] : (NCH == 7 ? u[i] : 0.0);
+                            }
+                        } else {
+                            double q2[4];
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) {
+                                const double o = __ldg(A.occ + pass * np + n0 + i);
+                                if (NCH == 1) {
+                                    q2[i] = v[i] * v[i];
+                                    accs[i & 1] = fma(o, q2[i], accs[i & 1]);
+                                } else {
+                                    const double f = shfl_d(v[i], lane0);
+                                    accs[i & 1] = fma(times_occ(f, o, ch == 0 ? 0 : 1), v[i], accs[i & 1]);
+                                    if (NCH == 7) {
+                                        const double dv = shfl_d(v[i], lane0 + ((ch + 1) & 3));
+                                        acc1 = fma(times_occ(f, o, 1), u[i], acc1);
+                                        acc1 = fma(times_occ(dv, o, 1), dv, acc1);
+                                    }
+                                    if (A.mo_norm) q2[i] = ch == 0 ? v[i] * v[i] : 0.0;
+                                }
+                            }
+                            if (A.mo_norm) {
+                                // sums of q2[i] over the warp, four MOs at once: after two halving
+                                // exchanges lane l holds MO (l & 3) of its 4-lane group
+                                double s2[2], s1;
+#pragma unroll
+                                for (int i = 0; i < 4; ++i) q2[i] = valid ? q2[i] : 0.0;
+#pragma unroll
+                                for (int i = 0; i < 2; ++i) {
+                                    const double keep = (lane & 2) ? q2[i + 2] : q2[i], give = (lane & 2) ? q2[i] : q2[i + 2];
+                                    s2[i] = keep + shfl_d(give, lane ^ 2);
+                                }
+                                {
+                                    const double keep = (lane & 1) ? s2[1] : s2[0], give = (lane & 1) ? s2[0] : s2[1];
+                                    s1 = keep + shfl_d(give, lane ^ 1);
+                                }
+#pragma unroll
+                                for (int o = 4; o < 32; o *= 2) s1 += shfl_d(s1, lane ^ o);
+                                if (lane < 4 && n0 + lane < nmo) {
+                                    const int mo = pass * np + n0 + lane;
+                                    if (A.norm_smem)
+                                        S.norm[(warp - C::NGW) * A.npass * np + mo] += s1;
+                                    else
+                                        atomicAdd(A.mo_norm + mo, s1);
+                                }
+                                __syncwarp();
+                            }
+                        }
+                    }
+                    if (ng) {
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(S.acc_empty + 8 * ab);
+                        ++job;
+                    }
+                }
+            }
+            double acc0 = accs[0] + accs[1];
+            if (!MO_OUT && C::EPQ == 2) {
+                // the two halves of the MO sum meet in shared memory
+                if (half == 1) {
+                    if (round > 0 && !warp_wait(S, S.part_free + 8 * quad, (round - 1) & 1, status)) return;
+                    S.part[quad * 32 + lane] = acc0;
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(S.part_full + 8 * quad);
+                } else {
+                    if (!warp_wait(S, S.part_full + 8 * quad, round & 1, status)) return;
+                    acc0 += S.part[quad * 32 + lane];
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(S.part_free + 8 * quad);
+                }
+                ++round;
+            }
+            if (!MO_OUT && valid && half == 0) {
+                if (ch == 0) A.out[p] = acc0;
+                for (int d = 0; d < A.drv.n; ++d) {
+                    const int code = A.drv.code[d];
+                    if (code == 0) {
+                        // a density "derivative" of order 0: 2 occ MO^2
+                        if (ch == 0) A.dout[(long long)d * A.ld + p] = 2.0 * acc0;
+                    } else if (code < 4) {
+                        if (ch == code) A.dout[(long long)d * A.ld + p] = acc0;
+                    } else if (NCH == 7 && ch == code - 4) {
+                        A.dout[(long long)d * A.ld + p] = acc1;
+                    }
+                }
+            }
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(S.kfree + 8 * b);
+    }
+}
+
+// ------------------------------------------------------------------ tile warp
+// Bounds of a shell's operand values 2^-shift P R at one point, from the distance r and the
+// largest coordinate q = max(|x|, |y|, |z|) relative to its atom: with t = q, c = 1 and with
+// t = r, c = 2^-b (b = 0, 0, 1, 2, 3 for L = 0 .. 4: what the component shifts leave of r^L)
+//   |P| <= c t^L =: p0,
+//   |dP R| <= p1 R0 + 2 q1 R1,  p1 = c L t^(L-1), q1 = c t^(L+1),
+//   |ddP R| <= p2 R0 + 2 (2L+1) p0 R1 + 4 q2 R2,  p2 = c L(L-1) t^(L-2), q2 = c t^(L+2);
+// every factor is taken from the smaller of the two.
+struct Poly {
+    float p0, p1, p2, q1, q2;
+};
+__device__ __forceinline__ Poly poly1(int L, float t, float c)
+{
+    Poly f{c, 0.f, 0.f, 0.f, 0.f};
+    for (int i = 0; i < L; ++i) {
+        f.p2 = 2.f * f.p1 + f.p2 * t;
+        f.p1 = f.p0 + f.p1 * t;
+        f.p0 *= t;
+    }
+    f.q1 = f.p0 * t;
+    f.q2 = f.q1 * t;
+    return f;
+}
+__device__ __forceinline__ Poly poly(int L, float r, float q)
+{
+    const Poly a = poly1(L, q, 1.f), b = poly1(L, r, L < 2 ? 1.f : L == 2 ? 0.5f : L == 3 ? 0.25f : 0.125f);
+    return Poly{fminf(a.p0, b.p0), fminf(a.p1, b.p1), fminf(a.p2, b.p2), fminf(a.q1, b.q1), fminf(a.q2, b.q2)};
+}
+
+// Squared distances from an atom to the tile's box and its largest coordinate relative to
+// the atom, smallest and largest over the box.
+struct BoxRange {
+    float dmin, dmax, qmin, qmax;
+};
+__device__ __forceinline__ BoxRange box_range(const Args& A, int atom, double ox, double oy, double oz, const float (&lo)[3],
+                                              const float (&hi)[3])
+{
+    const float a[3] = {(float)(__ldg(A.B.atoms + 4 * atom) - ox), (float)(__ldg(A.B.atoms + 4 * atom + 1) - oy),
+                        (float)(__ldg(A.B.atoms + 4 * atom + 2) - oz)};
+    BoxRange o{0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        const float u = fmaxf(0.f, fmaxf(lo[c] - a[c], a[c] - hi[c]));
+        const float v = fmaxf(fabsf(lo[c] - a[c]), fabsf(hi[c] - a[c]));
+        o.dmin = fmaf(u, u, o.dmin);
+        o.dmax = fmaf(v, v, o.dmax);
+        o.qmin = fmaxf(o.qmin, u);
+        o.qmax = fmaxf(o.qmax, v);
+    }
+    return o;
+}
+
+// Raises top (log2, per channel class) to a shell's bound at squared distances dd:
+// sum over the primitives relative to the largest.
+template <int NCLS, int NQ>
+__device__ __forceinline__ void point_bounds(const float4* __restrict__ pl, int np, int L, const float (&dd)[NQ],
+                                             const float (&dq)[NQ], float (&top)[NQ][NCLS])
+{
+    float m[NQ], R0[NQ], R1[NQ], R2[NQ];
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        m[q] = -3.0e38f;
+        R0[q] = R1[q] = R2[q] = 0.f;
+    }
+    for (int i = 0; i < np; ++i) {
+        const float4 v = __ldg(pl + i);
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) m[q] = fmaxf(m[q], fmaf(-v.x, dd[q], v.y));
+    }
+    for (int i = 0; i < np; ++i) {
+        const float4 v = __ldg(pl + i);
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            const float e = exp2f(fmaf(-v.x, dd[q], v.y) - m[q]);
+            R0[q] += e;
+            if (NCLS > 1) R1[q] = fmaf(fabsf(v.z), e, R1[q]);
+            if (NCLS > 2) R2[q] = fmaf(v.z * v.z, e, R2[q]);
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        if (m[q] < -1.0e30f) continue;
+        const Poly f = poly(L, sqrtf(dd[q]), dq[q]);
+        top[q][0] = fmaxf(top[q][0], m[q] + __log2f(f.p0 * R0[q]));
+        if (NCLS > 1) top[q][1] = fmaxf(top[q][1], m[q] + __log2f(f.p1 * R0[q] + 2.f * f.q1 * R1[q]));
+        if (NCLS > 2)
+            top[q][2] = fmaxf(top[q][2],
+                              m[q] + __log2f(f.p2 * R0[q] + 2.f * (2 * L + 1) * f.p0 * R1[q] + 4.f * f.q2 * R2[q]));
+    }
+}
+
+template <int NCH>
+__device__ __forceinline__ void tile_role(const Args& A, const State& S, int tw)
+{
+    using C = Cfg<NCH>;
+    constexpr int NCLS = C::NCLS, NQ = 4;
+    const int lane = threadIdx.x & 31;
+    int* status = A.status;
+    const int nshell = A.B.nshell, nsub = A.nsub;
+    unsigned short* bigl = S.big + tw * MAX_BIG;
+    unsigned* pbits = S.pbits + tw * (MAX_PANELS / 32);
+    for (unsigned ord = tw;; ord += NTW) {
+        const int b = ord % NBUF;
+        const bool ok = ord < NBUF || warp_wait(S, S.kfree + 8 * b, ((ord / NBUF) - 1) & 1, status);
+        long long t = -1;
+        if (lane == 0 && ok) {
+            t = (long long)atomicAdd(A.counter, 1ull);
+            if (t >= A.ntiles) t = -1;
+        }
+        t = __shfl_sync(0xffffffffu, t, 0);
+        if (lane == 0) S.tile[b] = t;
+        if (t < 0) {
+            __syncwarp();
+            if (lane == 0) mbar_arrive(S.screened + 8 * b);
+            return;
+        }
+        // points relative to one of them (single precision keeps the distances to the
+        // nearby atoms); points at |coordinate| >= 2^60 or non-finite are set apart
+        float fx[NQ], fy[NQ], fz[NQ];
+        int special[NQ];
+        double ox = 0.0, oy = 0.0, oz = 0.0;
+        bool have = false;
+        float lo[3] = {3.0e38f, 3.0e38f, 3.0e38f}, hi[3] = {-3.0e38f, -3.0e38f, -3.0e38f};
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            special[q] = 0;
+            fx[q] = fy[q] = fz[q] = 0.f;
+            if (q >= nsub) continue;
+            long long p;
+            double x, y, z;
+            tile_point(A, t, q * 32 + lane, p, x, y, z);
+            if (NCH == 1) {
+                double* pt = S.pts + b * 3 * 128 + q * 32 + lane;
+                pt[0] = x;
+                pt[128] = y;
+                pt[256] = z;
+            }
+            const int h = max(__double2hiint(x) & 0x7FFFFFFF, max(__double2hiint(y) & 0x7FFFFFFF, __double2hiint(z) & 0x7FFFFFFF));
+            special[q] = h >= 0x7FF00000 ? ROW_NAN : h >= 0x43B00000 ? ROW_ZERO : 0;
+            const unsigned first = __ballot_sync(0xffffffffu, special[q] == 0);
+            if (!have && first) {
+                const int src = __ffs(first) - 1;
+                ox = shfl_d(x, src);
+                oy = shfl_d(y, src);
+                oz = shfl_d(z, src);
+                have = true;
+            }
+            if (special[q] == 0) {
+                fx[q] = (float)(x - ox);
+                fy[q] = (float)(y - oy);
+                fz[q] = (float)(z - oz);
+                lo[0] = fminf(lo[0], fx[q]);
+                hi[0] = fmaxf(hi[0], fx[q]);
+                lo[1] = fminf(lo[1], fy[q]);
+                hi[1] = fmaxf(hi[1], fy[q]);
+                lo[2] = fminf(lo[2], fz[q]);
+                hi[2] = fmaxf(hi[2], fz[q]);
+            }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                lo[c] = fminf(lo[c], __shfl_xor_sync(0xffffffffu, lo[c], o));
+                hi[c] = fmaxf(hi[c], __shfl_xor_sync(0xffffffffu, hi[c], o));
+            }
+        for (int i = lane; i < MAX_PANELS / 32; i += 32) pbits[i] = 0u;
+        __syncwarp();
+        unsigned char* nkeep = S.nkeep + b * MAX_SHELLS;
+        int npan = 0, nbig = 0;
+        const bool bad = __ldg(A.S.flags) != 0;  // a parameter or position that is not a number
+        float ref[3] = {-3.0e38f, -3.0e38f, -3.0e38f};
+        if (have && !bad) {
+            // what the scale of every point of the tile is known to reach: the largest
+            // lower bound of a shell over the tile's box (one primitive's share of it)
+            for (int s = lane; s < nshell; s += 32) {
+                const int4 rec = __ldg(A.S.shell + s);
+                const int L = rec.y & 0xFF, np = rec.w;
+                const BoxRange br = box_range(A, rec.x, ox, oy, oz, lo, hi);
+                float m = -3.0e38f, al = 0.f;
+                for (int q = 0; q < np; ++q) {
+                    const float4 v = __ldg(A.S.prim_lg + rec.z + q);
+                    const float l = v.y - fmaxf(v.x * br.dmin, v.x * br.dmax);
+                    al = l > m ? v.z : al;
+                    m = fmaxf(m, l);
+                }
+                const Poly f = poly(L, sqrtf(br.dmin), br.qmin);
+                float u[3];
+                u[0] = m + __log2f(f.p0);
+                u[1] = m + __log2f(f.p1 + 2.f * al * f.q1);
+                u[2] = m + __log2f(f.p2 + al * (2.f * (2 * L + 1) * f.p0 + 4.f * al * f.q2));
+#pragma unroll
+                for (int c = 0; c < NCLS; ++c) ref[c] = fmaxf(ref[c], u[c]);
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                for (int c = 0; c < NCLS; ++c) ref[c] = fmaxf(ref[c], __shfl_xor_sync(0xffffffffu, ref[c], o));
+            // upper bounds: kept shells and primitives, and the shells that may set a scale
+            for (int sb = 0; sb < nshell; sb += 32) {
+                const int s = sb + lane;
+                int nk = 0;
+                bool big = false;
+                if (s < nshell) {
+                    const int4 rec = __ldg(A.S.shell + s);
+                    const int L = rec.y & 0xFF, np = rec.w, pan = rec.y >> 16;
+                    const BoxRange br = box_range(A, rec.x, ox, oy, oz, lo, hi);
+                    const Poly f = poly(L, sqrtf(br.dmax), br.qmax);
+                    const float lnp = __log2f((float)np), l0 = __log2f(f.p0);
+                    for (int q = 0; q < np; ++q) {
+                        const float4 v = __ldg(A.S.prim_lg + rec.z + q);
+                        const float e = v.y - fminf(v.x * br.dmin, v.x * br.dmax), a = fabsf(v.z);
+                        float u[3];
+                        u[0] = e + l0;
+                        u[1] = e + __log2f(f.p1 + 2.f * a * f.q1);
+                        u[2] = e + __log2f(f.p2 + a * (2.f * (2 * L + 1) * f.p0 + 4.f * a * f.q2));
+#pragma unroll
+                        for (int c = 0; c < NCLS; ++c) {
+                            if (u[c] > fmaxf(ref[c] - KEEP_LOG2, ABS_FLOOR)) nk = q + 1;
+                            if (u[c] + lnp >= ref[c]) big = true;
+                        }
+                    }
+                    big = big && nk > 0;
+                    nkeep[s] = (unsigned char)nk;
+                    if (nk > 0) atomicOr(pbits + (pan >> 5), 1u << (pan & 31));
+                }
+                const unsigned mb = __ballot_sync(0xffffffffu, big);
+                const int at = nbig + __popc(mb & ((1u << lane) - 1u));
+                if (big && at < MAX_BIG) bigl[at] = (unsigned short)s;
+                nbig += __popc(mb);
+            }
+            __syncwarp();
+            for (int pb = 0; pb < A.S.npanel; pb += 32) {
+                const bool k = (pbits[pb >> 5] >> lane) & 1u;
+                const unsigned mk = __ballot_sync(0xffffffffu, k);
+                if (k) S.plist[b * MAX_PANELS + npan + __popc(mk & ((1u << lane) - 1u))] = (unsigned short)(pb + lane);
+                npan += __popc(mk);
+            }
+        }
+        // the scale of every point: the largest bound at the point itself
+        float top[NQ][NCLS];
+#pragma unroll
+        for (int q = 0; q < NQ; ++q)
+#pragma unroll
+            for (int c = 0; c < NCLS; ++c) top[q][c] = ref[c];
+        const bool every = nbig > MAX_BIG;  // (more candidates than the list holds: all shells)
+        for (int i = 0; i < (every ? nshell : nbig); ++i) {
+            const int s = every ? i : bigl[i];
+            const int4 rec = __ldg(A.S.shell + s);
+            const int L = rec.y & 0xFF, nk = nkeep[s];
+            const float ax = (float)(__ldg(A.B.atoms + 4 * rec.x) - ox), ay = (float)(__ldg(A.B.atoms + 4 * rec.x + 1) - oy),
+                        az = (float)(__ldg(A.B.atoms + 4 * rec.x + 2) - oz);
+            float dd[NQ], dq[NQ];
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) {
+                const float dx = fx[q] - ax, dy = fy[q] - ay, dz = fz[q] - az;
+                dd[q] = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+                dq[q] = fmaxf(fabsf(dx), fmaxf(fabsf(dy), fabsf(dz)));
+            }
+            point_bounds<NCLS>(A.S.prim_lg + rec.z, nk, L, dd, dq, top);
+        }
+        short* rowexp = S.rowexp + b * 3 * 128;
+#pragma unroll
+        for (int q = 0; q < NQ; ++q)
+#pragma unroll
+            for (int c = 0; c < NCLS; ++c) {
+                const float e = ceilf(fminf(fmaxf(top[q][c] + 0.1f, -950.f), 990.f));
+                if (q < nsub)
+                    rowexp[c * 128 + q * 32 + lane] = (short)((bad || top[q][c] > 985.f) ? ROW_NAN : special[q] ? special[q] : (int)e);
+            }
+        if (lane == 0) S.npan[b] = npan;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(S.screened + 8 * b);
+    }
+}
+
+// ------------------------------------------------------------------ the kernel
+template <int NCH, bool MO_OUT>
+__global__ void __launch_bounds__(Cfg<NCH>::NT, 1) split_kernel(const __grid_constant__ Args A)
+{
+    using C = Cfg<NCH>;
+    constexpr int NT = C::NT, NGW = C::NGW, NEW = C::NEW;
+    extern __shared__ unsigned char raw[];
+    const int tid = threadIdx.x, warp = tid >> 5;
+    unsigned char* base = (unsigned char*)(((uintptr_t)raw + 1023) & ~(uintptr_t)1023);
+    State S;
+    S.a_bytes = C::RG * ND * DT;
+    // (the coefficient digits' 32-byte swizzle repeats every 256 bytes; slots start at 1 KB)
+    S.slot_bytes = (S.a_bytes + (uint32_t)(ND * A.np * PK * 2) + 1023u) & ~1023u;
+    S.slots = base;
+    unsigned char* q = base + (size_t)A.nslot * S.slot_bytes;
+    S.tab = (uint64_t*)q;
+    q += TABN * 8;
+    S.tile = (long long*)q;
+    q += NBUF * 8;
+    uint64_t* bar = (uint64_t*)q;
+    q += NBAR * 8;
+    S.part = (double*)q;
+    q += 4 * 32 * 8;
+    S.norm = (double*)q;
+    if (A.norm_smem) q += (size_t)NEW * A.npass * A.np * 8;
+    S.pts = (double*)q;
+    if (NCH == 1) q += NBUF * 3 * 128 * 8;
+    S.rowexp = (short*)q;
+    q += NBUF * 2 * 3 * 128;
+    S.npan = (int*)q;
+    q += NBUF * 4;
+    S.last_use = (int*)q;
+    q += MAX_SLOTS * 4;
+    S.abort_flag = (int*)q;
+    uint32_t* tmem_slot = (uint32_t*)(q + 4);
+    q += 8;
+    S.pbits = (unsigned*)q;
+    q += NTW * MAX_PANELS / 8;
+    S.plist = (unsigned short*)q;
+    q += NBUF * MAX_PANELS * 2;
+    S.big = (unsigned short*)q;
+    q += NTW * MAX_BIG * 2;
+    S.nkeep = q;
+    S.full = smem_u32(bar);
+    S.empty = smem_u32(bar + MAX_SLOTS);
+    S.bfull = smem_u32(bar + 2 * MAX_SLOTS);
+    S.acc_full = smem_u32(bar + 3 * MAX_SLOTS);
+    S.acc_empty = smem_u32(bar + 3 * MAX_SLOTS + 2);
+    S.screened = smem_u32(bar + 3 * MAX_SLOTS + 4);
+    S.kfree = smem_u32(bar + 3 * MAX_SLOTS + 4 + NBUF);
+    S.part_full = smem_u32(bar + 3 * MAX_SLOTS + 4 + 2 * NBUF);
+    S.part_free = smem_u32(bar + 3 * MAX_SLOTS + 8 + 2 * NBUF);
+    S.drain = smem_u32(bar + 3 * MAX_SLOTS + 12 + 2 * NBUF);
+    // operand slots start as zeros: columns that no shell of a panel owns stay finite
+    // (their coefficients are zero)
+    for (int i = tid; i < (int)(A.nslot * S.slot_bytes / 16); i += NT) ((uint4*)S.slots)[i] = make_uint4(0, 0, 0, 0);
+    for (int i = tid; i < TABN; i += NT) S.tab[i] = __ldg(A.S.exp_tab + i);
+    if (A.norm_smem)
+        for (int i = tid; i < NEW * A.npass * A.np; i += NT) S.norm[i] = 0.0;
+    if (tid == 0) {
+        for (int s = 0; s < A.nslot; ++s) {
+            mbar_init(S.full + 8 * s, C::TEAM);
+            mbar_init(S.empty + 8 * s, 1);
+            mbar_init(S.bfull + 8 * s, 1);
+            S.last_use[s] = -1;
+        }
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(S.acc_full + 8 * s, 1);
+            mbar_init(S.acc_empty + 8 * s, NEW);
+        }
+        for (int s = 0; s < NBUF; ++s) {
+            mbar_init(S.screened + 8 * s, 1);
+            mbar_init(S.kfree + 8 * s, NGW + NEW + 1);
+        }
+        for (int s = 0; s < 4; ++s) {
+            mbar_init(S.part_full + 8 * s, 1);
+            mbar_init(S.part_free + 8 * s, 1);
+        }
+        mbar_init(S.drain, 1);
+        *S.abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                     "r"(A.tm_cols));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    fence_proxy_async();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    S.tmem = *tmem_slot;
+
+    if (warp < NGW)
+        gen_role<NCH>(A, S);
+    else if (warp < NGW + NEW)
+        epi_role<NCH, MO_OUT>(A, S);
+    else if (warp == NGW + NEW)
+        mma_role<NCH>(A, S);
+    else
+        tile_role<NCH>(A, S, warp - (NGW + NEW + 1));
+
+    __syncwarp();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    // no coefficient copy may land after the CTA has left (all have, unless a wait gave up)
+    if (tid < A.nslot && S.last_use[tid] >= 0) mbar_drain(S.bfull + 8 * tid, S.last_use[tid] & 1);
+    if (!MO_OUT && A.mo_norm && A.norm_smem)
+        for (int i = tid; i < A.nmo; i += NT) {
+            double t = 0.0;
+            for (int w = 0; w < NEW; ++w) t += S.norm[w * A.npass * A.np + i];
+            atomicAdd(A.mo_norm + i, t);
+        }
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(S.tmem), "r"(A.tm_cols));
+}
+
+// Digits of the MO coefficients times the column norms and scales, one block per MO
+// column of the operand; block 0 also zeroes the tile counter.
+__global__ void __launch_bounds__(256) split_pack_kernel(SplitDev S, int nmo, int np, int ncart,
+                                                         const double* __restrict__ C, const double* __restrict__ occ,
+                                                         unsigned char* __restrict__ bpack, int* __restrict__ fexp,
+                                                         double* __restrict__ occ_pad, unsigned long long* counter)
+{
+    __shared__ unsigned long long top;
+    const int mo = blockIdx.x, pass = mo / np, n = mo % np, ncol = S.npanel * PK;
+    if (threadIdx.x == 0) top = 0;
+    __syncthreads();
+    auto value = [&](int i) -> double {
+        const int r = S.col_cart[i];
+        if (mo >= nmo || r < 0) return 0.0;
+        return C[(long long)mo * ncart + r] * S.col_g[i];
+    };
+    // magnitudes compare like their bit patterns (NaN and infinity last)
+    unsigned long long m = 0;
+    for (int i = threadIdx.x; i < ncol; i += blockDim.x) {
+        const unsigned long long u = (unsigned long long)__double_as_longlong(value(i)) & 0x7FFFFFFFFFFFFFFFull;
+        m = u > m ? u : m;
+    }
+    atomicMax(&top, m);
+    __syncthreads();
+    const int ex = (int)(top >> 52);
+    // exponent F with |c| < 0.99 2^F
+    int F = ex == 0 ? -1022 : ex - 1022;
+    if (((top >> 44) & 0xFF) >= 0xFA) ++F;
+    if (F < -900) F = -900;
+    const bool nan = ex == 0x7FF;
+    if (threadIdx.x == 0) {
+        fexp[mo] = nan ? MO_NAN : F;
+        occ_pad[mo] = (mo < nmo && occ) ? occ[mo] : 0.0;
+        if (mo == 0) *counter = 0ull;
+    }
+    for (int i = threadIdx.x; i < ncol; i += blockDim.x) {
+        const uint64_t t = nan ? 0x0080808080808080ull : digits7(value(i), F + 1030);
+        unsigned char* tile = bpack + ((size_t)pass * S.npanel + i / PK) * (size_t)(ND * np * PK * 2);
+#pragma unroll
+        for (int j = 0; j < ND; ++j) {
+            const int d = (int)((t >> (8 * (6 - j))) & 0xFF) - 128;
+            *(__half*)(tile + b_off(j * np + n, i % PK)) = __int2half_rn(d);
+        }
+    }
+}
+
+}  // namespace sp
+
+// ---------------------------------------------------------------- host side
+SplitLayout split_layout(const std::vector<Shell>& shells, const std::vector<int>& comp_row,
+                         const std::vector<double>& comp_g, const int* order)
+{
+    // panels of 16 columns, whole shells; a shell goes to the oldest of the last four
+    // open panels with room
+    const int n = (int)shells.size();
+    std::vector<std::vector<int>> pan;
+    std::vector<int> used;
+    for (int i = 0; i < n; ++i) {
+        const int s = order ? order[i] : i, nc = ncanon(shells[s].L);
+        int at = -1;
+        const int lo = (int)pan.size() > 4 ? (int)pan.size() - 4 : 0;
+        for (int p = lo; p < (int)pan.size() && at < 0; ++p)
+            if (used[p] + nc <= OKG_SPLIT_PK) at = p;
+        if (at < 0) {
+            at = (int)pan.size();
+            pan.emplace_back();
+            used.push_back(0);
+        }
+        pan[at].push_back(s);
+        used[at] += nc;
+    }
+    SplitLayout m;
+    m.panel.push_back(0);
+    m.col_cart.assign(pan.size() * OKG_SPLIT_PK, -1);
+    m.col_g.assign(pan.size() * OKG_SPLIT_PK, 0.0);
+    for (size_t p = 0; p < pan.size(); ++p) {
+        int col = 0;
+        for (int s : pan[p]) {
+            const Shell& sh = shells[s];
+            m.shell.push_back(make_int4(sh.atom, sh.L | (col << 8) | ((int)p << 16), sh.prim0, sh.nprim));
+            for (int q = 0; q < ncanon(sh.L); ++q) {
+                const size_t c = p * OKG_SPLIT_PK + col + q;
+                const int r = comp_row[sh.comp0 + q];
+                if (r >= 0) {
+                    m.col_cart[c] = sh.cart0 + r;
+                    m.col_g[c] = ldexp(comp_g[sh.comp0 + q],
+                                       sp::norm_shift(canon_l(sh.L, q, 0), canon_l(sh.L, q, 1), canon_l(sh.L, q, 2)));
+                }
+            }
+            col += ncanon(sh.L);
+        }
+        m.panel.push_back((int)m.shell.size());
+    }
+    return m;
+}
+
+const uint64_t* split_exp_table()
+{
+    static const std::vector<uint64_t> t = [] {
+        std::vector<uint64_t> v(OKG_SPLIT_EXP);
+        for (int j = 0; j < OKG_SPLIT_EXP; ++j)
+            v[j] = (uint64_t)roundl(ldexpl(exp2l(-(long double)j / OKG_SPLIT_EXP), 63));
+        return v;
+    }();
+    return t.data();
+}
+
+namespace {
+
+constexpr int MAX_DEVICES = 64;
+
+// Raised by a kernel whose bounded wait expired: one page-locked word per process,
+// written by the device and read by okg_wait_status after the stream was waited for.
+int* status_word()
+{
+    static int* const w = [] {
+        int* p = nullptr;
+        if (cudaHostAlloc((void**)&p, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return (int*)nullptr;
+        }
+        *p = 0;
+        return p;
+    }();
+    return w;
+}
+
+// The library's own stream-ordered pool for the coefficient digits of a call (a few MB):
+// safe for any number of threads and streams; up to 64 MB stay mapped between calls.
+cudaMemPool_t workspace_pool(int device)
+{
+    static std::mutex lock;
+    static cudaMemPool_t pools[MAX_DEVICES] = {};
+    if (device < 0 || device >= MAX_DEVICES) return nullptr;
+    std::lock_guard<std::mutex> hold(lock);
+    if (!pools[device]) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        cudaMemPool_t p = nullptr;
+        if (cudaMemPoolCreate(&p, &props) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return nullptr;
+        }
+        uint64_t keep = 64ull << 20;
+        cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
+        pools[device] = p;
+    }
+    return pools[device];
+}
+
+int sm_count(int device)
+{
+    static int n[MAX_DEVICES] = {};
+    if (device < 0 || device >= MAX_DEVICES) return 1;
+    if (!n[device]) {
+        int v = 0;
+        cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, device);
+        n[device] = v > 0 ? v : 1;
+    }
+    return n[device];
+}
+
+int current_device()
+{
+    int d = 0;
+    cudaGetDevice(&d);
+    return d;
+}
+
+template <int NCH, bool MO_OUT>
+int launch(sp::Args& A, int nblk, size_t smem, cudaStream_t st)
+{
+    // (set on every launch: the attribute belongs to the current device)
+    cudaError_t e = cudaFuncSetAttribute(sp::split_kernel<NCH, MO_OUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)smem);
+    if (e != cudaSuccess) return cuda_status(e, "FP64 tensor-core path: shared memory");
+    sp::split_kernel<NCH, MO_OUT><<<nblk, sp::Cfg<NCH>::NT, smem, st>>>(A);
+    return cuda_status(cudaGetLastError(), "FP64 tensor-core path: launch");
+}
+
+template <int NCH>
+int run(const okg_basis* b, const Grid& g, const SplitCall& c, cudaStream_t st, bool& done)
+{
+    using C = sp::Cfg<NCH>;
+    const int npmax = C::RG == 1 ? 64 : 32;  // 7 accumulators per MO and row tile in 512 TMEM columns
+    sp::Args A{};
+    A.B = b->dev;
+    A.S = b->split;
+    A.g = g;
+    A.nmo = c.nmo;
+    A.npass = (c.nmo + npmax - 1) / npmax;
+    A.np = ((c.nmo + A.npass - 1) / A.npass + 15) & ~15;
+    A.drv = c.drv;
+    A.out = c.out;
+    A.dout = c.dout;
+    A.mo_norm = c.mo_norm;
+    A.ld = c.ld;
+    A.brick = g.regular && g.offset == 0 && g.npts == (long long)g.nx * g.ny * g.nz;
+    const int device = current_device(), sms = sm_count(device);
+    // 128-point tiles share one screening; with fewer than four of them per SM, calls with
+    // derivatives take 32-point tiles, which spread over the SMs
+    A.nsub = 4;
+    for (;;) {
+        if (A.brick) {
+            A.nby = (g.ny + 3) / 4;
+            A.nbz = (g.nz + 7) / 8;
+            A.ntiles = (long long)((g.nx + A.nsub - 1) / A.nsub) * A.nby * A.nbz;
+        } else {
+            A.ntiles = (g.npts + 32 * A.nsub - 1) / (32 * A.nsub);
+        }
+        if (A.nsub == 1 || NCH == 1 || A.ntiles >= 4ll * sms) break;
+        A.nsub = 1;
+    }
+    const int acc_cols = C::RG * sp::ND * A.np;
+    A.nacc = 2 * acc_cols <= 512 ? 2 : 1;
+    A.tm_cols = 32;
+    while ((int)A.tm_cols < A.nacc * acc_cols) A.tm_cols *= 2;
+    const size_t slot = ((size_t)C::RG * sp::ND * sp::DT + (size_t)sp::ND * A.np * sp::PK * 2 + 1023) & ~(size_t)1023;
+    const size_t norm = (size_t)C::NEW * A.npass * A.np * 8;
+    A.norm_smem = c.mo_norm && norm <= 16384;
+    const size_t fixed = 1024 + sp::AUX_BYTES + (A.norm_smem ? norm : 0) + (NCH == 1 ? sp::NBUF * 3 * 128 * 8 : 0);
+    A.nslot = (int)((sp::SMEM_MAX - fixed) / slot);
+    if (A.nslot > sp::MAX_SLOTS) A.nslot = sp::MAX_SLOTS;
+    if (A.nslot < 2) return OKG_OK;
+    const int nblk = (int)(A.ntiles < sms ? A.ntiles : sms);
+    int* status = status_word();
+    cudaMemPool_t pool = workspace_pool(device);
+    if (!status || !pool) return OKG_OK;
+    A.status = status;
+    const int nrow = A.npass * A.np;
+    auto up = [](size_t v) { return (v + 255) & ~(size_t)255; };
+    const size_t o_fexp = 256, o_occ = o_fexp + up(4 * (size_t)nrow), o_b = o_occ + up(8 * (size_t)nrow),
+                 o_phi = o_b + up((size_t)nrow * b->split.npanel * sp::ND * sp::PK * 2),
+                 bytes = o_phi + (b->split.npanel > sp::GROUP ? (size_t)nblk * C::RG * A.np * 128 * 8 : 0);
+    char* ws = nullptr;
+    if (cudaMallocFromPoolAsync((void**)&ws, bytes, pool, st) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return OKG_OK;  // no room for the digits: the caller's other path needs none
+    }
+    A.counter = (unsigned long long*)ws;
+    A.fexp = (const int*)(ws + o_fexp);
+    A.occ = (const double*)(ws + o_occ);
+    A.bpack = (const unsigned char*)(ws + o_b);
+    A.phi = b->split.npanel > sp::GROUP ? (double*)(ws + o_phi) : nullptr;
+    sp::split_pack_kernel<<<nrow, 256, 0, st>>>(b->split, c.nmo, A.np, b->ncart, c.C, c.occ, (unsigned char*)(ws + o_b),
+                                                (int*)(ws + o_fexp), (double*)(ws + o_occ), A.counter);
+    int s = cuda_status(cudaGetLastError(), "FP64 tensor-core path: coefficient digits");
+    const size_t smem = fixed + A.nslot * slot;
+    if (!s) s = c.mo_out ? launch<NCH, true>(A, nblk, smem, st) : launch<NCH, false>(A, nblk, smem, st);
+    const cudaError_t e = cudaFreeAsync(ws, st);
+    if (!s) s = cuda_status(e, "FP64 tensor-core path: workspace");
+    done = s == OKG_OK;
+    return s;
+}
+}  // namespace
+
+int split_run(const okg_basis* b, const Grid& g, const SplitCall& c, cudaStream_t st, bool& done)
+{
+    done = false;
+    if (c.need & ~0x7Fu) return OKG_OK;  // mixed second derivatives
+    // Few points do not fill the chip with operand tiles (a tile's latency is 60 us for a
+    // 3-atom, 130 us for a 12-atom molecule), while fused64_kernel spreads 8 points per CTA
+    // and takes 32 / 70 us for up to 8 points per SM.  Measured (3 atoms | 12 atoms | 40
+    // spherical atoms, fused64 against this path, us): values 3000 points 54:71 | 131:153 |
+    // 542:898, 10000 points 176:72 | 514:155 | 2394:918; gradients 1000 points 49:65 |
+    // 111:130 | 1004:616, 3000 points 94:64 | 243:133 | 2100:692; second derivatives 1000
+    // points 62:86 | 147:198 | 1439:1533, 3000 points 121:84 | 328:199 | 2915:1658.
+    const bool values = (c.need & ~1u) == 0;
+    const bool contraction = (c.need & ~0xFu) == 0 && !values && (long long)c.nmo * b->ncart >= 32768;
+    if (!contraction && g.npts < (values ? 32 : 16) * sm_count(current_device())) return OKG_OK;
+    if (b->nshell > sp::MAX_SHELLS || b->split.npanel > sp::MAX_PANELS || b->dev.max_nprim > 255) return OKG_OK;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+        (void)cudaGetLastError();
+        return OKG_OK;  // (a captured call keeps to the kernel without a workspace)
+    }
+    if ((c.need & ~1u) == 0) return run<1>(b, g, c, st, done);
+    if ((c.need & ~0xFu) == 0) return run<4>(b, g, c, st, done);
+    return run<7>(b, g, c, st, done);
+}
+}  // namespace okg
+
+extern "C" int okg_wait_status(int* status)
+{
+    int* w = okg::status_word();
+    const int v = w ? *(volatile int*)w : 0;
+    if (status) *status = v;
+    if (!v) return OKG_OK;
+    *(volatile int*)w = 0;
+    return okg::set_error(OKG_ERR_TIMEOUT, "FP64 tensor-core path: a device wait expired; the results are incomplete");
+}

@@ -1,0 +1,63 @@
+// Host interface and device tables of the FP64 path on the tensor cores (okg_split64.cu).
+#pragma once
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include <vector>
+
+#define OKG_SPLIT_PK 16     // columns of an operand panel: one MMA K-step
+#define OKG_SPLIT_EXP 2048  // entries of the exponential's table
+
+namespace okg {
+
+// A primitive for the radial sums: alpha log2(e) = A 2^ea, w, -2 alpha w, 4 alpha^2 w.
+struct alignas(16) SplitPrim {
+    uint64_t A;
+    int special;  // alpha <= 0 or subnormal: the exponential is taken in FP64
+    int ea;
+    double w, w1, w2, neg_alpha;
+};
+
+struct SplitDev {
+    const int4* shell;      // nshell, panel by panel: {atom, L | first column << 8 | panel << 16, first primitive, primitives}
+    const int* panel;       // npanel + 1: first entry of each panel in shell
+    const int* col_cart;    // npanel x 16: listed Cartesian row of each column, or -1
+    const double* col_g;    // npanel x 16: angular norm of each column times its 2^shift
+    const float4* prim_lg;  // nprim: {alpha log2(e), log2 |w|, alpha, 0}, ascending alpha per shell
+    const SplitPrim* prim;  // nprim, ascending alpha per shell
+    const uint64_t* exp_tab;  // 2^(63 - j / 2048), rounded
+    const int* flags;       // non-zero: a parameter or position is not a number
+    int npanel;
+};
+
+// One primitive (alpha, w) as the FP64 tensor-core path's bounds and radial sums read it;
+// false if a parameter is not a number (an exponent of +infinity drops its primitive).
+__device__ __forceinline__ bool split_prim(double2 p, float4& lg, SplitPrim& o)
+{
+    const bool inf = p.x > 1.0e300;
+    // log2 |w| from exponent field and mantissa (|w| beyond the range of a float keeps its size)
+    const long long wb = __double_as_longlong(p.y);
+    const int we = (int)((wb >> 52) & 0x7FF);
+    const float lw = we == 0 ? -3.0e38f
+                             : (float)(we - 1023) + log2f((float)__longlong_as_double((wb & 0xFFFFFFFFFFFFFll) | 0x3FF0000000000000ll));
+    lg = inf ? make_float4(0.f, -3.0e38f, 0.f, 0.f) : make_float4((float)(p.x * 1.4426950408889634), lw, (float)p.x, 0.f);
+    // alpha log2(e) = A 2^ea with a 64-bit mantissa
+    const long long bits = __double_as_longlong(p.x);
+    const int ex = (int)((bits >> 52) & 0x7FF);
+    const uint64_t m = (((uint64_t)bits & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull) << 11;
+    const uint64_t l2e = 0xB8AA3B295C17F0BCull;  // log2(e) 2^63
+    uint64_t h = __umul64hi(m, l2e);
+    o.ea = ex - 1086 + 1;
+    if (!(h >> 63)) {
+        h = (h << 1) | ((m * l2e) >> 63);
+        --o.ea;
+    }
+    o.A = h;
+    o.special = !(p.x > 0.0) || ex == 0;
+    o.w = inf ? 0.0 : p.y;
+    o.w1 = inf ? 0.0 : -2.0 * p.x * p.y;
+    o.w2 = inf ? 0.0 : 4.0 * p.x * p.x * p.y;
+    o.neg_alpha = -p.x;
+    return inf || (isfinite(p.x) && isfinite(p.y));
+}
+}  // namespace okg
