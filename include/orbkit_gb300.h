@@ -130,6 +130,12 @@ int okg_rho(const okg_basis* basis, const okg_grid* grid, int nmo, const double*
             int ndrv, const int* h_drv, int exact_mixed, double* d_rho, double* d_drho, int64_t ld,
             double* d_mo_norm, okg_stream stream);
 
+/* MO coefficients of a spherical basis <-> its Cartesian rows: C_cart[m, c] = sum_r T[r, c]
+ * C_sph[m, r] (the C_eff of the calls above) and the transposed map of gradients, with T
+ * the spherical transform of okg_basis_create. */
+int okg_fold_coeff(const okg_basis* basis, int nmo, const double* d_csph, double* d_ccart, okg_stream stream);
+int okg_unfold_coeff(const okg_basis* basis, int nmo, const double* d_ccart, double* d_csph, okg_stream stream);
+
 /* Whether a device wait of an okg_rho / okg_eval_mo call expired (OKG_ERR_TIMEOUT; the
  * outputs of that call are then incomplete) since the last query; clears the record.  The
  * device writes it during the call: query it after waiting for the call's stream.  Large

@@ -49,6 +49,8 @@ SIGNATURES = {
                                    ctypes.c_int, _vp, ctypes.c_int64, _vp]),
     "okg_rho": (ctypes.c_int, [_vp, ctypes.POINTER(OkgGrid), ctypes.c_int, _vp, _vp, ctypes.c_int, _c_int_p,
                                ctypes.c_int, _vp, _vp, ctypes.c_int64, _vp, _vp]),
+    "okg_fold_coeff": (ctypes.c_int, [_vp, ctypes.c_int, _vp, _vp, _vp]),
+    "okg_unfold_coeff": (ctypes.c_int, [_vp, ctypes.c_int, _vp, _vp, _vp]),
     "okg_wait_status": (ctypes.c_int, [_c_int_p]),
     "okg_mixed_plan_create": (ctypes.c_int, [_vp, ctypes.c_int, ctypes.POINTER(_vp)]),
     "okg_mixed_plan_destroy": (ctypes.c_int, [_vp]),

@@ -115,9 +115,7 @@ class DensityModel:
                                             _lib.ptr(g_rho), _lib.ptr(g_grad), self.npts, prec, _lib.ptr(dC),
                                             _lib.ptr(dprim), _lib.ptr(dgeo), _lib.ptr(self._work), nbytes.value,
                                             _lib.stream_handle()))
-        if self.basis.spherical:
-            dC = dC @ self.basis.T_dev.T
-        return dC, dprim, dgeo
+        return self.basis.c_grad(dC), dprim, dgeo
 
 
 def _grad_fn():

@@ -116,16 +116,6 @@ class DeviceBasis:
         self.spherical = f["spherical"]
         self.nao = len(f["sph_ptr"]) - 1 if self.spherical else self.ncart
         self.device = torch.device(device)
-        if self.spherical:
-            T = numpy.zeros((self.nao, self.ncart))
-            for r in range(self.nao):
-                for t in range(f["sph_ptr"][r], f["sph_ptr"][r + 1]):
-                    T[r, f["sph_idx"][t]] += f["sph_coef"][t]
-            self.T = T
-            self.T_dev = torch.from_numpy(T).to(self.device)
-        else:
-            self.T = None
-            self.T_dev = None
         h = ctypes.c_void_p()
         ip = lambda a: a.ctypes.data_as(ctypes.POINTER(ctypes.c_int)) if a is not None else None
         dp = lambda a: a.ctypes.data_as(ctypes.POINTER(ctypes.c_double)) if a is not None else None
@@ -156,6 +146,25 @@ class DeviceBasis:
         _lib.check(self._L.okg_basis_set_params(self._h, _lib.ptr(self.geo), _lib.ptr(self.prim),
                                                 _lib.stream_handle(stream)))
 
+    @property
+    def T(self):
+        """Dense (nao, ncart) spherical transform (None for a Cartesian basis)."""
+        if not self.spherical:
+            return None
+        f = self.flat
+        T = numpy.zeros((self.nao, self.ncart))
+        numpy.add.at(T, (numpy.repeat(numpy.arange(self.nao), numpy.diff(f["sph_ptr"])), f["sph_idx"]), f["sph_coef"])
+        return T
+
+    def c_grad(self, grad):
+        """Gradient with respect to C_eff (nmo, ncart) -> with respect to the MO coefficients (nmo, nao)."""
+        import torch
+        if not self.spherical:
+            return grad
+        out = torch.empty((grad.shape[0], self.nao), dtype=torch.float64, device=self.device)
+        _lib.check(self._L.okg_unfold_coeff(self._h, grad.shape[0], _lib.ptr(grad), _lib.ptr(out), _lib.stream_handle()))
+        return out
+
     def c_eff(self, coeffs):
         """MO coefficients (nmo, nao) -> Cartesian-basis coefficients (nmo, ncart) on the device."""
         import torch
@@ -165,12 +174,9 @@ class DeviceBasis:
         if C.shape[1] != self.nao:
             raise ValueError("MO coefficients have %d columns, the basis has %d AOs" % (C.shape[1], self.nao))
         if self.spherical:
-            # C_eff = C_sph . T by the FP64 contraction kernel (T's Cartesian columns
-            # play the role of grid points)
             C = C.contiguous()
             out = torch.empty((C.shape[0], self.ncart), dtype=torch.float64, device=self.device)
-            _lib.check(self._L.okg_mo_from_ao(C.shape[0], self.nao, _lib.ptr(C), _lib.ptr(self.T_dev), self.ncart,
-                                              self.ncart, _lib.ptr(out), self.ncart, _lib.stream_handle()))
+            _lib.check(self._L.okg_fold_coeff(self._h, C.shape[0], _lib.ptr(C), _lib.ptr(out), _lib.stream_handle()))
             return out
         return C.contiguous()
 

@@ -394,6 +394,30 @@ extern "C" int okg_basis_create(int natom, int nshell, const int* h_shell_atom, 
     const size_t o_spr = lay.take(sizeof(SplitPrim) * nprim);
     const size_t o_sfl = lay.take(sizeof(int));
     const size_t o_exp = lay.take(sizeof(uint64_t) * OKG_SPLIT_EXP);
+    // the transform by Cartesian row; entries of the same spherical row added up in order
+    std::vector<int> cart_ptr(ncart + 1, 0), cart_srow, sph_cart;
+    std::vector<double> cart_coef;
+    if (nsph > 0) {
+        std::vector<std::vector<std::pair<int, double>>> by(ncart);
+        for (int r = 0; r < nsph; ++r)
+            for (int t = h_sph_ptr[r]; t < h_sph_ptr[r + 1]; ++t) {
+                auto& v = by[h_sph_cart[t]];
+                if (!v.empty() && v.back().first == r) v.back().second += h_sph_coef[t];
+                else v.push_back({r, h_sph_coef[t]});
+                sph_cart.push_back(h_sph_cart[t]);
+            }
+        for (int c = 0; c < ncart; ++c) {
+            for (const auto& e : by[c]) {
+                cart_srow.push_back(e.first);
+                cart_coef.push_back(e.second);
+            }
+            cart_ptr[c + 1] = (int)cart_srow.size();
+        }
+    }
+    const size_t o_cptr = lay.take(sizeof(int) * (ncart + 1));
+    const size_t o_crw = lay.take(sizeof(int) * (cart_srow.size() + 1));
+    const size_t o_ccf = lay.take(sizeof(double) * (cart_coef.size() + 1));
+    const size_t o_scart = lay.take(sizeof(int) * (sph_cart.size() + 1));
     const size_t bytes = lay.take(0);
     char* blk = nullptr;
     cudaError_t e = cudaMalloc((void**)&blk, bytes);
@@ -446,6 +470,19 @@ extern "C" int okg_basis_create(int natom, int nshell, const int* h_shell_atom, 
     if (e == cudaSuccess) e = upload_split(b, split_layout(shells, comp_row, comp_g, nullptr));
     if (e == cudaSuccess)
         e = cudaMemcpy(blk + o_exp, split_exp_table(), sizeof(uint64_t) * OKG_SPLIT_EXP, cudaMemcpyHostToDevice);
+    b->cart_ptr = (const int*)(blk + o_cptr);
+    b->cart_srow = (const int*)(blk + o_crw);
+    b->cart_coef = (const double*)(blk + o_ccf);
+    b->sph_cart = (const int*)(blk + o_scart);
+    if (e == cudaSuccess && nsph > 0) {
+        auto put = [](void* dst, const auto& v) {
+            return cudaMemcpy(dst, v.data(), sizeof(v[0]) * v.size(), cudaMemcpyHostToDevice);
+        };
+        e = put(blk + o_cptr, cart_ptr);
+        if (e == cudaSuccess) e = put(blk + o_crw, cart_srow);
+        if (e == cudaSuccess) e = put(blk + o_ccf, cart_coef);
+        if (e == cudaSuccess) e = put(blk + o_scart, sph_cart);
+    }
     if (e != cudaSuccess) {
         cudaFree(blk);
         free(b);

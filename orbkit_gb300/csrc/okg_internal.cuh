@@ -251,6 +251,13 @@ __host__ __device__ inline bool need_r2(unsigned m) { return (m & (CH_HESS_D | C
 struct okg_basis {
     okg::BasisDev dev;
     okg::SplitDev split;  // tables of the FP64 path on the tensor cores
+    // the spherical transform by Cartesian row (device; spherical bases): per listed row the
+    // spherical rows that contain it, ascending, and their coefficients
+    const int* cart_ptr;
+    const int* cart_srow;
+    const double* cart_coef;
+    // and by spherical row: listed Cartesian row of each entry (sph_ptr, sph_coef in dev)
+    const int* sph_cart;
     void* dev_block;  // single device allocation holding every table
     size_t dev_bytes;
     int* h_shell_L;   // unused (kept zero)
