@@ -18,31 +18,59 @@ from . import _lib
 from .tools import get_cart2sph
 
 
+def _shell_transform(comps, lms):
+    """(entries per row, component of each entry, coefficient) of one shell listing the
+    Cartesian components ``comps`` and the real harmonics ``lms``."""
+    count, pos, coef = [], [], []
+    for l, m in lms:
+        want, cf, fac = get_cart2sph(l, m)
+        for c, f in zip(want, cf):
+            hit = [i for i, v in enumerate(comps) if v == tuple(c)]
+            if not hit:
+                return None
+            pos.append(hit[-1])
+            coef.append(f * fac)
+        count.append(len(want))
+    return numpy.array(count), numpy.array(pos), numpy.array(coef, dtype=numpy.float64)
+
+
 def spherical_csr(ao_spec):
     """CSR (ptr, listed Cartesian row, coefficient) of the spherical transform,
     following orbkit's cartesian2spherical: for each listed (lx,ly,lz) of the
     Schlegel-Frisch combination the last matching row of the shell is used and
-    the coefficient is coef * global factor."""
-    lxlylz = ao_spec.get_lxlylz()
-    assign = ao_spec.get_assign_lxlylz_to_cont()
-    rows = {}
-    for i, j in enumerate(assign):
-        rows.setdefault(int(j), []).append(i)
-    ptr, idx, coef = [0], [], []
-    for (j0, k0) in ao_spec.get_old_ao_spherical():
-        comps, cf, fac = get_cart2sph(*k0)
-        for c, f in zip(comps, cf):
-            hit = None
-            for i in rows[int(j0)]:
-                if tuple(int(v) for v in lxlylz[i]) == tuple(c):
-                    hit = i
-            if hit is None:
-                raise ValueError("spherical component %s missing from shell %d" % (c, j0))
-            idx.append(hit)
-            coef.append(f * fac)
-        ptr.append(len(idx))
-    return (numpy.array(ptr, dtype=numpy.intc), numpy.array(idx, dtype=numpy.intc),
-            numpy.array(coef, dtype=numpy.float64))
+    the coefficient is coef * global factor.  Shells that list the same components and
+    harmonics share one small table (a few kinds per basis)."""
+    lxlylz = numpy.asarray(ao_spec.get_lxlylz()).reshape(-1, 3)
+    assign = numpy.asarray(ao_spec.get_assign_lxlylz_to_cont())
+    order = numpy.argsort(assign, kind="stable")
+    comps = [tuple(v) for v in lxlylz[order].tolist()]
+    bounds = numpy.searchsorted(assign[order], numpy.arange(int(assign.max()) + 2 if len(assign) else 1)).tolist()
+    # runs of spherical rows of one shell
+    kinds, runs = {}, []
+    old = ao_spec.get_old_ao_spherical()
+    i = 0
+    while i < len(old):
+        shell, j = int(old[i][0]), i
+        lms = []
+        while j < len(old) and int(old[j][0]) == shell:
+            lms.append((int(old[j][1][0]), int(old[j][1][1])))
+            j += 1
+        first, last = bounds[shell], bounds[shell + 1]
+        key = (tuple(comps[first:last]), tuple(lms))
+        if key not in kinds:
+            kinds[key] = (len(kinds), _shell_transform(*key))
+            if kinds[key][1] is None:
+                raise ValueError("spherical component missing from shell %d" % shell)
+        runs.append((kinds[key][0], first))
+        i = j
+    if not runs:
+        return numpy.zeros(1, dtype=numpy.intc), numpy.zeros(0, dtype=numpy.intc), numpy.zeros(0)
+    tables = [t for _, t in sorted(kinds.values(), key=lambda v: v[0])]
+    count = numpy.concatenate([tables[k][0] for k, _ in runs])
+    idx = order[numpy.concatenate([tables[k][1] + first for k, first in runs])]
+    coef = numpy.concatenate([tables[k][2] for k, _ in runs])
+    ptr = numpy.concatenate(([0], numpy.cumsum(count)))
+    return ptr.astype(numpy.intc), idx.astype(numpy.intc), coef
 
 
 def flatten(ao_spec):

@@ -202,38 +202,44 @@ MixedLayout mixed_layout(const std::vector<Shell>& shells, const std::vector<int
     return m;
 }
 
-// Upload a mixed layout into the basis block (capacity: one chunk per shell).
-cudaError_t upload_mixed(okg_basis* b, const MixedLayout& m)
-{
-    BasisDev& d = b->dev;
-    cudaError_t e = cudaMemcpy((void*)d.mshells, m.mshells.data(), sizeof(Shell) * m.mshells.size(),
-                               cudaMemcpyHostToDevice);
-    if (e == cudaSuccess)
-        e = cudaMemcpy((void*)d.mchunks, m.mchunks.data(), sizeof(int4) * m.mchunks.size(), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess)
-        e = cudaMemcpy((void*)d.mcol_cart, m.mcol_cart.data(), sizeof(int) * m.mcol_cart.size(),
-                       cudaMemcpyHostToDevice);
-    if (e == cudaSuccess)
-        e = cudaMemcpy((void*)d.mcol_g, m.mcol_g.data(), sizeof(double) * m.mcol_g.size(), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) d.nmchunk = (int)m.mchunks.size();
-    return e;
-}
+// Tables in a host image of the basis block (one upload).
+struct Image {
+    std::vector<char> bytes;
+    template <typename T>
+    void put(size_t off, const std::vector<T>& v)
+    {
+        if (!v.empty()) memcpy(bytes.data() + off, v.data(), sizeof(T) * v.size());
+    }
+};
 
-// Upload the FP64 tensor-core path's panels (capacity: one panel per shell).
-cudaError_t upload_split(okg_basis* b, const SplitLayout& m)
+// Offsets of the tables that depend on the shell order, one contiguous range of the block
+// [begin, end) with room for one chunk and one panel per shell.
+struct OrderOffsets {
+    size_t msh, mch, mcc, mcg, ssh, spn, scc, scg, begin, end;
+};
+
+void put_order(okg_basis* b, Image& im, const OrderOffsets& o, size_t base, const MixedLayout& m, const SplitLayout& s)
 {
-    SplitDev& d = b->split;
-    auto put = [](const void* dst, const auto& v) {
-        return cudaMemcpy((void*)dst, v.data(), sizeof(v[0]) * v.size(), cudaMemcpyHostToDevice);
-    };
-    cudaError_t e = put(d.shell, m.shell);
-    if (e == cudaSuccess) e = put(d.panel, m.panel);
-    if (e == cudaSuccess) e = put(d.col_cart, m.col_cart);
-    if (e == cudaSuccess) e = put(d.col_g, m.col_g);
-    if (e == cudaSuccess) d.npanel = (int)m.panel.size() - 1;
-    return e;
+    im.put(o.msh - base, m.mshells);
+    im.put(o.mch - base, m.mchunks);
+    im.put(o.mcc - base, m.mcol_cart);
+    im.put(o.mcg - base, m.mcol_g);
+    im.put(o.ssh - base, s.shell);
+    im.put(o.spn - base, s.panel);
+    im.put(o.scc - base, s.col_cart);
+    im.put(o.scg - base, s.col_g);
+    b->dev.nmchunk = (int)m.mchunks.size();
+    b->split.npanel = (int)s.panel.size() - 1;
 }
 }  // namespace
+
+// What okg_basis_set_mixed_order needs of the basis on the host.
+struct okg_basis_host {
+    std::vector<Shell> shells;
+    std::vector<int> comp_row;
+    std::vector<double> comp_g;
+    OrderOffsets order;
+};
 
 extern "C" int okg_basis_create(int natom, int nshell, const int* h_shell_atom, const int* h_shell_ncart,
                                 const int* h_shell_nprim, const int* h_lxlylz, int is_normalized,
@@ -359,9 +365,6 @@ extern "C" int okg_basis_create(int natom, int nshell, const int* h_shell_atom, 
         chunks.push_back(make_int4(s0, nshell, k0, k));
     }
 
-    // mixed-path chunks in basis order (okg_basis_set_mixed_order may choose another)
-    const MixedLayout mixed = mixed_layout(shells, comp_row, comp_g, nullptr);
-
     okg_basis* b = (okg_basis*)calloc(1, sizeof(okg_basis));
     if (!b) return set_error(OKG_ERR_ALLOC, "okg_basis_create: host allocation");
     Layout lay;
@@ -382,14 +385,16 @@ extern "C" int okg_basis_create(int natom, int nshell, const int* h_shell_atom, 
     const size_t o_asp = lay.take(sizeof(int) * (natom + 1));
     const size_t o_ash = lay.take(sizeof(int) * nshell);
     const size_t o_padj = lay.take(sizeof(double) * 2 * nprim);
-    const size_t o_msh = lay.take(sizeof(Shell) * nshell);
-    const size_t o_mch = lay.take(sizeof(int4) * nshell);
-    const size_t o_mcc = lay.take(sizeof(int) * OKG_MKC * nshell);
-    const size_t o_mcg = lay.take(sizeof(double) * OKG_MKC * nshell);
-    const size_t o_ssh = lay.take(sizeof(int4) * nshell);
-    const size_t o_spn = lay.take(sizeof(int) * (nshell + 1));
-    const size_t o_scc = lay.take(sizeof(int) * OKG_SPLIT_PK * nshell);
-    const size_t o_scg = lay.take(sizeof(double) * OKG_SPLIT_PK * nshell);
+    OrderOffsets oo;
+    oo.begin = oo.msh = lay.take(sizeof(Shell) * nshell);
+    oo.mch = lay.take(sizeof(int4) * nshell);
+    oo.mcc = lay.take(sizeof(int) * OKG_MKC * nshell);
+    oo.mcg = lay.take(sizeof(double) * OKG_MKC * nshell);
+    oo.ssh = lay.take(sizeof(int4) * nshell);
+    oo.spn = lay.take(sizeof(int) * (nshell + 1));
+    oo.scc = lay.take(sizeof(int) * OKG_SPLIT_PK * nshell);
+    oo.scg = lay.take(sizeof(double) * OKG_SPLIT_PK * nshell);
+    oo.end = lay.take(0);
     const size_t o_slg = lay.take(sizeof(float4) * nprim);
     const size_t o_spr = lay.take(sizeof(SplitPrim) * nprim);
     const size_t o_sfl = lay.take(sizeof(int));
@@ -425,11 +430,6 @@ extern "C" int okg_basis_create(int natom, int nshell, const int* h_shell_atom, 
         free(b);
         return cuda_status(e, "okg_basis_create: cudaMalloc");
     }
-    e = cudaMemset(blk, 0, bytes);
-    if (e == cudaSuccess) e = cudaMemcpy(blk + o_shells, shells.data(), sizeof(Shell) * nshell, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(blk + o_primL, prim_L.data(), sizeof(int) * nprim, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess)
-        e = cudaMemcpy(blk + o_patom, prim_atom.data(), sizeof(int) * nprim, cudaMemcpyHostToDevice);
     // shells of each atom (CSR), for the cusp points of the mixed path
     std::vector<int> atom_shell_ptr(natom + 1, 0), atom_shells(nshell);
     for (int s = 0; s < nshell; ++s) atom_shell_ptr[shells[s].atom + 1]++;
@@ -438,56 +438,50 @@ extern "C" int okg_basis_create(int natom, int nshell, const int* h_shell_atom, 
         std::vector<int> fill(atom_shell_ptr.begin(), atom_shell_ptr.end() - 1);
         for (int s = 0; s < nshell; ++s) atom_shells[fill[shells[s].atom]++] = s;
     }
-    if (e == cudaSuccess)
-        e = cudaMemcpy(blk + o_asp, atom_shell_ptr.data(), sizeof(int) * (natom + 1), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(blk + o_ash, atom_shells.data(), sizeof(int) * nshell, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess)
-        e = cudaMemcpy(blk + o_crow, comp_row.data(), sizeof(int) * comp_row.size(), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess)
-        e = cudaMemcpy(blk + o_cg, comp_g.data(), sizeof(double) * comp_g.size(), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess)
-        e = cudaMemcpy(blk + o_sptr, sph_ptr.data(), sizeof(int) * sph_ptr.size(), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && !sph_cidx.empty())
-        e = cudaMemcpy(blk + o_scid, sph_cidx.data(), sizeof(int) * sph_cidx.size(), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && !sph_coef.empty())
-        e = cudaMemcpy(blk + o_scoef, sph_coef.data(), sizeof(double) * sph_coef.size(), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess)
-        e = cudaMemcpy(blk + o_chunks, chunks.data(), sizeof(int4) * chunks.size(), cudaMemcpyHostToDevice);
+    Image im;
+    im.bytes.assign(bytes, 0);
+    im.put(o_shells, shells);
+    im.put(o_primL, prim_L);
+    im.put(o_patom, prim_atom);
+    im.put(o_asp, atom_shell_ptr);
+    im.put(o_ash, atom_shells);
+    im.put(o_crow, comp_row);
+    im.put(o_cg, comp_g);
+    im.put(o_sptr, sph_ptr);
+    im.put(o_scid, sph_cidx);
+    im.put(o_scoef, sph_coef);
+    im.put(o_chunks, chunks);
+    memcpy(im.bytes.data() + o_exp, split_exp_table(), sizeof(uint64_t) * OKG_SPLIT_EXP);
+    im.put(o_cptr, cart_ptr);
+    im.put(o_crw, cart_srow);
+    im.put(o_ccf, cart_coef);
+    im.put(o_scart, sph_cart);
+    // columns in basis order (okg_basis_set_mixed_order may choose another)
+    put_order(b, im, oo, 0, mixed_layout(shells, comp_row, comp_g, nullptr), split_layout(shells, comp_row, comp_g, nullptr));
+    e = cudaMemcpy(blk, im.bytes.data(), bytes, cudaMemcpyHostToDevice);
     BasisDev& d = b->dev;
-    d.mshells = (const Shell*)(blk + o_msh);
-    d.mchunks = (const int4*)(blk + o_mch);
-    d.mcol_cart = (const int*)(blk + o_mcc);
-    d.mcol_g = (const double*)(blk + o_mcg);
-    if (e == cudaSuccess) e = upload_mixed(b, mixed);
-    b->split.shell = (const int4*)(blk + o_ssh);
-    b->split.panel = (const int*)(blk + o_spn);
-    b->split.col_cart = (const int*)(blk + o_scc);
-    b->split.col_g = (const double*)(blk + o_scg);
+    d.mshells = (const Shell*)(blk + oo.msh);
+    d.mchunks = (const int4*)(blk + oo.mch);
+    d.mcol_cart = (const int*)(blk + oo.mcc);
+    d.mcol_g = (const double*)(blk + oo.mcg);
+    b->split.shell = (const int4*)(blk + oo.ssh);
+    b->split.panel = (const int*)(blk + oo.spn);
+    b->split.col_cart = (const int*)(blk + oo.scc);
+    b->split.col_g = (const double*)(blk + oo.scg);
     b->split.prim_lg = (const float4*)(blk + o_slg);
     b->split.prim = (const SplitPrim*)(blk + o_spr);
     b->split.flags = (const int*)(blk + o_sfl);
     b->split.exp_tab = (const uint64_t*)(blk + o_exp);
-    if (e == cudaSuccess) e = upload_split(b, split_layout(shells, comp_row, comp_g, nullptr));
-    if (e == cudaSuccess)
-        e = cudaMemcpy(blk + o_exp, split_exp_table(), sizeof(uint64_t) * OKG_SPLIT_EXP, cudaMemcpyHostToDevice);
     b->cart_ptr = (const int*)(blk + o_cptr);
     b->cart_srow = (const int*)(blk + o_crw);
     b->cart_coef = (const double*)(blk + o_ccf);
     b->sph_cart = (const int*)(blk + o_scart);
-    if (e == cudaSuccess && nsph > 0) {
-        auto put = [](void* dst, const auto& v) {
-            return cudaMemcpy(dst, v.data(), sizeof(v[0]) * v.size(), cudaMemcpyHostToDevice);
-        };
-        e = put(blk + o_cptr, cart_ptr);
-        if (e == cudaSuccess) e = put(blk + o_crw, cart_srow);
-        if (e == cudaSuccess) e = put(blk + o_ccf, cart_coef);
-        if (e == cudaSuccess) e = put(blk + o_scart, sph_cart);
-    }
     if (e != cudaSuccess) {
         cudaFree(blk);
         free(b);
         return cuda_status(e, "okg_basis_create: upload");
     }
+    b->host = new okg_basis_host{std::move(shells), std::move(comp_row), std::move(comp_g), oo};
     b->dev_block = blk;
     b->dev_bytes = bytes;
     d.atoms = (const double*)(blk + o_atoms);
@@ -524,7 +518,7 @@ extern "C" int okg_basis_create(int natom, int nshell, const int* h_shell_atom, 
     for (int l = 0; l <= OKG_MAX_L; ++l) b->l_hist[l] = l_hist[l];
     b->is_normalized = is_normalized ? 1 : 0;
     b->prim_L = (int*)(blk + o_primL);
-    b->ncomp = (int)comp_row.size();
+    b->ncomp = (int)b->host->comp_row.size();
     b->mixed_locked = 0;
     cudaGetDevice(&b->device);
     *out = b;
@@ -543,23 +537,20 @@ extern "C" int okg_basis_set_mixed_order(okg_basis* b, const int* h_order)
             return set_error(OKG_ERR_ARG, "okg_basis_set_mixed_order: order is not a permutation of the shells");
         seen[h_order[i]] = 1;
     }
-    std::vector<Shell> shells(n);
-    std::vector<int> comp_row(b->ncomp);
-    std::vector<double> comp_g(b->ncomp);
-    cudaError_t e = cudaMemcpy(shells.data(), b->dev.shells, sizeof(Shell) * n, cudaMemcpyDeviceToHost);
-    if (e == cudaSuccess)
-        e = cudaMemcpy(comp_row.data(), b->dev.comp_row, sizeof(int) * b->ncomp, cudaMemcpyDeviceToHost);
-    if (e == cudaSuccess)
-        e = cudaMemcpy(comp_g.data(), b->dev.comp_g, sizeof(double) * b->ncomp, cudaMemcpyDeviceToHost);
-    if (e == cudaSuccess) e = upload_mixed(b, mixed_layout(shells, comp_row, comp_g, h_order));
-    if (e == cudaSuccess) e = upload_split(b, split_layout(shells, comp_row, comp_g, h_order));
-    return cuda_status(e, "okg_basis_set_mixed_order");
+    const okg_basis_host& h = *b->host;
+    Image im;
+    im.bytes.assign(h.order.end - h.order.begin, 0);
+    put_order(b, im, h.order, h.order.begin, mixed_layout(h.shells, h.comp_row, h.comp_g, h_order),
+              split_layout(h.shells, h.comp_row, h.comp_g, h_order));
+    return cuda_status(cudaMemcpy((char*)b->dev_block + h.order.begin, im.bytes.data(), im.bytes.size(), cudaMemcpyHostToDevice),
+                       "okg_basis_set_mixed_order");
 }
 
 extern "C" int okg_basis_destroy(okg_basis* b)
 {
     if (!b) return OKG_OK;
     cudaError_t e = cudaFree(b->dev_block);
+    delete b->host;
     free(b);
     return cuda_status(e, "okg_basis_destroy");
 }

@@ -248,7 +248,9 @@ __host__ __device__ inline bool need_r2(unsigned m) { return (m & (CH_HESS_D | C
 }  // namespace okg
 
 // Host-side helpers shared by the translation units (okg_api.cu).
+struct okg_basis_host;
 struct okg_basis {
+    okg_basis_host* host;  // tables kept on the host (okg_basis.cu)
     okg::BasisDev dev;
     okg::SplitDev split;  // tables of the FP64 path on the tensor cores
     // the spherical transform by Cartesian row (device; spherical bases): per listed row the
