@@ -5,8 +5,9 @@
 // (orbkit/cy_overlap.pyx:78-163) and get_overlap (orbkit/c_non-grid-based.c:9-52).
 //
 // Per call, a table holds what a primitive pair shares across all component pairs of
-// its two shells (p, the prefactor, P - A; ov_pairs_kernel).  Then one thread per
-// output Cartesian pair (I, J).  It walks the primitives of I (outer)
+// its two shells (1/(2p), the prefactor, P - A; ov_pairs_kernel).  Then one thread per
+// bra row and ket shell (ao_overlap_shell_kernel; kets in the canonical component order), or
+// per output Cartesian pair (I, J) (any other ket).  It walks the primitives of I (outer)
 // and of J (inner), which is the order orbkit's flattened primitive loop adds them
 // to aoom[I, J].  The 1D factors are evaluated with orbkit's operations and
 // rounding (IEEE divisions, no FMA contraction): the two terms of a derivative can
@@ -55,6 +56,21 @@ struct OvRow {
 
 __device__ __forceinline__ int lcomp(int packed, int d) { return (packed >> (8 * d)) & 0xff; }
 
+// (n / 2p) rounded once, n = a - 1 >= 1: multiples of the pair's 1/(2p) and 3/(2p) by a power
+// of two are exact, so the IEEE division is left for n = 5, 7, 9, ...
+__device__ __forceinline__ double recur(int n, double h1, double h3, double p)
+{
+    switch (n) {
+    case 1: return h1;
+    case 2: return 2.0 * h1;
+    case 3: return h3;
+    case 4: return 4.0 * h1;
+    case 6: return 2.0 * h3;
+    case 8: return 8.0 * h1;
+    default: return (double)n / (2.0 * p);
+    }
+}
+
 // s(la, lb) along one axis (and, for the derivative axis, s(la, lb - 1) and
 // s(la, lb + 1)).  v holds s(a, k) for a >= la after transfer round k.
 __device__ __forceinline__ void os_axis(double xpa, double ab, double p, int la, int lb, bool deriv, double* v,
@@ -78,21 +94,38 @@ __device__ __forceinline__ void os_axis(double xpa, double ab, double p, int la,
 
 // Quantities of a primitive pair (bra primitive i at its atom in geo_a, ket primitive j
 // at its atom in geo_b) shared by every Cartesian component pair of the two shells:
-// p = alpha + beta, pref = exp(-mu R^2) (pi/p)^(3/2) (0 where the exponential
-// underflows) and P - A per axis.  Evaluated once per call into a table of
+// 1/(2p) and 3/(2p) of p = alpha + beta, pref = exp(-mu R^2) (pi/p)^(3/2) (0 where the
+// exponential underflows) and P - A per axis.  Evaluated once per call into a table of
 // nprim x nprim entries when the plan holds one, with the same operations as the
 // element kernel's own evaluation.
 struct alignas(16) OvPair {
-    double pref, p, xpa[3], pad;
+    double pref, h1, xpa[3], h3;  // h1 = 1 / (2p), h3 = 3 / (2p)
 };
 
+// n / p rounded once, y = 1/p rounded once: two Newton corrections of the quotient with exact
+// remainders (P. W. Markstein, IBM J. Res. Dev. 34 (1990) 111); p and n far from the ends of
+// the exponent range.
+__device__ __forceinline__ double quotient(double n, double p, double y)
+{
+    double q = n * y;
+    q = fma(fma(-q, p, n), y, q);
+    return fma(fma(-q, p, n), y, q);
+}
+
+// Per call about 100 FP64 operations per entry were 0.23 ms for 1128 primitives (87 % of the
+// FP64 pipe), a third of a matrix: the exponential in integers, corrected quotients instead
+// of four IEEE divisions and half the entries leave about a third of that.
+// SYM: bra and ket at the same positions; entries (i, j) and (j, i) share everything but
+// which atom P - A refers to, so the threads below the diagonal leave and the others write
+// both (bit for bit what two threads would).
+template <bool SYM>
 __global__ void ov_pairs_kernel(int nprim, const double2* __restrict__ prim, const int* __restrict__ prim_atom,
                                 const double* __restrict__ geo_a, const double* __restrict__ geo_b,
-                                OvPair* __restrict__ pairs)
+                                const uint64_t* __restrict__ tab, OvPair* __restrict__ pairs)
 {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     const int i = blockIdx.y * blockDim.y + threadIdx.y;
-    if (i >= nprim || j >= nprim) return;
+    if (i >= nprim || j >= nprim || (SYM && j < i)) return;
     const double al = prim[i].x, be = prim[j].x;
     double A[3], B[3];
     double rr = 0.0;
@@ -104,22 +137,184 @@ __global__ void ov_pairs_kernel(int nprim, const double2* __restrict__ prim, con
         rr = fma(ab, ab, rr);
     }
     OvPair e;
-    const double inv_p = 1.0 / (al + be);
+    const double p = al + be, inv_p = 1.0 / p;
+    const bool plain = p > 1.0e-100 && p < 1.0e100;  // (and finite)
+    e.h1 = 0.5 * inv_p;
+    e.h3 = plain ? quotient(1.5, p, inv_p) : 3.0 / (2.0 * p);
     const double arg = al * be * inv_p * rr;
-    e.p = al + be;
     if (arg > 746.0) {
         e.pref = 0.0;  // exp(-arg) is 0 in double
     } else {
+        uint64_t m;
+        int x;
+        split_mantissa(arg, m, x);
         const double t = M_PI * inv_p;
-        e.pref = exp(-arg) * t * sqrt(t);
+        // (negative or non-finite arguments: alpha or beta out of their usual range)
+        const double ex = arg >= 0.0 ? exp_neg(m, x, 0xB8AA3B295C17F0BCull, -63, tab) : exp(-arg);
+        e.pref = ex * t * sqrt(t);
     }
+    double P[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-        const double P = __dadd_rn(__dmul_rn(al, A[d]), __dmul_rn(be, B[d])) / e.p;
-        e.xpa[d] = -(A[d] - P);
+        const double n = __dadd_rn(__dmul_rn(al, A[d]), __dmul_rn(be, B[d]));
+        P[d] = plain && fabs(n) < 1.0e100 && (fabs(n) > 1.0e-100 || n == 0.0) ? quotient(n, p, inv_p) : n / p;
+        e.xpa[d] = -(A[d] - P[d]);
     }
-    e.pad = 0.0;
     pairs[(long long)i * nprim + j] = e;
+    if (SYM && j != i) {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) e.xpa[d] = -(B[d] - P[d]);
+        pairs[(long long)j * nprim + i] = e;
+    }
+}
+
+// Elements of one bra row with every component of a ket shell in the canonical (Molden)
+// order, the common case: a warp takes one bra row I and 32 ket shells of one (L, primitive
+// count), so the loops are uniform.  Per primitive pair the one-dimensional factors
+// s(la, 0 .. L (+ 1)) are built once per axis and shared by the shell's components, with the
+// operations and the rounding of the one-element kernel below (the elements are the same
+// bits): for a d shell 6 components share them, for f 10.  Bound by the FP64 pipe (62-74 %
+// active).  120 atoms, 1560 Cartesian rows, one matrix with its pair table and transform:
+// 0.95 ms with the one-element kernel, 0.46 ms with this one (a derivative matrix).
+struct OvKet {
+    int prim0, nprim, atom, rp0, row0;  // first primitive, count, atom, first norm, first row
+};
+
+template <int LB, bool DRV>
+__device__ __forceinline__ void axis_factors(double xpa, double ab, double h1, double h3, double p, int la,
+                                             double (&sb)[LB + 2])
+{
+    constexpr int N = LB + (DRV ? 2 : 1);
+    double w[N];
+    // s(0), s(1), ... up to s(la), then the window s(la) .. s(la + N - 1)
+    double prev = 0.0, cur = 1.0;
+    for (int a = 1; a <= la; ++a) {
+        const double nxt = a == 1 ? xpa : __dadd_rn(__dmul_rn(xpa, cur), __dmul_rn(recur(a - 1, h1, h3, p), prev));
+        prev = cur;
+        cur = nxt;
+    }
+    w[0] = cur;
+#pragma unroll
+    for (int i = 1; i < N; ++i) {
+        const int a = la + i;
+        const double nxt = a == 1 ? xpa : __dadd_rn(__dmul_rn(xpa, cur), __dmul_rn(recur(a - 1, h1, h3, p), prev));
+        prev = cur;
+        cur = nxt;
+        w[i] = cur;
+    }
+    sb[0] = w[0];
+#pragma unroll
+    for (int k = 1; k < N; ++k) {
+#pragma unroll
+        for (int i = 0; i < N - k; ++i) w[i] = __dadd_rn(w[i + 1], __dmul_rn(ab, w[i]));
+        sb[k] = w[0];
+    }
+}
+
+struct OvShellArgs {
+    int nrow;
+    const OvRow* rows;
+    const OvKet* kets;
+    int shell0[OKG_MAX_L + 2];   // ket shells of each L
+    int block0[OKG_MAX_L + 2];   // first block column of each L, highest L first
+    const double2* prim;
+    const double* pnorm;
+    const double* geo_a;
+    const double* geo_b;
+    const OvPair* pairs;
+    int nprim;
+    double* out;
+    long long ld;
+};
+
+template <int LB, int DD>  // DD: derivative axis, or -1
+__device__ __forceinline__ void shell_elements(const OvShellArgs& G, int bx)
+{
+    const int nrow = G.nrow, nprim = G.nprim, nket = G.shell0[LB + 1] - G.shell0[LB];
+    const OvRow* __restrict__ rows = G.rows;
+    const OvKet* __restrict__ kets = G.kets + G.shell0[LB];
+    const double2* __restrict__ prim = G.prim;
+    const double* __restrict__ pnorm = G.pnorm;
+    const double* __restrict__ geo_a = G.geo_a;
+    const double* __restrict__ geo_b = G.geo_b;
+    const OvPair* __restrict__ pairs = G.pairs;
+    double* __restrict__ out = G.out;
+    const long long ld = G.ld;
+    constexpr int NC = (LB + 1) * (LB + 2) / 2;
+    const int jk = bx * 32 + threadIdx.x;
+    const int I = blockIdx.y * blockDim.y + threadIdx.y;
+    if (I >= nrow) return;
+    const bool live = jk < nket;
+    const OvRow ri = rows[I];
+    const OvKet kt = kets[live ? jk : nket - 1];
+    double AB[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) AB[d] = geo_a[3 * ri.atom + d] - geo_b[3 * kt.atom + d];
+    const int la[3] = {lcomp(ri.la, 0), lcomp(ri.la, 1), lcomp(ri.la, 2)};
+    double acc[NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) acc[c] = 0.0;
+    // (the lanes of a warp may differ in the primitive count at the end of a group)
+    const int np = __reduce_max_sync(0xffffffffu, kt.nprim);
+    for (int ip = 0; ip < ri.nprim; ++ip) {
+        const double2 pa = prim[ri.prim0 + ip];
+        const double na = pnorm[ri.rp0 + ip];
+        for (int jp = 0; jp < np; ++jp) {
+            const bool on = jp < kt.nprim;
+            const double2* e = reinterpret_cast<const double2*>(pairs + (long long)(ri.prim0 + ip) * nprim + kt.prim0 +
+                                                               (on ? jp : 0));
+            const double2 e0 = e[0], e1 = e[1], e2 = e[2];
+            if (__all_sync(0xffffffffu, !on || e0.x == 0.0)) continue;  // the pair adds exactly 0
+            if (!on) continue;
+            const double2 pb = prim[kt.prim0 + jp];
+            const double p = pa.x + pb.x;
+            double s[3][LB + 2];
+            axis_factors<LB, DD == 0>(e1.x, AB[0], e0.y, e2.y, p, la[0], s[0]);
+            axis_factors<LB, DD == 1>(e1.y, AB[1], e0.y, e2.y, p, la[1], s[1]);
+            axis_factors<LB, DD == 2>(e2.x, AB[2], e0.y, e2.y, p, la[2], s[2]);
+            [&]<int... J>(std::integer_sequence<int, J...>) {
+                (
+                    [&] {
+                        constexpr int b[3] = {canon_l(LB, J, 0), canon_l(LB, J, 1), canon_l(LB, J, 2)};
+                        const double nb = pnorm[kt.rp0 + J * kt.nprim + jp];
+                        if constexpr (DD < 0) {
+                            const double v = __dmul_rn(__dmul_rn(__dmul_rn(e0.x, s[0][b[0]]), s[1][b[1]]), s[2][b[2]]);
+                            acc[J] = __dadd_rn(acc[J], __dmul_rn(__dmul_rn(__dmul_rn(__dmul_rn(pa.y, pb.y), na), nb), v));
+                        } else {
+                            constexpr int lbd = b[DD < 0 ? 0 : DD];
+                            if constexpr (lbd > 0) {
+                                const double v = __dmul_rn(__dmul_rn(__dmul_rn(e0.x, s[0][b[0] - (DD == 0)]), s[1][b[1] - (DD == 1)]),
+                                                           s[2][b[2] - (DD == 2)]);
+                                const double t = __dmul_rn(__dmul_rn(__dmul_rn((double)lbd * pa.y, pb.y), na), nb);
+                                acc[J] = __dadd_rn(acc[J], __dmul_rn(t, v));
+                            }
+                            const double v = __dmul_rn(__dmul_rn(__dmul_rn(e0.x, s[0][b[0] + (DD == 0)]), s[1][b[1] + (DD == 1)]),
+                                                       s[2][b[2] + (DD == 2)]);
+                            const double t = __dmul_rn(__dmul_rn(__dmul_rn(__dmul_rn(-2.0 * pb.x, pa.y), pb.y), na), nb);
+                            acc[J] = __dadd_rn(acc[J], __dmul_rn(t, v));
+                        }
+                    }(),
+                    ...);
+            }(std::make_integer_sequence<int, NC>{});
+        }
+    }
+    if (live) {
+        double* o = out + (long long)I * ld + kt.row0;
+#pragma unroll
+        for (int c = 0; c < NC; ++c) o[c] = acc[c];
+    }
+}
+
+// All ket shells in one launch (separate launches per L left a partly filled last wave each).
+template <int DD>
+__global__ void __launch_bounds__(128, 4) ao_overlap_shell_kernel(const __grid_constant__ OvShellArgs G)
+{
+    const int bx = blockIdx.x;
+    if (bx >= G.block0[0]) shell_elements<0, DD>(G, bx - G.block0[0]);
+    else if (bx >= G.block0[1]) shell_elements<1, DD>(G, bx - G.block0[1]);
+    else if (bx >= G.block0[2]) shell_elements<2, DD>(G, bx - G.block0[2]);
+    else if (bx >= G.block0[3]) shell_elements<3, DD>(G, bx - G.block0[3]);
+    else shell_elements<4, DD>(G, bx - G.block0[4]);
 }
 
 // A warp computes 32 elements of one bra row I.  Its kets are consecutive in the
@@ -167,7 +362,7 @@ __global__ void __launch_bounds__(256) ao_overlap_kernel(int nrow, const OvRow* 
                                                                    rj.prim0 + jp);
                 const double2 e0 = e[0], e1 = e[1], e2 = e[2];
                 pref = e0.x;
-                p = e0.y;
+                p = al + be;
                 xpa_t[0] = e1.x;
                 xpa_t[1] = e1.y;
                 xpa_t[2] = e2.x;
@@ -235,12 +430,18 @@ __global__ void aoom_transform_kernel(int nout, const int* __restrict__ ptr, con
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     const int r = blockIdx.y * blockDim.y + threadIdx.y;
     if (r >= nout || s >= nout) return;
+    const int i0 = ptr[r], i1 = ptr[r + 1], j0 = ptr[s], j1 = ptr[s + 1];
+    // (most rows are one Cartesian row with coefficient 1: its element as it is)
+    if (!renorm && i1 - i0 == 1 && j1 - j0 == 1 && coef[i0] == 1.0 && coef[j0] == 1.0) {
+        out[(long long)r * ld + s] = S[(long long)cart[i0] * lds + cart[j0]] + 0.0;
+        return;
+    }
     double acc = 0.0;
-    for (int i = ptr[r]; i < ptr[r + 1]; ++i) {
+    for (int i = i0; i < i1; ++i) {
         const int a = cart[i];
         const double ka = coef[i];
         const double na = renorm ? renorm[a] : 1.0;
-        for (int j = ptr[s]; j < ptr[s + 1]; ++j) {
+        for (int j = j0; j < j1; ++j) {
             const int b = cart[j];
             double sab = S[(long long)a * lds + b];
             if (renorm) sab = __dmul_rn(__dmul_rn(na, renorm[b]), sab);
@@ -255,6 +456,13 @@ __global__ void aoom_transform_kernel(int nout, const int* __restrict__ ptr, con
 using namespace okg;
 
 struct okg_overlap_plan {
+    // ket shells whose rows are the canonical components in order, sorted by (L, primitives):
+    // [shell0[L], shell0[L + 1]) per L; all kets of the plan, or none (canonical = 0)
+    OvKet* kets = nullptr;
+    uint64_t* exp_tab = nullptr;  // 2^(63 - j/2048), for the pair table
+    int shell0[OKG_MAX_L + 2] = {};
+    int canonical = 0;
+    std::vector<int> h_shell_ncart;
     int* ket_order = nullptr;  // kets sorted by (primitive count, exponents): the kernel's column order
     int* prim_atom = nullptr;  // atom of every primitive
     OvPair* pairs = nullptr;   // nprim x nprim primitive-pair table (NULL above OV_PAIR_TABLE_MAX bytes)
@@ -300,6 +508,39 @@ static std::vector<int> ov_ket_order(const std::vector<OvRow>& rows)
     return o;
 }
 
+// The plan's ket shells for the shell kernel; empty if a shell's listed rows are not the
+// canonical components of one L in order (explicit component lists, shifted exponents).
+static std::vector<OvKet> ov_canonical_kets(const std::vector<OvRow>& rows, const std::vector<int>& ncart, int (&shell0)[OKG_MAX_L + 2])
+{
+    std::vector<OvKet> k;
+    std::vector<int> ls;
+    int r0 = 0;
+    for (size_t s = 0; s < ncart.size(); r0 += ncart[s], ++s) {
+        int L = -1;
+        for (int l = 0; l <= OKG_MAX_L; ++l)
+            if (ncart[s] == ncanon(l)) L = l;
+        if (L < 0) return {};
+        for (int c = 0; c < ncart[s]; ++c)
+            for (int d = 0; d < 3; ++d)
+                if (((rows[r0 + c].lb >> (8 * d)) & 0xff) != canon_l(L, c, d)) return {};
+        k.push_back(OvKet{rows[r0].prim0, rows[r0].nprim, rows[r0].atom, rows[r0].rp0, r0});
+        ls.push_back(L);
+    }
+    std::vector<int> o(k.size());
+    for (size_t i = 0; i < o.size(); ++i) o[i] = (int)i;
+    std::stable_sort(o.begin(), o.end(), [&](int a, int b) {
+        return ls[a] != ls[b] ? ls[a] < ls[b] : k[a].nprim < k[b].nprim;
+    });
+    std::vector<OvKet> sorted;
+    for (int l = 0; l <= OKG_MAX_L + 1; ++l) shell0[l] = 0;
+    for (int i : o) {
+        sorted.push_back(k[i]);
+        ++shell0[ls[i] + 1];
+    }
+    for (int l = 1; l <= OKG_MAX_L + 1; ++l) shell0[l] += shell0[l - 1];
+    return sorted;
+}
+
 static void ov_free(okg_overlap_plan* p)
 {
     if (!p) return;
@@ -314,6 +555,8 @@ static void ov_free(okg_overlap_plan* p)
     cudaFree(p->ket_order);
     cudaFree(p->prim_atom);
     cudaFree(p->pairs);
+    cudaFree(p->kets);
+    cudaFree(p->exp_tab);
     delete p;
 }
 
@@ -366,6 +609,7 @@ extern "C" int okg_overlap_plan_create(int natom, int nshell, const int* h_shell
             P->h_lxa.insert(P->h_lxa.end(), l, l + 3);
             nrp += np;
         }
+        P->h_shell_ncart.push_back(nc);
         ncart += nc;
         nprim += np;
     }
@@ -443,7 +687,8 @@ extern "C" int okg_overlap_plan_create(int natom, int nshell, const int* h_shell
         prim_atom.reserve(nprim);
         for (int sh = 0; sh < nshell; ++sh)
             for (int q = 0; q < h_shell_nprim[sh]; ++q) prim_atom.push_back(h_shell_atom[sh]);
-        if ((st = ov_upload(&P->prim_atom, prim_atom.data(), prim_atom.size(), "okg_overlap_plan_create"))) {
+        if ((st = ov_upload(&P->prim_atom, prim_atom.data(), prim_atom.size(), "okg_overlap_plan_create")) ||
+            (st = ov_upload(&P->exp_tab, split_exp_table(), (size_t)OKG_SPLIT_EXP, "okg_overlap_plan_create"))) {
             ov_free(P);
             return st;
         }
@@ -452,6 +697,15 @@ extern "C" int okg_overlap_plan_create(int natom, int nshell, const int* h_shell
             ov_free(P);
             return cuda_status(e, "okg_overlap_plan_create: primitive-pair table");
         }
+    }
+    const std::vector<OvKet> kets = ov_canonical_kets(P->h_rows, P->h_shell_ncart, P->shell0);
+    P->canonical = !kets.empty();
+    e = cudaMalloc((void**)&P->kets, sizeof(OvKet) * nshell);
+    if (e == cudaSuccess && P->canonical)
+        e = cudaMemcpy(P->kets, kets.data(), sizeof(OvKet) * kets.size(), cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) {
+        ov_free(P);
+        return cuda_status(e, "okg_overlap_plan_create: ket shells");
     }
     *out = P;
     return OKG_OK;
@@ -493,9 +747,47 @@ extern "C" int okg_overlap_plan_set_ket(okg_overlap_plan* plan, const int* h_lxl
                                     cudaMemcpyHostToDevice),
                          "okg_overlap_plan_set_ket");
     if (st) return st;
+    const std::vector<OvKet> kets = ov_canonical_kets(plan->h_rows, plan->h_shell_ncart, plan->shell0);
+    plan->canonical = !kets.empty();
+    if (plan->canonical) {
+        st = cuda_status(cudaMemcpy(plan->kets, kets.data(), sizeof(OvKet) * kets.size(), cudaMemcpyHostToDevice),
+                         "okg_overlap_plan_set_ket");
+        if (st) return st;
+    }
     const std::vector<int> order = ov_ket_order(plan->h_rows);
     return cuda_status(cudaMemcpy(plan->ket_order, order.data(), order.size() * sizeof(int), cudaMemcpyHostToDevice),
                        "okg_overlap_plan_set_ket");
+}
+
+static void ov_shells(const okg_overlap_plan* P, const double* ga, const double* gb, int drv, double* S, long long lds,
+                      cudaStream_t st)
+{
+    OvShellArgs G;
+    G.nrow = P->ncart;
+    G.rows = P->rows;
+    G.kets = P->kets;
+    int nb = 0;
+    for (int l = 0; l <= OKG_MAX_L + 1; ++l) G.shell0[l] = P->shell0[l];
+    for (int l = OKG_MAX_L; l >= 0; --l) {
+        G.block0[l] = nb;
+        nb += (P->shell0[l + 1] - P->shell0[l] + 31) / 32;
+    }
+    G.block0[OKG_MAX_L + 1] = 0;
+    G.prim = P->prim;
+    G.pnorm = P->pnorm;
+    G.geo_a = ga;
+    G.geo_b = gb;
+    G.pairs = P->pairs;
+    G.nprim = P->nprim;
+    G.out = S;
+    G.ld = lds;
+    const dim3 blk(32, 4), grd(nb, (P->ncart + 3) / 4);
+    switch (drv) {
+    case 0: ao_overlap_shell_kernel<-1><<<grd, blk, 0, st>>>(G); break;
+    case 1: ao_overlap_shell_kernel<0><<<grd, blk, 0, st>>>(G); break;
+    case 2: ao_overlap_shell_kernel<1><<<grd, blk, 0, st>>>(G); break;
+    default: ao_overlap_shell_kernel<2><<<grd, blk, 0, st>>>(G); break;
+    }
 }
 
 extern "C" int okg_ao_overlap(okg_overlap_plan* plan, const double* d_geo_a, const double* d_geo_b, int drv,
@@ -515,10 +807,18 @@ extern "C" int okg_ao_overlap(okg_overlap_plan* plan, const double* d_geo_a, con
     const dim3 grd((plan->ncart + 31) / 32, (plan->ncart + 7) / 8);
     if (plan->pairs) {
         const dim3 gpp((plan->nprim + 31) / 32, (plan->nprim + 7) / 8);
-        ov_pairs_kernel<<<gpp, blk, 0, st>>>(plan->nprim, plan->prim, plan->prim_atom, d_geo_a, d_geo_b, plan->pairs);
-        ao_overlap_kernel<true><<<grd, blk, 0, st>>>(plan->ncart, plan->rows, plan->ket_order, plan->prim,
-                                                    plan->pnorm, d_geo_a, d_geo_b, plan->pairs, plan->nprim, drv,
-                                                    S, lds);
+        if (d_geo_a == d_geo_b)
+            ov_pairs_kernel<true><<<gpp, blk, 0, st>>>(plan->nprim, plan->prim, plan->prim_atom, d_geo_a, d_geo_b,
+                                                       plan->exp_tab, plan->pairs);
+        else
+            ov_pairs_kernel<false><<<gpp, blk, 0, st>>>(plan->nprim, plan->prim, plan->prim_atom, d_geo_a, d_geo_b,
+                                                        plan->exp_tab, plan->pairs);
+        if (plan->canonical)
+            ov_shells(plan, d_geo_a, d_geo_b, drv, S, lds, st);
+        else
+            ao_overlap_kernel<true><<<grd, blk, 0, st>>>(plan->ncart, plan->rows, plan->ket_order, plan->prim,
+                                                        plan->pnorm, d_geo_a, d_geo_b, plan->pairs, plan->nprim, drv,
+                                                        S, lds);
     } else {
         ao_overlap_kernel<false><<<grd, blk, 0, st>>>(plan->ncart, plan->rows, plan->ket_order, plan->prim,
                                                      plan->pnorm, d_geo_a, d_geo_b, nullptr, 0, drv, S, lds);

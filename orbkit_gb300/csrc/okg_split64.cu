@@ -251,35 +251,6 @@ __device__ __forceinline__ void mma_f16(uint32_t d, uint64_t a, uint64_t b, uint
 }
 
 // ------------------------------------------------------------------ FP64 AO values
-// e^(-alpha rr) as an FP64 value in integer arithmetic (the FP64 pipe is what bounds this
-// kernel: an FP64 exponential took 9 of its operations per primitive and point, this one
-// takes none).  mr 2^er = rr with a 64-bit mantissa; A 2^ea = alpha log2(e) likewise.
-//   u = alpha log2(e) rr from the upper half of mr A, as a fixed-point number with 53
-//   fraction bits: integer part k, 11 bits j, remainder f (42 bits);
-//   e = 2^-k 2^(-j/2048) 2^-f, 2^(-j/2048) from a table of 64-bit fixed-point numbers
-//   (table-driven exponential after P. T. P. Tang, ACM TOMS 15 (1989)) and
-//   2^-f = 1 - f (c1 - f (c2 - f (c3 - f c4))), c_n = (ln 2)^n / n! (f < 2^-11: the first
-//   term left out is below 2^-65), the inner terms in 32 bits.
-// Error before the final rounding: 0.7 2^-53 relative (the truncation of u).
-__device__ __forceinline__ double exp_neg(uint64_t mr, int er, uint64_t A, int ea, const uint64_t* __restrict__ tab)
-{
-    int s = -(er + ea) - 117;
-    const uint64_t Y = __umul64hi(mr, A) >> (s > 63 ? 63 : s < 0 ? 0 : s);
-    const int k = (int)(Y >> 53);
-    const uint64_t T = tab[(unsigned)(Y >> 42) & (TABN - 1)];
-    const uint64_t F = Y << 22;
-    const unsigned fh = (unsigned)(F >> 32);
-    const unsigned r3 = 3814213304u - (__umulhi(fh, 2643811198u) >> 13);
-    const unsigned r2 = 4127059964u - (__umulhi(fh, r3) >> 13);
-    const uint64_t c = 0xB17217F7D1CF79ACull - (((uint64_t)fh * r2) >> 13);
-    const uint64_t E = T - (__umul64hi(T, __umul64hi(F, c)) >> 11);
-    const int lz = __clz((int)(E >> 32));
-    const uint64_t n = E << lz;
-    const uint64_t m = (n >> 11) + ((n >> 10) & 1);
-    const uint64_t bits = m + ((uint64_t)(unsigned)(1022 - lz - k) << 52);
-    return (s < 0 || k > 1000) ? 0.0 : __longlong_as_double((long long)bits);
-}
-
 __device__ __noinline__ double slow_exp(double x) { return exp(x); }
 
 // position of x^a y^b z^c among the monomials of its degree
@@ -437,10 +408,9 @@ __device__ __forceinline__ void gen_shell(const Args& A, const State& S, uint32_
                                           double X, double Y, double Z, int row, int e0, int e1, int e2)
 {
     const double rr = X * X + Y * Y + Z * Z;
-    // rr = mr 2^er, mr with its top bit set (rr = 0: a value far below any alpha's range)
-    const unsigned rh = (unsigned)__double2hiint(rr), rl = (unsigned)__double2loint(rr);
-    const int er = (int)(rh >> 20) - 1086;
-    const uint64_t mr = ((uint64_t)__funnelshift_l(rl, (rh & 0xFFFFFu) | 0x100000u, 11) << 32) | (uint64_t)(rl << 11);
+    uint64_t mr;
+    int er;
+    split_mantissa(rr, mr, er);
     // radial sums R0 = sum w e, S1 = -2 sum w alpha e, S2 = 4 sum w alpha^2 e
     double R0 = 0.0, S1 = 0.0, S2 = 0.0;
 #pragma unroll 1

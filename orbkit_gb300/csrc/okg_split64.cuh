@@ -60,4 +60,40 @@ __device__ __forceinline__ bool split_prim(double2 p, float4& lg, SplitPrim& o)
     o.neg_alpha = -p.x;
     return inf || (isfinite(p.x) && isfinite(p.y));
 }
+// e^(-alpha rr) as an FP64 value in integer arithmetic (the FP64 pipe bounds the
+// kernels that use it, and an FP64 exponential takes 9 to 18 of its operations, this one
+// none).  mr 2^er = rr with a 64-bit mantissa; A 2^ea = alpha log2(e) likewise.
+//   u = alpha log2(e) rr from the upper half of mr A, as a fixed-point number with 53
+//   fraction bits: integer part k, 11 bits j, remainder f (42 bits);
+//   e = 2^-k 2^(-j/2048) 2^-f, 2^(-j/2048) from a table of 64-bit fixed-point numbers
+//   (table-driven exponential after P. T. P. Tang, ACM TOMS 15 (1989)) and
+//   2^-f = 1 - f (c1 - f (c2 - f (c3 - f c4))), c_n = (ln 2)^n / n! (f < 2^-11: the first
+//   term left out is below 2^-65), the inner terms in 32 bits.
+// Error before the final rounding: 0.7 2^-53 relative (the truncation of u).
+__device__ __forceinline__ double exp_neg(uint64_t mr, int er, uint64_t A, int ea, const uint64_t* __restrict__ tab)
+{
+    int s = -(er + ea) - 117;
+    const uint64_t Y = __umul64hi(mr, A) >> (s > 63 ? 63 : s < 0 ? 0 : s);
+    const int k = (int)(Y >> 53);
+    const uint64_t T = tab[(unsigned)(Y >> 42) & (OKG_SPLIT_EXP - 1)];
+    const uint64_t F = Y << 22;
+    const unsigned fh = (unsigned)(F >> 32);
+    const unsigned r3 = 3814213304u - (__umulhi(fh, 2643811198u) >> 13);
+    const unsigned r2 = 4127059964u - (__umulhi(fh, r3) >> 13);
+    const uint64_t c = 0xB17217F7D1CF79ACull - (((uint64_t)fh * r2) >> 13);
+    const uint64_t E = T - (__umul64hi(T, __umul64hi(F, c)) >> 11);
+    const int lz = __clz((int)(E >> 32));
+    const uint64_t n = E << lz;
+    const uint64_t m = (n >> 11) + ((n >> 10) & 1);
+    const uint64_t bits = m + ((uint64_t)(unsigned)(1022 - lz - k) << 52);
+    return (s < 0 || k > 1000) ? 0.0 : __longlong_as_double((long long)bits);
+}
+
+// rr >= 0 as mr 2^er, mr with its top bit set (rr = 0: a value far below any exponent's range).
+__device__ __forceinline__ void split_mantissa(double rr, uint64_t& mr, int& er)
+{
+    const unsigned rh = (unsigned)__double2hiint(rr), rl = (unsigned)__double2loint(rr);
+    er = (int)(rh >> 20) - 1086;
+    mr = ((uint64_t)__funnelshift_l(rl, (rh & 0xFFFFFu) | 0x100000u, 11) << 32) | (uint64_t)(rl << 11);
+}
 }  // namespace okg
