@@ -10,6 +10,7 @@
 // contraction), so for the same MO grids the results are orbkit's to the bit.
 // Term tables are read by every thread of a warp at the same address (broadcast
 // through L1); MO values are read coalesced.
+#include "okg_digits.cuh"
 #include "okg_internal.cuh"
 
 namespace okg {
@@ -119,6 +120,218 @@ __global__ void __launch_bounds__(128) ci_quad_kernel(long long npts, const doub
     }
 }
 
+// The same quadratic forms with the matrix-vector product on the tensor cores: per 128 points
+// the MO values become exact digit operands (okg_digits.cuh), t_b = sum_a Q^T[b][a] MO_a comes
+// back as FP64 values, and the FP64 pipe is left with t_b MO_b (NMO FMAs per point) or
+// t_b dMO_b (3 NMO) of the NMO^2 (+ 3 NMO).  The coefficient digits are made by every CTA for
+// itself (at most 64 x 64 values) and stay in shared memory; the MO values are read twice
+// (scale, then digits: the second time from L1).
+struct CiSplit {
+    long long npts, ld;
+    const double* mo;
+    const double* drv;
+    const double* qt;
+    int nmo, ldq, np;  // np: nmo rounded up to 16 (= ldq)
+    double scale;
+    double* out;
+    int* status;
+    unsigned tm_cols;
+};
+
+constexpr int CI_SPLIT_MAX = 64;  // MOs: 7 accumulators per MO in 512 TMEM columns
+
+static size_t ci_split_smem(int np)
+{
+    return 1024 + (size_t)(np / 16) * (sp::ND * sp::DT + sp::ND * np * 32) + 3 * 3 * 128 * 8 + 4 * 128 * 8 + 64 * 4 + 64;
+}
+
+template <int G>
+__device__ __forceinline__ unsigned long long largest(const unsigned long long* tops, int r)
+{
+    unsigned long long m = tops[r];
+#pragma unroll
+    for (int g = 1; g < G; ++g) m = tops[g * 128 + r] > m ? tops[g * 128 + r] : m;
+    return m;
+}
+
+// G threads per point (G warps per 32 accumulator rows).  Phases alternate in a CTA (digits,
+// MMAs, accumulators), so their latency shows: with more than 32 MOs one CTA of 512 threads
+// per SM (42 MOs, 2^20 points: rho 2.26 ms with the DFMA kernel, 0.92 with G = 2, 0.72 with
+// G = 4; flux 4.07, 1.09, 0.88), up to 32 MOs two CTAs of 256 (24 MOs: rho 0.93, 0.35 with
+// G = 2, 0.48 with G = 4; 8 MOs: 0.24, 0.16, 0.27).
+template <bool FLUX, int G>
+__global__ void __launch_bounds__(128 * G, 4 / G) ci_split_kernel(const __grid_constant__ CiSplit A)
+{
+    using namespace sp;
+    extern __shared__ unsigned char raw[];
+    unsigned char* base = (unsigned char*)(((uintptr_t)raw + 1023) & ~(uintptr_t)1023);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int np = A.np, KP = np / 16, bpanel = ND * np * 32;
+    unsigned char* Bs = base + (size_t)KP * ND * DT;
+    double* part = (double*)(Bs + (size_t)KP * bpanel);            // 3 x 3 x 128
+    unsigned long long* tops = (unsigned long long*)(part + 9 * 128);  // 4 x 128
+    int* fexp = (int*)(tops + 512);
+    uint64_t* bar = (uint64_t*)(fexp + CI_SPLIT_MAX);
+    uint32_t* tmem_slot = (uint32_t*)(bar + 1);
+    const uint32_t bar_a = smem_u32(bar);
+    // coefficient digits
+    for (int b = warp; b < np; b += 4 * G) {
+        unsigned long long m = 0;
+        for (int a = lane; a < A.nmo && b < A.nmo; a += 32) {
+            const unsigned long long u = (unsigned long long)__double_as_longlong(A.qt[(long long)b * A.ldq + a]) & 0x7FFFFFFFFFFFFFFFull;
+            m = u > m ? u : m;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const unsigned long long u = __shfl_xor_sync(0xffffffffu, m, o);
+            m = u > m ? u : m;
+        }
+        const bool nan = (m >> 52) == 0x7FF;
+        const int F = scale_of(m);
+        if (lane == 0) fexp[b] = nan ? MO_NAN : F;
+        for (int a = lane; a < np; a += 32) {
+            const double v = (a < A.nmo && b < A.nmo) ? A.qt[(long long)b * A.ldq + a] : 0.0;
+            const uint64_t t = nan ? 0x0080808080808080ull : digits7(v, F + 1030);
+#pragma unroll
+            for (int j = 0; j < ND; ++j)
+                *(__half*)(Bs + (a >> 4) * bpanel + b_off(j * np + b, a & 15)) = __int2half_rn((int)((t >> (8 * (6 - j))) & 0xFF) - 128);
+        }
+    }
+    if (tid == 0) {
+        mbar_init(bar_a, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(A.tm_cols));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    fence_proxy_async();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+    const int r = tid & 127, part4 = tid >> 7;
+    const long long ntiles = (A.npts + 127) / 128, dstride = (long long)A.nmo * A.ld;
+    const int h0 = part4 * KP * (16 / G), h1 = h0 + KP * (16 / G);  // this thread's MOs
+    uint32_t parity = 0;
+    for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x, parity ^= 1) {
+        const long long p = tile * 128 + r < A.npts ? tile * 128 + r : A.npts - 1;
+        unsigned long long m = 0;
+#pragma unroll 8
+        for (int a = h0; a < h1; ++a) {
+            const unsigned long long u = a < A.nmo ? (unsigned long long)__double_as_longlong(A.mo[(long long)a * A.ld + p]) & 0x7FFFFFFFFFFFFFFFull : 0ull;
+            m = u > m ? u : m;
+        }
+        tops[part4 * 128 + r] = m;
+        __syncthreads();
+        m = largest<G>(tops, r);
+        const int E = scale_of(m), rs = E + 1030;
+#pragma unroll 4
+        for (int a = h0; a < h1; ++a)
+            put1(a < A.nmo ? A.mo[(long long)a * A.ld + p] : 0.0, rs, smem_u32(base) + (a >> 4) * (ND * DT) + a_off(r, a & 15));
+        fence_proxy_async();
+        __syncthreads();
+        if (tid == 0) {
+            tc_fence_after();
+            const int dmax = 256 / np;
+#pragma unroll 1
+            for (int k = 0; k < KP; ++k)
+#pragma unroll 1
+                for (int i = 0; i < ND; ++i) {
+                    const uint64_t ad = a_desc(smem_u32(base) + (uint32_t)(k * ND + i) * DT);
+#pragma unroll 1
+                    for (int j = 0; j < ND - i; j += dmax) {
+                        const int nd = ND - i - j < dmax ? ND - i - j : dmax;
+                        mma_f16(tmem + (uint32_t)((i + j) * np), ad, b_desc(smem_u32(Bs) + (uint32_t)(k * bpanel + j * np * 32)),
+                                idesc(nd * np), (k > 0 || i > 0) ? 1u : 0u);
+                    }
+                }
+            mma_commit(bar_a);
+        }
+        const bool ok = mbar_wait(bar_a, parity, A.status, WAIT_LIMIT);
+        if (!__syncthreads_and(ok)) {
+            parity ^= 1;
+            break;
+        }
+        tc_fence_after();
+        // accumulators: warps w, w + 4, ... share 32 rows, every G-th group of 4 MOs each
+        const int quad = warp & 3, row = quad * 32 + lane, hf = warp >> 2;
+        const long long q = tile * 128 + row;
+        const bool valid = q < A.npts;
+        const long long pr = valid ? q : A.npts - 1;
+        const unsigned long long mr = largest<G>(tops, row);
+        const int rowx = (mr >> 52) == 0x7FF ? ROW_NAN : scale_of(mr);
+        double acc[3] = {0.0, 0.0, 0.0};
+#pragma unroll 1
+        for (int n0 = 4 * hf; n0 < A.nmo; n0 += 4 * G) {
+            Acc4 va;
+            double t[4];
+            acc_load(va, tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)n0, np);
+            const int4 f4 = *(const int4*)(fexp + n0);
+            double x[FLUX ? 3 : 1][4];
+            const double* src = FLUX ? A.drv : A.mo;
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int d = 0; d < (FLUX ? 3 : 1); ++d)
+                    x[d][i] = n0 + i < A.nmo ? src[d * dstride + (long long)(n0 + i) * A.ld + pr] : 0.0;
+            acc_wait(va);
+            acc_values(va, rowx, f4, t);
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int d = 0; d < (FLUX ? 3 : 1); ++d)
+                    if (n0 + i < A.nmo) acc[d] = fma(t[i], x[d][i], acc[d]);
+        }
+        if (hf > 0)
+            for (int d = 0; d < (FLUX ? 3 : 1); ++d) part[((hf - 1) * 3 + d) * 128 + row] = acc[d];
+        tc_fence_before();
+        __syncthreads();
+        if (hf == 0 && valid)
+            for (int d = 0; d < (FLUX ? 3 : 1); ++d) {
+                double t = acc[d];
+                for (int h = 0; h < G - 1; ++h) t += part[(h * 3 + d) * 128 + row];
+                A.out[d * A.npts + q] = A.scale * t;
+            }
+    }
+    // (after an expired wait: the MMAs issued last complete before the CTA leaves)
+    if (tid == 0 && blockIdx.x < ntiles) mbar_drain(bar_a, parity ^ 1);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(A.tm_cols));
+}
+
+// Runs the quadratic form on the tensor cores where it is one for them.
+template <bool FLUX>
+static int ci_split(long long npts, const double* mo, const double* drv, long long ld, int nmo, const double* qt, double scale,
+                    double* out, cudaStream_t st, bool& done)
+{
+    done = false;
+    if (nmo > CI_SPLIT_MAX) return OKG_OK;
+    int* status = split_status_word();
+    if (!status) return OKG_OK;
+    CiSplit A{npts, ld, mo, drv, qt, nmo, (nmo + 15) / 16 * 16, (nmo + 15) / 16 * 16, scale, out, status, 32};
+    while ((int)A.tm_cols < sp::ND * A.np) A.tm_cols *= 2;
+    const size_t smem = ci_split_smem(A.np);
+    int dev = 0, sms = 1;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int per = A.np <= 32 ? 2 : 1;  // CTAs per SM
+    const long long ntiles = (npts + 127) / 128, cap = (long long)sms * per;
+    const unsigned nblk = (unsigned)(ntiles < cap ? ntiles : cap);
+    auto go = [&](auto kernel, int threads) -> int {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return cuda_status(e, "detCI quadratic form: shared memory");
+        kernel<<<nblk, threads, smem, st>>>(A);
+        return OKG_OK;
+    };
+    const int s = per == 2 ? go(ci_split_kernel<FLUX, 2>, 256) : go(ci_split_kernel<FLUX, 4>, 512);
+    if (s) return s;
+    done = true;
+    return cuda_status(cudaGetLastError(), "detCI quadratic form launch");
+}
+
 }  // namespace okg
 
 using namespace okg;
@@ -184,6 +397,9 @@ extern "C" int okg_ci_rho_matrix(int64_t npts, const double* d_mo, int64_t ld, i
         return set_error(OKG_ERR_ARG, "okg_ci_rho_matrix: bad argument (NULL pointer, npts < 0, ld < npts, nmo <= 0)");
     if (((uintptr_t)d_qt & 15) != 0) return set_error(OKG_ERR_ARG, "okg_ci_rho_matrix: d_qt not 16-byte aligned");
     if (npts == 0) return OKG_OK;
+    bool done = false;
+    const int s = ci_split<false>(npts, d_mo, nullptr, ld, nmo, d_qt, 1.0, d_rho, (cudaStream_t)stream, done);
+    if (s || done) return s;
     const unsigned nblk = (unsigned)((npts + 127) / 128);
     ci_quad_kernel<false><<<nblk, 128, 0, (cudaStream_t)stream>>>(npts, d_mo, nullptr, ld, nmo, d_qt, 1.0, d_rho);
     return cuda_status(cudaGetLastError(), "okg_ci_rho_matrix launch");
@@ -196,6 +412,9 @@ extern "C" int okg_ci_flux_matrix(int64_t npts, const double* d_mo, const double
         return set_error(OKG_ERR_ARG, "okg_ci_flux_matrix: bad argument (NULL pointer, npts < 0, ld < npts, nmo <= 0)");
     if (((uintptr_t)d_qt & 15) != 0) return set_error(OKG_ERR_ARG, "okg_ci_flux_matrix: d_qt not 16-byte aligned");
     if (npts == 0) return OKG_OK;
+    bool done = false;
+    const int s = ci_split<true>(npts, d_mo, d_drv, ld, nmo, d_qt, scale, d_j, (cudaStream_t)stream, done);
+    if (s || done) return s;
     const unsigned nblk = (unsigned)((npts + 127) / 128);
     ci_quad_kernel<true><<<nblk, 128, 0, (cudaStream_t)stream>>>(npts, d_mo, d_drv, ld, nmo, d_qt, scale, d_j);
     return cuda_status(cudaGetLastError(), "okg_ci_flux_matrix launch");

@@ -330,6 +330,9 @@ SplitLayout split_layout(const std::vector<Shell>& shells, const std::vector<int
                          const std::vector<double>& comp_g, const int* order);
 const uint64_t* split_exp_table();                   // host, OKG_SPLIT_EXP entries
 
+// Page-locked word that a kernel raises when a bounded wait expires (okg_wait_status).
+int* split_status_word();
+
 struct SplitCall {
     int nmo;
     const double* C;    // nmo x ncart

@@ -38,24 +38,20 @@
 // integer code (digits, exponentials, conversion of the accumulators), which is why the
 // kernel runs with 23 warps of 80 registers: 8 generation warps in lock step with 128
 // registers took 21.2 ms.
-#include <cuda_fp16.h>
 #include <math.h>
 
 #include <mutex>
 #include <vector>
 
+#include "okg_digits.cuh"
 #include "okg_internal.cuh"
 #include "okg_split64.cuh"
-#include "okg_tc.cuh"
 
 namespace okg {
 namespace sp {
 
 using namespace mx;
 
-constexpr int ND = 7;                   // digits of an operand
-constexpr int PK = OKG_SPLIT_PK;        // columns of a panel: one MMA K-step
-constexpr int DT = 128 * PK * 2;        // bytes of one digit of one 128-row operand tile
 constexpr int GROUP = 10;               // panels per accumulation (exact FP32 sums: see the header)
 constexpr int MAX_SHELLS = 2048;
 constexpr int MAX_PANELS = 768;
@@ -64,8 +60,6 @@ constexpr int NTW = 2;                  // tile warps, each with every second bu
 constexpr int MAX_BIG = 512;
 constexpr int TABN = OKG_SPLIT_EXP;     // entries of the 2^(j/2048) table
 constexpr int SMEM_MAX = 232448;
-constexpr int ROW_NAN = 30000, ROW_ZERO = 30001;  // row exponents of points without finite AO values
-constexpr int MO_NAN = 200000;                      // exponent of an MO with a non-finite coefficient
 constexpr float KEEP_LOG2 = 62.0f;
 constexpr float ABS_FLOOR = -1000.0f;   // values below 2^-1000 are dropped
 
@@ -189,67 +183,6 @@ __device__ __forceinline__ bool warp_wait(const State& S, uint32_t bar, uint32_t
     return __all_sync(0xffffffffu, wait(S, bar, parity, status));
 }
 
-// ------------------------------------------------------------------ digits
-// v = t 2^(E - 55), t rounded to an integer of 7 balanced base-256 digits; returned
-// biased by 128 per digit (byte b holds digit + 128), rs0 = E + 1030.  Integer
-// instructions only; |v| < 0.99 2^E.
-__device__ __forceinline__ uint64_t digits7(double v, int rs0)
-{
-    const int hi = __double2hiint(v);
-    const unsigned lo = (unsigned)__double2loint(v);
-    const int ex = (hi >> 20) & 0x7FF;
-    const unsigned mh = ((unsigned)hi & 0xFFFFFu) | 0x100000u;
-    const uint64_t m = ((uint64_t)__funnelshift_l(lo, mh, 10) << 32) | (uint64_t)(lo << 10);
-    int s = rs0 - 1 - ex;
-    s = s < 7 ? 7 : s > 63 ? 63 : s;
-    const uint64_t q = ((m >> s) + 1) >> 1;
-    const uint64_t neg = (uint64_t)(long long)(hi >> 31);
-    return ((q ^ neg) - neg) + 0x0080808080808080ull;
-}
-
-// Two biased digit bytes (byte b of two values) -> two FP16 digits.
-__device__ __forceinline__ uint32_t digit_pair(uint32_t w0, uint32_t w1, int b)
-{
-    const uint32_t r = (__byte_perm(w0, w1, (uint32_t)(b | (b << 4) | ((4 + b) << 8) | (b << 12))) & 0x00FF00FFu) | 0x64006400u;
-    const __half2 h = __hsub2(*reinterpret_cast<const __half2*>(&r), __half2(__ushort_as_half(0x6480), __ushort_as_half(0x6480)));
-    return *reinterpret_cast<const uint32_t*>(&h);
-}
-
-// byte offset of (row m, column k) in a 128 x 16 FP16 digit tile: M-major, 128-byte
-// swizzle (64 rows per 128-byte line, lines of 8 columns per atom)
-__device__ __forceinline__ uint32_t a_off(int m, int k)
-{
-    return (uint32_t)((m >> 6) * 1024 + (k >> 3) * 2048 + (k & 7) * 128 + ((((m >> 3) ^ k) & 7) << 4) + ((m & 7) << 1));
-}
-
-// byte offset of (row n, column k) of the coefficient digits: K-major, 32-byte rows,
-// 32-byte swizzle
-__host__ __device__ __forceinline__ uint32_t b_off(int n, int k)
-{
-    return (uint32_t)((n >> 3) * 256 + (n & 7) * 32 + ((((k >> 3) ^ (n >> 2)) & 1) << 4) + ((k & 7) << 1));
-}
-
-__device__ __forceinline__ uint64_t a_desc(uint32_t addr)
-{
-    return (uint64_t)((addr >> 4) & 0x3FFF) | ((uint64_t)(1024 >> 4) << 16) | ((uint64_t)(2048 >> 4) << 32) |
-           ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
-}
-__device__ __forceinline__ uint64_t b_desc(uint32_t addr)
-{
-    return (uint64_t)((addr >> 4) & 0x3FFF) | ((uint64_t)1 << 16) | ((uint64_t)(256 >> 4) << 32) | ((uint64_t)1 << 46) |
-           ((uint64_t)6 << 61);
-}
-// kind::f16, A = B = FP16, D = FP32, M-major A, K-major B, M = 128
-__host__ __device__ constexpr uint32_t idesc(int n) { return (1u << 4) | (1u << 15) | ((uint32_t)(n >> 3) << 17) | (8u << 24); }
-
-__device__ __forceinline__ void mma_f16(uint32_t d, uint64_t a, uint64_t b, uint32_t id, uint32_t acc)
-{
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d),
-        "l"(a), "l"(b), "r"(id), "r"(acc));
-}
-
 // ------------------------------------------------------------------ FP64 AO values
 __device__ __noinline__ double slow_exp(double x) { return exp(x); }
 
@@ -348,28 +281,7 @@ __device__ __forceinline__ void shell_values(double X, double Y, double Z, doubl
     }(std::make_integer_sequence<int, N>{});
 }
 
-__device__ __forceinline__ void sts16(uint32_t a, unsigned v) { asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "h"((unsigned short)v) : "memory"); }
 __device__ __forceinline__ void sts64(uint32_t a, uint32_t x, uint32_t y) { asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(a), "r"(x), "r"(y) : "memory"); }
-
-// Digits of one column value (value channel alone) into the 7 digit tiles.  A call, like
-// put4: the digit code appears once instead of once per component and angular momentum
-// (inlined, the kernel's hot code was far beyond the instruction cache: 30 % of its
-// instruction requests missed).
-__device__ __noinline__ void put1(double v, int rs, uint32_t a)
-{
-    const uint64_t t = digits7(v, rs);
-    const uint32_t lo = (uint32_t)t, hi = (uint32_t)(t >> 32);
-    // digit 0 is the most significant byte (byte 6)
-    const uint32_t h20 = digit_pair(hi, hi >> 16, 0), h1 = digit_pair(hi, hi, 1);
-    const uint32_t h64 = digit_pair(lo, lo >> 16, 0), h53 = digit_pair(lo, lo >> 16, 1);
-    sts16(a + 0 * DT, h20 >> 16);
-    sts16(a + 1 * DT, h1);
-    sts16(a + 2 * DT, h20);
-    sts16(a + 3 * DT, h53 >> 16);
-    sts16(a + 4 * DT, h64 >> 16);
-    sts16(a + 5 * DT, h53);
-    sts16(a + 6 * DT, h64);
-}
 
 // Digits of four rows (channels of a point) of a column.
 __device__ __noinline__ void put4(double v0, double v1, double v2, double v3, int rs0, int rs1, uint32_t a)
@@ -628,65 +540,6 @@ __device__ __forceinline__ void mma_role(const Args& A, const State& S)
 }
 
 // ------------------------------------------------------------------ epilogue
-// Seven accumulators of four MOs (columns n0 .. n0 + 3) of this lane's row.
-struct Acc4 {
-    uint32_t r[7][4];
-};
-__device__ __forceinline__ void acc_load(Acc4& a, uint32_t taddr, int np)
-{
-#pragma unroll
-    for (int w = 0; w < 7; ++w)
-        asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
-                     : "=r"(a.r[w][0]), "=r"(a.r[w][1]), "=r"(a.r[w][2]), "=r"(a.r[w][3])
-                     : "r"(taddr + (uint32_t)(w * np)));
-}
-// (the loaded registers are operands: no use of them moves before the wait)
-__device__ __forceinline__ void acc_wait(Acc4& a)
-{
-    asm volatile("tcgen05.wait::ld.sync.aligned;"
-                 : "+r"(a.r[0][0]), "+r"(a.r[0][1]), "+r"(a.r[0][2]), "+r"(a.r[0][3]), "+r"(a.r[1][0]), "+r"(a.r[1][1]), "+r"(a.r[1][2]), "+r"(a.r[1][3]), "+r"(a.r[2][0]), "+r"(a.r[2][1]), "+r"(a.r[2][2]), "+r"(a.r[2][3]), "+r"(a.r[3][0]), "+r"(a.r[3][1]), "+r"(a.r[3][2]), "+r"(a.r[3][3]), "+r"(a.r[4][0]), "+r"(a.r[4][1]), "+r"(a.r[4][2]), "+r"(a.r[4][3]), "+r"(a.r[5][0]), "+r"(a.r[5][1]), "+r"(a.r[5][2]), "+r"(a.r[5][3]), "+r"(a.r[6][0]), "+r"(a.r[6][1]), "+r"(a.r[6][2]), "+r"(a.r[6][3]));
-}
-
-__device__ __forceinline__ int f2i(uint32_t r) { return __float2int_rn(__uint_as_float(r)); }
-
-// sum_w acc_w 2^(-8 w) 2^x as an FP64 value, rounded once, in integer arithmetic (a
-// conversion on the FP64 pipe would cost its bound): t = sum acc_w 2^(40 - 8 w) in 64
-// bits, x = scale - 40 included by the caller.
-__device__ __forceinline__ double combine7(const int (&a)[7], int x)
-{
-    const long long lo = (long long)a[4] * 256 + a[5] + ((a[6] + 128) >> 8);
-    const long long t = (((long long)(a[0] * 256 + a[1])) << 32) + ((long long)(a[2] * 256 + a[3]) << 16) + lo;
-    const unsigned long long neg = (unsigned long long)(t >> 63);
-    const unsigned long long u = ((unsigned long long)t ^ neg) - neg;
-    const int lz = __clzll((long long)u);
-    const unsigned long long n = u << (lz & 63);
-    const unsigned long long m = (n >> 11) + ((n >> 10) & 1);  // 53 bits, rounded
-    const int e = 1023 + 63 - lz + x;                          // biased exponent of the leading bit
-    if (u == 0 || e <= 0) return 0.0;
-    if (e >= 0x7FF) return __hiloint2double((int)(0x7FF00000u | (unsigned)(neg & 0x80000000u)), 0);
-    const unsigned long long bits = ((unsigned long long)(unsigned)(e - 1) << 52) + m;
-    return __longlong_as_double((long long)(bits | (neg & 0x8000000000000000ull)));
-}
-
-// Accumulators of four MOs -> FP64 values of this lane's row.
-__device__ __forceinline__ void acc_values(const Acc4& a, int rowx, const int4& f4, double (&v)[4])
-{
-    const int f[4] = {f4.x, f4.y, f4.z, f4.w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int t[7] = {f2i(a.r[0][i]), f2i(a.r[1][i]), f2i(a.r[2][i]), f2i(a.r[3][i]), f2i(a.r[4][i]), f2i(a.r[5][i]), f2i(a.r[6][i])};
-        // a = t 2^(E - 55), c = s 2^(F - 55); leading digits weigh 2^48: products 2^(E + F - 14)
-        v[i] = combine7(t, rowx + f[i] - 54);
-        if (rowx >= ROW_NAN || f[i] == MO_NAN) v[i] = (rowx == ROW_ZERO && f[i] != MO_NAN) ? 0.0 : __longlong_as_double(0x7FF8000000000000ll);
-    }
-}
-
-__device__ __forceinline__ double shfl_d(double v, int src)
-{
-    return __hiloint2double(__shfl_sync(0xffffffffu, __double2hiint(v), src),
-                            __shfl_sync(0xffffffffu, __double2loint(v), src));
-}
-
 // o 2^x v: through the exponent field where the occupation o is a power of two (2, 1, ...;
 // the FP64 pipe is the bound), the same value as the product.
 __device__ __forceinline__ double times_occ(double v, double o, int x)
@@ -1291,10 +1144,7 @@ __global__ void __launch_bounds__(256) split_pack_kernel(SplitDev S, int nmo, in
     atomicMax(&top, m);
     __syncthreads();
     const int ex = (int)(top >> 52);
-    // exponent F with |c| < 0.99 2^F
-    int F = ex == 0 ? -1022 : ex - 1022;
-    if (((top >> 44) & 0xFF) >= 0xFA) ++F;
-    if (F < -900) F = -900;
+    const int F = scale_of(top);
     const bool nan = ex == 0x7FF;
     if (threadIdx.x == 0) {
         fexp[mo] = nan ? MO_NAN : F;
@@ -1373,13 +1223,9 @@ const uint64_t* split_exp_table()
     return t.data();
 }
 
-namespace {
-
-constexpr int MAX_DEVICES = 64;
-
 // Raised by a kernel whose bounded wait expired: one page-locked word per process,
 // written by the device and read by okg_wait_status after the stream was waited for.
-int* status_word()
+int* split_status_word()
 {
     static int* const w = [] {
         int* p = nullptr;
@@ -1392,6 +1238,10 @@ int* status_word()
     }();
     return w;
 }
+
+namespace {
+
+constexpr int MAX_DEVICES = 64;
 
 // The library's own stream-ordered pool for the coefficient digits of a call (a few MB):
 // safe for any number of threads and streams; up to 64 MB stay mapped between calls.
@@ -1493,7 +1343,7 @@ int run(const okg_basis* b, const Grid& g, const SplitCall& c, cudaStream_t st, 
     if (A.nslot > sp::MAX_SLOTS) A.nslot = sp::MAX_SLOTS;
     if (A.nslot < 2) return OKG_OK;
     const int nblk = (int)(A.ntiles < sms ? A.ntiles : sms);
-    int* status = status_word();
+    int* status = split_status_word();
     cudaMemPool_t pool = workspace_pool(device);
     if (!status || !pool) return OKG_OK;
     A.status = status;
@@ -1552,7 +1402,7 @@ int split_run(const okg_basis* b, const Grid& g, const SplitCall& c, cudaStream_
 
 extern "C" int okg_wait_status(int* status)
 {
-    int* w = okg::status_word();
+    int* w = okg::split_status_word();
     const int v = w ? *(volatile int*)w : 0;
     if (status) *status = v;
     if (!v) return OKG_OK;

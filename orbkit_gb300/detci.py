@@ -79,6 +79,15 @@ def _zero_terms(zero):
 
 
 def _sing_terms(sing):
+    # plain lists of numbers and of index pairs convert in one go; anything else (ragged
+    # rows, objects) entry by entry
+    try:
+        coef, pairs = numpy.asarray(sing[0]), numpy.asarray(sing[1])
+        if coef.ndim == 1 and coef.dtype.kind in "fiu" and pairs.ndim == 2 and pairs.shape[1] >= 2 and \
+                pairs.dtype.kind in "iu" and len(coef) == len(pairs):
+            return coef.astype(numpy.float64), numpy.ascontiguousarray(pairs[:, :2], dtype=numpy.int32)
+    except ValueError:
+        pass
     coef = numpy.asarray([float(c) for c in sing[0]], dtype=numpy.float64)
     pairs = numpy.asarray([[int(p[0]), int(p[1])] for p in sing[1]], dtype=numpy.int32).reshape(-1, 2)
     return coef, pairs
@@ -95,8 +104,11 @@ def _covered(npts, slice_length):
 
 
 def _out(t, shape, was_tensor):
-    return t.reshape(tuple(t.shape[:-1]) + tuple(shape)) if was_tensor else t.cpu().numpy().reshape(
-        tuple(t.shape[:-1]) + tuple(shape))
+    if was_tensor:
+        return t.reshape(tuple(t.shape[:-1]) + tuple(shape))
+    out = t.cpu().numpy().reshape(tuple(t.shape[:-1]) + tuple(shape))
+    _lib.check(_lib.load().okg_wait_status(None))
+    return out
 
 
 def _qt_device(qt_rows, nmo):
