@@ -159,6 +159,32 @@ __device__ __forceinline__ double shfl_d(double v, int src)
                             __shfl_sync(0xffffffffu, __double2loint(v), src));
 }
 
+// The same for two MOs (half the registers).
+struct Acc2 {
+    uint32_t r[7][2];
+};
+__device__ __forceinline__ void acc2_load(Acc2& a, uint32_t taddr, int np)
+{
+#pragma unroll
+    for (int w = 0; w < 7; ++w)
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0,%1}, [%2];" : "=r"(a.r[w][0]), "=r"(a.r[w][1]) : "r"(taddr + (uint32_t)(w * np)));
+}
+__device__ __forceinline__ void acc2_wait(Acc2& a)
+{
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(a.r[0][0]), "+r"(a.r[0][1]), "+r"(a.r[1][0]), "+r"(a.r[1][1]), "+r"(a.r[2][0]), "+r"(a.r[2][1]), "+r"(a.r[3][0]), "+r"(a.r[3][1]), "+r"(a.r[4][0]), "+r"(a.r[4][1]), "+r"(a.r[5][0]), "+r"(a.r[5][1]), "+r"(a.r[6][0]), "+r"(a.r[6][1]));
+}
+__device__ __forceinline__ void acc2_values(const Acc2& a, int rowx, const int2& f2, double (&v)[2])
+{
+    const int f[2] = {f2.x, f2.y};
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int t[7] = {f2i(a.r[0][i]), f2i(a.r[1][i]), f2i(a.r[2][i]), f2i(a.r[3][i]), f2i(a.r[4][i]), f2i(a.r[5][i]), f2i(a.r[6][i])};
+        v[i] = combine7(t, rowx + f[i] - 54);
+        if (rowx >= ROW_NAN || f[i] == MO_NAN) v[i] = (rowx == ROW_ZERO && f[i] != MO_NAN) ? 0.0 : __longlong_as_double(0x7FF8000000000000ll);
+    }
+}
+
 // Exponent F with |v| < 0.99 2^F for the magnitude bits `top` of the largest |v| (finite).
 __device__ __forceinline__ int scale_of(unsigned long long top)
 {

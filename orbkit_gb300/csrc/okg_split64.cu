@@ -26,18 +26,19 @@
 // Tile: 128 operand rows (2 x 128 with second derivatives): 128 points x 1 channel, or
 // 32 points x (value, d/dx, d/dy, d/dz) [+ 32 x (xx, yy, zz, unused)].  Persistent CTAs,
 // one per SM, tiles handed out by a device counter; warps of a CTA:
-//   8 generation warps  FP64 radial sums and polynomials of the kept shells, digits
-//                       written to the panel's operand slot (ring of slots);
-//   4 epilogue warps    accumulators -> FP64 MO values (integer arithmetic) -> outputs;
+//   generation warps (8, values alone 12)  FP64 radial sums and polynomials of the kept
+//                       shells, digits written to the panel's operand slot (ring of slots);
+//   epilogue warps (8, second derivatives 4)  accumulators -> FP64 MO values (integer
+//                       arithmetic) -> outputs;
 //   1 MMA warp, 1 coefficient loader (bulk copies), 1 tile warp (screening, scales).
 // Every wait is bounded and raises the status word instead of hanging (okg_wait_status).
 //
-// What bounds it (20 atoms, 180 AOs, 40 MOs, 160^3 points, density and gradient): 16.6 ms
-// against 234 ms of the DFMA kernel, per 32-point tile and SM 39 K cycles, of which the
-// FP64 pipe needs about 9 K and the tensor cores 4 K; the rest is the latency of the
-// integer code (digits, exponentials, conversion of the accumulators), which is why the
-// kernel runs with 23 warps of 80 registers: 8 generation warps in lock step with 128
-// registers took 21.2 ms.
+// What bounds it (20 atoms, 180 AOs, 40 MOs, 160^3 points, density and gradient): 15.2 to
+// 16.7 ms (four runs) against 254 ms of the DFMA kernel; per 32-point tile and SM the FP64
+// pipe needs 13 K and the tensor cores 4 K of about 39 K cycles, the rest is the latency of
+// the integer code (digits, exponentials, conversion of the accumulators) behind a chain:
+// with more than 32 MOs only one set of accumulators fits tensor memory, and the MMAs of a
+// tile wait until the epilogue has read the previous tile's.
 #include <math.h>
 
 #include <mutex>
@@ -60,6 +61,7 @@ constexpr int NTW = 2;                  // tile warps, each with every second bu
 constexpr int MAX_BIG = 512;
 constexpr int TABN = OKG_SPLIT_EXP;     // entries of the 2^(j/2048) table
 constexpr int SMEM_MAX = 232448;
+enum { OUT_RHO = 0, OUT_MO = 1 };
 constexpr float KEEP_LOG2 = 62.0f;
 constexpr float ABS_FLOOR = -1000.0f;   // values below 2^-1000 are dropped
 
@@ -69,13 +71,15 @@ struct Cfg {
     static constexpr int PTS = NCH == 1 ? 128 : 32;   // points of an operand tile
     static constexpr int SUB = PTS / 32;              // points per lane of an operand tile
     static constexpr int NCLS = NCH == 1 ? 1 : NCH == 4 ? 2 : 3;
-    // Warps.  Most of the kernel's time is latency (integer digit and exponential code, a
-    // slow FP64 pipe), so values and gradients run with 23 warps of 80 registers; second
-    // derivatives need 128 registers (15 warps).
+    // Warps: most of the kernel's time is latency (integer digit and exponential code, a slow
+    // FP64 pipe), so as many warps as their registers allow.  20 atoms, 96^3 | 12 atoms, 64^3
+    // points, ms: values with 3 teams (23 warps of 80 registers) 1.25 | 0.32, with 2 teams
+    // (19 warps of 96) 1.32 | 0.32; gradients with 3 teams 3.82 | 0.87, with 2 teams 3.64 |
+    // 0.77 (12 epilogue warps: 3.96 | 0.94); second derivatives need 128 registers (15 warps).
     static constexpr int TEAM = 4;                         // generation warps working on one panel
-    static constexpr int NTEAM = NCH == 7 ? 2 : 3;         // panels under generation at a time
-    static constexpr int NGW = TEAM * NTEAM;
+    static constexpr int NTEAM = NCH == 1 ? 3 : 2;         // panels under generation at a time
     static constexpr int EPQ = NCH == 7 ? 1 : 2;           // epilogue warps per 32 accumulator rows
+    static constexpr int NGW = TEAM * NTEAM;
     static constexpr int NEW = 4 * EPQ;
     static constexpr int NT = 32 * (NGW + NEW + NTW + 1);
 };
@@ -101,6 +105,7 @@ struct Args {
     int nslot, nacc;              // operand slots, accumulator sets
     unsigned tm_cols;
     int norm_smem;                // the MO norms are summed in shared memory
+    int tab_smem;                 // exponents and occupations of the MOs are kept in shared memory
 };
 
 // ------------------------------------------------------------------ tile geometry
@@ -149,7 +154,9 @@ struct State {
     unsigned short* big;    // NTW x MAX_BIG (tile warps)
     unsigned* pbits;        // NTW x MAX_PANELS / 32 (tile warps)
     double* norm;           // 8 x npass np, when A.norm_smem
-    double* part;           // 4 x 32: density sums of the second epilogue warp of a row group
+    double* occ;            // npass np each, when A.tab_smem
+    int* fexp;
+    double* part;           // (EPQ - 1) x 4 x 32: density sums of a row group's other epilogue warps
     int* last_use;          // nslot: last phase whose coefficient copy was requested, or -1
     int* abort_flag;
     uint32_t full, empty, bfull;          // nslot mbarriers each, 8 B apart
@@ -163,7 +170,7 @@ constexpr int MAX_SLOTS = 6;
 constexpr int NBAR = 3 * MAX_SLOTS + 4 + 2 * NBUF + 8 + 1;
 constexpr int AUX_BYTES = TABN * 8 + NBUF * 8 + NBUF * 4 + MAX_SLOTS * 4 + 8 + NBUF * 2 * 3 * 128 + NBUF * MAX_PANELS * 2 +
                           NBUF * MAX_SHELLS + NTW * MAX_BIG * 2 + NTW * MAX_PANELS / 8 +
-                          NBAR * 8 + 4 * 32 * 8 + 64;
+                          NBAR * 8 + 64;
 
 // Bounded wait that also ends when another role gave up.
 __device__ __forceinline__ bool wait(const State& S, uint32_t bar, uint32_t parity, int* status)
@@ -221,59 +228,55 @@ __host__ __device__ constexpr int norm_shift(int a, int b, int c)
 // Values, gradients and pure second derivatives of every canonical component of a shell:
 // with S0 = R0, S1 = -2 R1, S2 = 4 R2,
 //   chi = P S0,  d_x chi = P x S1 + a (P/x) S0,  d_xx chi = P x^2 S2 + (2a + 1) P S1 + a (a-1) (P/x^2) S0,
-// about 1.5 FP64 operations per value (monomials built with the radial sum as a factor).
+// about 1.5 FP64 operations per value.  Kept between components are only the monomials of
+// degree L - 1 times the radial sums (3 + 3 for a d shell): with all values of a shell formed
+// first (19 for a d shell) the registers around the calls of put4 went to local memory, and
+// its traffic through what shared memory leaves of the L1 cost more than the arithmetic.
 template <int L, int NCH, typename Sink>
 __device__ __forceinline__ void shell_values(double X, double Y, double Z, double R0, double S1, double S2, Sink&& sink)
 {
-    constexpr int N = (L + 1) * (L + 2) / 2;
-    double V[N], Vm[L > 0 ? N - L - 1 : 1], Vmm[L > 1 ? N - 2 * L - 1 : 1];
-    double G[NCH >= 4 ? (L + 2) * (L + 3) / 2 : 1], G0[NCH == 7 ? N : 1];
-    double H[NCH == 7 ? (L + 3) * (L + 4) / 2 : 1];
+    constexpr int N = (L + 1) * (L + 2) / 2, M = L > 0 ? L * (L + 1) / 2 : 1, MM = L > 1 ? L * (L - 1) / 2 : 1;
+    double V[M], G[NCH >= 4 ? M : 1], H[NCH == 7 ? M : 1], W[NCH == 7 ? MM : 1];
     V[0] = R0;
+    if constexpr (NCH >= 4) G[0] = S1;
+    if constexpr (NCH == 7) H[0] = S2;
     if constexpr (L >= 2) {
         raise_to<0, L - 2>(V, X, Y, Z);
-        if constexpr (NCH == 7)
-            for (int i = 0; i < N - 2 * L - 1; ++i) Vmm[i] = V[i];
+        if constexpr (NCH == 7) {
+#pragma unroll
+            for (int i = 0; i < MM; ++i) W[i] = V[i];
+        }
         raise<L - 1>(V, X, Y, Z);
-    }
-    if constexpr (L >= 1) {
-        if constexpr (NCH >= 4)
-            for (int i = 0; i < N - L - 1; ++i) Vm[i] = V[i];
-        raise<L>(V, X, Y, Z);
-    }
-    if constexpr (NCH >= 4) {
-        G[0] = S1;
-        raise_to<0, L>(G, X, Y, Z);
-        if constexpr (NCH == 7)
-            for (int i = 0; i < N; ++i) G0[i] = G[i];
-        raise<L + 1>(G, X, Y, Z);
-    }
-    if constexpr (NCH == 7) {
-        H[0] = S2;
-        raise_to<0, L + 2>(H, X, Y, Z);
+        if constexpr (NCH >= 4) raise_to<0, L - 1>(G, X, Y, Z);
+        if constexpr (NCH == 7) raise_to<0, L - 1>(H, X, Y, Z);
     }
     [&]<int... J>(std::integer_sequence<int, J...>) {
         (
             [&] {
                 constexpr int a = canon_l(L, J, 0), b = canon_l(L, J, 1), c = canon_l(L, J, 2);
+                // P = x_d (P / x_d) along an axis with a non-zero exponent
+                constexpr int d = a > 0 ? 0 : b > 0 ? 1 : 2;
+                constexpr int m = L == 0 ? 0 : midx(a - (d == 0), b - (d == 1), c - (d == 2));
+                const double xd = d == 0 ? X : d == 1 ? Y : Z;
                 double v[NCH];
-                v[0] = V[midx(a, b, c)];
+                v[0] = L == 0 ? R0 : xd * V[m];
                 if constexpr (NCH >= 4) {
-                    v[1] = G[midx(a + 1, b, c)];
-                    v[2] = G[midx(a, b + 1, c)];
-                    v[3] = G[midx(a, b, c + 1)];
-                    if constexpr (a > 0) v[1] = fma((double)a, Vm[midx(a - 1, b, c)], v[1]);
-                    if constexpr (b > 0) v[2] = fma((double)b, Vm[midx(a, b - 1, c)], v[2]);
-                    if constexpr (c > 0) v[3] = fma((double)c, Vm[midx(a, b, c - 1)], v[3]);
-                }
-                if constexpr (NCH == 7) {
-                    const double g0 = G0[midx(a, b, c)];
-                    v[4] = fma((double)(2 * a + 1), g0, H[midx(a + 2, b, c)]);
-                    v[5] = fma((double)(2 * b + 1), g0, H[midx(a, b + 2, c)]);
-                    v[6] = fma((double)(2 * c + 1), g0, H[midx(a, b, c + 2)]);
-                    if constexpr (a > 1) v[4] = fma((double)(a * (a - 1)), Vmm[midx(a - 2, b, c)], v[4]);
-                    if constexpr (b > 1) v[5] = fma((double)(b * (b - 1)), Vmm[midx(a, b - 2, c)], v[5]);
-                    if constexpr (c > 1) v[6] = fma((double)(c * (c - 1)), Vmm[midx(a, b, c - 2)], v[6]);
+                    const double g = L == 0 ? S1 : xd * G[m];  // P S1
+                    v[1] = g * X;
+                    v[2] = g * Y;
+                    v[3] = g * Z;
+                    if constexpr (a > 0) v[1] = fma((double)a, V[midx(a - 1, b, c)], v[1]);
+                    if constexpr (b > 0) v[2] = fma((double)b, V[midx(a, b - 1, c)], v[2]);
+                    if constexpr (c > 0) v[3] = fma((double)c, V[midx(a, b, c - 1)], v[3]);
+                    if constexpr (NCH == 7) {
+                        const double h = L == 0 ? S2 : xd * H[m];  // P S2
+                        v[4] = fma((double)(2 * a + 1), g, (h * X) * X);
+                        v[5] = fma((double)(2 * b + 1), g, (h * Y) * Y);
+                        v[6] = fma((double)(2 * c + 1), g, (h * Z) * Z);
+                        if constexpr (a > 1) v[4] = fma((double)(a * (a - 1)), W[midx(a - 2, b, c)], v[4]);
+                        if constexpr (b > 1) v[5] = fma((double)(b * (b - 1)), W[midx(a, b - 2, c)], v[5]);
+                        if constexpr (c > 1) v[6] = fma((double)(c * (c - 1)), W[midx(a, b, c - 2)], v[6]);
+                    }
                 }
                 sink(J, norm_shift(a, b, c), v);
             }(),
@@ -478,13 +481,39 @@ __device__ __forceinline__ void gen_role(const Args& A, const State& S)
     __syncwarp();
 }
 
+// The MMAs of a panel: digit i of the AOs times digits 0 .. 6 - i of the coefficients side by
+// side in N (neighbouring accumulators), DM digits per instruction (N <= 256).  Straight-line
+// code with the descriptors advanced in their address words: in nested loops an instruction
+// took the issuing thread 200 to 320 cycles, whatever its N.
+template <int DM, int RG>
+__device__ __forceinline__ void issue_panel(uint32_t acc, uint32_t sa, uint32_t sb, int np, uint32_t more)
+{
+    const uint64_t a0 = a_desc(sa), b0 = b_desc(sb);
+    const uint32_t ahi = (uint32_t)(a0 >> 32), bhi = (uint32_t)(b0 >> 32), bstep = (uint32_t)(np * PK * 2) >> 4;
+    const uint32_t id0 = idesc(0), idn = (uint32_t)(np >> 3) << 17;
+#pragma unroll
+    for (int rg = 0; rg < RG; ++rg)
+#pragma unroll
+        for (int i = 0; i < ND; ++i)
+#pragma unroll
+            for (int j = 0; j < ND - i; j += DM) {
+                const int nd = ND - i - j < DM ? ND - i - j : DM;
+                const uint32_t alo = (uint32_t)a0 + (uint32_t)((rg * ND + i) * (DT >> 4)), blo = (uint32_t)b0 + j * bstep;
+                asm volatile(
+                    "{\n\t.reg .pred p;\n\t.reg .b64 ad, bd;\n\tmov.b64 ad, {%1, %2};\n\tmov.b64 bd, {%3, %4};\n\t"
+                    "setp.ne.b32 p, %6, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], ad, bd, %5, p;\n\t}\n" ::"r"(
+                        acc + (uint32_t)((rg * ND + i + j) * np)),
+                    "r"(alo), "r"(ahi), "r"(blo), "r"(bhi), "r"(id0 + (uint32_t)nd * idn), "r"(i > 0 ? 1u : more));
+            }
+}
+
 template <int NCH>
 __device__ __forceinline__ void mma_role(const Args& A, const State& S)
 {
     if ((threadIdx.x & 31) != 0) return;
     using C = Cfg<NCH>;
     int* status = A.status;
-    const int np = A.np, dmax = 256 / np;  // digits per instruction (N <= 256)
+    const int np = A.np;
     unsigned seq = 0, job = 0;
     bool ok = true, issued = false;
     TileSeq ts;
@@ -512,20 +541,10 @@ __device__ __forceinline__ void mma_role(const Args& A, const State& S)
                 }
                 tc_fence_after();
                 const uint32_t sa = smem_u32(S.slots + sl * S.slot_bytes), sb = sa + S.a_bytes;
-#pragma unroll 1
-                for (int rg = 0; rg < C::RG; ++rg)
-#pragma unroll 1
-                    for (int i = 0; i < ND; ++i) {
-                        // digit i of the AOs times digits 0 .. 6 - i of the coefficients:
-                        // neighbouring accumulators, one instruction per dmax digits
-                        const uint64_t ad = a_desc(sa + (uint32_t)(rg * ND + i) * DT);
-#pragma unroll 1
-                        for (int j = 0; j < ND - i; j += dmax) {
-                            const int nd = ND - i - j < dmax ? ND - i - j : dmax;
-                            mma_f16(acc + (uint32_t)((rg * ND + i + j) * np), ad, b_desc(sb + (uint32_t)(j * np * PK * 2)),
-                                    idesc(nd * np), (pi > p0 || i > 0) ? 1u : 0u);
-                        }
-                    }
+                const uint32_t more = pi > p0 ? 1u : 0u;
+                if (np <= 32) issue_panel<7, C::RG>(acc, sa, sb, np, more);
+                else if (np <= 48) issue_panel<5, C::RG>(acc, sa, sb, np, more);
+                else issue_panel<4, C::RG>(acc, sa, sb, np, more);
                 mma_commit(S.empty + 8 * sl);
                 issued = true;
             }
@@ -553,12 +572,12 @@ __device__ __forceinline__ double times_occ(double v, double o, int x)
     return (x ? 2.0 * o : o) * v;
 }
 
-template <int NCH, bool MO_OUT>
+template <int NCH, int MODE>
 __device__ __forceinline__ void epi_role(const Args& A, const State& S)
 {
     using C = Cfg<NCH>;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, quad = warp & 3;
-    const int half = (warp - C::NGW) >> 2;            // of a row group's EPQ warps: MOs 4 half, 4 half + 4 EPQ, ...
+    const int half = (warp - C::NGW) >> 2;            // of a row group's EPQ warps: MOs 2 half, 2 half + 2 EPQ, ...
     const int row = quad * 32 + lane;                 // accumulator row
     const int pt = NCH == 1 ? row : row >> 2;         // point of the tile
     const int ch = NCH == 1 ? 0 : lane & 3;           // channel (of the first row tile)
@@ -581,7 +600,8 @@ __device__ __forceinline__ void epi_role(const Args& A, const State& S)
             const bool valid = tile_point(A, tile, sub * 32 + pt, p, px, py, pz);
             double accs[2] = {0.0, 0.0}, acc1 = 0.0;
             for (int pass = 0; pass < A.npass; ++pass) {
-                const int* fexp = A.fexp + pass * np;
+                const int* fexp = (A.tab_smem ? S.fexp : A.fexp) + pass * np;
+                const double* occ = (A.tab_smem ? S.occ : A.occ) + pass * np;
                 for (int gr = 0; gr < (ng ? ng : 1); ++gr) {
                     const unsigned ab = job % (unsigned)A.nacc, ause = job / (unsigned)A.nacc;
                     const bool last = gr + 1 >= ng;
@@ -591,21 +611,21 @@ __device__ __forceinline__ void epi_role(const Args& A, const State& S)
                         tc_fence_after();
                     }
                     const int nmo = A.nmo - pass * np < np ? A.nmo - pass * np : np;  // MOs of this pass
-                    Acc4 va, ua;
+                    Acc2 va, ua;
 #pragma unroll 1
-                    for (int n0 = 4 * half; n0 < nmo; n0 += 4 * C::EPQ) {
-                        double v[4], u[4];
-                        const int4 f4 = __ldg((const int4*)(fexp + n0));
+                    for (int n0 = 2 * half; n0 < nmo; n0 += 2 * C::EPQ) {
+                        double v[2], u[2];
+                        const int2 f2 = *(const int2*)(fexp + n0);
                         if (ng) {
-                            acc_load(va, taddr + (uint32_t)n0, np);
-                            if (NCH == 7) acc_load(ua, taddr + (uint32_t)(ND * np + n0), np);
-                            acc_wait(va);
-                            if (NCH == 7) acc_wait(ua);
-                            acc_values(va, rx0, f4, v);
-                            if (NCH == 7) acc_values(ua, rx1, f4, u);
+                            acc2_load(va, taddr + (uint32_t)n0, np);
+                            if (NCH == 7) acc2_load(ua, taddr + (uint32_t)(ND * np + n0), np);
+                            acc2_wait(va);
+                            if (NCH == 7) acc2_wait(ua);
+                            acc2_values(va, rx0, f2, v);
+                            if (NCH == 7) acc2_values(ua, rx1, f2, u);
                             if (ng > 1) {
 #pragma unroll
-                                for (int i = 0; i < 4; ++i) {
+                                for (int i = 0; i < 2; ++i) {
                                     double* q = phi + (size_t)(n0 + i) * 128;
                                     if (gr > 0) v[i] += *q;
                                     if (!last) *q = v[i];
@@ -618,27 +638,27 @@ __device__ __forceinline__ void epi_role(const Args& A, const State& S)
                             }
                         } else {
                             // no shell reaches this tile: zeros (or NaN where the input has it)
-                            const int f[4] = {f4.x, f4.y, f4.z, f4.w};
+                            const int f[2] = {f2.x, f2.y};
 #pragma unroll
-                            for (int i = 0; i < 4; ++i)
+                            for (int i = 0; i < 2; ++i)
                                 v[i] = u[i] = (rx0 == ROW_NAN || f[i] == MO_NAN) ? __longlong_as_double(0x7FF8000000000000ll) : 0.0;
                         }
                         if (!last) continue;
-                        if (MO_OUT) {
+                        if (MODE == OUT_MO) {
                             for (int d = 0; d < A.drv.n; ++d) {
                                 const int code = A.drv.code[d];
                                 const bool first = code < 4;
                                 if (!valid || (first ? ch != code : (NCH != 7 || ch != code - 4))) continue;
                                 double* out = A.out + ((long long)d * A.nmo + pass * np + n0) * A.ld + p;
 #pragma unroll
-                                for (int i = 0; i < 4; ++i)
+                                for (int i = 0; i < 2; ++i)
                                     if (n0 + i < nmo) out[i * A.ld] = first ? v[i] : (NCH == 7 ? u[i] : 0.0);
                             }
                         } else {
-                            double q2[4];
+                            double q2[2];
 #pragma unroll
-                            for (int i = 0; i < 4; ++i) {
-                                const double o = __ldg(A.occ + pass * np + n0 + i);
+                            for (int i = 0; i < 2; ++i) {
+                                const double o = occ[n0 + i];
                                 if (NCH == 1) {
                                     q2[i] = v[i] * v[i];
                                     accs[i & 1] = fma(o, q2[i], accs[i & 1]);
@@ -654,23 +674,15 @@ __device__ __forceinline__ void epi_role(const Args& A, const State& S)
                                 }
                             }
                             if (A.mo_norm) {
-                                // sums of q2[i] over the warp, four MOs at once: after two halving
-                                // exchanges lane l holds MO (l & 3) of its 4-lane group
-                                double s2[2], s1;
+                                // sums of q2[i] over the warp, two MOs at once: after one halving
+                                // exchange lane l holds MO (l & 1)
 #pragma unroll
-                                for (int i = 0; i < 4; ++i) q2[i] = valid ? q2[i] : 0.0;
+                                for (int i = 0; i < 2; ++i) q2[i] = valid ? q2[i] : 0.0;
+                                const double keep = (lane & 1) ? q2[1] : q2[0], give = (lane & 1) ? q2[0] : q2[1];
+                                double s1 = keep + shfl_d(give, lane ^ 1);
 #pragma unroll
-                                for (int i = 0; i < 2; ++i) {
-                                    const double keep = (lane & 2) ? q2[i + 2] : q2[i], give = (lane & 2) ? q2[i] : q2[i + 2];
-                                    s2[i] = keep + shfl_d(give, lane ^ 2);
-                                }
-                                {
-                                    const double keep = (lane & 1) ? s2[1] : s2[0], give = (lane & 1) ? s2[0] : s2[1];
-                                    s1 = keep + shfl_d(give, lane ^ 1);
-                                }
-#pragma unroll
-                                for (int o = 4; o < 32; o *= 2) s1 += shfl_d(s1, lane ^ o);
-                                if (lane < 4 && n0 + lane < nmo) {
+                                for (int o = 2; o < 32; o *= 2) s1 += shfl_d(s1, lane ^ o);
+                                if (lane < 2 && n0 + lane < nmo) {
                                     const int mo = pass * np + n0 + lane;
                                     if (A.norm_smem)
                                         S.norm[(warp - C::NGW) * A.npass * np + mo] += s1;
@@ -690,22 +702,23 @@ __device__ __forceinline__ void epi_role(const Args& A, const State& S)
                 }
             }
             double acc0 = accs[0] + accs[1];
-            if (!MO_OUT && C::EPQ == 2) {
-                // the two halves of the MO sum meet in shared memory
-                if (half == 1) {
+            if (MODE == OUT_RHO && C::EPQ > 1) {
+                // the shares of the MO sum meet in shared memory
+                if (half > 0) {
                     if (round > 0 && !warp_wait(S, S.part_free + 8 * quad, (round - 1) & 1, status)) return;
-                    S.part[quad * 32 + lane] = acc0;
+                    S.part[((half - 1) * 4 + quad) * 32 + lane] = acc0;
                     __syncwarp();
                     if (lane == 0) mbar_arrive(S.part_full + 8 * quad);
                 } else {
                     if (!warp_wait(S, S.part_full + 8 * quad, round & 1, status)) return;
-                    acc0 += S.part[quad * 32 + lane];
+#pragma unroll
+                    for (int h = 1; h < C::EPQ; ++h) acc0 += S.part[((h - 1) * 4 + quad) * 32 + lane];
                     __syncwarp();
                     if (lane == 0) mbar_arrive(S.part_free + 8 * quad);
                 }
                 ++round;
             }
-            if (!MO_OUT && valid && half == 0) {
+            if (MODE == OUT_RHO && valid && half == 0) {
                 if (ch == 0) A.out[p] = acc0;
                 for (int d = 0; d < A.drv.n; ++d) {
                     const int code = A.drv.code[d];
@@ -1002,7 +1015,7 @@ __device__ __forceinline__ void tile_role(const Args& A, const State& S, int tw)
 }
 
 // ------------------------------------------------------------------ the kernel
-template <int NCH, bool MO_OUT>
+template <int NCH, int MODE>
 __global__ void __launch_bounds__(Cfg<NCH>::NT, 1) split_kernel(const __grid_constant__ Args A)
 {
     using C = Cfg<NCH>;
@@ -1023,9 +1036,18 @@ __global__ void __launch_bounds__(Cfg<NCH>::NT, 1) split_kernel(const __grid_con
     uint64_t* bar = (uint64_t*)q;
     q += NBAR * 8;
     S.part = (double*)q;
-    q += 4 * 32 * 8;
+    if (C::EPQ > 1) q += (C::EPQ - 1) * 4 * 32 * 8;
     S.norm = (double*)q;
     if (A.norm_smem) q += (size_t)NEW * A.npass * A.np * 8;
+    S.occ = (double*)q;
+    S.fexp = (int*)(S.occ + A.npass * A.np);
+    if (A.tab_smem) {
+        q += (size_t)A.npass * A.np * 12;
+        for (int i = tid; i < A.npass * A.np; i += NT) {
+            S.occ[i] = __ldg(A.occ + i);
+            S.fexp[i] = __ldg(A.fexp + i);
+        }
+    }
     S.pts = (double*)q;
     if (NCH == 1) q += NBUF * 3 * 128 * 8;
     S.rowexp = (short*)q;
@@ -1076,7 +1098,7 @@ __global__ void __launch_bounds__(Cfg<NCH>::NT, 1) split_kernel(const __grid_con
             mbar_init(S.kfree + 8 * s, NGW + NEW + 1);
         }
         for (int s = 0; s < 4; ++s) {
-            mbar_init(S.part_full + 8 * s, 1);
+            mbar_init(S.part_full + 8 * s, C::EPQ > 1 ? C::EPQ - 1 : 1);
             mbar_init(S.part_free + 8 * s, 1);
         }
         mbar_init(S.drain, 1);
@@ -1097,7 +1119,7 @@ __global__ void __launch_bounds__(Cfg<NCH>::NT, 1) split_kernel(const __grid_con
     if (warp < NGW)
         gen_role<NCH>(A, S);
     else if (warp < NGW + NEW)
-        epi_role<NCH, MO_OUT>(A, S);
+        epi_role<NCH, MODE>(A, S);
     else if (warp == NGW + NEW)
         mma_role<NCH>(A, S);
     else
@@ -1109,7 +1131,7 @@ __global__ void __launch_bounds__(Cfg<NCH>::NT, 1) split_kernel(const __grid_con
     tc_fence_after();
     // no coefficient copy may land after the CTA has left (all have, unless a wait gave up)
     if (tid < A.nslot && S.last_use[tid] >= 0) mbar_drain(S.bfull + 8 * tid, S.last_use[tid] & 1);
-    if (!MO_OUT && A.mo_norm && A.norm_smem)
+    if (MODE == OUT_RHO && A.mo_norm && A.norm_smem)
         for (int i = tid; i < A.nmo; i += NT) {
             double t = 0.0;
             for (int w = 0; w < NEW; ++w) t += S.norm[w * A.npass * A.np + i];
@@ -1287,14 +1309,14 @@ int current_device()
     return d;
 }
 
-template <int NCH, bool MO_OUT>
+template <int NCH, int MODE>
 int launch(sp::Args& A, int nblk, size_t smem, cudaStream_t st)
 {
     // (set on every launch: the attribute belongs to the current device)
-    cudaError_t e = cudaFuncSetAttribute(sp::split_kernel<NCH, MO_OUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(sp::split_kernel<NCH, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem);
     if (e != cudaSuccess) return cuda_status(e, "FP64 tensor-core path: shared memory");
-    sp::split_kernel<NCH, MO_OUT><<<nblk, sp::Cfg<NCH>::NT, smem, st>>>(A);
+    sp::split_kernel<NCH, MODE><<<nblk, sp::Cfg<NCH>::NT, smem, st>>>(A);
     return cuda_status(cudaGetLastError(), "FP64 tensor-core path: launch");
 }
 
@@ -1338,7 +1360,11 @@ int run(const okg_basis* b, const Grid& g, const SplitCall& c, cudaStream_t st, 
     const size_t slot = ((size_t)C::RG * sp::ND * sp::DT + (size_t)sp::ND * A.np * sp::PK * 2 + 1023) & ~(size_t)1023;
     const size_t norm = (size_t)C::NEW * A.npass * A.np * 8;
     A.norm_smem = c.mo_norm && norm <= 16384;
-    const size_t fixed = 1024 + sp::AUX_BYTES + (A.norm_smem ? norm : 0) + (NCH == 1 ? sp::NBUF * 3 * 128 * 8 : 0);
+    const size_t tab = (size_t)A.npass * A.np * 12;
+    const size_t fixed0 = 1024 + sp::AUX_BYTES + (A.norm_smem ? norm : 0) + (NCH == 1 ? sp::NBUF * 3 * 128 * 8 : 0) + (C::EPQ - 1) * 4 * 32 * 8;
+    // (the MO table only where it does not cost an operand slot)
+    A.tab_smem = tab <= 8192 && (sp::SMEM_MAX - fixed0 - tab) / slot == (sp::SMEM_MAX - fixed0) / slot;
+    const size_t fixed = fixed0 + (A.tab_smem ? tab : 0);
     A.nslot = (int)((sp::SMEM_MAX - fixed) / slot);
     if (A.nslot > sp::MAX_SLOTS) A.nslot = sp::MAX_SLOTS;
     if (A.nslot < 2) return OKG_OK;
@@ -1366,7 +1392,7 @@ int run(const okg_basis* b, const Grid& g, const SplitCall& c, cudaStream_t st, 
                                                 (int*)(ws + o_fexp), (double*)(ws + o_occ), A.counter);
     int s = cuda_status(cudaGetLastError(), "FP64 tensor-core path: coefficient digits");
     const size_t smem = fixed + A.nslot * slot;
-    if (!s) s = c.mo_out ? launch<NCH, true>(A, nblk, smem, st) : launch<NCH, false>(A, nblk, smem, st);
+    if (!s) s = c.mo_out ? launch<NCH, sp::OUT_MO>(A, nblk, smem, st) : launch<NCH, sp::OUT_RHO>(A, nblk, smem, st);
     const cudaError_t e = cudaFreeAsync(ws, st);
     if (!s) s = cuda_status(e, "FP64 tensor-core path: workspace");
     done = s == OKG_OK;
