@@ -1,8 +1,8 @@
 """Differentiable rho and grad rho: a torch.autograd.Function over the GPU kernels.
 
 Forward: okg_rho (FP64 path), or the tensor-core mixed path for precision="fp32".
-Backward: the hand-written adjoint kernel okg_rho_backward (FP64 or FP32
-arithmetic), which recomputes AO tiles instead of storing them and returns
+Backward: the hand-written adjoint okg_rho_backward (FP64 or FP32 arithmetic), which
+recomputes the AOs instead of keeping them from the forward pass and returns
 dL/dC (MO coefficients, in the output AO basis), dL/dalpha and dL/dc (primitive
 exponents and contraction coefficients, in ao_spec.get_prim_coeffs() order) and
 dL/dR (nuclear coordinates).

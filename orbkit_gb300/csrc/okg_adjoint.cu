@@ -1,7 +1,9 @@
 // Adjoint of the fused density path: given cotangents of rho and grad rho on a
 // grid, the gradients of a loss with respect to the MO coefficients, the primitive
-// exponents and contraction coefficients, and the nuclear coordinates.  AO tiles
-// are recomputed, never stored.
+// exponents and contraction coefficients, and the nuclear coordinates.  This is the
+// one-kernel form, for more than 64 MOs and FP32 calls of fewer than 2048 points (and for
+// a workspace too small for the other): AO tiles are recomputed, never stored.  The other
+// calls take the pipeline of okg_adjoint_split.cu.
 //
 // Forward being differentiated (orbkit/core.py:266-300 with the AO kernel of
 // orbkit/c_grid-based.c:9-79):
@@ -436,6 +438,8 @@ extern "C" int okg_rho_backward_workspace(const okg_basis* b, const okg_grid* gr
     const long long ntiles = (grid->npts + adj::P - 1) / adj::P;
     *bytes = precision == 32 ? adj::workspace_bytes<float>(b, nmo, adj::block_count<float>(ntiles))
                              : adj::workspace_bytes<double>(b, nmo, adj::block_count<double>(ntiles));
+    const size_t split = adjoint_split_bytes(b, grid->npts, nmo, precision);
+    if (split > *bytes) *bytes = split;
     return OKG_OK;
 }
 
@@ -463,6 +467,12 @@ extern "C" int okg_rho_backward(const okg_basis* b, const okg_grid* gr, int nmo,
         return set_error(OKG_ERR_ARG, "okg_rho_backward: regular grid range outside Nx*Ny*Nz");
     if (ld < g.npts) return set_error(OKG_ERR_ARG, "okg_rho_backward: ld < npts");
     cudaStream_t st = (cudaStream_t)stream;
+    if (work_bytes >= adjoint_split_bytes(b, g.npts, nmo, precision)) {
+        bool done = false;
+        const int s = adjoint_split_run(b, g, nmo, d_coeff, d_occ, d_g_rho, d_g_grad, ld, precision, d_dcoeff, d_dprim, d_dgeo,
+                                        d_work, st, done);
+        if (s || done) return s;
+    }
     if (precision == 64)
         return adj::run<double>(b, g, nmo, d_coeff, d_occ, d_g_rho, d_g_grad, ld, d_dcoeff, d_dprim, d_dgeo, d_work,
                                 work_bytes, st);

@@ -86,13 +86,15 @@ __global__ void prim_weights_kernel(const double* __restrict__ prim_in, const in
 // sorted order; *flags is raised by a parameter or position that is not a number.
 __global__ void sort_prim_mx_kernel(const Shell* __restrict__ shells, int nshell, PrimMx* __restrict__ prim_mx,
                                     double2* __restrict__ prim_cusp, const double* __restrict__ atoms, int natom,
-                                    float4* __restrict__ split_lg, SplitPrim* __restrict__ split_pr, int* __restrict__ flags)
+                                    float4* __restrict__ split_lg, SplitPrim* __restrict__ split_pr,
+                                    int* __restrict__ split_place, int* __restrict__ flags)
 {
     int s = blockIdx.x * blockDim.x + threadIdx.x;
     for (int i = s; i < natom; i += gridDim.x * blockDim.x)
         if (!isfinite(atoms[4 * i]) || !isfinite(atoms[4 * i + 1]) || !isfinite(atoms[4 * i + 2])) atomicOr(flags, 1);
     if (s >= nshell) return;
     const int p0 = shells[s].prim0, np = shells[s].nprim;
+    for (int i = 0; i < np; ++i) split_place[p0 + i] = p0 + i;
     for (int i = 1; i < np; ++i) {
         const PrimMx v = prim_mx[p0 + i];
         const double2 c = prim_cusp[p0 + i];
@@ -100,10 +102,12 @@ __global__ void sort_prim_mx_kernel(const Shell* __restrict__ shells, int nshell
         while (j >= 0 && prim_mx[p0 + j].a2 > v.a2) {
             prim_mx[p0 + j + 1] = prim_mx[p0 + j];
             prim_cusp[p0 + j + 1] = prim_cusp[p0 + j];
+            split_place[p0 + j + 1] = split_place[p0 + j];
             --j;
         }
         prim_mx[p0 + j + 1] = v;
         prim_cusp[p0 + j + 1] = c;
+        split_place[p0 + j + 1] = p0 + i;
     }
     for (int i = 0; i < np; ++i)
         if (!split_prim(prim_cusp[p0 + i], split_lg[p0 + i], split_pr[p0 + i])) atomicOr(flags, 1);
@@ -397,6 +401,7 @@ extern "C" int okg_basis_create(int natom, int nshell, const int* h_shell_atom, 
     oo.end = lay.take(0);
     const size_t o_slg = lay.take(sizeof(float4) * nprim);
     const size_t o_spr = lay.take(sizeof(SplitPrim) * nprim);
+    const size_t o_spl = lay.take(sizeof(int) * nprim);
     const size_t o_sfl = lay.take(sizeof(int));
     const size_t o_exp = lay.take(sizeof(uint64_t) * OKG_SPLIT_EXP);
     // the transform by Cartesian row; entries of the same spherical row added up in order
@@ -470,6 +475,7 @@ extern "C" int okg_basis_create(int natom, int nshell, const int* h_shell_atom, 
     b->split.col_g = (const double*)(blk + oo.scg);
     b->split.prim_lg = (const float4*)(blk + o_slg);
     b->split.prim = (const SplitPrim*)(blk + o_spr);
+    b->split.prim_place = (const int*)(blk + o_spl);
     b->split.flags = (const int*)(blk + o_sfl);
     b->split.exp_tab = (const uint64_t*)(blk + o_exp);
     b->cart_ptr = (const int*)(blk + o_cptr);
@@ -579,6 +585,6 @@ extern "C" int okg_basis_set_params(okg_basis* b, const double* d_geo, const dou
     sort_prim_mx_kernel<<<(b->nshell + 127) / 128, 128, 0, st>>>(b->dev.shells, b->nshell, (PrimMx*)b->dev.prim_mx,
                                                                  (double2*)b->dev.prim_cusp, b->dev.atoms, b->natom,
                                                                  (float4*)b->split.prim_lg, (SplitPrim*)b->split.prim,
-                                                                 (int*)b->split.flags);
+                                                                 (int*)b->split.prim_place, (int*)b->split.flags);
     return cuda_status(cudaGetLastError(), "okg_basis_set_params");
 }

@@ -344,7 +344,19 @@ struct SplitCall {
     double* dout;
     double* mo_norm;
     long long ld;
+    // cotangents of rho and grad rho (the adjoint): out receives W and V (2 x nmo x ld), need = 0xF
+    const double* g_rho = nullptr;
+    const double* g_grad = nullptr;
+    long long g_ld = 0;
+    bool wv_float = false;  // W and V as floats
 };
 // Runs the call on the tensor cores if it is one for them (done = true), else leaves it.
 int split_run(const okg_basis* b, const Grid& g, const SplitCall& c, cudaStream_t st, bool& done);
+
+// Adjoint through the tensor cores (okg_adjoint_split.cu): workspace, and the call (done =
+// false: not one for it, nothing was written to the outputs).
+size_t adjoint_split_bytes(const okg_basis* b, long long npts, int nmo, int precision);
+int adjoint_split_run(const okg_basis* b, const Grid& g, int nmo, const double* C, const double* occ, const double* grho,
+                      const double* ggrad, long long ld, int precision, double* dC, double* dprim, double* dgeo, void* work,
+                      cudaStream_t st, bool& done);
 }  // namespace okg

@@ -61,7 +61,7 @@ constexpr int NTW = 2;                  // tile warps, each with every second bu
 constexpr int MAX_BIG = 512;
 constexpr int TABN = OKG_SPLIT_EXP;     // entries of the 2^(j/2048) table
 constexpr int SMEM_MAX = 232448;
-enum { OUT_RHO = 0, OUT_MO = 1 };
+enum { OUT_RHO = 0, OUT_MO = 1, OUT_WV = 2 };
 constexpr float KEEP_LOG2 = 62.0f;
 constexpr float ABS_FLOOR = -1000.0f;   // values below 2^-1000 are dropped
 
@@ -96,7 +96,11 @@ struct Args {
     double* phi;                  // per CTA [RG][np][128] partial MO values (bases beyond GROUP panels)
     int* status;                  // raised when a wait expires
     DrvList drv;
-    double* out;                  // MO output: ndrv x nmo x ld; density: rho
+    double* out;                  // MO output: ndrv x nmo x ld; density: rho; cotangents: W, V (2 x nmo x ld)
+    const double* g_rho;          // cotangents of rho, and of grad rho (3 x g_ld, or null)
+    const double* g_grad;
+    long long g_ld;
+    int wv_float;
     double* dout;                 // density: ndrv x ld
     double* mo_norm;              // density: nmo sums of MO^2, or null
     long long ld, ntiles;
@@ -599,6 +603,8 @@ __device__ __forceinline__ void epi_role(const Args& A, const State& S)
             double px, py, pz;
             const bool valid = tile_point(A, tile, sub * 32 + pt, p, px, py, pz);
             double accs[2] = {0.0, 0.0}, acc1 = 0.0;
+            double cot = 0.0;  // this channel's cotangent at the point
+            if (MODE == OUT_WV && valid) cot = ch == 0 ? A.g_rho[p] : A.g_grad ? A.g_grad[(ch - 1) * A.g_ld + p] : 0.0;
             for (int pass = 0; pass < A.npass; ++pass) {
                 const int* fexp = (A.tab_smem ? S.fexp : A.fexp) + pass * np;
                 const double* occ = (A.tab_smem ? S.occ : A.occ) + pass * np;
@@ -644,7 +650,23 @@ __device__ __forceinline__ void epi_role(const Args& A, const State& S)
                                 v[i] = u[i] = (rx0 == ROW_NAN || f[i] == MO_NAN) ? __longlong_as_double(0x7FF8000000000000ll) : 0.0;
                         }
                         if (!last) continue;
-                        if (MODE == OUT_MO) {
+                        if (MODE == OUT_WV) {
+                            // cotangents of the MOs: W = 2 occ (g_rho MO + sum_d g_d d_d MO), V = 2 occ MO
+#pragma unroll
+                            for (int i = 0; i < 2; ++i) {
+                                const double o = occ[n0 + i];
+                                const double f = shfl_d(v[i], lane0);
+                                double w = v[i] * cot;
+                                w += shfl_d(w, lane ^ 1);
+                                w += shfl_d(w, lane ^ 2);
+                                if (valid && n0 + i < nmo && ch < 2) {
+                                    const long long at = (long long)(ch * A.nmo + pass * np + n0 + i) * A.ld + p;
+                                    const double v2 = times_occ(ch == 0 ? w : f, o, 1);
+                                    if (A.wv_float) ((float*)A.out)[at] = (float)v2;
+                                    else A.out[at] = v2;
+                                }
+                            }
+                        } else if (MODE == OUT_MO) {
                             for (int d = 0; d < A.drv.n; ++d) {
                                 const int code = A.drv.code[d];
                                 const bool first = code < 4;
@@ -1336,6 +1358,10 @@ int run(const okg_basis* b, const Grid& g, const SplitCall& c, cudaStream_t st, 
     A.out = c.out;
     A.dout = c.dout;
     A.mo_norm = c.mo_norm;
+    A.g_rho = c.g_rho;
+    A.g_grad = c.g_grad;
+    A.g_ld = c.g_ld;
+    A.wv_float = c.wv_float;
     A.ld = c.ld;
     A.brick = g.regular && g.offset == 0 && g.npts == (long long)g.nx * g.ny * g.nz;
     const int device = current_device(), sms = sm_count(device);
@@ -1392,7 +1418,13 @@ int run(const okg_basis* b, const Grid& g, const SplitCall& c, cudaStream_t st, 
                                                 (int*)(ws + o_fexp), (double*)(ws + o_occ), A.counter);
     int s = cuda_status(cudaGetLastError(), "FP64 tensor-core path: coefficient digits");
     const size_t smem = fixed + A.nslot * slot;
-    if (!s) s = c.mo_out ? launch<NCH, sp::OUT_MO>(A, nblk, smem, st) : launch<NCH, sp::OUT_RHO>(A, nblk, smem, st);
+    if (!s) {
+        if (c.g_rho) {
+            if constexpr (NCH == 4) s = launch<NCH, sp::OUT_WV>(A, nblk, smem, st);
+        } else {
+            s = c.mo_out ? launch<NCH, sp::OUT_MO>(A, nblk, smem, st) : launch<NCH, sp::OUT_RHO>(A, nblk, smem, st);
+        }
+    }
     const cudaError_t e = cudaFreeAsync(ws, st);
     if (!s) s = cuda_status(e, "FP64 tensor-core path: workspace");
     done = s == OKG_OK;
@@ -1413,7 +1445,7 @@ int split_run(const okg_basis* b, const Grid& g, const SplitCall& c, cudaStream_
     // points 62:86 | 147:198 | 1439:1533, 3000 points 121:84 | 328:199 | 2915:1658.
     const bool values = (c.need & ~1u) == 0;
     const bool contraction = (c.need & ~0xFu) == 0 && !values && (long long)c.nmo * b->ncart >= 32768;
-    if (!contraction && g.npts < (values ? 32 : 16) * sm_count(current_device())) return OKG_OK;
+    if (!c.g_rho && !contraction && g.npts < (values ? 32 : 16) * sm_count(current_device())) return OKG_OK;
     if (b->nshell > sp::MAX_SHELLS || b->split.npanel > sp::MAX_PANELS || b->dev.max_nprim > 255) return OKG_OK;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {

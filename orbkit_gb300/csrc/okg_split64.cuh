@@ -25,6 +25,7 @@ struct SplitDev {
     const double* col_g;    // npanel x 16: angular norm of each column times its 2^shift
     const float4* prim_lg;  // nprim: {alpha log2(e), log2 |w|, alpha, 0}, ascending alpha per shell
     const SplitPrim* prim;  // nprim, ascending alpha per shell
+    const int* prim_place;  // nprim: place of each sorted primitive in the caller's order
     const uint64_t* exp_tab;  // 2^(63 - j / 2048), rounded
     const int* flags;       // non-zero: a parameter or position is not a number
     int npanel;
