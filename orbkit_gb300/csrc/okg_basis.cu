@@ -80,36 +80,62 @@ __global__ void prim_weights_kernel(const double* __restrict__ prim_in, const in
 
 // Mixed path: order each shell's primitives by ascending exponent, so that a
 // tile keeps a prefix of them when screening (the radial sums do not depend on
-// the order).  One thread per shell, insertion sort (a handful of primitives).
-// The FP64 {alpha, w} copy used for the cusp points of the mixed path is sorted
-// along (same permutation), and the FP64 tensor-core path's tables are filled in the
-// sorted order; *flags is raised by a parameter or position that is not a number.
+// the order).  The FP64 {alpha, w} copy used for the cusp points of the mixed path is
+// sorted along (same permutation, split_place), and the FP64 tensor-core path's tables
+// are filled in the sorted order; *flags is raised by a parameter or position that is not
+// a number.  Latency bounds it (a few hundred shells): a warp per shell and a lane per
+// primitive, whose place is the number of smaller exponents (equal ones by index).  One
+// thread per shell, inserting through global memory, took 13.8 us against 4.4 us (12 atoms);
+// that form is left for
+// more than 32 primitives and exponents that are not numbers.
 __global__ void sort_prim_mx_kernel(const Shell* __restrict__ shells, int nshell, PrimMx* __restrict__ prim_mx,
                                     double2* __restrict__ prim_cusp, const double* __restrict__ atoms, int natom,
                                     float4* __restrict__ split_lg, SplitPrim* __restrict__ split_pr,
                                     int* __restrict__ split_place, int* __restrict__ flags)
 {
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
-    for (int i = s; i < natom; i += gridDim.x * blockDim.x)
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, lane = t & 31, s = t >> 5;
+    for (int i = t; i < natom; i += gridDim.x * blockDim.x)
         if (!isfinite(atoms[4 * i]) || !isfinite(atoms[4 * i + 1]) || !isfinite(atoms[4 * i + 2])) atomicOr(flags, 1);
     if (s >= nshell) return;
     const int p0 = shells[s].prim0, np = shells[s].nprim;
-    for (int i = 0; i < np; ++i) split_place[p0 + i] = p0 + i;
-    for (int i = 1; i < np; ++i) {
-        const PrimMx v = prim_mx[p0 + i];
-        const double2 c = prim_cusp[p0 + i];
-        int j = i - 1;
-        while (j >= 0 && prim_mx[p0 + j].a2 > v.a2) {
-            prim_mx[p0 + j + 1] = prim_mx[p0 + j];
-            prim_cusp[p0 + j + 1] = prim_cusp[p0 + j];
-            split_place[p0 + j + 1] = split_place[p0 + j];
-            --j;
-        }
-        prim_mx[p0 + j + 1] = v;
-        prim_cusp[p0 + j + 1] = c;
-        split_place[p0 + j + 1] = p0 + i;
+    const bool on = np <= 32 && lane < np;
+    PrimMx v{};
+    double2 c = make_double2(0.0, 0.0);
+    if (on) {
+        v = prim_mx[p0 + lane];
+        c = prim_cusp[p0 + lane];
     }
-    for (int i = 0; i < np; ++i)
+    if (np <= 32 && !__any_sync(0xffffffffu, on && isnan(v.a2))) {
+        int place = 0;
+        for (int j = 0; j < np; ++j) {
+            const double other = __shfl_sync(0xffffffffu, v.a2, j);
+            place += other < v.a2 || (other == v.a2 && j < lane);
+        }
+        __syncwarp();
+        if (on) {
+            prim_mx[p0 + place] = v;
+            prim_cusp[p0 + place] = c;
+            split_place[p0 + place] = p0 + lane;
+        }
+    } else if (lane == 0) {
+        for (int i = 0; i < np; ++i) split_place[p0 + i] = p0 + i;
+        for (int i = 1; i < np; ++i) {
+            v = prim_mx[p0 + i];
+            c = prim_cusp[p0 + i];
+            int j = i - 1;
+            while (j >= 0 && prim_mx[p0 + j].a2 > v.a2) {
+                prim_mx[p0 + j + 1] = prim_mx[p0 + j];
+                prim_cusp[p0 + j + 1] = prim_cusp[p0 + j];
+                split_place[p0 + j + 1] = split_place[p0 + j];
+                --j;
+            }
+            prim_mx[p0 + j + 1] = v;
+            prim_cusp[p0 + j + 1] = c;
+            split_place[p0 + j + 1] = p0 + i;
+        }
+    }
+    __syncwarp();
+    for (int i = lane; i < np; i += 32)
         if (!split_prim(prim_cusp[p0 + i], split_lg[p0 + i], split_pr[p0 + i])) atomicOr(flags, 1);
 }
 
@@ -582,7 +608,7 @@ extern "C" int okg_basis_set_params(okg_basis* b, const double* d_geo, const dou
                                                                  (double*)b->dev.prim, (float*)b->dev.prim32,
                                                                  (PrimMx*)b->dev.prim_mx, (double*)b->dev.prim_adj,
                                                                  (double2*)b->dev.prim_cusp);
-    sort_prim_mx_kernel<<<(b->nshell + 127) / 128, 128, 0, st>>>(b->dev.shells, b->nshell, (PrimMx*)b->dev.prim_mx,
+    sort_prim_mx_kernel<<<(b->nshell + 3) / 4, 128, 0, st>>>(b->dev.shells, b->nshell, (PrimMx*)b->dev.prim_mx,
                                                                  (double2*)b->dev.prim_cusp, b->dev.atoms, b->natom,
                                                                  (float4*)b->split.prim_lg, (SplitPrim*)b->split.prim,
                                                                  (int*)b->split.prim_place, (int*)b->split.flags);
