@@ -86,8 +86,7 @@ __global__ void prim_weights_kernel(const double* __restrict__ prim_in, const in
 // a number.  Latency bounds it (a few hundred shells): a warp per shell and a lane per
 // primitive, whose place is the number of smaller exponents (equal ones by index).  One
 // thread per shell, inserting through global memory, took 13.8 us against 4.4 us (12 atoms);
-// that form is left for
-// more than 32 primitives and exponents that are not numbers.
+// that form is left for more than 32 primitives and exponents that are not numbers.
 __global__ void sort_prim_mx_kernel(const Shell* __restrict__ shells, int nshell, PrimMx* __restrict__ prim_mx,
                                     double2* __restrict__ prim_cusp, const double* __restrict__ atoms, int natom,
                                     float4* __restrict__ split_lg, SplitPrim* __restrict__ split_pr,
