@@ -136,10 +136,11 @@ int okg_rho(const okg_basis* basis, const okg_grid* grid, int nmo, const double*
 int okg_fold_coeff(const okg_basis* basis, int nmo, const double* d_csph, double* d_ccart, okg_stream stream);
 int okg_unfold_coeff(const okg_basis* basis, int nmo, const double* d_ccart, double* d_csph, okg_stream stream);
 
-/* Whether a device wait of an okg_rho / okg_eval_mo call expired (OKG_ERR_TIMEOUT; the
- * outputs of that call are then incomplete) since the last query; clears the record.  The
- * device writes it during the call: query it after waiting for the call's stream.  Large
- * calls run on the tensor cores with waits between the warps of a block, each bounded. */
+/* Whether a device wait of an okg_rho, okg_eval_mo, okg_rho_backward or okg_ci_*_matrix
+ * call expired (OKG_ERR_TIMEOUT; the outputs of that call are then incomplete) since the
+ * last query; clears the record.  The device writes it during the call: query it after
+ * waiting for the call's stream.  Large calls run on the tensor cores with waits between
+ * the warps of a block, each bounded. */
 int okg_wait_status(int* status);
 
 /* ------------------------------------------------ operations on given grids
@@ -257,10 +258,11 @@ int okg_batch_status(okg_batch* batch, int* device_status);
  * orbkit/c_support.c:28-188); AO tiles are recomputed, not stored.
  * Outputs (overwritten): d_dcoeff (nmo x ncart, w.r.t. C_eff), d_dprim (nprim x 2:
  * d/dalpha, d/dc in ao_spec.get_prim_coeffs() order), d_dgeo (natom x 3).
- * precision: 64 or 32 (arithmetic of the backward).  Any nmo: above 48 MOs the AO
- * tiles of the MO pass are recomputed per block of 48 MOs.  d_work is caller
- * memory of at least okg_rho_backward_workspace bytes (per-CTA partial sums,
- * reduced in a fixed order: results are deterministic). */
+ * precision: 64 or 32 (arithmetic of the backward).  Up to 64 MOs (in FP32 from 2048
+ * points on) the contractions run on the tensor cores over runs of points; else, above
+ * 48 MOs, the AO tiles of the MO pass are recomputed per block of 48 MOs.  d_work is
+ * caller memory of at least okg_rho_backward_workspace bytes (about 1 GB of
+ * intermediates at most, and partial sums, reduced in a fixed order). */
 int okg_rho_backward_workspace(const okg_basis* basis, const okg_grid* grid, int nmo, int precision, size_t* bytes);
 int okg_rho_backward(const okg_basis* basis, const okg_grid* grid, int nmo, const double* d_coeff,
                      const double* d_occ, const double* d_g_rho, const double* d_g_grad, int64_t ld, int precision,
