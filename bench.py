@@ -702,7 +702,7 @@ def _single_workload(args, name, flush, L):
     pk, pk_kind = peaks()
     tflops = 8.0 * p.nmo * b.nao * npts / (kms * 1e-3) / 1e12
     fma64 = 4.0 * p.nmo * b.ncart * n64 / (fp64_ms * 1e-3)
-    fpk = fp64_fma_peak()
+    digits = 28 * 2 * fma64 / 1e12  # the FP64 path's products as digit products on the tensor cores
     res = {"value": npts / (ms * 1e-3), "ms_per_step": ms,
            "config": {"workload": name, "npts": npts, "nao": b.nao, "ncart": b.ncart, "nmo": p.nmo,
                       "spherical": b.spherical, "path": "mixed",
@@ -716,11 +716,11 @@ def _single_workload(args, name, flush, L):
                         "kernel": "rho_mixed_kernel", "kernel_ms": kms,
                         "peak_source": "bf16 burst, %s (MEASURED_PEAKS.json)" % pk_kind,
                         "algorithmic": "8*NMO*NAO FLOP per point (value + 3 derivatives of C.AO)",
-                        "fp64_path": {"bound": "fp64", "achieved": fma64, "peak": fpk, "unit": "FMA/s",
-                                      "frac": fma64 / fpk, "kernel": "fused64_kernel", "kernel_ms": fp64_ms,
-                                      "traffic": profile_traffic("fused64_kernel_" + name),
-                                      "algorithmic": "4*NMO*NCART FMA per point (C.AO for value + 3 derivatives)",
-                                      "peak_source": "2 DFMA/clk/SM x SMs x max SM clock"}},
+                        "fp64_path": {"bound": "latency", "achieved": digits, "peak": pk["bf16_tflops"], "unit": "TFLOP/s",
+                                      "frac": digits / pk["bf16_tflops"], "kernel": "split_kernel", "kernel_ms": fp64_ms,
+                                      "fma_per_s": fma64, "traffic": None,
+                                      "algorithmic": "28 digit products for each of 4*NMO*NCART FMA per point (C.AO for "
+                                                     "value + 3 derivatives), screened ones included"}},
            "gpu_launches": args.steps * 2}
     if not args.no_cpu_baseline:
         rate, cores, n, dt = cpu_rate(qc, gx, gy, gz, target_s=8.0)
@@ -866,14 +866,10 @@ def _detci_workload(args, flush):
     r_m, j_m = rho.clone(), j.clone()
     ms_terms = _time_ms(step_terms, max(2, args.steps // 2), 1, flush)
     err = max(float((r_m - rho).abs().max() / rho.abs().max()), float((j_m - j).abs().max() / j.abs().max()))
-    # FMAs the quadratic forms issue per point: rho visits a <= b in chunks of 16, the
-    # flux all (a, b) plus three accumulations per b
-    ch = (nmo + 15) // 16
-    fma_rho = sum(16 * (nmo - 16 * c) for c in range(ch)) + sum(nmo - 16 * c for c in range(ch))
-    fma_jab = ch * nmo * (16 + 3)
-    fma_rate = (fma_rho + fma_jab) * npts / (ms * 1e-3)
-    peak = fp64_fma_peak()
-    diag = ctypes_fp64_rate(_lib.load())
+    # bytes a point cannot do without: MO values (rho, flux), three derivatives, 4 results; the
+    # matrix-vector products run on the tensor cores
+    gbs = 8 * (5 * nmo + 4) * npts / (ms * 1e-3) / 1e9
+    pk, pk_kind = peaks()
     res = {"metric": "grid points/s for the CI transition density + flux density from MO grids",
            "unit": "grid points/s", "value": npts / (ms * 1e-3), "ms_per_step": ms, "dtype": "f64",
            "config": {"workload": "detci: %d zero + %d single terms over %d MOs, %d points (rho then jab)"
@@ -882,10 +878,10 @@ def _detci_workload(args, flush):
                       "term_order": {"value": npts / (ms_terms * 1e-3), "ms_per_step": ms_terms,
                                      "api": "okg_ci_rho + okg_ci_jab (exact=True)"},
                       "max_normwise_diff_vs_term_order": err},
-           "roofline": {"bound": "fp64", "achieved": fma_rate, "peak": peak, "unit": "FMA/s",
-                        "frac": fma_rate / peak, "traffic": None,
-                        "note": "FMAs issued per point %d (rho) + %d (flux); peak = 2 DFMA/clk/SM x SMs x max "
-                                "clock; the FMA-chain diagnostic reaches %.3g" % (fma_rho, fma_jab, diag or 0)},
+           "roofline": {"bound": "latency", "achieved": gbs, "peak": pk["hbm_gbs"], "unit": "GB/s",
+                        "frac": gbs / pk["hbm_gbs"], "traffic": None, "kernel": "ci_split_kernel",
+                        "peak_source": "copy, %s (MEASURED_PEAKS.json)" % pk_kind,
+                        "algorithmic": "8*(5*NMO + 4) bytes per point (rho and flux)"},
            "gpu_launches": 2}
     if not args.no_cpu_baseline:
         okref = _oracle()
