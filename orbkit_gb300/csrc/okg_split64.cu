@@ -64,6 +64,11 @@ constexpr int SMEM_MAX = 232448;
 enum { OUT_RHO = 0, OUT_MO = 1, OUT_WV = 2 };
 constexpr float KEEP_LOG2 = 62.0f;
 constexpr float ABS_FLOOR = -1000.0f;   // values below 2^-1000 are dropped
+// Up to which sqrt(alpha) times the error of a coordinate single precision places a tile's
+// points.  With an error x per coordinate log2 e^(-alpha d^2) errs by
+// 1.443 alpha (2 sqrt(3) d x + 3 x^2); where alpha d^2 <= 735 (beyond ABS_FLOOR nothing counts)
+// that is 136 sqrt(alpha) x + 4.3 alpha x^2, here 0.05 at most, which the scales have to spare.
+constexpr float WIDE = 3.6e-4f;
 
 template <int NCH>
 struct Cfg {
@@ -812,11 +817,11 @@ __device__ __forceinline__ BoxRange box_range(const Args& A, int atom, double ox
     return o;
 }
 
-// Raises top (log2, per channel class) to a shell's bound at squared distances dd:
-// sum over the primitives relative to the largest.
+// Raises top (log2, per channel class) to a shell's bound at squared distances dd (coordinates
+// within err): sum over the primitives relative to the largest.
 template <int NCLS, int NQ>
 __device__ __forceinline__ void point_bounds(const float4* __restrict__ pl, int np, int L, const float (&dd)[NQ],
-                                             const float (&dq)[NQ], float (&top)[NQ][NCLS])
+                                             const float (&dq)[NQ], float err, float (&top)[NQ][NCLS])
 {
     float m[NQ], R0[NQ], R1[NQ], R2[NQ];
 #pragma unroll
@@ -842,12 +847,52 @@ __device__ __forceinline__ void point_bounds(const float4* __restrict__ pl, int 
 #pragma unroll
     for (int q = 0; q < NQ; ++q) {
         if (m[q] < -1.0e30f) continue;
-        const Poly f = poly(L, sqrtf(dd[q]), dq[q]);
+        const Poly f = poly(L, sqrtf(dd[q]) + 2.f * err, dq[q] + err);
         top[q][0] = fmaxf(top[q][0], m[q] + __log2f(f.p0 * R0[q]));
         if (NCLS > 1) top[q][1] = fmaxf(top[q][1], m[q] + __log2f(f.p1 * R0[q] + 2.f * f.q1 * R1[q]));
         if (NCLS > 2)
             top[q][2] = fmaxf(top[q][2],
                               m[q] + __log2f(f.p2 * R0[q] + 2.f * (2 * L + 1) * f.p0 * R1[q] + 4.f * f.q2 * R2[q]));
+    }
+}
+
+// A point that is set apart: non-finite, or |coordinate| >= 2^60; else 0.
+__device__ __forceinline__ int special_point(double x, double y, double z)
+{
+    const int h = max(__double2hiint(x) & 0x7FFFFFFF, max(__double2hiint(y) & 0x7FFFFFFF, __double2hiint(z) & 0x7FFFFFFF));
+    return h >= 0x7FF00000 ? ROW_NAN : h >= 0x43B00000 ? ROW_ZERO : 0;
+}
+// Row exponent of a point with the bound `top` (log2): 0.1 for the roundings of the bound, 0.05 for
+// those of the coordinates.
+__device__ __forceinline__ int row_scale(int special, float top)
+{
+    return special ? special : top > 985.f ? ROW_NAN : (int)ceilf(fminf(fmaxf(top + 0.15f, -950.f), 990.f));
+}
+
+// The points' scales of a tile beyond WIDE, with FP64 differences to the atoms: every kept shell,
+// point after point (a call of its own: few tiles need it).
+template <int NCH>
+__device__ __noinline__ void wide_scales(const Args& A, long long t, const unsigned char* nkeep, short* rowexp, float r0,
+                                         float r1, float r2)
+{
+    constexpr int NCLS = Cfg<NCH>::NCLS;
+    const int lane = threadIdx.x & 31;
+    const float ref[3] = {r0, r1, r2};
+#pragma unroll 1
+    for (int q = 0; q < A.nsub; ++q) {
+        long long p;
+        double x, y, z;
+        tile_point(A, t, q * 32 + lane, p, x, y, z);
+        float top[1][NCLS];
+        for (int c = 0; c < NCLS; ++c) top[0][c] = ref[c];
+        for (int s = 0; s < A.B.nshell; ++s) {
+            const int4 rec = __ldg(A.S.shell + s);
+            const double* at = A.B.atoms + 4 * rec.x;
+            const float dx = (float)(x - __ldg(at)), dy = (float)(y - __ldg(at + 1)), dz = (float)(z - __ldg(at + 2));
+            const float dd[1] = {fmaf(dx, dx, fmaf(dy, dy, dz * dz))}, dq[1] = {fmaxf(fabsf(dx), fmaxf(fabsf(dy), fabsf(dz)))};
+            point_bounds<NCLS>(A.S.prim_lg + rec.z, nkeep[s], rec.y & 0xFF, dd, dq, 0.f, top);
+        }
+        for (int c = 0; c < NCLS; ++c) rowexp[c * 128 + q * 32 + lane] = (short)row_scale(special_point(x, y, z), top[0][c]);
     }
 }
 
@@ -876,8 +921,8 @@ __device__ __forceinline__ void tile_role(const Args& A, const State& S, int tw)
             if (lane == 0) mbar_arrive(S.screened + 8 * b);
             return;
         }
-        // points relative to one of them (single precision keeps the distances to the
-        // nearby atoms); points at |coordinate| >= 2^60 or non-finite are set apart
+        // points relative to one of them, in single precision (see WIDE); points at
+        // |coordinate| >= 2^60 or non-finite are set apart
         float fx[NQ], fy[NQ], fz[NQ];
         int special[NQ];
         double ox = 0.0, oy = 0.0, oz = 0.0;
@@ -897,8 +942,7 @@ __device__ __forceinline__ void tile_role(const Args& A, const State& S, int tw)
                 pt[128] = y;
                 pt[256] = z;
             }
-            const int h = max(__double2hiint(x) & 0x7FFFFFFF, max(__double2hiint(y) & 0x7FFFFFFF, __double2hiint(z) & 0x7FFFFFFF));
-            special[q] = h >= 0x7FF00000 ? ROW_NAN : h >= 0x43B00000 ? ROW_ZERO : 0;
+            special[q] = special_point(x, y, z);
             const unsigned first = __ballot_sync(0xffffffffu, special[q] == 0);
             if (!have && first) {
                 const int src = __ffs(first) - 1;
@@ -926,6 +970,18 @@ __device__ __forceinline__ void tile_role(const Args& A, const State& S, int tw)
                 lo[c] = fminf(lo[c], __shfl_xor_sync(0xffffffffu, lo[c], o));
                 hi[c] = fmaxf(hi[c], __shfl_xor_sync(0xffffffffu, hi[c], o));
             }
+        // The coordinates relative to the origin point (of points and atoms) are rounded to floats,
+        // so differences err by up to 2^-23 of the tile's extent, besides their own rounding: the
+        // box is widened by that, and where it counts (WIDE) the points' differences are FP64.
+        float ext = 0.f;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) ext = have ? fmaxf(ext, fmaxf(fabsf(lo[c]), fabsf(hi[c]))) : 0.f;
+        float err = 2.0e-7f * ext, amax = 0.f;  // 2^-23 + 2^-24 (the widened edge's rounding) = 1.8e-7
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            lo[c] -= err;
+            hi[c] += err;
+        }
         for (int i = lane; i < MAX_PANELS / 32; i += 32) pbits[i] = 0u;
         __syncwarp();
         unsigned char* nkeep = S.nkeep + b * MAX_SHELLS;
@@ -981,6 +1037,7 @@ __device__ __forceinline__ void tile_role(const Args& A, const State& S, int tw)
                             if (u[c] > fmaxf(ref[c] - KEEP_LOG2, ABS_FLOOR)) nk = q + 1;
                             if (u[c] + lnp >= ref[c]) big = true;
                         }
+                        if (nk == q + 1) amax = fmaxf(amax, a);
                     }
                     big = big && nk > 0;
                     nkeep[s] = (unsigned char)nk;
@@ -998,6 +1055,16 @@ __device__ __forceinline__ void tile_role(const Args& A, const State& S, int tw)
                 if (k) S.plist[b * MAX_PANELS + npan + __popc(mk & ((1u << lane) - 1u))] = (unsigned short)(pb + lane);
                 npan += __popc(mk);
             }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+        short* rowexp = S.rowexp + b * 3 * 128;
+        if (sqrtf(amax) * err > WIDE) {
+            wide_scales<NCH>(A, t, nkeep, rowexp, ref[0], NCLS > 1 ? ref[1] : 0.f, NCLS > 2 ? ref[2] : 0.f);
+            if (lane == 0) S.npan[b] = npan;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(S.screened + 8 * b);
+            continue;
         }
         // the scale of every point: the largest bound at the point itself
         float top[NQ][NCLS];
@@ -1019,17 +1086,13 @@ __device__ __forceinline__ void tile_role(const Args& A, const State& S, int tw)
                 dd[q] = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
                 dq[q] = fmaxf(fabsf(dx), fmaxf(fabsf(dy), fabsf(dz)));
             }
-            point_bounds<NCLS>(A.S.prim_lg + rec.z, nk, L, dd, dq, top);
+            point_bounds<NCLS>(A.S.prim_lg + rec.z, nk, L, dd, dq, err, top);
         }
-        short* rowexp = S.rowexp + b * 3 * 128;
 #pragma unroll
         for (int q = 0; q < NQ; ++q)
 #pragma unroll
-            for (int c = 0; c < NCLS; ++c) {
-                const float e = ceilf(fminf(fmaxf(top[q][c] + 0.1f, -950.f), 990.f));
-                if (q < nsub)
-                    rowexp[c * 128 + q * 32 + lane] = (short)((bad || top[q][c] > 985.f) ? ROW_NAN : special[q] ? special[q] : (int)e);
-            }
+            for (int c = 0; c < NCLS; ++c)
+                if (q < nsub) rowexp[c * 128 + q * 32 + lane] = (short)(bad ? ROW_NAN : row_scale(special[q], top[q][c]));
         if (lane == 0) S.npan[b] = npan;
         __syncwarp();
         if (lane == 0) mbar_arrive(S.screened + 8 * b);
