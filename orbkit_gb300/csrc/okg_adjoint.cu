@@ -3,7 +3,8 @@
 // exponents and contraction coefficients, and the nuclear coordinates.  This is the
 // one-kernel form, for more than 64 MOs and FP32 calls of fewer than 2048 points (and for
 // a workspace too small for the other): AO tiles are recomputed, never stored.  The other
-// calls take the pipeline of okg_adjoint_split.cu.
+// calls take the pipeline of okg_adjoint_split.cu, and run this form after it where the
+// pipeline raised its redo word (values out of the digits' range).
 //
 // Forward being differentiated (orbkit/core.py:266-300 with the AO kernel of
 // orbkit/c_grid-based.c:9-79):
@@ -56,6 +57,7 @@ struct Args {
     T* part_g;  // [nblk][NW][natom][3]
     T* part_w;  // nmo > NMOMAX: [nblk][2][nmo][P] (W and V of the CTA's tile), else null
     long long ntiles;
+    const int* go;  // null, or the word that has to be raised for the call to run
 };
 
 template <typename T>
@@ -141,6 +143,7 @@ __device__ __forceinline__ void shell_sums_L(int L, T X, T Y, T Z, T gx, T gy, T
 template <typename T, bool BIG>
 __global__ void __launch_bounds__(NT, ctas_per_sm<T>()) adjoint_kernel(BasisDev B, Grid g, Args<T> A)
 {
+    if (A.go && *A.go == 0) return;
     extern __shared__ __align__(16) unsigned char sm_raw[];
     T* AO_s = (T*)sm_raw;            // 10 x KC x P
     T* C_s = AO_s + 10 * KC * P;     // NMOMAX x KC
@@ -351,15 +354,22 @@ __global__ void __launch_bounds__(NT, ctas_per_sm<T>()) adjoint_kernel(BasisDev 
     }
 }
 
+// Sums over the blocks b (part_g: and their NW consecutive sub-slots) of part[b][.][j], in order.
 template <typename T>
-__global__ void reduce_kernel(const T* __restrict__ part, long long n, int nblk, int inner, double* __restrict__ out)
+__global__ void reduce_kernel(Args<T> A, int nblk, long long nc, long long np, long long ng, double* __restrict__ dC,
+                              double* __restrict__ dprim, double* __restrict__ dgeo)
 {
-    // out[j] = sum over blocks b (and `inner` consecutive sub-slots) of part[b][.][j], fixed order
+    if (A.go && *A.go == 0) return;
     long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    const bool c = j < nc, p = !c && j - nc < np;
+    const T* part = c ? A.part_c : p ? A.part_p : A.part_g;
+    double* out = c ? dC : p ? dprim : dgeo;
+    const long long n = c ? nc : p ? np : ng;
+    j -= c ? 0 : p ? nc : nc + np;
     if (j >= n) return;
+    const int slots = c || p ? nblk : nblk * NW;
     double s = 0.0;
-    for (int b = 0; b < nblk; ++b)
-        for (int w = 0; w < inner; ++w) s += (double)part[((long long)b * inner + w) * n + j];
+    for (int b = 0; b < slots; ++b) s += (double)part[(long long)b * n + j];
     out[j] = s;
 }
 
@@ -385,7 +395,7 @@ static int block_count(long long ntiles)
 template <typename T>
 static int run(const okg_basis* b, const Grid& g, int nmo, const double* C, const double* occ, const double* grho,
                const double* ggrad, long long ld, double* dC, double* dprim, double* dgeo, void* work,
-               size_t work_bytes, cudaStream_t st)
+               size_t work_bytes, const int* go, cudaStream_t st)
 {
     const long long ntiles = (g.npts + P - 1) / P;
     const int nblk = block_count<T>(ntiles);
@@ -403,6 +413,7 @@ static int run(const okg_basis* b, const Grid& g, int nmo, const double* C, cons
     A.part_g = A.part_p + (size_t)nblk * 2 * b->nprim;
     A.part_w = nmo > NMOMAX ? A.part_g + (size_t)nblk * NW * b->natom * 3 : nullptr;
     A.ntiles = ntiles;
+    A.go = go;
     const size_t smem = sizeof(T) * (10 * KC * P + NMOMAX * KC + 2 * NMOMAX * P + 3 * KC * P);
     static bool configured = false;
     if (!configured) {
@@ -417,13 +428,25 @@ static int run(const okg_basis* b, const Grid& g, int nmo, const double* C, cons
         adjoint_kernel<T, true><<<nblk, NT, smem, st>>>(b->dev, g, A);
     else
         adjoint_kernel<T, false><<<nblk, NT, smem, st>>>(b->dev, g, A);
-    long long n = (long long)nmo * b->ncart;
-    reduce_kernel<T><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(A.part_c, n, nblk, 1, dC);
-    n = 2ll * b->nprim;
-    reduce_kernel<T><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(A.part_p, n, nblk, 1, dprim);
-    n = 3ll * b->natom;
-    reduce_kernel<T><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(A.part_g, n, nblk, NW, dgeo);
+    const long long nc = (long long)nmo * b->ncart, np = 2ll * b->nprim, ng = 3ll * b->natom;
+    reduce_kernel<T><<<(unsigned)((nc + np + ng + 255) / 256), 256, 0, st>>>(A, nblk, nc, np, ng, dC, dprim, dgeo);
     return cuda_status(cudaGetLastError(), "okg_rho_backward launch");
+}
+
+static size_t one_kernel_bytes(const okg_basis* b, long long npts, int nmo, int precision)
+{
+    const long long ntiles = (npts + P - 1) / P;
+    return precision == 32 ? workspace_bytes<float>(b, nmo, block_count<float>(ntiles))
+                           : workspace_bytes<double>(b, nmo, block_count<double>(ntiles));
+}
+
+// Workspace of the pipeline, with room for the one-kernel form after it and a redo word beyond
+// both; 0 if the call is not one for it.
+constexpr size_t REDO_BYTES = 256;
+static size_t pipeline_bytes(const okg_basis* b, long long npts, int nmo, int precision)
+{
+    const size_t split = adjoint_split_bytes(b, npts, nmo, precision), one = one_kernel_bytes(b, npts, nmo, precision);
+    return split ? ((split > one ? split : one) + 255) / 256 * 256 + REDO_BYTES : 0;
 }
 
 }  // namespace adj
@@ -435,11 +458,9 @@ extern "C" int okg_rho_backward_workspace(const okg_basis* b, const okg_grid* gr
                                           size_t* bytes)
 {
     if (!b || !grid || !bytes || nmo <= 0) return set_error(OKG_ERR_ARG, "okg_rho_backward_workspace: bad argument");
-    const long long ntiles = (grid->npts + adj::P - 1) / adj::P;
-    *bytes = precision == 32 ? adj::workspace_bytes<float>(b, nmo, adj::block_count<float>(ntiles))
-                             : adj::workspace_bytes<double>(b, nmo, adj::block_count<double>(ntiles));
-    const size_t split = adjoint_split_bytes(b, grid->npts, nmo, precision);
-    if (split > *bytes) *bytes = split;
+    *bytes = adj::one_kernel_bytes(b, grid->npts, nmo, precision);
+    const size_t all = adj::pipeline_bytes(b, grid->npts, nmo, precision);
+    if (all) *bytes = all;
     return OKG_OK;
 }
 
@@ -467,15 +488,19 @@ extern "C" int okg_rho_backward(const okg_basis* b, const okg_grid* gr, int nmo,
         return set_error(OKG_ERR_ARG, "okg_rho_backward: regular grid range outside Nx*Ny*Nz");
     if (ld < g.npts) return set_error(OKG_ERR_ARG, "okg_rho_backward: ld < npts");
     cudaStream_t st = (cudaStream_t)stream;
-    if (work_bytes >= adjoint_split_bytes(b, g.npts, nmo, precision)) {
+    const int* go = nullptr;
+    const size_t all = adj::pipeline_bytes(b, g.npts, nmo, precision);
+    if (all && work_bytes >= all) {
         bool done = false;
+        int* redo = (int*)((char*)d_work + all - adj::REDO_BYTES);
         const int s = adjoint_split_run(b, g, nmo, d_coeff, d_occ, d_g_rho, d_g_grad, ld, precision, d_dcoeff, d_dprim, d_dgeo,
-                                        d_work, st, done);
-        if (s || done) return s;
+                                        d_work, redo, st, done);
+        if (s) return s;
+        if (done) go = redo;
     }
     if (precision == 64)
         return adj::run<double>(b, g, nmo, d_coeff, d_occ, d_g_rho, d_g_grad, ld, d_dcoeff, d_dprim, d_dgeo, d_work,
-                                work_bytes, st);
+                                work_bytes, go, st);
     return adj::run<float>(b, g, nmo, d_coeff, d_occ, d_g_rho, d_g_grad, ld, d_dcoeff, d_dprim, d_dgeo, d_work,
-                           work_bytes, st);
+                           work_bytes, go, st);
 }

@@ -16,6 +16,8 @@
 //   4. dC_ik = sum_r W_i chi_k + V_i G_k: digit products with the points as the summed index,
 //      64 points per accumulation, FP64 sums of those;
 //   5. partial sums added in a fixed order.
+// What the digits cannot hold (values that are not finite, a call that step 1 gives up) raises
+// the call's redo word, and the one-kernel form, launched at the end, computes the call.
 // FP32 precision: W, V, A, B, chi and G are floats, the products of steps 2 and 4 take 4
 // digits (31 bits), step 3 computes in FP32.
 //
@@ -137,7 +139,6 @@ __device__ __forceinline__ void acc_doubles(const AccN<D>& a, int rowx, const in
 #pragma unroll
         for (int w = 0; w < 7; ++w) t[w] = w < D ? f2i(a.r[w < D ? w : 0][i]) : 0;
         v[i] = combine7(t, rowx + f[i] - 54);
-        if (rowx >= ROW_NAN || f[i] == MO_NAN) v[i] = __longlong_as_double(0x7FF8000000000000ll);
     }
 }
 // ... as floats: 4 weights, sums below 2^22, so the upper and lower pair are exact in 32 bits
@@ -153,7 +154,6 @@ __device__ __forceinline__ void acc_floats(const AccN<4>& a, int rowx, const int
         x = x < -250 ? -250 : x > 250 ? 250 : x;
         const int x1 = x / 2, x2 = x - x1;
         v[i] = t * __int_as_float((127 + x1) << 23) * __int_as_float((127 + x2) << 23);
-        if (rowx >= ROW_NAN || f[i] == MO_NAN) v[i] = __int_as_float(0x7FC00000);
     }
 }
 
@@ -188,6 +188,7 @@ struct ColArgs {
     int nmo, ncart, kp;
     T* out;            // 2 x ncart x ld
     int* status;
+    int* redo;         // raised where a value is not finite
 };
 
 template <typename T>
@@ -226,7 +227,8 @@ __global__ void __launch_bounds__(128 * ColCfg<T>::G, ColCfg<T>::CTAS) column_ke
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) m = DG::shfl_max(m, o);
         const int F = DG::scale(m);
-        if (lane == 0) fexp[b] = DG::special(m) ? MO_NAN : F;
+        if (DG::special(m)) *(volatile int*)A.redo = 1;
+        if (lane == 0) fexp[b] = F;
         for (int a = lane; a < KP * 16; a += 32)
             DG::put((a < A.nmo && b < ncol) ? as<T>(A.C[(long long)a * A.ncart + n_first + b]) : T(0), F,
                     smem_u32(Bs) + (a >> 4) * bpanel + b_off(b, a & 15), np * 32);
@@ -301,7 +303,8 @@ __global__ void __launch_bounds__(128 * ColCfg<T>::G, ColCfg<T>::CTAS) column_ke
         U mr = 0;
 #pragma unroll
         for (int g = 0; g < G; ++g) mr = max(mr, tops[g * 128 + row]);
-        const int rowx = DG::special(mr) ? ROW_NAN : DG::scale(mr);
+        if (DG::special(mr)) *(volatile int*)A.redo = 1;
+        const int rowx = DG::scale(mr);
 #pragma unroll 1
         for (int n0 = 4 * (warp >> 2); n0 < ncol; n0 += 4 * G) {
             AccN<D> va;
@@ -339,6 +342,7 @@ struct RowArgs {
     double* part;     // nslot x ncart x nmo
     int slot0;
     int* status;
+    int* redo;        // raised where a value is not finite
     unsigned tm_cols;
 };
 
@@ -366,7 +370,8 @@ __device__ __forceinline__ Pair<T> load_row(const T* __restrict__ src, long long
 // Their digits into the K-major tiles (row `row` of panels panel_bytes apart, digits
 // digit_bytes apart); the row's scale.
 template <typename T>
-__device__ __forceinline__ int put_row(const Pair<T>& x, int lane, uint32_t base, uint32_t panel_bytes, uint32_t digit_bytes, int row)
+__device__ __forceinline__ int put_row(const Pair<T>& x, int lane, uint32_t base, uint32_t panel_bytes, uint32_t digit_bytes, int row,
+                                       int* redo)
 {
     using DG = Dg<T>;
     typename DG::U m = max(DG::magnitude(x.v[0]), DG::magnitude(x.v[1]));
@@ -376,7 +381,8 @@ __device__ __forceinline__ int put_row(const Pair<T>& x, int lane, uint32_t base
 #pragma unroll
     for (int h = 0; h < 2; ++h)
         DG::put(x.v[h], E, base + (uint32_t)(2 * h + (lane >> 4)) * panel_bytes + b_off(row, lane & 15), digit_bytes);
-    return DG::special(m) ? ROW_NAN : E;
+    if (DG::special(m)) *(volatile int*)redo = 1;
+    return E;
 }
 
 template <typename T>
@@ -440,10 +446,10 @@ __global__ void __launch_bounds__(512, 1) row_kernel(const __grid_constant__ Row
                     const bool left = k < nrow;
                     const int rw = left ? k : k - nrow;
                     const int e = put_row(x[u], lane, left ? smem_u32(base) : smem_u32(Bs), left ? (uint32_t)(D * DT) : (uint32_t)bpanel,
-                                          left ? (uint32_t)DT : (uint32_t)(np * 32), rw);
+                                          left ? (uint32_t)DT : (uint32_t)(np * 32), rw, A.redo);
                     if (lane == 0) {
                         if (left) rexp[rw] = e;
-                        else fexp[rw] = e == ROW_NAN ? MO_NAN : e;
+                        else fexp[rw] = e;
                     }
                 }
             }
@@ -533,6 +539,7 @@ struct ShellArgs {
     double* part_g;        // nslot x nshell x 3
     int slot0;
     long long per;         // points of a slot (multiple of 32)
+    int* redo;             // raised where a cotangent is not finite
 };
 
 // Coordinates of points visited in ascending order, 32 or fewer apart: the indices of a
@@ -644,9 +651,9 @@ __device__ __forceinline__ void shell_polynomials(const T (&Av)[(L + 1) * (L + 2
 }
 
 // e^(-alpha rr)
-__device__ __forceinline__ double gauss(double rr, uint64_t mr, int er, const SplitPrim* pr, double alpha, const uint64_t* tab)
+__device__ __forceinline__ double gauss(double, uint64_t mr, int er, const SplitPrim* pr, double, const uint64_t* tab)
 {
-    return pr->special ? exp(-alpha * rr) : exp_neg(mr, er, pr->A, pr->ea, tab);
+    return exp_neg(mr, er, pr->A, pr->ea, tab);
 }
 __device__ __forceinline__ float gauss(float rr, uint64_t, int, const SplitPrim*, float alpha, const uint64_t*) { return expf(-alpha * rr); }
 
@@ -688,16 +695,13 @@ __device__ __forceinline__ void run_shell(const ShellArgs<T>& A, const Shell& sh
         // exponents and coefficients: floats in registers, doubles (whose sums take those) read again
         constexpr bool HELD = sizeof(T) == 4;
         T U0[QB], U1[QB], U2[QB], al_[HELD ? QB : 1], w_[HELD ? QB : 1];
-        unsigned always = 0;
 #pragma unroll
         for (int q = 0; q < QB; ++q) {
             U0[q] = U1[q] = U2[q] = T(0);
             if (q >= nq) continue;
-            const T wq = as<T>(prims[q].w);
-            if (!(wq - wq == T(0)) || prims[q].special) always |= 1u << q;
             if constexpr (HELD) {
                 al_[q] = as<T>(-prims[q].neg_alpha);
-                w_[q] = wq;
+                w_[q] = as<T>(prims[q].w);
             }
         }
         auto al = [&](int q) -> T {
@@ -742,7 +746,7 @@ __device__ __forceinline__ void run_shell(const ShellArgs<T>& A, const Shell& sh
                 e[q] = T(0);
                 if (q >= nq) continue;
                 const T aq = al(q);
-                if (!(always >> q & 1) && !__any_sync(0xffffffffu, !underflows(aq, rr))) continue;
+                if (!__any_sync(0xffffffffu, !underflows(aq, rr))) continue;
                 live |= 1u << q;
                 e[q] = gauss(rr, mr, er, prims + q, aq, A.S.exp_tab);
                 const T we = w(q) * e[q];
@@ -774,8 +778,8 @@ __device__ __forceinline__ void run_shell(const ShellArgs<T>& A, const Shell& sh
             T F = o.Pa;
             if constexpr (L > 0) F += gx * o.dB[0] + gy * o.dB[1] + gz * o.dB[2];
             const T Tt = gX * o.Pb, T2 = T(2) * Tt;
-            // (a cotangent that is not finite reaches every primitive, as 0 times it is not 0)
-            if (__any_sync(0xffffffffu, !(F - F == T(0) && Tt - Tt == T(0)))) live = 0xFFFFFFFFu;
+            // (a cotangent that is not finite would reach every primitive, as 0 times it is not 0)
+            if (!(F - F == T(0) && Tt - Tt == T(0))) *(volatile int*)A.redo = 1;
             if (q0 == 0) {
                 const T s1F = S1 * F + S2 * Tt, s1b = S1 * o.Pb;
                 dR[0] += s1F * X + s1b * gx;
@@ -922,7 +926,7 @@ static int sm_count()
 
 template <typename T>
 static int run(const okg_basis* b, const Grid& g, int nmo, const double* C, const double* occ, const double* grho, const double* ggrad,
-               long long ld, double* dC, double* dprim, double* dgeo, char* work, const Plan& P, cudaStream_t st, bool& done)
+               long long ld, double* dC, double* dprim, double* dgeo, char* work, const Plan& P, int* redo, cudaStream_t st, bool& done)
 {
     int* status = split_status_word();
     if (!status) return OKG_OK;
@@ -935,6 +939,8 @@ static int run(const okg_basis* b, const Grid& g, int nmo, const double* C, cons
     cudaError_t e = cudaFuncSetAttribute(column_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cs);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(row_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rs);
     if (e != cudaSuccess) return cuda_status(e, "okg_rho_backward: shared memory");
+    e = cudaMemsetAsync(redo, 0, sizeof(int), st);
+    if (e != cudaSuccess) return cuda_status(e, "okg_rho_backward: memset");
     const int passes = (b->ncart + 63) / 64, sms = sm_count();
     for (int r = 0; r < P.nruns; ++r) {
         const long long i0 = r * P.run, n = g.npts - i0 < P.run ? g.npts - i0 : P.run;
@@ -952,21 +958,22 @@ static int run(const okg_basis* b, const Grid& g, int nmo, const double* C, cons
         c.g_rho = grho + i0;
         c.g_grad = ggrad ? ggrad + i0 : nullptr;
         c.g_ld = ld;
+        c.redo = redo;
         bool wv = false;
-        int s = split_run(b, gr, c, st, wv);
+        int s = split_run(b, gr, c, SplitGeneral{}, st, wv);
         if (s || !wv) return s;
         const long long tiles = (n + 127) / 128;
         int gx = (sms * ColCfg<T>::CTAS + 2 * passes - 1) / (2 * passes);
         if (gx > tiles) gx = (int)tiles;
-        column_kernel<T><<<dim3(gx, passes, 2), 128 * ColCfg<T>::G, cs, st>>>(ColArgs<T>{n, P.run, X, C, nmo, b->ncart, kp, AB, status});
+        column_kernel<T><<<dim3(gx, passes, 2), 128 * ColCfg<T>::G, cs, st>>>(ColArgs<T>{n, P.run, X, C, nmo, b->ncart, kp, AB, status, redo});
         long long per = ((n + P.nchunk - 1) / P.nchunk + 31) / 32 * 32;
-        const ShellArgs<T> sa{b->dev, b->split, gr, c.g_grad, ld, P.run, AB, Y, pp, pg, r * P.nchunk, per};
+        const ShellArgs<T> sa{b->dev, b->split, gr, c.g_grad, ld, P.run, AB, Y, pp, pg, r * P.nchunk, per, redo};
         shell_kernel<T, false><<<dim3(b->nshell, P.nchunk / 4), 128, 0, st>>>(sa);
         if (b->max_l > 2) shell_kernel<T, true><<<dim3(b->nshell, P.nchunk / 4), 128, 0, st>>>(sa);
         unsigned tm = 32;
         while ((int)tm < Dg<T>::D * np) tm *= 2;
         row_kernel<T><<<dim3(P.nbx, (b->ncart + 127) / 128), 512, rs, st>>>(
-            RowArgs<T>{n, P.run, X, Y, nmo, b->ncart, np, pc, r * P.nbx, status, tm});
+            RowArgs<T>{n, P.run, X, Y, nmo, b->ncart, np, pc, r * P.nbx, status, redo, tm});
     }
     dcoeff_kernel<<<(nmo * b->ncart + 31) / 32, dim3(32, 8), 0, st>>>(pc, P.nruns * P.nbx, nmo, b->ncart, dC);
     finish_kernel<<<(b->nprim + b->natom + 3) / 4, 128, 0, st>>>(b->dev, b->split, pp, pg, P.nruns * P.nchunk, dprim, dgeo);
@@ -985,15 +992,15 @@ size_t adjoint_split_bytes(const okg_basis* b, long long npts, int nmo, int prec
 
 int adjoint_split_run(const okg_basis* b, const Grid& g, int nmo, const double* C, const double* occ, const double* grho,
                       const double* ggrad, long long ld, int precision, double* dC, double* dprim, double* dgeo, void* work,
-                      cudaStream_t st, bool& done)
+                      int* redo, cudaStream_t st, bool& done)
 {
     done = false;
     if (!adjs::takes(g.npts, nmo, precision)) return OKG_OK;
     const int sms = adjs::sm_count();
     if (precision == 32)
         return adjs::run<float>(b, g, nmo, C, occ, grho, ggrad, ld, dC, dprim, dgeo, (char*)work,
-                                adjs::make_plan<float>(b, g.npts, nmo, sms), st, done);
+                                adjs::make_plan<float>(b, g.npts, nmo, sms), redo, st, done);
     return adjs::run<double>(b, g, nmo, C, occ, grho, ggrad, ld, dC, dprim, dgeo, (char*)work,
-                             adjs::make_plan<double>(b, g.npts, nmo, sms), st, done);
+                             adjs::make_plan<double>(b, g.npts, nmo, sms), redo, st, done);
 }
 }  // namespace okg

@@ -82,8 +82,8 @@ __global__ void prim_weights_kernel(const double* __restrict__ prim_in, const in
 // tile keeps a prefix of them when screening (the radial sums do not depend on
 // the order).  The FP64 {alpha, w} copy used for the cusp points of the mixed path is
 // sorted along (same permutation, split_place), and the FP64 tensor-core path's tables
-// are filled in the sorted order; *flags is raised by a parameter or position that is not
-// a number.  Latency bounds it (a few hundred shells): a warp per shell and a lane per
+// are filled in the sorted order; *flags is raised by a parameter or position out of their
+// range (split_prim).  Latency bounds it (a few hundred shells): a warp per shell and a lane per
 // primitive, whose place is the number of smaller exponents (equal ones by index).  One
 // thread per shell, inserting through global memory, took 13.8 us against 4.4 us (12 atoms);
 // that form is left for more than 32 primitives and exponents that are not numbers.
@@ -94,7 +94,8 @@ __global__ void sort_prim_mx_kernel(const Shell* __restrict__ shells, int nshell
 {
     const int t = blockIdx.x * blockDim.x + threadIdx.x, lane = t & 31, s = t >> 5;
     for (int i = t; i < natom; i += gridDim.x * blockDim.x)
-        if (!isfinite(atoms[4 * i]) || !isfinite(atoms[4 * i + 1]) || !isfinite(atoms[4 * i + 2])) atomicOr(flags, 1);
+        for (int d = 0; d < 3; ++d)
+            if (!(fabs(atoms[4 * i + d]) < 536870912.0)) atomicOr(flags, 1);
     if (s >= nshell) return;
     const int p0 = shells[s].prim0, np = shells[s].nprim;
     const bool on = np <= 32 && lane < np;

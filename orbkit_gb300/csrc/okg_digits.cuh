@@ -16,7 +16,7 @@ constexpr int ND = 7;                   // digits of an operand
 constexpr int PK = OKG_SPLIT_PK;        // columns of a panel: one MMA K-step
 constexpr int DT = 128 * PK * 2;        // bytes of one digit of one 128-row operand tile
 constexpr int ROW_NAN = 30000, ROW_ZERO = 30001;  // row exponents of points without finite values
-constexpr int MO_NAN = 200000;                    // exponent of a column with a non-finite coefficient
+constexpr int MO_NAN = 200000;                    // exponent of a column with coefficients out of range
 
 // v = t 2^(E - 55), t rounded to an integer of 7 balanced base-256 digits; returned
 // biased by 128 per digit (byte b holds digit + 128), rs0 = E + 1030.  Integer
@@ -181,7 +181,7 @@ __device__ __forceinline__ void acc2_values(const Acc2& a, int rowx, const int2&
     for (int i = 0; i < 2; ++i) {
         const int t[7] = {f2i(a.r[0][i]), f2i(a.r[1][i]), f2i(a.r[2][i]), f2i(a.r[3][i]), f2i(a.r[4][i]), f2i(a.r[5][i]), f2i(a.r[6][i])};
         v[i] = combine7(t, rowx + f[i] - 54);
-        if (rowx >= ROW_NAN || f[i] == MO_NAN) v[i] = (rowx == ROW_ZERO && f[i] != MO_NAN) ? 0.0 : __longlong_as_double(0x7FF8000000000000ll);
+        if (rowx >= ROW_NAN) v[i] = rowx == ROW_ZERO ? 0.0 : __longlong_as_double(0x7FF8000000000000ll);
     }
 }
 

@@ -39,6 +39,10 @@ struct FusedArgs {
     double* dout;       // rho mode: ndrv x ld
     double* mo_norm;    // rho mode: nmo or null
     long long ld;
+    // after a tensor-core run of the same call: nothing to do unless *go is raised, but the MO
+    // norms of that run to be added
+    const int* go;
+    const double* norm_part;
 };
 
 template <int NCH>
@@ -74,125 +78,136 @@ __global__ void __launch_bounds__(FP * FG) fused64_kernel(BasisDev B, Grid g, Fu
     const int tid = threadIdx.x;
     const int pl = tid % FP;
     const int grp = tid / FP;
-    const long long p = (long long)blockIdx.x * FP + pl;
-    const bool valid = p < g.npts;
-    double x, y, z;
-    grid_point(g, valid ? p : g.npts - 1, x, y, z);
-    constexpr unsigned chmask = (1u << NCH) - 1u;
-    constexpr int MOPASS = FG * MB;
-
-    double rho_part = 0.0;
-    double drho_part[10];
-#pragma unroll
-    for (int d = 0; d < 10; ++d) drho_part[d] = 0.0;
-
-    for (int mo0 = 0; mo0 < A.nmo; mo0 += MOPASS) {
-        double acc[MB][NCH];
-#pragma unroll
-        for (int m = 0; m < MB; ++m)
-#pragma unroll
-            for (int c = 0; c < NCH; ++c) acc[m][c] = 0.0;
-
-        for (int ci = 0; ci < B.nchunk; ++ci) {
-            const int4 ck = B.chunks[ci];
-            const int kc = ck.w - ck.z;
-            __syncthreads();  // previous chunk fully consumed
-            for (int i = tid; i < MOPASS * OKG_KC; i += FT) {
-                const int m = i / OKG_KC, kk = i % OKG_KC;
-                const int mo = mo0 + m;
-                C_s[i] = (mo < A.nmo && kk < kc) ? A.C[(long long)mo * B.ncart + ck.z + kk] : 0.0;
-            }
-            int last_atom = -1;
-            double X = 0, Y = 0, Z = 0, rr = 0;
-            for (int s = ck.x + grp; s < ck.y; s += FG) {
-                const Shell sh = B.shells[s];
-                if (sh.atom != last_atom) {
-                    X = x - B.atoms[4 * sh.atom];
-                    Y = y - B.atoms[4 * sh.atom + 1];
-                    Z = z - B.atoms[4 * sh.atom + 2];
-                    rr = X * X + Y * Y + Z * Z;
-                    last_atom = sh.atom;
-                }
-                const Radial<double> r = radial64(B.prim, sh.prim0, sh.nprim, rr, NCH > 1, NCH > 4);
-                const int rowbase = sh.cart0 - ck.z;
-                shell_eval_L(sh.L, X, Y, Z, r, chmask, A.mixed_ref != 0, [&](int ch, int j, double v) {
-                    const int row = B.comp_row[sh.comp0 + j];
-                    if (row < 0) return;
-                    AO_s[(ch * OKG_KC + rowbase + row) * FP + pl] = v * B.comp_g[sh.comp0 + j];
-                });
-            }
-            __syncthreads();
-            const double* Cg = C_s + grp * MB * OKG_KC;
-            for (int kk = 0; kk < kc; ++kk) {
-                double a[NCH];
-#pragma unroll
-                for (int c = 0; c < NCH; ++c) a[c] = AO_s[(c * OKG_KC + kk) * FP + pl];
-#pragma unroll
-                for (int m = 0; m < MB; ++m) {
-                    const double cm = Cg[m * OKG_KC + kk];
-#pragma unroll
-                    for (int c = 0; c < NCH; ++c) acc[m][c] = fma(cm, a[c], acc[m][c]);
-                }
-            }
-        }
-
-        // epilogue of this MO pass
-#pragma unroll
-        for (int m = 0; m < MB; ++m) {
-            const int mo = mo0 + grp * MB + m;
-            if (mo >= A.nmo) break;
-            if (MO_OUT) {
-                if (valid)
-                    for (int d = 0; d < A.drv.n; ++d)
-                        A.out[((long long)d * A.nmo + mo) * A.ld + p] = pick<NCH>(acc[m], A.drv.code[d]);
-            } else {
-                const double o = A.occ[mo];
-                const double v0 = acc[m][0];
-                rho_part += o * (v0 * v0);
-                const double o2 = o * 2;
-#pragma unroll
-                for (int d = 0; d < 10; ++d) {
-                    if (d >= A.drv.n) break;
-                    const int code = A.drv.code[d];
-                    double t = (o2 * pick<NCH>(acc[m], code)) * v0;
-                    if (code >= 4) {
-                        int ca, cb;
-                        second_pair(code, ca, cb);
-                        t += o2 * (pick<NCH>(acc[m], ca) * pick<NCH>(acc[m], cb));
-                    }
-                    drho_part[d] += t;
-                }
-                if (A.mo_norm) {
-                    double q = valid ? v0 * v0 : 0.0;
-#pragma unroll
-                    for (int off = 16; off > 0; off >>= 1) q += __shfl_xor_sync(0xffffffffu, q, off);
-                    if ((tid & 31) == 0) atomicAdd(A.mo_norm + mo, q);
-                }
-            }
-        }
+    if (A.go && *A.go == 0) {
+        if (!MO_OUT && A.norm_part && blockIdx.x == 0)
+            for (int i = tid; i < A.nmo; i += FT) atomicAdd(A.mo_norm + i, A.norm_part[i]);
+        return;
     }
+    for (long long p0 = (long long)blockIdx.x * FP; p0 < g.npts; p0 += (long long)gridDim.x * FP) {
+        const long long p = p0 + pl;
+        const bool valid = p < g.npts;
+        double x, y, z;
+        grid_point(g, valid ? p : g.npts - 1, x, y, z);
+        constexpr unsigned chmask = (1u << NCH) - 1u;
+        constexpr int MOPASS = FG * MB;
 
-    if (!MO_OUT) {
-        // reduce the FG group partials per point, in fixed order
-        __syncthreads();
-        double* red = smem;  // FG x (1 + 10) x FP
-        red[(grp * 11 + 0) * FP + pl] = rho_part;
+        double rho_part = 0.0;
+        double drho_part[10];
 #pragma unroll
-        for (int d = 0; d < 10; ++d)
-            if (d < A.drv.n) red[(grp * 11 + 1 + d) * FP + pl] = drho_part[d];
-        __syncthreads();
-        if (grp == 0 && valid) {
-            double r = 0.0;
-            for (int q = 0; q < FG; ++q) r += red[(q * 11) * FP + pl];
-            A.out[p] = r;
-            for (int d = 0; d < A.drv.n; ++d) {
-                double t = 0.0;
-                for (int q = 0; q < FG; ++q) t += red[(q * 11 + 1 + d) * FP + pl];
-                A.dout[(long long)d * A.ld + p] = t;
+        for (int d = 0; d < 10; ++d) drho_part[d] = 0.0;
+
+        for (int mo0 = 0; mo0 < A.nmo; mo0 += MOPASS) {
+            double acc[MB][NCH];
+#pragma unroll
+            for (int m = 0; m < MB; ++m)
+#pragma unroll
+                for (int c = 0; c < NCH; ++c) acc[m][c] = 0.0;
+
+            for (int ci = 0; ci < B.nchunk; ++ci) {
+                const int4 ck = B.chunks[ci];
+                const int kc = ck.w - ck.z;
+                __syncthreads();  // previous chunk fully consumed
+                for (int i = tid; i < MOPASS * OKG_KC; i += FT) {
+                    const int m = i / OKG_KC, kk = i % OKG_KC;
+                    const int mo = mo0 + m;
+                    C_s[i] = (mo < A.nmo && kk < kc) ? A.C[(long long)mo * B.ncart + ck.z + kk] : 0.0;
+                }
+                int last_atom = -1;
+                double X = 0, Y = 0, Z = 0, rr = 0;
+                for (int s = ck.x + grp; s < ck.y; s += FG) {
+                    const Shell sh = B.shells[s];
+                    if (sh.atom != last_atom) {
+                        X = x - B.atoms[4 * sh.atom];
+                        Y = y - B.atoms[4 * sh.atom + 1];
+                        Z = z - B.atoms[4 * sh.atom + 2];
+                        rr = X * X + Y * Y + Z * Z;
+                        last_atom = sh.atom;
+                    }
+                    const Radial<double> r = radial64(B.prim, sh.prim0, sh.nprim, rr, NCH > 1, NCH > 4);
+                    const int rowbase = sh.cart0 - ck.z;
+                    shell_eval_L(sh.L, X, Y, Z, r, chmask, A.mixed_ref != 0, [&](int ch, int j, double v) {
+                        const int row = B.comp_row[sh.comp0 + j];
+                        if (row < 0) return;
+                        AO_s[(ch * OKG_KC + rowbase + row) * FP + pl] = v * B.comp_g[sh.comp0 + j];
+                    });
+                }
+                __syncthreads();
+                const double* Cg = C_s + grp * MB * OKG_KC;
+                for (int kk = 0; kk < kc; ++kk) {
+                    double a[NCH];
+#pragma unroll
+                    for (int c = 0; c < NCH; ++c) a[c] = AO_s[(c * OKG_KC + kk) * FP + pl];
+#pragma unroll
+                    for (int m = 0; m < MB; ++m) {
+                        const double cm = Cg[m * OKG_KC + kk];
+#pragma unroll
+                        for (int c = 0; c < NCH; ++c) acc[m][c] = fma(cm, a[c], acc[m][c]);
+                    }
+                }
+            }
+
+            // epilogue of this MO pass
+#pragma unroll
+            for (int m = 0; m < MB; ++m) {
+                const int mo = mo0 + grp * MB + m;
+                if (mo >= A.nmo) break;
+                if (MO_OUT) {
+                    if (valid)
+                        for (int d = 0; d < A.drv.n; ++d)
+                            A.out[((long long)d * A.nmo + mo) * A.ld + p] = pick<NCH>(acc[m], A.drv.code[d]);
+                } else {
+                    const double o = A.occ[mo];
+                    const double v0 = acc[m][0];
+                    rho_part += o * (v0 * v0);
+                    const double o2 = o * 2;
+#pragma unroll
+                    for (int d = 0; d < 10; ++d) {
+                        if (d >= A.drv.n) break;
+                        const int code = A.drv.code[d];
+                        double t = (o2 * pick<NCH>(acc[m], code)) * v0;
+                        if (code >= 4) {
+                            int ca, cb;
+                            second_pair(code, ca, cb);
+                            t += o2 * (pick<NCH>(acc[m], ca) * pick<NCH>(acc[m], cb));
+                        }
+                        drho_part[d] += t;
+                    }
+                    if (A.mo_norm) {
+                        double q = valid ? v0 * v0 : 0.0;
+#pragma unroll
+                        for (int off = 16; off > 0; off >>= 1) q += __shfl_xor_sync(0xffffffffu, q, off);
+                        if ((tid & 31) == 0) atomicAdd(A.mo_norm + mo, q);
+                    }
+                }
+            }
+        }
+
+        if (!MO_OUT) {
+            // reduce the FG group partials per point, in fixed order
+            __syncthreads();
+            double* red = smem;  // FG x (1 + 10) x FP
+            red[(grp * 11 + 0) * FP + pl] = rho_part;
+#pragma unroll
+            for (int d = 0; d < 10; ++d)
+                if (d < A.drv.n) red[(grp * 11 + 1 + d) * FP + pl] = drho_part[d];
+            __syncthreads();
+            if (grp == 0 && valid) {
+                double r = 0.0;
+                for (int q = 0; q < FG; ++q) r += red[(q * 11) * FP + pl];
+                A.out[p] = r;
+                for (int d = 0; d < A.drv.n; ++d) {
+                    double t = 0.0;
+                    for (int q = 0; q < FG; ++q) t += red[(q * 11 + 1 + d) * FP + pl];
+                    A.dout[(long long)d * A.ld + p] = t;
+                }
             }
         }
     }
 }
+
+// Blocks of a launch that rarely has anything to do: one resident set (the empty launch of a
+// block per 64 points would take 1 us per 300 of them).
+constexpr long long GO_BLOCKS = 304;
 
 template <int NCH, int MB, bool MO_OUT, int FPx = FP, int FGx = FG>
 static int launch_fused(const okg_basis* b, const Grid& g, const FusedArgs& A, cudaStream_t st)
@@ -207,7 +222,8 @@ static int launch_fused(const okg_basis* b, const Grid& g, const FusedArgs& A, c
         if (e != cudaSuccess) return cuda_status(e, "fused64: smem attribute");
         configured = true;
     }
-    const long long nblk = (g.npts + FPx - 1) / FPx;
+    long long nblk = (g.npts + FPx - 1) / FPx;
+    if (A.go && nblk > GO_BLOCKS) nblk = GO_BLOCKS;
     fused64_kernel<NCH, MB, MO_OUT, FPx, FGx><<<(unsigned)nblk, FPx * FGx, smem, st>>>(b->dev, g, A);
     return cuda_status(cudaGetLastError(), "fused64 launch");
 }
@@ -236,6 +252,12 @@ static int dispatch_fused(const okg_basis* b, const Grid& g, const FusedArgs& A,
     return launch_fused<10, 4, MO_OUT>(b, g, A, st);
 }
 
+template <typename F>
+static SplitGeneral general_call(const F& f)
+{
+    return SplitGeneral{[](const void* self, const int* go, const double* norm) { return (*(const F*)self)(go, norm); }, &f};
+}
+
 }  // namespace okg
 
 using namespace okg;
@@ -259,8 +281,13 @@ extern "C" int okg_eval_mo(const okg_basis* b, const okg_grid* grid, int nmo, co
     A.ld = ld;
     bool done = false;
     const SplitCall sc{nmo, d_coeff, nullptr, A.drv, mask | 1u, true, d_out, nullptr, nullptr, ld};
-    if ((st = split_run(b, g, sc, (cudaStream_t)stream, done)) || done) return st;
-    return dispatch_fused<true>(b, g, A, mask | 1u, (cudaStream_t)stream);
+    const auto general = [&](const int* go, const double*) {
+        FusedArgs F = A;
+        F.go = go;
+        return dispatch_fused<true>(b, g, F, mask | 1u, (cudaStream_t)stream);
+    };
+    if ((st = split_run(b, g, sc, general_call(general), (cudaStream_t)stream, done)) || done) return st;
+    return general(nullptr, nullptr);
 }
 
 extern "C" int okg_rho(const okg_basis* b, const okg_grid* grid, int nmo, const double* d_coeff, const double* d_occ,
@@ -297,8 +324,14 @@ extern "C" int okg_rho(const okg_basis* b, const okg_grid* grid, int nmo, const 
     A.ld = ld;
     bool done = false;
     const SplitCall sc{nmo, d_coeff, d_occ, A.drv, need, false, d_rho, d_drho, d_mo_norm, ld};
-    if ((st = split_run(b, g, sc, (cudaStream_t)stream, done)) || done) return st;
-    // (the MO-norm sums reduce over warps of one MO group: 64-point CTAs only)
-    if (g.npts <= FEW_MAX_POINTS && !A.mo_norm) return dispatch_few(b, g, A, need, (cudaStream_t)stream);
-    return dispatch_fused<false>(b, g, A, need, (cudaStream_t)stream);
+    const auto general = [&](const int* go, const double* norm_part) {
+        FusedArgs F = A;
+        F.go = go;
+        F.norm_part = norm_part;
+        // (the MO-norm sums reduce over warps of one MO group: 64-point CTAs only)
+        if (g.npts <= FEW_MAX_POINTS && !A.mo_norm) return dispatch_few(b, g, F, need, (cudaStream_t)stream);
+        return dispatch_fused<false>(b, g, F, need, (cudaStream_t)stream);
+    };
+    if ((st = split_run(b, g, sc, general_call(general), (cudaStream_t)stream, done)) || done) return st;
+    return general(nullptr, nullptr);
 }

@@ -349,14 +349,24 @@ struct SplitCall {
     const double* g_grad = nullptr;
     long long g_ld = 0;
     bool wv_float = false;  // W and V as floats
+    // (the cotangents' caller) device word raised instead of running the DFMA kernel after it
+    int* redo = nullptr;
 };
-// Runs the call on the tensor cores if it is one for them (done = true), else leaves it.
-int split_run(const okg_basis* b, const Grid& g, const SplitCall& c, cudaStream_t st, bool& done);
+// The call by the DFMA kernel, run if *go is not zero, else norm_part (or null) added to the
+// MO norms.
+struct SplitGeneral {
+    int (*run)(const void* self, const int* go, const double* norm_part);
+    const void* self;
+};
+// Runs the call on the tensor cores if it is one for them (done = true), else leaves it.  What
+// turns out on the device to be out of their range is computed by `general` after them.
+int split_run(const okg_basis* b, const Grid& g, const SplitCall& c, const SplitGeneral& general, cudaStream_t st, bool& done);
 
 // Adjoint through the tensor cores (okg_adjoint_split.cu): workspace, and the call (done =
-// false: not one for it, nothing was written to the outputs).
+// false: not one for it, nothing was written to the outputs).  *redo (device): zero after the
+// call, or the outputs are not valid (a value out of the digits' range).
 size_t adjoint_split_bytes(const okg_basis* b, long long npts, int nmo, int precision);
 int adjoint_split_run(const okg_basis* b, const Grid& g, int nmo, const double* C, const double* occ, const double* grho,
                       const double* ggrad, long long ld, int precision, double* dC, double* dprim, double* dgeo, void* work,
-                      cudaStream_t st, bool& done);
+                      int* redo, cudaStream_t st, bool& done);
 }  // namespace okg

@@ -23,6 +23,10 @@
 // cannot change a digit and is left out, and so are panels of 16 columns without a kept
 // shell.  Bounds are taken per channel class (values, first, second derivatives).
 //
+// Range.  What the digits cannot hold (a basis whose flags are raised, see split_prim; MOs
+// whose largest coefficient is not finite or not between 2^-900 and 2^1000; points at
+// |coordinate| >= 2^170; AO values from 2^985 on) raises the call's redo word, and the DFMA kernel, launched after this one, computes the call.
+//
 // Tile: 128 operand rows (2 x 128 with second derivatives): 128 points x 1 channel, or
 // 32 points x (value, d/dx, d/dy, d/dz) [+ 32 x (xx, yy, zz, unused)].  Persistent CTAs,
 // one per SM, tiles handed out by a device counter; warps of a CTA:
@@ -64,6 +68,9 @@ constexpr int SMEM_MAX = 232448;
 enum { OUT_RHO = 0, OUT_MO = 1, OUT_WV = 2 };
 constexpr float KEEP_LOG2 = 62.0f;
 constexpr float ABS_FLOOR = -1000.0f;   // values below 2^-1000 are dropped
+// e^(-alpha d^2) w below 2^-3000 is nothing whatever the polynomial (below 2^192 for points and
+// atoms within 2^31 of each other), which may leave the range of a float there
+constexpr float NOTHING = -3000.0f;
 // Up to which sqrt(alpha) times the error of a coordinate single precision places a tile's
 // points.  With an error x per coordinate log2 e^(-alpha d^2) errs by
 // 1.443 alpha (2 sqrt(3) d x + 3 x^2); where alpha d^2 <= 735 (beyond ABS_FLOOR nothing counts)
@@ -99,6 +106,7 @@ struct Args {
     const double* occ;            // [npass np] occupations, zero padded
     unsigned long long* counter;  // tile counter, zero at launch
     double* phi;                  // per CTA [RG][np][128] partial MO values (bases beyond GROUP panels)
+    int* redo;                    // raised when the call is not one for the digits after all
     int* status;                  // raised when a wait expires
     DrvList drv;
     double* out;                  // MO output: ndrv x nmo x ld; density: rho; cotangents: W, V (2 x nmo x ld)
@@ -200,8 +208,6 @@ __device__ __forceinline__ bool warp_wait(const State& S, uint32_t bar, uint32_t
 }
 
 // ------------------------------------------------------------------ FP64 AO values
-__device__ __noinline__ double slow_exp(double x) { return exp(x); }
-
 // position of x^a y^b z^c among the monomials of its degree
 __host__ __device__ constexpr int midx(int a, int b, int c) { return (b + c) * (b + c + 1) / 2 + c; }
 
@@ -342,8 +348,7 @@ __device__ __forceinline__ void gen_shell(const Args& A, const State& S, uint32_
         const SplitPrim* pr = A.S.prim + prim0 + q;
         const ulonglong2 ae = __ldg((const ulonglong2*)pr);
         const double2 w01 = __ldg((const double2*)pr + 1);
-        double e = exp_neg(mr, er, ae.x, (int)(ae.y >> 32), S.tab);
-        if ((int)ae.y) e = slow_exp(__ldg(&pr->neg_alpha) * rr);  // alpha <= 0
+        const double e = exp_neg(mr, er, ae.x, (int)ae.y, S.tab);
         R0 = fma(w01.x, e, R0);
         if (NCH >= 4) S1 = fma(w01.y, e, S1);
         if (NCH == 7) S2 = fma(__ldg(&pr->w2), e, S2);
@@ -649,10 +654,8 @@ __device__ __forceinline__ void epi_role(const Args& A, const State& S)
                             }
                         } else {
                             // no shell reaches this tile: zeros (or NaN where the input has it)
-                            const int f[2] = {f2.x, f2.y};
 #pragma unroll
-                            for (int i = 0; i < 2; ++i)
-                                v[i] = u[i] = (rx0 == ROW_NAN || f[i] == MO_NAN) ? __longlong_as_double(0x7FF8000000000000ll) : 0.0;
+                            for (int i = 0; i < 2; ++i) v[i] = u[i] = rx0 == ROW_NAN ? __longlong_as_double(0x7FF8000000000000ll) : 0.0;
                         }
                         if (!last) continue;
                         if (MODE == OUT_WV) {
@@ -840,13 +843,13 @@ __device__ __forceinline__ void point_bounds(const float4* __restrict__ pl, int 
         for (int q = 0; q < NQ; ++q) {
             const float e = exp2f(fmaf(-v.x, dd[q], v.y) - m[q]);
             R0[q] += e;
-            if (NCLS > 1) R1[q] = fmaf(fabsf(v.z), e, R1[q]);
+            if (NCLS > 1) R1[q] = fmaf(v.z, e, R1[q]);
             if (NCLS > 2) R2[q] = fmaf(v.z * v.z, e, R2[q]);
         }
     }
 #pragma unroll
     for (int q = 0; q < NQ; ++q) {
-        if (m[q] < -1.0e30f) continue;
+        if (m[q] < NOTHING) continue;
         const Poly f = poly(L, sqrtf(dd[q]) + 2.f * err, dq[q] + err);
         top[q][0] = fmaxf(top[q][0], m[q] + __log2f(f.p0 * R0[q]));
         if (NCLS > 1) top[q][1] = fmaxf(top[q][1], m[q] + __log2f(f.p1 * R0[q] + 2.f * f.q1 * R1[q]));
@@ -856,17 +859,22 @@ __device__ __forceinline__ void point_bounds(const float4* __restrict__ pl, int 
     }
 }
 
-// A point that is set apart: non-finite, or |coordinate| >= 2^60; else 0.
+// A point that is set apart: NaN where a coordinate is NaN, 0 at |coordinate| >= 2^30 (every AO
+// is exactly 0 there, see split_prim; from 2^170 on a polynomial may overflow and 0 times it is
+// not 0: ROW_OUT); else 0.
+constexpr int ROW_OUT = 30002;
 __device__ __forceinline__ int special_point(double x, double y, double z)
 {
+    if (x != x || y != y || z != z) return ROW_NAN;
     const int h = max(__double2hiint(x) & 0x7FFFFFFF, max(__double2hiint(y) & 0x7FFFFFFF, __double2hiint(z) & 0x7FFFFFFF));
-    return h >= 0x7FF00000 ? ROW_NAN : h >= 0x43B00000 ? ROW_ZERO : 0;
+    return h >= 0x4A900000 ? ROW_OUT : h >= 0x41D00000 ? ROW_ZERO : 0;
 }
 // Row exponent of a point with the bound `top` (log2): 0.1 for the roundings of the bound, 0.05 for
 // those of the coordinates.
-__device__ __forceinline__ int row_scale(int special, float top)
+__device__ __forceinline__ int row_scale(int special, float top, int* redo)
 {
-    return special ? special : top > 985.f ? ROW_NAN : (int)ceilf(fminf(fmaxf(top + 0.15f, -950.f), 990.f));
+    if (special == ROW_OUT || (!special && !(top <= 985.f))) *(volatile int*)redo = 1;
+    return special ? special : (int)ceilf(fminf(fmaxf(top + 0.15f, -950.f), 990.f));
 }
 
 // The points' scales of a tile beyond WIDE, with FP64 differences to the atoms: every kept shell,
@@ -892,7 +900,7 @@ __device__ __noinline__ void wide_scales(const Args& A, long long t, const unsig
             const float dd[1] = {fmaf(dx, dx, fmaf(dy, dy, dz * dz))}, dq[1] = {fmaxf(fabsf(dx), fmaxf(fabsf(dy), fabsf(dz)))};
             point_bounds<NCLS>(A.S.prim_lg + rec.z, nkeep[s], rec.y & 0xFF, dd, dq, 0.f, top);
         }
-        for (int c = 0; c < NCLS; ++c) rowexp[c * 128 + q * 32 + lane] = (short)row_scale(special_point(x, y, z), top[0][c]);
+        for (int c = 0; c < NCLS; ++c) rowexp[c * 128 + q * 32 + lane] = (short)row_scale(special_point(x, y, z), top[0][c], A.redo);
     }
 }
 
@@ -921,8 +929,7 @@ __device__ __forceinline__ void tile_role(const Args& A, const State& S, int tw)
             if (lane == 0) mbar_arrive(S.screened + 8 * b);
             return;
         }
-        // points relative to one of them, in single precision (see WIDE); points at
-        // |coordinate| >= 2^60 or non-finite are set apart
+        // points relative to one of them, in single precision (see WIDE), some set apart
         float fx[NQ], fy[NQ], fz[NQ];
         int special[NQ];
         double ox = 0.0, oy = 0.0, oz = 0.0;
@@ -986,9 +993,8 @@ __device__ __forceinline__ void tile_role(const Args& A, const State& S, int tw)
         __syncwarp();
         unsigned char* nkeep = S.nkeep + b * MAX_SHELLS;
         int npan = 0, nbig = 0;
-        const bool bad = __ldg(A.S.flags) != 0;  // a parameter or position that is not a number
         float ref[3] = {-3.0e38f, -3.0e38f, -3.0e38f};
-        if (have && !bad) {
+        if (have) {
             // what the scale of every point of the tile is known to reach: the largest
             // lower bound of a shell over the tile's box (one primitive's share of it)
             for (int s = lane; s < nshell; s += 32) {
@@ -998,7 +1004,7 @@ __device__ __forceinline__ void tile_role(const Args& A, const State& S, int tw)
                 float m = -3.0e38f, al = 0.f;
                 for (int q = 0; q < np; ++q) {
                     const float4 v = __ldg(A.S.prim_lg + rec.z + q);
-                    const float l = v.y - fmaxf(v.x * br.dmin, v.x * br.dmax);
+                    const float l = v.y - v.x * br.dmax;
                     al = l > m ? v.z : al;
                     m = fmaxf(m, l);
                 }
@@ -1008,7 +1014,7 @@ __device__ __forceinline__ void tile_role(const Args& A, const State& S, int tw)
                 u[1] = m + __log2f(f.p1 + 2.f * al * f.q1);
                 u[2] = m + __log2f(f.p2 + al * (2.f * (2 * L + 1) * f.p0 + 4.f * al * f.q2));
 #pragma unroll
-                for (int c = 0; c < NCLS; ++c) ref[c] = fmaxf(ref[c], u[c]);
+                for (int c = 0; c < NCLS; ++c) ref[c] = m < NOTHING ? ref[c] : fmaxf(ref[c], u[c]);
             }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1)
@@ -1027,7 +1033,8 @@ __device__ __forceinline__ void tile_role(const Args& A, const State& S, int tw)
                     const float lnp = __log2f((float)np), l0 = __log2f(f.p0);
                     for (int q = 0; q < np; ++q) {
                         const float4 v = __ldg(A.S.prim_lg + rec.z + q);
-                        const float e = v.y - fminf(v.x * br.dmin, v.x * br.dmax), a = fabsf(v.z);
+                        const float e = v.y - v.x * br.dmin, a = v.z;
+                        if (e < NOTHING) continue;
                         float u[3];
                         u[0] = e + l0;
                         u[1] = e + __log2f(f.p1 + 2.f * a * f.q1);
@@ -1092,7 +1099,7 @@ __device__ __forceinline__ void tile_role(const Args& A, const State& S, int tw)
         for (int q = 0; q < NQ; ++q)
 #pragma unroll
             for (int c = 0; c < NCLS; ++c)
-                if (q < nsub) rowexp[c * 128 + q * 32 + lane] = (short)(bad ? ROW_NAN : row_scale(special[q], top[q][c]));
+                if (q < nsub) rowexp[c * 128 + q * 32 + lane] = (short)row_scale(special[q], top[q][c], A.redo);
         if (lane == 0) S.npan[b] = npan;
         __syncwarp();
         if (lane == 0) mbar_arrive(S.screened + 8 * b);
@@ -1107,6 +1114,12 @@ __global__ void __launch_bounds__(Cfg<NCH>::NT, 1) split_kernel(const __grid_con
     constexpr int NT = C::NT, NGW = C::NGW, NEW = C::NEW;
     extern __shared__ unsigned char raw[];
     const int tid = threadIdx.x, warp = tid >> 5;
+    bool out = __ldg(A.S.flags) != 0;
+    for (int i = tid; i < A.npass * A.np; i += NT) out |= __ldg(A.fexp + i) == MO_NAN;
+    if (__syncthreads_or(out)) {
+        if (tid == 0) *(volatile int*)A.redo = 1;
+        return;
+    }
     unsigned char* base = (unsigned char*)(((uintptr_t)raw + 1023) & ~(uintptr_t)1023);
     State S;
     S.a_bytes = C::RG * ND * DT;
@@ -1227,11 +1240,13 @@ __global__ void __launch_bounds__(Cfg<NCH>::NT, 1) split_kernel(const __grid_con
 }
 
 // Digits of the MO coefficients times the column norms and scales, one block per MO
-// column of the operand; block 0 also zeroes the tile counter.
+// column of the operand, which also zeroes its sum of MO^2 (if there are such); block 0 zeroes
+// the tile counter and the redo word.
 __global__ void __launch_bounds__(256) split_pack_kernel(SplitDev S, int nmo, int np, int ncart,
                                                          const double* __restrict__ C, const double* __restrict__ occ,
                                                          unsigned char* __restrict__ bpack, int* __restrict__ fexp,
-                                                         double* __restrict__ occ_pad, unsigned long long* counter)
+                                                         double* __restrict__ occ_pad, unsigned long long* counter,
+                                                         int* redo, double* norm)
 {
     __shared__ unsigned long long top;
     const int mo = blockIdx.x, pass = mo / np, n = mo % np, ncol = S.npanel * PK;
@@ -1252,11 +1267,16 @@ __global__ void __launch_bounds__(256) split_pack_kernel(SplitDev S, int nmo, in
     __syncthreads();
     const int ex = (int)(top >> 52);
     const int F = scale_of(top);
-    const bool nan = ex == 0x7FF;
+    // (coefficients from 2^1000 on may overflow in a sum, MOs below 2^-900 lose digits)
+    const bool nan = ex >= 2023 || (ex < 123 && top != 0);
     if (threadIdx.x == 0) {
         fexp[mo] = nan ? MO_NAN : F;
         occ_pad[mo] = (mo < nmo && occ) ? occ[mo] : 0.0;
-        if (mo == 0) *counter = 0ull;
+        if (norm) norm[mo] = 0.0;
+        if (mo == 0) {
+            *counter = 0ull;
+            *redo = 0;
+        }
     }
     for (int i = threadIdx.x; i < ncol; i += blockDim.x) {
         const uint64_t t = nan ? 0x0080808080808080ull : digits7(value(i), F + 1030);
@@ -1406,7 +1426,7 @@ int launch(sp::Args& A, int nblk, size_t smem, cudaStream_t st)
 }
 
 template <int NCH>
-int run(const okg_basis* b, const Grid& g, const SplitCall& c, cudaStream_t st, bool& done)
+int run(const okg_basis* b, const Grid& g, const SplitCall& c, const SplitGeneral& general, cudaStream_t st, bool& done)
 {
     using C = sp::Cfg<NCH>;
     const int npmax = C::RG == 1 ? 64 : 32;  // 7 accumulators per MO and row tile in 512 TMEM columns
@@ -1420,7 +1440,6 @@ int run(const okg_basis* b, const Grid& g, const SplitCall& c, cudaStream_t st, 
     A.drv = c.drv;
     A.out = c.out;
     A.dout = c.dout;
-    A.mo_norm = c.mo_norm;
     A.g_rho = c.g_rho;
     A.g_grad = c.g_grad;
     A.g_ld = c.g_ld;
@@ -1464,7 +1483,8 @@ int run(const okg_basis* b, const Grid& g, const SplitCall& c, cudaStream_t st, 
     A.status = status;
     const int nrow = A.npass * A.np;
     auto up = [](size_t v) { return (v + 255) & ~(size_t)255; };
-    const size_t o_fexp = 256, o_occ = o_fexp + up(4 * (size_t)nrow), o_b = o_occ + up(8 * (size_t)nrow),
+    const size_t o_fexp = 256, o_occ = o_fexp + up(4 * (size_t)nrow), o_norm = o_occ + up(8 * (size_t)nrow),
+                 o_b = o_norm + (c.mo_norm ? up(8 * (size_t)nrow) : 0),
                  o_phi = o_b + up((size_t)nrow * b->split.npanel * sp::ND * sp::PK * 2),
                  bytes = o_phi + (b->split.npanel > sp::GROUP ? (size_t)nblk * C::RG * A.np * 128 * 8 : 0);
     char* ws = nullptr;
@@ -1473,12 +1493,14 @@ int run(const okg_basis* b, const Grid& g, const SplitCall& c, cudaStream_t st, 
         return OKG_OK;  // no room for the digits: the caller's other path needs none
     }
     A.counter = (unsigned long long*)ws;
+    A.redo = c.redo ? c.redo : (int*)(ws + 8);
+    A.mo_norm = c.mo_norm ? (double*)(ws + o_norm) : nullptr;
     A.fexp = (const int*)(ws + o_fexp);
     A.occ = (const double*)(ws + o_occ);
     A.bpack = (const unsigned char*)(ws + o_b);
     A.phi = b->split.npanel > sp::GROUP ? (double*)(ws + o_phi) : nullptr;
     sp::split_pack_kernel<<<nrow, 256, 0, st>>>(b->split, c.nmo, A.np, b->ncart, c.C, c.occ, (unsigned char*)(ws + o_b),
-                                                (int*)(ws + o_fexp), (double*)(ws + o_occ), A.counter);
+                                                (int*)(ws + o_fexp), (double*)(ws + o_occ), A.counter, (int*)(ws + 8), A.mo_norm);
     int s = cuda_status(cudaGetLastError(), "FP64 tensor-core path: coefficient digits");
     const size_t smem = fixed + A.nslot * slot;
     if (!s) {
@@ -1486,6 +1508,7 @@ int run(const okg_basis* b, const Grid& g, const SplitCall& c, cudaStream_t st, 
             if constexpr (NCH == 4) s = launch<NCH, sp::OUT_WV>(A, nblk, smem, st);
         } else {
             s = c.mo_out ? launch<NCH, sp::OUT_MO>(A, nblk, smem, st) : launch<NCH, sp::OUT_RHO>(A, nblk, smem, st);
+            if (!s) s = general.run(general.self, A.redo, A.mo_norm);
         }
     }
     const cudaError_t e = cudaFreeAsync(ws, st);
@@ -1495,7 +1518,7 @@ int run(const okg_basis* b, const Grid& g, const SplitCall& c, cudaStream_t st, 
 }
 }  // namespace
 
-int split_run(const okg_basis* b, const Grid& g, const SplitCall& c, cudaStream_t st, bool& done)
+int split_run(const okg_basis* b, const Grid& g, const SplitCall& c, const SplitGeneral& general, cudaStream_t st, bool& done)
 {
     done = false;
     if (c.need & ~0x7Fu) return OKG_OK;  // mixed second derivatives
@@ -1515,9 +1538,9 @@ int split_run(const okg_basis* b, const Grid& g, const SplitCall& c, cudaStream_
         (void)cudaGetLastError();
         return OKG_OK;  // (a captured call keeps to the kernel without a workspace)
     }
-    if ((c.need & ~1u) == 0) return run<1>(b, g, c, st, done);
-    if ((c.need & ~0xFu) == 0) return run<4>(b, g, c, st, done);
-    return run<7>(b, g, c, st, done);
+    if ((c.need & ~1u) == 0) return run<1>(b, g, c, general, st, done);
+    if ((c.need & ~0xFu) == 0) return run<4>(b, g, c, general, st, done);
+    return run<7>(b, g, c, general, st, done);
 }
 }  // namespace okg
 

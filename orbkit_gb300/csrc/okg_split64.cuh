@@ -13,8 +13,7 @@ namespace okg {
 // A primitive for the radial sums: alpha log2(e) = A 2^ea, w, -2 alpha w, 4 alpha^2 w.
 struct alignas(16) SplitPrim {
     uint64_t A;
-    int special;  // alpha <= 0 or subnormal: the exponential is taken in FP64
-    int ea;
+    int ea, unused;
     double w, w1, w2, neg_alpha;
 };
 
@@ -27,21 +26,22 @@ struct SplitDev {
     const SplitPrim* prim;  // nprim, ascending alpha per shell
     const int* prim_place;  // nprim: place of each sorted primitive in the caller's order
     const uint64_t* exp_tab;  // 2^(63 - j / 2048), rounded
-    const int* flags;       // non-zero: a parameter or position is not a number
+    const int* flags;       // non-zero: a parameter or position out of the tables' range
     int npanel;
 };
 
-// One primitive (alpha, w) as the FP64 tensor-core path's bounds and radial sums read it;
-// false if a parameter is not a number (an exponent of +infinity drops its primitive).
+// One primitive (alpha, w) as the FP64 tensor-core path's bounds and radial sums read it; false
+// if it is out of their range, 1e-9 <= alpha <= 1e37 and finite w (such a basis takes the DFMA
+// kernels).  With |positions| < 2^29 and alpha >= 1e-9 every AO is exactly zero at
+// |coordinate| >= 2^30; above 1e37 alpha log2(e) leaves the range of a float.
 __device__ __forceinline__ bool split_prim(double2 p, float4& lg, SplitPrim& o)
 {
-    const bool inf = p.x > 1.0e300;
     // log2 |w| from exponent field and mantissa (|w| beyond the range of a float keeps its size)
     const long long wb = __double_as_longlong(p.y);
     const int we = (int)((wb >> 52) & 0x7FF);
     const float lw = we == 0 ? -3.0e38f
                              : (float)(we - 1023) + log2f((float)__longlong_as_double((wb & 0xFFFFFFFFFFFFFll) | 0x3FF0000000000000ll));
-    lg = inf ? make_float4(0.f, -3.0e38f, 0.f, 0.f) : make_float4((float)(p.x * 1.4426950408889634), lw, (float)p.x, 0.f);
+    lg = make_float4((float)(p.x * 1.4426950408889634), lw, (float)p.x, 0.f);
     // alpha log2(e) = A 2^ea with a 64-bit mantissa
     const long long bits = __double_as_longlong(p.x);
     const int ex = (int)((bits >> 52) & 0x7FF);
@@ -54,12 +54,12 @@ __device__ __forceinline__ bool split_prim(double2 p, float4& lg, SplitPrim& o)
         --o.ea;
     }
     o.A = h;
-    o.special = !(p.x > 0.0) || ex == 0;
-    o.w = inf ? 0.0 : p.y;
-    o.w1 = inf ? 0.0 : -2.0 * p.x * p.y;
-    o.w2 = inf ? 0.0 : 4.0 * p.x * p.x * p.y;
+    o.unused = 0;
+    o.w = p.y;
+    o.w1 = -2.0 * p.x * p.y;
+    o.w2 = 4.0 * p.x * p.x * p.y;
     o.neg_alpha = -p.x;
-    return inf || (isfinite(p.x) && isfinite(p.y));
+    return p.x >= 1.0e-9 && p.x <= 1.0e37 && isfinite(p.y);
 }
 // e^(-alpha rr) as an FP64 value in integer arithmetic (the FP64 pipe bounds the
 // kernels that use it, and an FP64 exponential takes 9 to 18 of its operations, this one
