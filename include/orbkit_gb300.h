@@ -136,12 +136,15 @@ int okg_rho(const okg_basis* basis, const okg_grid* grid, int nmo, const double*
 int okg_fold_coeff(const okg_basis* basis, int nmo, const double* d_csph, double* d_ccart, okg_stream stream);
 int okg_unfold_coeff(const okg_basis* basis, int nmo, const double* d_ccart, double* d_csph, okg_stream stream);
 
-/* Whether a device wait of an okg_rho, okg_eval_mo, okg_rho_backward or okg_ci_*_matrix
- * call expired (OKG_ERR_TIMEOUT; the outputs of that call are then incomplete) since the
- * last query; clears the record.  The device writes it during the call: query it after
- * waiting for the call's stream.  Large calls run on the tensor cores with waits between
- * the warps of a block, each bounded. */
+/* Large okg_rho, okg_eval_mo, okg_rho_backward and okg_ci_*_matrix calls run on the tensor
+ * cores with bounded waits between the warps of a block.  Where a wait expires the call's
+ * general kernel computes the outputs on the device behind it, so that they are complete
+ * in any case: okg_wait_status reports OKG_OK and 0, and need not be called.
+ * okg_set_wait_limit sets the polls per wait (default 2^24, >= 0) in the calls that the
+ * calling host thread makes from then on; one poll, or none, makes waits expire on purpose,
+ * which is how that path is tested. */
 int okg_wait_status(int* status);
+int okg_set_wait_limit(long long polls);
 
 /* ------------------------------------------------ operations on given grids
  * FP64 operations on AO / MO values the caller already holds on the device, every

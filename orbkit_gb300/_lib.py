@@ -52,6 +52,7 @@ SIGNATURES = {
     "okg_fold_coeff": (ctypes.c_int, [_vp, ctypes.c_int, _vp, _vp, _vp]),
     "okg_unfold_coeff": (ctypes.c_int, [_vp, ctypes.c_int, _vp, _vp, _vp]),
     "okg_wait_status": (ctypes.c_int, [_c_int_p]),
+    "okg_set_wait_limit": (ctypes.c_int, [ctypes.c_longlong]),
     "okg_mixed_plan_create": (ctypes.c_int, [_vp, ctypes.c_int, ctypes.POINTER(_vp)]),
     "okg_mixed_plan_destroy": (ctypes.c_int, [_vp]),
     "okg_mixed_set_coeffs": (ctypes.c_int, [_vp, _vp, _vp, _vp]),

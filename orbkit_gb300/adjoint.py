@@ -81,7 +81,6 @@ class DensityModel:
 
     def _forward(self, C):
         import torch
-        _lib.check(self._L.okg_wait_status(None))  # (of the calls before this one: no synchronisation)
         Ceff = self.basis.c_eff(C.detach())
         rho = torch.empty(self.npts, dtype=torch.float64, device=self.device)
         grad = torch.empty((3, self.npts), dtype=torch.float64, device=self.device)
@@ -101,7 +100,6 @@ class DensityModel:
 
     def _backward(self, C, g_rho, g_grad):
         import torch
-        _lib.check(self._L.okg_wait_status(None))  # (of the calls before this one: no synchronisation)
         Ceff = self.basis.c_eff(C.detach())
         prec = 64 if self.precision == "fp64" else 32
         nbytes = ctypes.c_size_t(0)

@@ -161,10 +161,9 @@ class _Result:
             self.pinned[index].copy_(part, non_blocking=True)
 
     def finish(self):
-        """The array, complete; raises if a device wait of the evaluation expired."""
+        """The array, complete."""
         if self.pinned is not None:
             _torch().cuda.current_stream().synchronize()
-        _lib.check(_lib.load().okg_wait_status(None))
         return self.array
 
 

@@ -16,8 +16,8 @@
 //   4. dC_ik = sum_r W_i chi_k + V_i G_k: digit products with the points as the summed index,
 //      64 points per accumulation, FP64 sums of those;
 //   5. partial sums added in a fixed order.
-// What the digits cannot hold (values that are not finite, a call that step 1 gives up) raises
-// the call's redo word, and the one-kernel form, launched at the end, computes the call.
+// What the digits cannot hold (values that are not finite, a call that step 1 gives up), and a
+// wait that expires, raises the call's redo word, and the one-kernel form, launched at the end, computes the call.
 // FP32 precision: W, V, A, B, chi and G are floats, the products of steps 2 and 4 take 4
 // digits (31 bits), step 3 computes in FP32.
 //
@@ -57,7 +57,7 @@ struct Dg<double> {
     static constexpr int D = 7;
     using U = unsigned long long;
     static __device__ __forceinline__ U magnitude(double v) { return (U)__double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFull; }
-    static __device__ __forceinline__ bool special(U m) { return (m >> 52) == 0x7FF; }
+    static __device__ __forceinline__ bool special(U m) { return too_large(m); }
     static __device__ __forceinline__ int scale(U m) { return scale_of(m); }
     static __device__ __forceinline__ U shfl_max(U m, int o)
     {
@@ -86,7 +86,7 @@ struct Dg<float> {
     static constexpr int D = 4;
     using U = unsigned;
     static __device__ __forceinline__ U magnitude(float v) { return __float_as_uint(v) & 0x7FFFFFFFu; }
-    static __device__ __forceinline__ bool special(U m) { return (m >> 23) == 0xFF; }
+    static __device__ __forceinline__ bool special(U m) { return (m >> 23) >= 0xF8; }
     static __device__ __forceinline__ int scale(U m)
     {
         const int ex = (int)(m >> 23);
@@ -187,8 +187,8 @@ struct ColArgs {
     const double* C;   // nmo x ncart
     int nmo, ncart, kp;
     T* out;            // 2 x ncart x ld
-    int* status;
-    int* redo;         // raised where a value is not finite
+    int* redo;         // raised where a value is not finite or a wait expires
+    long long limit;   // polls of a wait
 };
 
 template <typename T>
@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(128 * ColCfg<T>::G, ColCfg<T>::CTAS) column_ke
             mma_commit(bar_a);
         }
         if (tile + gridDim.x < ntiles) fetch(tile + gridDim.x);
-        const bool ok = mbar_wait(bar_a, parity, A.status, WAIT_LIMIT);
+        const bool ok = mbar_wait(bar_a, parity, A.redo, A.limit);
         if (!__syncthreads_and(ok)) {
             parity ^= 1;
             break;
@@ -341,8 +341,8 @@ struct RowArgs {
     int nmo, ncart, np;
     double* part;     // nslot x ncart x nmo
     int slot0;
-    int* status;
-    int* redo;        // raised where a value is not finite
+    int* redo;        // raised where a value is not finite or a wait expires
+    long long limit;  // polls of a wait
     unsigned tm_cols;
 };
 
@@ -472,7 +472,7 @@ __global__ void __launch_bounds__(512, 1) row_kernel(const __grid_constant__ Row
                 mma_commit(bar_a);
             }
             issued = true;
-            const bool ok = mbar_wait(bar_a, parity, A.status, WAIT_LIMIT);
+            const bool ok = mbar_wait(bar_a, parity, A.redo, A.limit);
             good = __syncthreads_and(ok);
             if (!good) continue;
             tc_fence_after();
@@ -928,8 +928,7 @@ template <typename T>
 static int run(const okg_basis* b, const Grid& g, int nmo, const double* C, const double* occ, const double* grho, const double* ggrad,
                long long ld, double* dC, double* dprim, double* dgeo, char* work, const Plan& P, int* redo, cudaStream_t st, bool& done)
 {
-    int* status = split_status_word();
-    if (!status) return OKG_OK;
+    const long long limit = split_wait_limit();
     T* X = (T*)(work + P.o_x);
     T* AB = (T*)(work + P.o_ab);
     T* Y = (T*)(work + P.o_y);
@@ -965,7 +964,7 @@ static int run(const okg_basis* b, const Grid& g, int nmo, const double* C, cons
         const long long tiles = (n + 127) / 128;
         int gx = (sms * ColCfg<T>::CTAS + 2 * passes - 1) / (2 * passes);
         if (gx > tiles) gx = (int)tiles;
-        column_kernel<T><<<dim3(gx, passes, 2), 128 * ColCfg<T>::G, cs, st>>>(ColArgs<T>{n, P.run, X, C, nmo, b->ncart, kp, AB, status, redo});
+        column_kernel<T><<<dim3(gx, passes, 2), 128 * ColCfg<T>::G, cs, st>>>(ColArgs<T>{n, P.run, X, C, nmo, b->ncart, kp, AB, redo, limit});
         long long per = ((n + P.nchunk - 1) / P.nchunk + 31) / 32 * 32;
         const ShellArgs<T> sa{b->dev, b->split, gr, c.g_grad, ld, P.run, AB, Y, pp, pg, r * P.nchunk, per, redo};
         shell_kernel<T, false><<<dim3(b->nshell, P.nchunk / 4), 128, 0, st>>>(sa);
@@ -973,7 +972,7 @@ static int run(const okg_basis* b, const Grid& g, int nmo, const double* C, cons
         unsigned tm = 32;
         while ((int)tm < Dg<T>::D * np) tm *= 2;
         row_kernel<T><<<dim3(P.nbx, (b->ncart + 127) / 128), 512, rs, st>>>(
-            RowArgs<T>{n, P.run, X, Y, nmo, b->ncart, np, pc, r * P.nbx, status, redo, tm});
+            RowArgs<T>{n, P.run, X, Y, nmo, b->ncart, np, pc, r * P.nbx, redo, limit, tm});
     }
     dcoeff_kernel<<<(nmo * b->ncart + 31) / 32, dim3(32, 8), 0, st>>>(pc, P.nruns * P.nbx, nmo, b->ncart, dC);
     finish_kernel<<<(b->nprim + b->natom + 3) / 4, 128, 0, st>>>(b->dev, b->split, pp, pg, P.nruns * P.nchunk, dprim, dgeo);

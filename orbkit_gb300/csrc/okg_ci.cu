@@ -79,13 +79,10 @@ __global__ void ci_flux_kernel(long long npts, const double* __restrict__ mo, co
 #define CI_CH 16
 
 template <bool FLUX>
-__global__ void __launch_bounds__(128) ci_quad_kernel(long long npts, const double* __restrict__ mo,
-                                                      const double* __restrict__ drv, long long ld, int nmo,
-                                                      const double* __restrict__ qt, double scale,
-                                                      double* __restrict__ out)
+__device__ __forceinline__ void quad_point(long long npts, const double* __restrict__ mo, const double* __restrict__ drv,
+                                           long long ld, int nmo, const double* __restrict__ qt, double scale,
+                                           double* __restrict__ out, long long p)
 {
-    const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= npts) return;
     const long long dstride = (long long)nmo * ld;
     double acc0 = 0.0, acc1 = 0.0, acc2 = 0.0;
     for (int a0 = 0; a0 < nmo; a0 += CI_CH) {
@@ -120,12 +117,23 @@ __global__ void __launch_bounds__(128) ci_quad_kernel(long long npts, const doub
     }
 }
 
+template <bool FLUX>
+__global__ void __launch_bounds__(128) ci_quad_kernel(long long npts, const double* __restrict__ mo,
+                                                      const double* __restrict__ drv, long long ld, int nmo,
+                                                      const double* __restrict__ qt, double scale,
+                                                      double* __restrict__ out)
+{
+    const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (p < npts) quad_point<FLUX>(npts, mo, drv, ld, nmo, qt, scale, out, p);
+}
+
 // The same quadratic forms with the matrix-vector product on the tensor cores: per 128 points
 // the MO values become exact digit operands (okg_digits.cuh), t_b = sum_a Q^T[b][a] MO_a comes
 // back as FP64 values, and the FP64 pipe is left with t_b MO_b (NMO FMAs per point) or
 // t_b dMO_b (3 NMO) of the NMO^2 (+ 3 NMO).  The coefficient digits are made by every CTA for
 // itself (at most 64 x 64 values) and stay in shared memory; the MO values are read twice
-// (scale, then digits: the second time from L1).
+// (scale, then digits: the second time from L1).  Points and coefficients beyond the digits'
+// range, and what a block has left when a wait expires, are evaluated as in ci_quad_kernel.
 struct CiSplit {
     long long npts, ld;
     const double* mo;
@@ -134,9 +142,15 @@ struct CiSplit {
     int nmo, ldq, np;  // np: nmo rounded up to 16 (= ldq)
     double scale;
     double* out;
-    int* status;
+    long long limit;  // polls of a wait
     unsigned tm_cols;
 };
+
+template <bool FLUX>
+__device__ __noinline__ void direct_point(const CiSplit& A, long long p)
+{
+    quad_point<FLUX>(A.npts, A.mo, A.drv, A.ld, A.nmo, A.qt, A.scale, A.out, p);
+}
 
 constexpr int CI_SPLIT_MAX = 64;  // MOs: 7 accumulators per MO in 512 TMEM columns
 
@@ -175,6 +189,7 @@ __global__ void __launch_bounds__(128 * G, 4 / G) ci_split_kernel(const __grid_c
     uint32_t* tmem_slot = (uint32_t*)(bar + 1);
     const uint32_t bar_a = smem_u32(bar);
     // coefficient digits
+    bool direct = false;
     for (int b = warp; b < np; b += 4 * G) {
         unsigned long long m = 0;
         for (int a = lane; a < A.nmo && b < A.nmo; a += 32) {
@@ -186,12 +201,12 @@ __global__ void __launch_bounds__(128 * G, 4 / G) ci_split_kernel(const __grid_c
             const unsigned long long u = __shfl_xor_sync(0xffffffffu, m, o);
             m = u > m ? u : m;
         }
-        const bool nan = (m >> 52) == 0x7FF;
+        direct |= too_large(m) || vanishing(m);
         const int F = scale_of(m);
-        if (lane == 0) fexp[b] = nan ? MO_NAN : F;
+        if (lane == 0) fexp[b] = F;
         for (int a = lane; a < np; a += 32) {
             const double v = (a < A.nmo && b < A.nmo) ? A.qt[(long long)b * A.ldq + a] : 0.0;
-            const uint64_t t = nan ? 0x0080808080808080ull : digits7(v, F + 1030);
+            const uint64_t t = digits7(v, F + 1030);
 #pragma unroll
             for (int j = 0; j < ND; ++j)
                 *(__half*)(Bs + (a >> 4) * bpanel + b_off(j * np + b, a & 15)) = __int2half_rn((int)((t >> (8 * (6 - j))) & 0xFF) - 128);
@@ -207,14 +222,16 @@ __global__ void __launch_bounds__(128 * G, 4 / G) ci_split_kernel(const __grid_c
     }
     fence_proxy_async();
     tc_fence_before();
-    __syncthreads();
+    direct = __syncthreads_or(direct);
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     const int r = tid & 127, part4 = tid >> 7;
     const long long ntiles = (A.npts + 127) / 128, dstride = (long long)A.nmo * A.ld;
     const int h0 = part4 * KP * (16 / G), h1 = h0 + KP * (16 / G);  // this thread's MOs
     uint32_t parity = 0;
-    for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x, parity ^= 1) {
+    bool issued = false;
+    long long tile = blockIdx.x;
+    for (; !direct && tile < ntiles; tile += gridDim.x, parity ^= 1) {
         const long long p = tile * 128 + r < A.npts ? tile * 128 + r : A.npts - 1;
         unsigned long long m = 0;
 #pragma unroll 8
@@ -248,8 +265,9 @@ __global__ void __launch_bounds__(128 * G, 4 / G) ci_split_kernel(const __grid_c
                 }
             mma_commit(bar_a);
         }
-        const bool ok = mbar_wait(bar_a, parity, A.status, WAIT_LIMIT);
-        if (!__syncthreads_and(ok)) {
+        issued = true;
+        direct = __syncthreads_or(!mbar_try_for(bar_a, parity, A.limit));
+        if (direct) {
             parity ^= 1;
             break;
         }
@@ -260,7 +278,7 @@ __global__ void __launch_bounds__(128 * G, 4 / G) ci_split_kernel(const __grid_c
         const bool valid = q < A.npts;
         const long long pr = valid ? q : A.npts - 1;
         const unsigned long long mr = largest<G>(tops, row);
-        const int rowx = (mr >> 52) == 0x7FF ? ROW_NAN : scale_of(mr);
+        const int rowx = scale_of(mr);
         double acc[3] = {0.0, 0.0, 0.0};
 #pragma unroll 1
         for (int n0 = 4 * hf; n0 < A.nmo; n0 += 4 * G) {
@@ -287,7 +305,9 @@ __global__ void __launch_bounds__(128 * G, 4 / G) ci_split_kernel(const __grid_c
             for (int d = 0; d < (FLUX ? 3 : 1); ++d) part[((hf - 1) * 3 + d) * 128 + row] = acc[d];
         tc_fence_before();
         __syncthreads();
-        if (hf == 0 && valid)
+        if (hf == 0 && valid && too_large(mr))
+            direct_point<FLUX>(A, q);
+        else if (hf == 0 && valid)
             for (int d = 0; d < (FLUX ? 3 : 1); ++d) {
                 double t = acc[d];
                 for (int h = 0; h < G - 1; ++h) t += part[(h * 3 + d) * 128 + row];
@@ -295,7 +315,9 @@ __global__ void __launch_bounds__(128 * G, 4 / G) ci_split_kernel(const __grid_c
             }
     }
     // (after an expired wait: the MMAs issued last complete before the CTA leaves)
-    if (tid == 0 && blockIdx.x < ntiles) mbar_drain(bar_a, parity ^ 1);
+    if (tid == 0 && issued) mbar_drain(bar_a, parity ^ 1);
+    for (; tile < ntiles; tile += gridDim.x)
+        if (tid < 128 && tile * 128 + tid < A.npts) direct_point<FLUX>(A, tile * 128 + tid);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -309,9 +331,7 @@ static int ci_split(long long npts, const double* mo, const double* drv, long lo
 {
     done = false;
     if (nmo > CI_SPLIT_MAX) return OKG_OK;
-    int* status = split_status_word();
-    if (!status) return OKG_OK;
-    CiSplit A{npts, ld, mo, drv, qt, nmo, (nmo + 15) / 16 * 16, (nmo + 15) / 16 * 16, scale, out, status, 32};
+    CiSplit A{npts, ld, mo, drv, qt, nmo, (nmo + 15) / 16 * 16, (nmo + 15) / 16 * 16, scale, out, split_wait_limit(), 32};
     while ((int)A.tm_cols < sp::ND * A.np) A.tm_cols *= 2;
     const size_t smem = ci_split_smem(A.np);
     int dev = 0, sms = 1;

@@ -149,7 +149,6 @@ __device__ __forceinline__ void acc_values(const Acc4& a, int rowx, const int4& 
         const int t[7] = {f2i(a.r[0][i]), f2i(a.r[1][i]), f2i(a.r[2][i]), f2i(a.r[3][i]), f2i(a.r[4][i]), f2i(a.r[5][i]), f2i(a.r[6][i])};
         // a = t 2^(E - 55), c = s 2^(F - 55); leading digits weigh 2^48: products 2^(E + F - 14)
         v[i] = combine7(t, rowx + f[i] - 54);
-        if (rowx >= ROW_NAN || f[i] == MO_NAN) v[i] = (rowx == ROW_ZERO && f[i] != MO_NAN) ? 0.0 : __longlong_as_double(0x7FF8000000000000ll);
     }
 }
 
@@ -184,6 +183,11 @@ __device__ __forceinline__ void acc2_values(const Acc2& a, int rowx, const int2&
         if (rowx >= ROW_NAN) v[i] = rowx == ROW_ZERO ? 0.0 : __longlong_as_double(0x7FF8000000000000ll);
     }
 }
+
+// Magnitude bits of a largest |v| too large for sums of digit products (a partial sum may
+// overflow, or it is not finite), or (vanishing) too small for all digits.
+__device__ __forceinline__ bool too_large(unsigned long long top) { return (top >> 52) >= 2023; }
+__device__ __forceinline__ bool vanishing(unsigned long long top) { return top != 0 && (top >> 52) < 123; }
 
 // Exponent F with |v| < 0.99 2^F for the magnitude bits `top` of the largest |v| (finite).
 __device__ __forceinline__ int scale_of(unsigned long long top)

@@ -330,8 +330,8 @@ SplitLayout split_layout(const std::vector<Shell>& shells, const std::vector<int
                          const std::vector<double>& comp_g, const int* order);
 const uint64_t* split_exp_table();                   // host, OKG_SPLIT_EXP entries
 
-// Page-locked word that a kernel raises when a bounded wait expires (okg_wait_status).
-int* split_status_word();
+// Polls of the bounded device waits of a call from this host thread.
+long long split_wait_limit();
 
 struct SplitCall {
     int nmo;
@@ -364,7 +364,7 @@ int split_run(const okg_basis* b, const Grid& g, const SplitCall& c, const Split
 
 // Adjoint through the tensor cores (okg_adjoint_split.cu): workspace, and the call (done =
 // false: not one for it, nothing was written to the outputs).  *redo (device): zero after the
-// call, or the outputs are not valid (a value out of the digits' range).
+// call, or the outputs are not valid (a value out of the digits' range, an expired wait).
 size_t adjoint_split_bytes(const okg_basis* b, long long npts, int nmo, int precision);
 int adjoint_split_run(const okg_basis* b, const Grid& g, int nmo, const double* C, const double* occ, const double* grho,
                       const double* ggrad, long long ld, int precision, double* dC, double* dprim, double* dgeo, void* work,

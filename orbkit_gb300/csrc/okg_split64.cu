@@ -25,7 +25,7 @@
 //
 // Range.  What the digits cannot hold (a basis whose flags are raised, see split_prim; MOs
 // whose largest coefficient is not finite or not between 2^-900 and 2^1000; points at
-// |coordinate| >= 2^170; AO values from 2^985 on) raises the call's redo word, and the DFMA kernel, launched after this one, computes the call.
+// |coordinate| >= 2^170; AO values from 2^985 on), and a wait that expires, raises the call's redo word, and the DFMA kernel, launched after this one, computes the call.
 //
 // Tile: 128 operand rows (2 x 128 with second derivatives): 128 points x 1 channel, or
 // 32 points x (value, d/dx, d/dy, d/dz) [+ 32 x (xx, yy, zz, unused)].  Persistent CTAs,
@@ -35,7 +35,8 @@
 //   epilogue warps (8, second derivatives 4)  accumulators -> FP64 MO values (integer
 //                       arithmetic) -> outputs;
 //   1 MMA warp, 1 coefficient loader (bulk copies), 1 tile warp (screening, scales).
-// Every wait is bounded and raises the status word instead of hanging (okg_wait_status).
+// Every wait is bounded: one that expires raises the redo word, and the block drains its copies
+// and MMAs in flight and leaves.
 //
 // What bounds it (20 atoms, 180 AOs, 40 MOs, 160^3 points, density and gradient): 15.2 to
 // 16.7 ms (four runs) against 254 ms of the DFMA kernel; per 32-point tile and SM the FP64
@@ -106,8 +107,8 @@ struct Args {
     const double* occ;            // [npass np] occupations, zero padded
     unsigned long long* counter;  // tile counter, zero at launch
     double* phi;                  // per CTA [RG][np][128] partial MO values (bases beyond GROUP panels)
-    int* redo;                    // raised when the call is not one for the digits after all
-    int* status;                  // raised when a wait expires
+    int* redo;                    // raised when the call is not one for the digits after all, or a wait expires
+    long long limit;              // polls of a wait
     DrvList drv;
     double* out;                  // MO output: ndrv x nmo x ld; density: rho; cotangents: W, V (2 x nmo x ld)
     const double* g_rho;          // cotangents of rho, and of grad rho (3 x g_ld, or null)
@@ -190,21 +191,21 @@ constexpr int AUX_BYTES = TABN * 8 + NBUF * 8 + NBUF * 4 + MAX_SLOTS * 4 + 8 + N
                           NBAR * 8 + 64;
 
 // Bounded wait that also ends when another role gave up.
-__device__ __forceinline__ bool wait(const State& S, uint32_t bar, uint32_t parity, int* status)
+__device__ __forceinline__ bool wait(const Args& A, const State& S, uint32_t bar, uint32_t parity)
 {
-    for (long long it = 0; it < WAIT_LIMIT; ++it) {
+    for (long long it = 0; it < A.limit; ++it) {
         if (mbar_try(bar, parity)) return true;
         if ((it & 255) == 255 && *(volatile int*)S.abort_flag) return false;
     }
-    atomicExch(status, 1);
+    *(volatile int*)A.redo = 1;
     *(volatile int*)S.abort_flag = 1;
     return false;
 }
 
 // One answer for the warp (collective instructions follow).
-__device__ __forceinline__ bool warp_wait(const State& S, uint32_t bar, uint32_t parity, int* status)
+__device__ __forceinline__ bool warp_wait(const Args& A, const State& S, uint32_t bar, uint32_t parity)
 {
-    return __all_sync(0xffffffffu, wait(S, bar, parity, status));
+    return __all_sync(0xffffffffu, wait(A, S, bar, parity));
 }
 
 // ------------------------------------------------------------------ FP64 AO values
@@ -372,13 +373,13 @@ struct TileSeq {
     unsigned ord = 0, ended = 0;
     // next buffer, or -1 (all sequences ended, or the wait gave up)
     template <bool WARP>
-    __device__ __forceinline__ int next(const State& S, int* status, long long& tile)
+    __device__ __forceinline__ int next(const Args& A, const State& S, long long& tile)
     {
         for (;; ++ord) {
             if ((ended >> (ord % NTW)) & 1u) continue;
             const int b = ord % NBUF;
-            const bool ok = WARP ? warp_wait(S, S.screened + 8 * b, (ord / NBUF) & 1, status)
-                                 : wait(S, S.screened + 8 * b, (ord / NBUF) & 1, status);
+            const bool ok = WARP ? warp_wait(A, S, S.screened + 8 * b, (ord / NBUF) & 1)
+                                 : wait(A, S, S.screened + 8 * b, (ord / NBUF) & 1);
             if (!ok) return -1;
             tile = S.tile[b];
             if (tile >= 0) {
@@ -399,14 +400,13 @@ __device__ __forceinline__ void gen_role(const Args& A, const State& S)
 {
     using C = Cfg<NCH>;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, team = warp / C::TEAM, tw = warp % C::TEAM;
-    int* status = A.status;
     const uint32_t bytes = (uint32_t)(ND * A.np * PK * 2);
     unsigned seq = 0, turn = 0;
     TileSeq ts;
     long long tile;
     bool ok = true;
     while (ok) {
-        const int b = ts.next<true>(S, status, tile);
+        const int b = ts.next<true>(A, S, tile);
         if (b < 0) break;
         const int npan = S.npan[b];
         const unsigned short* plist = S.plist + b * MAX_PANELS;
@@ -438,7 +438,7 @@ __device__ __forceinline__ void gen_role(const Args& A, const State& S)
                     nk = nkeep[s0 + lane];
                 }
                 const unsigned kept = __ballot_sync(0xffffffffu, nk > 0);
-                if (use > 0 && !warp_wait(S, S.empty + 8 * sl, (use - 1) & 1, status)) {
+                if (use > 0 && !warp_wait(A, S, S.empty + 8 * sl, (use - 1) & 1)) {
                     ok = false;
                     break;
                 }
@@ -526,20 +526,19 @@ __device__ __forceinline__ void mma_role(const Args& A, const State& S)
 {
     if ((threadIdx.x & 31) != 0) return;
     using C = Cfg<NCH>;
-    int* status = A.status;
     const int np = A.np;
     unsigned seq = 0, job = 0;
     bool ok = true, issued = false;
     TileSeq ts;
     long long tile;
     while (ok) {
-        const int b = ts.next<false>(S, status, tile);
+        const int b = ts.next<false>(A, S, tile);
         if (b < 0) break;
         const int npan = S.npan[b], ng = ngroups(npan);
         for (int pg = 0; ok && pg < A.nsub / C::SUB * A.npass * ng; ++pg, ++job) {
             const int gr = pg % ng;
             const unsigned ab = job % (unsigned)A.nacc, ause = job / (unsigned)A.nacc;
-            if (ause > 0 && !wait(S, S.acc_empty + 8 * ab, (ause - 1) & 1, status)) {
+            if (ause > 0 && !wait(A, S, S.acc_empty + 8 * ab, (ause - 1) & 1)) {
                 ok = false;
                 break;
             }
@@ -548,8 +547,8 @@ __device__ __forceinline__ void mma_role(const Args& A, const State& S)
             const int p0 = group_begin(npan, ng, gr), p1 = group_begin(npan, ng, gr + 1);
             for (int pi = p0; pi < p1; ++pi, ++seq) {
                 const unsigned sl = seq % (unsigned)A.nslot, ph = (seq / (unsigned)A.nslot) & 1;
-                if (!wait(S, S.bfull + 8 * sl, ph, status) ||
-                    !wait(S, S.full + 8 * sl, ph, status)) {
+                if (!wait(A, S, S.bfull + 8 * sl, ph) ||
+                    !wait(A, S, S.full + 8 * sl, ph)) {
                     ok = false;
                     break;
                 }
@@ -596,14 +595,13 @@ __device__ __forceinline__ void epi_role(const Args& A, const State& S)
     const int pt = NCH == 1 ? row : row >> 2;         // point of the tile
     const int ch = NCH == 1 ? 0 : lane & 3;           // channel (of the first row tile)
     const int lane0 = NCH == 1 ? lane : lane & ~3;    // lane of the point's value
-    int* status = A.status;
     const int np = A.np;
     double* phi = A.phi ? A.phi + (size_t)blockIdx.x * C::RG * np * 128 + row : nullptr;
     unsigned job = 0, round = 0;
     TileSeq ts;
     long long tile;
     for (;;) {
-        const int b = ts.next<true>(S, status, tile);
+        const int b = ts.next<true>(A, S, tile);
         if (b < 0) return;
         const int npan = S.npan[b], ng = ngroups(npan);
         const short* rowexp = S.rowexp + b * 3 * 128;
@@ -623,7 +621,7 @@ __device__ __forceinline__ void epi_role(const Args& A, const State& S)
                     const bool last = gr + 1 >= ng;
                     uint32_t taddr = S.tmem + ab * (uint32_t)(C::RG * ND * np) + ((uint32_t)(quad * 32) << 16);
                     if (ng) {
-                        if (!warp_wait(S, S.acc_full + 8 * ab, ause & 1, status)) return;
+                        if (!warp_wait(A, S, S.acc_full + 8 * ab, ause & 1)) return;
                         tc_fence_after();
                     }
                     const int nmo = A.nmo - pass * np < np ? A.nmo - pass * np : np;  // MOs of this pass
@@ -735,12 +733,12 @@ __device__ __forceinline__ void epi_role(const Args& A, const State& S)
             if (MODE == OUT_RHO && C::EPQ > 1) {
                 // the shares of the MO sum meet in shared memory
                 if (half > 0) {
-                    if (round > 0 && !warp_wait(S, S.part_free + 8 * quad, (round - 1) & 1, status)) return;
+                    if (round > 0 && !warp_wait(A, S, S.part_free + 8 * quad, (round - 1) & 1)) return;
                     S.part[((half - 1) * 4 + quad) * 32 + lane] = acc0;
                     __syncwarp();
                     if (lane == 0) mbar_arrive(S.part_full + 8 * quad);
                 } else {
-                    if (!warp_wait(S, S.part_full + 8 * quad, round & 1, status)) return;
+                    if (!warp_wait(A, S, S.part_full + 8 * quad, round & 1)) return;
 #pragma unroll
                     for (int h = 1; h < C::EPQ; ++h) acc0 += S.part[((h - 1) * 4 + quad) * 32 + lane];
                     __syncwarp();
@@ -910,13 +908,12 @@ __device__ __forceinline__ void tile_role(const Args& A, const State& S, int tw)
     using C = Cfg<NCH>;
     constexpr int NCLS = C::NCLS, NQ = 4;
     const int lane = threadIdx.x & 31;
-    int* status = A.status;
     const int nshell = A.B.nshell, nsub = A.nsub;
     unsigned short* bigl = S.big + tw * MAX_BIG;
     unsigned* pbits = S.pbits + tw * (MAX_PANELS / 32);
     for (unsigned ord = tw;; ord += NTW) {
         const int b = ord % NBUF;
-        const bool ok = ord < NBUF || warp_wait(S, S.kfree + 8 * b, ((ord / NBUF) - 1) & 1, status);
+        const bool ok = ord < NBUF || warp_wait(A, S, S.kfree + 8 * b, ((ord / NBUF) - 1) & 1);
         long long t = -1;
         if (lane == 0 && ok) {
             t = (long long)atomicAdd(A.counter, 1ull);
@@ -1265,10 +1262,8 @@ __global__ void __launch_bounds__(256) split_pack_kernel(SplitDev S, int nmo, in
     }
     atomicMax(&top, m);
     __syncthreads();
-    const int ex = (int)(top >> 52);
     const int F = scale_of(top);
-    // (coefficients from 2^1000 on may overflow in a sum, MOs below 2^-900 lose digits)
-    const bool nan = ex >= 2023 || (ex < 123 && top != 0);
+    const bool nan = too_large(top) || vanishing(top);
     if (threadIdx.x == 0) {
         fexp[mo] = nan ? MO_NAN : F;
         occ_pad[mo] = (mo < nmo && occ) ? occ[mo] : 0.0;
@@ -1350,21 +1345,9 @@ const uint64_t* split_exp_table()
     return t.data();
 }
 
-// Raised by a kernel whose bounded wait expired: one page-locked word per process,
-// written by the device and read by okg_wait_status after the stream was waited for.
-int* split_status_word()
-{
-    static int* const w = [] {
-        int* p = nullptr;
-        if (cudaHostAlloc((void**)&p, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
-            (void)cudaGetLastError();
-            return (int*)nullptr;
-        }
-        *p = 0;
-        return p;
-    }();
-    return w;
-}
+// Polls of the bounded waits in calls from this host thread (okg_set_wait_limit).
+static thread_local long long t_wait_limit = sp::WAIT_LIMIT;
+long long split_wait_limit() { return t_wait_limit; }
 
 namespace {
 
@@ -1477,10 +1460,9 @@ int run(const okg_basis* b, const Grid& g, const SplitCall& c, const SplitGenera
     if (A.nslot > sp::MAX_SLOTS) A.nslot = sp::MAX_SLOTS;
     if (A.nslot < 2) return OKG_OK;
     const int nblk = (int)(A.ntiles < sms ? A.ntiles : sms);
-    int* status = split_status_word();
     cudaMemPool_t pool = workspace_pool(device);
-    if (!status || !pool) return OKG_OK;
-    A.status = status;
+    if (!pool) return OKG_OK;
+    A.limit = split_wait_limit();
     const int nrow = A.npass * A.np;
     auto up = [](size_t v) { return (v + 255) & ~(size_t)255; };
     const size_t o_fexp = 256, o_occ = o_fexp + up(4 * (size_t)nrow), o_norm = o_occ + up(8 * (size_t)nrow),
@@ -1546,10 +1528,13 @@ int split_run(const okg_basis* b, const Grid& g, const SplitCall& c, const Split
 
 extern "C" int okg_wait_status(int* status)
 {
-    int* w = okg::split_status_word();
-    const int v = w ? *(volatile int*)w : 0;
-    if (status) *status = v;
-    if (!v) return OKG_OK;
-    *(volatile int*)w = 0;
-    return okg::set_error(OKG_ERR_TIMEOUT, "FP64 tensor-core path: a device wait expired; the results are incomplete");
+    if (status) *status = 0;
+    return OKG_OK;
+}
+
+extern "C" int okg_set_wait_limit(long long polls)
+{
+    if (polls < 0) return okg::set_error(OKG_ERR_ARG, "okg_set_wait_limit: polls < 0");
+    okg::t_wait_limit = polls;
+    return OKG_OK;
 }

@@ -35,12 +35,19 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity)
     return ok != 0;
 }
 
-// Bounded wait: returns false (and raises the status word) if the phase does not
-// complete within `limit` polls (WAIT_LIMIT unless the plan sets another).
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* status, long long limit)
+// Bounded wait: returns false if the phase does not complete within `limit` polls.
+__device__ __forceinline__ bool mbar_try_for(uint32_t bar, uint32_t parity, long long limit)
 {
     for (long long it = 0; it < limit; ++it)
         if (mbar_try(bar, parity)) return true;
+    return false;
+}
+
+// The same, also raising the status word if the phase does not
+// complete within `limit` polls (WAIT_LIMIT unless the plan sets another).
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* status, long long limit)
+{
+    if (mbar_try_for(bar, parity, limit)) return true;
     atomicExch(status, 1);
     return false;
 }
@@ -50,9 +57,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* st
 // such work always completes; false if even that expires.
 __device__ __forceinline__ bool mbar_drain(uint32_t bar, uint32_t parity)
 {
-    for (long long it = 0; it < WAIT_LIMIT; ++it)
-        if (mbar_try(bar, parity)) return true;
-    return false;
+    return mbar_try_for(bar, parity, WAIT_LIMIT);
 }
 
 // Whether any thread of the CTA raised the abort flag, the same answer for every

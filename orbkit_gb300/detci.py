@@ -106,9 +106,7 @@ def _covered(npts, slice_length):
 def _out(t, shape, was_tensor):
     if was_tensor:
         return t.reshape(tuple(t.shape[:-1]) + tuple(shape))
-    out = t.cpu().numpy().reshape(tuple(t.shape[:-1]) + tuple(shape))
-    _lib.check(_lib.load().okg_wait_status(None))
-    return out
+    return t.cpu().numpy().reshape(tuple(t.shape[:-1]) + tuple(shape))
 
 
 def _qt_device(qt_rows, nmo):
