@@ -935,8 +935,9 @@ static int run(const okg_basis* b, const Grid& g, int nmo, const double* C, cons
     double *pc = (double*)(work + P.o_pc), *pp = (double*)(work + P.o_pp), *pg = (double*)(work + P.o_pg);
     const int kp = (nmo + 15) / 16, np = kp * 16;
     const size_t cs = ColCfg<T>::smem(kp), rs = row_smem<T>(np);
-    cudaError_t e = cudaFuncSetAttribute(column_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cs);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(row_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rs);
+    // (the attributes are set to what the kernels take at most: other host threads launch under them)
+    cudaError_t e = cudaFuncSetAttribute(column_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ColCfg<T>::smem(NMO_MAX / 16));
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(row_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)row_smem<T>(NMO_MAX));
     if (e != cudaSuccess) return cuda_status(e, "okg_rho_backward: shared memory");
     e = cudaMemsetAsync(redo, 0, sizeof(int), st);
     if (e != cudaSuccess) return cuda_status(e, "okg_rho_backward: memset");

@@ -340,13 +340,14 @@ static int ci_split(long long npts, const double* mo, const double* drv, long lo
     const int per = A.np <= 32 ? 2 : 1;  // CTAs per SM
     const long long ntiles = (npts + 127) / 128, cap = (long long)sms * per;
     const unsigned nblk = (unsigned)(ntiles < cap ? ntiles : cap);
-    auto go = [&](auto kernel, int threads) -> int {
-        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // (the attribute is set to what the kernel takes at most: other host threads launch under it)
+    auto go = [&](auto kernel, int threads, int np_max) -> int {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ci_split_smem(np_max));
         if (e != cudaSuccess) return cuda_status(e, "detCI quadratic form: shared memory");
         kernel<<<nblk, threads, smem, st>>>(A);
         return OKG_OK;
     };
-    const int s = per == 2 ? go(ci_split_kernel<FLUX, 2>, 256) : go(ci_split_kernel<FLUX, 4>, 512);
+    const int s = per == 2 ? go(ci_split_kernel<FLUX, 2>, 256, 32) : go(ci_split_kernel<FLUX, 4>, 512, CI_SPLIT_MAX);
     if (s) return s;
     done = true;
     return cuda_status(cudaGetLastError(), "detCI quadratic form launch");

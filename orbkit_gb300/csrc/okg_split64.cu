@@ -1400,9 +1400,10 @@ int current_device()
 template <int NCH, int MODE>
 int launch(sp::Args& A, int nblk, size_t smem, cudaStream_t st)
 {
-    // (set on every launch: the attribute belongs to the current device)
+    // (set on every launch: the attribute belongs to the current device; always to the same
+    // size, as the device's other host threads launch under it)
     cudaError_t e = cudaFuncSetAttribute(sp::split_kernel<NCH, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
+                                         sp::SMEM_MAX);
     if (e != cudaSuccess) return cuda_status(e, "FP64 tensor-core path: shared memory");
     sp::split_kernel<NCH, MODE><<<nblk, sp::Cfg<NCH>::NT, smem, st>>>(A);
     return cuda_status(cudaGetLastError(), "FP64 tensor-core path: launch");
