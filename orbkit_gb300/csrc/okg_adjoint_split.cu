@@ -99,7 +99,8 @@ struct Dg<float> {
         const unsigned u = __float_as_uint(v);
         const int s = E + 126 - (int)((u >> 23) & 0xFF);
         const unsigned m = (u << 8) | 0x80000000u;
-        const unsigned q = ((m >> (s > 31 ? 31 : s < 0 ? 0 : s)) + 1) >> 1;
+        // (from s = 32 on v is below half a unit: the mantissa's leading bit is gone too)
+        const unsigned q = s > 31 ? 0u : ((m >> (s < 0 ? 0 : s)) + 1) >> 1;
         const unsigned neg = (unsigned)((int)u >> 31);
         const unsigned t = ((u & 0x7F800000u) ? ((q ^ neg) - neg) : 0u) + 0x80808080u;
         const uint32_t h20 = digit_pair(t, t >> 16, 1), h31 = digit_pair(t, t >> 16, 0);  // bytes 1 | 3, 0 | 2
