@@ -265,7 +265,8 @@ int okg_batch_status(okg_batch* batch, int* device_status);
  * points on) the contractions run on the tensor cores over runs of points; else, above
  * 48 MOs, the AO tiles of the MO pass are recomputed per block of 48 MOs.  d_work is
  * caller memory of at least okg_rho_backward_workspace bytes (about 1 GB of
- * intermediates at most, and partial sums, reduced in a fixed order). */
+ * intermediates at most, and partial sums of one resident set of blocks, whatever the
+ * number of points; reduced in a fixed order). */
 int okg_rho_backward_workspace(const okg_basis* basis, const okg_grid* grid, int nmo, int precision, size_t* bytes);
 int okg_rho_backward(const okg_basis* basis, const okg_grid* grid, int nmo, const double* d_coeff,
                      const double* d_occ, const double* d_g_rho, const double* d_g_grad, int64_t ld, int precision,

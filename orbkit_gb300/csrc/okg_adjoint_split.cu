@@ -340,8 +340,8 @@ struct RowArgs {
     const T* X;       // W, V: 2 x nmo x ld
     const T* Y;       // chi, G: 2 x ncart x ld
     int nmo, ncart, np;
-    double* part;     // nslot x ncart x nmo
-    int slot0;
+    double* part;     // gridDim.x x ncart x nmo: sums of a block's points, over all runs
+    bool first;       // first run: written, else added to
     int* redo;        // raised where a value is not finite or a wait expires
     long long limit;  // polls of a wait
     unsigned tm_cols;
@@ -494,14 +494,14 @@ __global__ void __launch_bounds__(512, 1) row_kernel(const __grid_constant__ Row
             __syncthreads();
         }
     if (tid == 0 && issued) mbar_drain(bar_a, parity ^ 1);
-    double* part = A.part + ((long long)(A.slot0 + blockIdx.x) * A.ncart + k0 + row) * A.nmo;
+    double* part = A.part + ((long long)blockIdx.x * A.ncart + k0 + row) * A.nmo;
     if (row < nrow)
 #pragma unroll
         for (int j = 0; j < 4; ++j)
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const int n = 4 * hf + 16 * j + i;
-                if (n < A.nmo) part[n] = acc[j][i];
+                if (n < A.nmo) part[n] = A.first ? acc[j][i] : part[n] + acc[j][i];
             }
     tc_fence_before();
     __syncthreads();
@@ -536,9 +536,9 @@ struct ShellArgs {
     long long g_ld, ld;
     const T* AB;           // A, B: 2 x ncart x ld
     T* Y;                  // chi, G: 2 x ncart x ld
-    double* part_p;        // nslot x nprim x 3: U0, U1, U2
+    double* part_p;        // nslot x nprim x 3: U0, U1, U2, over all runs
     double* part_g;        // nslot x nshell x 3
-    int slot0;
+    bool first;            // first run: written, else added to
     long long per;         // points of a slot (multiple of 32)
     int* redo;             // raised where a cotangent is not finite
 };
@@ -812,17 +812,18 @@ __device__ __forceinline__ void run_shell(const ShellArgs<T>& A, const Shell& sh
             if (q >= nq) continue;
             const T a = warp_total(U0[q]), b = warp_total(U1[q]), c = warp_total(U2[q]);
             if (lane == 0) {
-                double* o = A.part_p + ((long long)(A.slot0 + slot) * A.B.nprim + sh.prim0 + q0 + q) * 3;
-                o[0] = (double)a;
-                o[1] = (double)b;
-                o[2] = (double)c;
+                double* o = A.part_p + ((long long)slot * A.B.nprim + sh.prim0 + q0 + q) * 3;
+                o[0] = A.first ? (double)a : o[0] + (double)a;
+                o[1] = A.first ? (double)b : o[1] + (double)b;
+                o[2] = A.first ? (double)c : o[2] + (double)c;
             }
         }
     }
 #pragma unroll
     for (int u = 0; u < 3; ++u) {
         const T v = warp_total(dR[u]);
-        if (lane == 0) A.part_g[((long long)(A.slot0 + slot) * A.B.nshell + s) * 3 + u] = (double)v;
+        double* o = A.part_g + ((long long)slot * A.B.nshell + s) * 3 + u;
+        if (lane == 0) *o = A.first ? (double)v : *o + (double)v;
     }
 }
 
@@ -880,8 +881,8 @@ __global__ void __launch_bounds__(128) finish_kernel(BasisDev B, SplitDev S, con
 // ------------------------------------------------------------------ host side
 struct Plan {
     long long run;     // points of a run
-    int nruns, nchunk; // runs; slots of the shell kernel per run (multiple of 4)
-    int nbx;           // point slots of the row kernel per run
+    int nruns, nchunk; // runs; slots of the shell kernel (multiple of 4)
+    int nbx;           // point slots of the row kernel
     size_t o_x, o_ab, o_y, o_pc, o_pp, o_pg, bytes;
 };
 
@@ -911,9 +912,10 @@ static Plan make_plan(const okg_basis* b, long long npts, int nmo, int sms)
     P.o_ab = P.o_x + up256(2 * (size_t)nmo * ld * sizeof(T));
     P.o_y = P.o_ab + up256(2 * (size_t)b->ncart * ld * sizeof(T));
     P.o_pc = P.o_y + up256(2 * (size_t)b->ncart * ld * sizeof(T));
-    P.o_pp = P.o_pc + up256((size_t)P.nruns * P.nbx * b->ncart * nmo * 8);
-    P.o_pg = P.o_pp + up256((size_t)P.nruns * P.nchunk * b->nprim * 3 * 8);
-    P.bytes = P.o_pg + up256((size_t)P.nruns * P.nchunk * b->nshell * 3 * 8);
+    // (the runs follow one another on the stream and add to the same partial sums)
+    P.o_pp = P.o_pc + up256((size_t)P.nbx * b->ncart * nmo * 8);
+    P.o_pg = P.o_pp + up256((size_t)P.nchunk * b->nprim * 3 * 8);
+    P.bytes = P.o_pg + up256((size_t)P.nchunk * b->nshell * 3 * 8);
     return P;
 }
 
@@ -968,16 +970,16 @@ static int run(const okg_basis* b, const Grid& g, int nmo, const double* C, cons
         if (gx > tiles) gx = (int)tiles;
         column_kernel<T><<<dim3(gx, passes, 2), 128 * ColCfg<T>::G, cs, st>>>(ColArgs<T>{n, P.run, X, C, nmo, b->ncart, kp, AB, redo, limit});
         long long per = ((n + P.nchunk - 1) / P.nchunk + 31) / 32 * 32;
-        const ShellArgs<T> sa{b->dev, b->split, gr, c.g_grad, ld, P.run, AB, Y, pp, pg, r * P.nchunk, per, redo};
+        const ShellArgs<T> sa{b->dev, b->split, gr, c.g_grad, ld, P.run, AB, Y, pp, pg, r == 0, per, redo};
         shell_kernel<T, false><<<dim3(b->nshell, P.nchunk / 4), 128, 0, st>>>(sa);
         if (b->max_l > 2) shell_kernel<T, true><<<dim3(b->nshell, P.nchunk / 4), 128, 0, st>>>(sa);
         unsigned tm = 32;
         while ((int)tm < Dg<T>::D * np) tm *= 2;
         row_kernel<T><<<dim3(P.nbx, (b->ncart + 127) / 128), 512, rs, st>>>(
-            RowArgs<T>{n, P.run, X, Y, nmo, b->ncart, np, pc, r * P.nbx, redo, limit, tm});
+            RowArgs<T>{n, P.run, X, Y, nmo, b->ncart, np, pc, r == 0, redo, limit, tm});
     }
-    dcoeff_kernel<<<(nmo * b->ncart + 31) / 32, dim3(32, 8), 0, st>>>(pc, P.nruns * P.nbx, nmo, b->ncart, dC);
-    finish_kernel<<<(b->nprim + b->natom + 3) / 4, 128, 0, st>>>(b->dev, b->split, pp, pg, P.nruns * P.nchunk, dprim, dgeo);
+    dcoeff_kernel<<<(nmo * b->ncart + 31) / 32, dim3(32, 8), 0, st>>>(pc, P.nbx, nmo, b->ncart, dC);
+    finish_kernel<<<(b->nprim + b->natom + 3) / 4, 128, 0, st>>>(b->dev, b->split, pp, pg, P.nchunk, dprim, dgeo);
     done = true;
     return cuda_status(cudaGetLastError(), "okg_rho_backward launch");
 }
