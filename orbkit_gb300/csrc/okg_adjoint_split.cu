@@ -37,14 +37,14 @@ using namespace sp;
 
 constexpr int NMO_MAX = 64;
 
-// Which calls take this pipeline: up to 64 MOs (one accumulator set of the column kernel), and in
-// FP32 at least 2048 points.  Backward pass, one-kernel form | pipeline, us, FP64: 3 atoms, 5 MOs
+// Which calls take this pipeline: bases within the tables of step 1, up to 64 MOs (one
+// accumulator set of the column kernel), and in FP32 at least 2048 points.  Backward pass, one-kernel form | pipeline, us, FP64: 3 atoms, 5 MOs
 // and 50 points 215 | 158, 20 atoms, 60 MOs and 50 points 1679 | 333; FP32: 3 atoms and 500
 // points 106 | 152, 3000 points 225 | 156; 12 atoms, 40 MOs and 500 points 198 | 275, 3000 points
 // 315 | 282; 20 atoms and 500 points 457 | 397, 3000 points 574 | 412.
-static bool takes(long long npts, int nmo, int precision)
+static bool takes(const okg_basis* b, long long npts, int nmo, int precision)
 {
-    return nmo <= NMO_MAX && npts >= (precision == 32 ? 2048 : 1);
+    return split_basis(b) && nmo <= NMO_MAX && npts >= (precision == 32 ? 2048 : 1);
 }
 
 // Digit operands of the intermediates: doubles as 7 digits (55 bits), floats as 4 (31 bits,
@@ -988,7 +988,7 @@ static int run(const okg_basis* b, const Grid& g, int nmo, const double* C, cons
 
 size_t adjoint_split_bytes(const okg_basis* b, long long npts, int nmo, int precision)
 {
-    if (!adjs::takes(npts, nmo, precision)) return 0;
+    if (!adjs::takes(b, npts, nmo, precision)) return 0;
     const int sms = adjs::sm_count();
     return precision == 32 ? adjs::make_plan<float>(b, npts, nmo, sms).bytes : adjs::make_plan<double>(b, npts, nmo, sms).bytes;
 }
@@ -998,7 +998,7 @@ int adjoint_split_run(const okg_basis* b, const Grid& g, int nmo, const double* 
                       int* redo, cudaStream_t st, bool& done)
 {
     done = false;
-    if (!adjs::takes(g.npts, nmo, precision)) return OKG_OK;
+    if (!adjs::takes(b, g.npts, nmo, precision)) return OKG_OK;
     const int sms = adjs::sm_count();
     if (precision == 32)
         return adjs::run<float>(b, g, nmo, C, occ, grho, ggrad, ld, dC, dprim, dgeo, (char*)work,

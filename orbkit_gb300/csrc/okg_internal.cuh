@@ -358,6 +358,8 @@ struct SplitGeneral {
     int (*run)(const void* self, const int* go, const double* norm_part);
     const void* self;
 };
+// Whether the basis fits the tables of the kernel.
+bool split_basis(const okg_basis* b);
 // Runs the call on the tensor cores if it is one for them (done = true), else leaves it.  What
 // turns out on the device to be out of their range is computed by `general` after them.
 int split_run(const okg_basis* b, const Grid& g, const SplitCall& c, const SplitGeneral& general, cudaStream_t st, bool& done);

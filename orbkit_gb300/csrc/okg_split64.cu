@@ -1501,6 +1501,11 @@ int run(const okg_basis* b, const Grid& g, const SplitCall& c, const SplitGenera
 }
 }  // namespace
 
+bool split_basis(const okg_basis* b)
+{
+    return b->nshell <= sp::MAX_SHELLS && b->split.npanel <= sp::MAX_PANELS && b->dev.max_nprim <= 255;
+}
+
 int split_run(const okg_basis* b, const Grid& g, const SplitCall& c, const SplitGeneral& general, cudaStream_t st, bool& done)
 {
     done = false;
@@ -1515,7 +1520,7 @@ int split_run(const okg_basis* b, const Grid& g, const SplitCall& c, const Split
     const bool values = (c.need & ~1u) == 0;
     const bool contraction = (c.need & ~0xFu) == 0 && !values && (long long)c.nmo * b->ncart >= 32768;
     if (!c.g_rho && !contraction && g.npts < (values ? 32 : 16) * sm_count(current_device())) return OKG_OK;
-    if (b->nshell > sp::MAX_SHELLS || b->split.npanel > sp::MAX_PANELS || b->dev.max_nprim > 255) return OKG_OK;
+    if (!split_basis(b)) return OKG_OK;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
         (void)cudaGetLastError();

@@ -36,3 +36,18 @@ def test_does_not_grow_with_the_points(core, nmo, precision):
     for npts in (1 << 22, 1 << 24, 1 << 27):
         gd.npts = npts
         assert workspace(b, gd, nmo, precision) <= 1.25 * 2 ** 30
+
+
+@pytest.mark.parametrize("precision", [64, 32])
+def test_bases_beyond_the_tables(core, precision):
+    """More shells than the tensor-core kernels' tables hold: the one-kernel form's workspace
+    (that of 65 MOs, but for the MOs)."""
+    import torch
+    from orbkit_gb300.orbitals import AOClass
+    rng = numpy.random.default_rng(3)
+    ao = AOClass([{"atom": i % 9, "type": "s", "pnum": 1, "coeffs": numpy.array([[rng.uniform(0.1, 9.0), 1.0]])} for i in range(2049)])
+    ao.update()
+    b = core.get_basis(rng.uniform(-3.0, 3.0, (9, 3)), ao, torch.device("cuda"))
+    qc = molecule("s")
+    _, _, _, xyz, gd, n = device_call(core, qc, near_points(qc, 6000))
+    assert workspace(b, gd, 64, precision) <= workspace(b, gd, 65, precision)
