@@ -268,6 +268,9 @@ int okg_batch_status(okg_batch* batch, int* device_status);
  * intermediates at most, and partial sums of one resident set of blocks, whatever the
  * number of points; reduced in a fixed order). */
 int okg_rho_backward_workspace(const okg_basis* basis, const okg_grid* grid, int nmo, int precision, size_t* bytes);
+/* The least workspace that okg_rho_backward takes: that of the form without intermediates,
+ * for a device without room for the other (2 to 5 times slower on large grids). */
+int okg_rho_backward_workspace_least(const okg_basis* basis, const okg_grid* grid, int nmo, int precision, size_t* bytes);
 int okg_rho_backward(const okg_basis* basis, const okg_grid* grid, int nmo, const double* d_coeff,
                      const double* d_occ, const double* d_g_rho, const double* d_g_grad, int64_t ld, int precision,
                      double* d_dcoeff, double* d_dprim, double* d_dgeo, void* d_work, size_t work_bytes,

@@ -24,6 +24,8 @@ from .qcinfo import unpack
 _SIGS = {
     "okg_rho_backward_workspace": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(_lib.OkgGrid), ctypes.c_int,
                                                   ctypes.c_int, ctypes.POINTER(ctypes.c_size_t)]),
+    "okg_rho_backward_workspace_least": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(_lib.OkgGrid), ctypes.c_int,
+                                                        ctypes.c_int, ctypes.POINTER(ctypes.c_size_t)]),
     "okg_rho_backward": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(_lib.OkgGrid), ctypes.c_int,
                                         ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p,
                                         ctypes.c_int64, ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p,
@@ -105,7 +107,13 @@ class DensityModel:
         nbytes = ctypes.c_size_t(0)
         _lib.check(self._L.okg_rho_backward_workspace(self.basis.handle, self.gd, self.nmo, prec, ctypes.byref(nbytes)))
         if self._work is None or self._work.numel() < nbytes.value:
-            self._work = torch.empty(nbytes.value, dtype=torch.uint8, device=self.device)
+            self._work = None
+            try:
+                self._work = torch.empty(nbytes.value, dtype=torch.uint8, device=self.device)
+            except torch.cuda.OutOfMemoryError:
+                # (the form without intermediates)
+                _lib.check(self._L.okg_rho_backward_workspace_least(self.basis.handle, self.gd, self.nmo, prec, ctypes.byref(nbytes)))
+                self._work = torch.empty(nbytes.value, dtype=torch.uint8, device=self.device)
         g_rho = g_rho.to(torch.float64).contiguous()
         g_grad = g_grad.to(torch.float64).contiguous()
         dC = torch.empty_like(Ceff)

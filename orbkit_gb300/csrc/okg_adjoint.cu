@@ -464,6 +464,15 @@ extern "C" int okg_rho_backward_workspace(const okg_basis* b, const okg_grid* gr
     return OKG_OK;
 }
 
+extern "C" int okg_rho_backward_workspace_least(const okg_basis* b, const okg_grid* grid, int nmo, int precision,
+                                                size_t* bytes)
+{
+    if (!b || !grid || !bytes || nmo <= 0)
+        return set_error(OKG_ERR_ARG, "okg_rho_backward_workspace_least: bad argument");
+    *bytes = adj::one_kernel_bytes(b, grid->npts, nmo, precision);
+    return OKG_OK;
+}
+
 extern "C" int okg_rho_backward(const okg_basis* b, const okg_grid* gr, int nmo, const double* d_coeff,
                                 const double* d_occ, const double* d_g_rho, const double* d_g_grad, int64_t ld,
                                 int precision, double* d_dcoeff, double* d_dprim, double* d_dgeo, void* d_work,

@@ -51,3 +51,45 @@ def test_bases_beyond_the_tables(core, precision):
     qc = molecule("s")
     _, _, _, xyz, gd, n = device_call(core, qc, near_points(qc, 6000))
     assert workspace(b, gd, 64, precision) <= workspace(b, gd, 65, precision)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_device_without_room(core, precision, monkeypatch):
+    """A fit step where the whole workspace cannot be allocated: the gradients of the form that
+    needs the least, and those of the other again once there is room."""
+    import torch
+    from orbkit_gb300.adjoint import DensityModel
+    qc = molecule("d", nmo=40)
+    pts = near_points(qc, 20000)
+    model = DensityModel(qc, pts[0], pts[1], pts[2], True, precision)
+    prim = qc.ao_spec.get_prim_coeffs()
+    par = [torch.tensor(numpy.array(v), dtype=torch.float64, device="cuda", requires_grad=True)
+           for v in (qc.mo_spec.get_coeffs(), prim[:, 0], prim[:, 1], qc.geo_spec)]
+
+    def step():
+        for p in par:
+            p.grad = None
+        rho, grad = model(*par)
+        (rho.sum() + (grad ** 2).sum()).backward()
+        return [p.grad.clone() for p in par]
+
+    usual = step()
+    whole = model._work.numel()
+    model._work = None
+    empty = torch.empty
+
+    def no_room(*a, **k):
+        if a and a[0] == whole:
+            raise torch.cuda.OutOfMemoryError("no room")
+        return empty(*a, **k)
+
+    monkeypatch.setattr(torch, "empty", no_room)
+    least = step()
+    assert model._work.numel() < whole
+    monkeypatch.undo()
+    again = step()
+    assert model._work.numel() == whole
+    bar = 1e-10 if precision == "fp64" else 2e-3  # (as in test_gpu_adjoint_split.py)
+    for u, l, a in zip(usual, least, again):
+        assert torch.equal(u, a)
+        assert float((u - l).abs().max() / u.abs().max()) <= bar
