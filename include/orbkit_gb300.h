@@ -146,6 +146,12 @@ int okg_unfold_coeff(const okg_basis* basis, int nmo, const double* d_ccart, dou
 int okg_wait_status(int* status);
 int okg_set_wait_limit(long long polls);
 
+/* Page-locked host memory, and the read-back of `rows` contiguous device rows of `width` bytes
+ * into host rows `pitch` bytes apart (asynchronous where the host memory is page-locked). */
+int okg_host_alloc(size_t bytes, void** out);
+int okg_host_free(void* p);
+int okg_read_rows(void* h_dst, size_t pitch, const void* d_src, size_t width, size_t rows, okg_stream stream);
+
 /* ------------------------------------------------ operations on given grids
  * FP64 operations on AO / MO values the caller already holds on the device, every
  * array row-major (row, point) with points contiguous and its own leading dimension

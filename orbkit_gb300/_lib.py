@@ -52,6 +52,9 @@ SIGNATURES = {
     "okg_fold_coeff": (ctypes.c_int, [_vp, ctypes.c_int, _vp, _vp, _vp]),
     "okg_unfold_coeff": (ctypes.c_int, [_vp, ctypes.c_int, _vp, _vp, _vp]),
     "okg_wait_status": (ctypes.c_int, [_c_int_p]),
+    "okg_host_alloc": (ctypes.c_int, [ctypes.c_size_t, ctypes.POINTER(_vp)]),
+    "okg_host_free": (ctypes.c_int, [_vp]),
+    "okg_read_rows": (ctypes.c_int, [_vp, ctypes.c_size_t, _vp, ctypes.c_size_t, ctypes.c_size_t, _vp]),
     "okg_set_wait_limit": (ctypes.c_int, [ctypes.c_longlong]),
     "okg_mixed_plan_create": (ctypes.c_int, [_vp, ctypes.c_int, ctypes.POINTER(_vp)]),
     "okg_mixed_plan_destroy": (ctypes.c_int, [_vp]),

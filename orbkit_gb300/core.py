@@ -23,6 +23,7 @@ import numpy
 from . import _lib
 from . import grid as _default_grid
 from .basis import get_basis
+from .hostmem import Result
 from .qcinfo import unpack
 from .tools import require, validate_drv
 
@@ -131,42 +132,6 @@ class _DeviceGrid:
         return g, xs
 
 
-# results between these sizes come back in page-locked memory (torch's caching host
-# allocator): 131 MB read back in 0.7 ms (3 ms with the pages newly locked), against 16 ms
-# through pageable memory into a fresh numpy array (page faults); below, the pageable copy
-# costs less than the allocator's bookkeeping
-PINNED_MIN_BYTES = 256 << 10
-PINNED_MAX_BYTES = 2 << 30
-
-
-class _Result:
-    """Host array of a result, filled part by part from device tensors."""
-
-    def __init__(self, *shape):
-        n = 8
-        for v in shape:
-            n *= int(v)
-        self.pinned = None
-        if PINNED_MIN_BYTES <= n <= PINNED_MAX_BYTES:
-            torch = _torch()
-            self.pinned = torch.empty(shape, dtype=torch.float64, pin_memory=True)
-            self.array = self.pinned.numpy()
-        else:
-            self.array = numpy.empty(shape)
-
-    def put(self, index, part):
-        if self.pinned is None:
-            self.array[index] = part.cpu().numpy()
-        else:
-            self.pinned[index].copy_(part, non_blocking=True)
-
-    def finish(self):
-        """The array, complete."""
-        if self.pinned is not None:
-            _torch().cuda.current_stream().synchronize()
-        return self.array
-
-
 def _slices(npts, bytes_per_point):
     step = max(1, min(npts, MAX_SLICE_BYTES // max(1, bytes_per_point)))
     return [(i, min(i + step, npts)) for i in range(0, npts, step)] or [(0, 0)]
@@ -203,33 +168,33 @@ def _eval(qc_geo, ao_spec, mo_spec, x, y, z, is_vector, what, drv_codes, exact_m
     em = 1 if exact_mixed else 0
     st = _lib.stream_handle()
     if what == "ao":
-        out = _Result(nd, b.nao, npts)
+        out = Result(nd, b.nao, npts)
         for (i, j) in _slices(npts, 8 * nd * b.nao):
             if j <= i:
                 continue
             gd, keep = g.slice(i, j)
             o = torch.empty((nd, b.nao, j - i), dtype=torch.float64, device=dev)
             _lib.check(L.okg_eval_ao(b.handle, gd, nd, codes, em, _lib.ptr(o), j - i, st))
-            out.put(numpy.s_[:, :, i:j], o)
+            out.put(i, j, o)
         return out.finish()
     C = b.c_eff(mo_spec.get_coeffs())
     nmo = C.shape[0]
     if what == "mo":
-        out = _Result(nd, nmo, npts)
+        out = Result(nd, nmo, npts)
         for (i, j) in _slices(npts, 8 * nd * nmo):
             if j <= i:
                 continue
             gd, keep = g.slice(i, j)
             o = torch.empty((nd, nmo, j - i), dtype=torch.float64, device=dev)
             _lib.check(L.okg_eval_mo(b.handle, gd, nmo, _lib.ptr(C), nd, codes, em, _lib.ptr(o), j - i, st))
-            out.put(numpy.s_[:, :, i:j], o)
+            out.put(i, j, o)
         return out.finish()
     if occ is None:
         occ = numpy.array([m["occ_num"] for m in mo_spec], dtype=numpy.float64)
     occ_d = torch.as_tensor(numpy.asarray(occ, dtype=numpy.float64), device=dev).contiguous()
     norm_d = torch.zeros(nmo, dtype=torch.float64, device=dev) if mo_norm else None
-    rho = _Result(npts)
-    drho = _Result(nd, npts)
+    rho = Result(npts)
+    drho = Result(nd, npts)
     for (i, j) in _slices(npts, 8 * (1 + nd)):
         if j <= i:
             continue
@@ -238,9 +203,9 @@ def _eval(qc_geo, ao_spec, mo_spec, x, y, z, is_vector, what, drv_codes, exact_m
         dr = torch.empty((max(nd, 1), j - i), dtype=torch.float64, device=dev)
         _lib.check(L.okg_rho(b.handle, gd, nmo, _lib.ptr(C), _lib.ptr(occ_d), nd, codes, em, _lib.ptr(r),
                              _lib.ptr(dr), j - i, _lib.ptr(norm_d), st))
-        rho.put(numpy.s_[i:j], r)
+        rho.put(i, j, r)
         if nd:
-            drho.put(numpy.s_[:, i:j], dr[:nd])
+            drho.put(i, j, dr[:nd])
     drho = drho.finish()
     rho = rho.finish()
     if mo_norm:
@@ -277,13 +242,13 @@ def mo_creator(ao_list, mo_spec):
     nmo, nao = coeffs.shape
     dev = torch.device("cuda", torch.cuda.current_device())
     C = torch.from_numpy(coeffs).to(dev)
-    out = _Result(nmo, npts)
+    out = Result(nmo, npts)
     st = _lib.stream_handle()
     for (i, j) in _point_steps(npts, 8 * (nao + nmo)):
         a = torch.from_numpy(numpy.ascontiguousarray(A[:, i:j])).to(dev)
         o = torch.empty((nmo, j - i), dtype=torch.float64, device=dev)
         _lib.check(L.okg_mo_from_ao(nmo, nao, _lib.ptr(C), _lib.ptr(a), j - i, j - i, _lib.ptr(o), j - i, st))
-        out.put(numpy.s_[:, i:j], o)
+        out.put(i, j, o)
     return out.finish().reshape((nmo,) + shape[1:])
 
 
@@ -306,14 +271,14 @@ def cartesian2spherical(ao_list, ao_spec):
     npts = A.shape[1]
     dev = torch.device("cuda", torch.cuda.current_device())
     d_ptr, d_idx, d_coef = (torch.from_numpy(numpy.ascontiguousarray(v)).to(dev) for v in (ptr, idx, coef))
-    out = _Result(nsph, npts)
+    out = Result(nsph, npts)
     st = _lib.stream_handle()
     for (i, j) in _point_steps(npts, 8 * (ncart + nsph)):
         a = torch.from_numpy(numpy.ascontiguousarray(A[:, i:j])).to(dev)
         o = torch.empty((nsph, j - i), dtype=torch.float64, device=dev)
         _lib.check(L.okg_cart2sph(nsph, ncart, _lib.ptr(d_ptr), _lib.ptr(d_idx), _lib.ptr(d_coef), _lib.ptr(a), j - i,
                                   j - i, _lib.ptr(o), j - i, st))
-        out.put(numpy.s_[:, i:j], o)
+        out.put(i, j, o)
     return out.finish().reshape((nsph,) + shape[1:])
 
 
@@ -491,7 +456,7 @@ def calc_mo_matrix(qc_a, qc_b=None, drv=None, numproc=1, slice_length=1e4, save_
     mo_b = mo_a if same else _MoGrids(qc_b, x, y, z, vec, exact_mixed)
     na, nb, nk = mo_a.nmo, mo_b.nmo, len(iket)
     npts = mo_a.g.npts
-    out = _Result(nk, na, nb, npts)
+    out = Result(nk, na, nb, npts)
     L = _lib.load()
     torch = _torch()
     for (i, j) in _point_steps(npts, 8 * (nk * na * nb + (len(drv) + 1) * max(na, nb))):
@@ -504,5 +469,5 @@ def calc_mo_matrix(qc_a, qc_b=None, drv=None, numproc=1, slice_length=1e4, save_
         o = torch.empty((nk, na, nb, j - i), dtype=torch.float64, device=mo_a.dev)
         _lib.check(L.okg_mo_products(nk, na, nb, _lib.ptr(bra), j - i, _lib.ptr(ket), j - i, j - i, _lib.ptr(o),
                                      j - i, _lib.stream_handle()))
-        out.put(numpy.s_[..., i:j], o)
+        out.put(i, j, o)
     return out.finish().reshape((nk, na, nb) + N)
