@@ -55,6 +55,8 @@ def spherical_csr(ao_spec):
         while j < len(old) and int(old[j][0]) == shell:
             lms.append((int(old[j][1][0]), int(old[j][1][1])))
             j += 1
+        if not 0 <= shell < len(bounds) - 1 or bounds[shell] == bounds[shell + 1]:
+            raise KeyError(shell)  # (no such shell)
         first, last = bounds[shell], bounds[shell + 1]
         key = (tuple(comps[first:last]), tuple(lms))
         if key not in kinds:
