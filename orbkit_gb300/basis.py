@@ -186,6 +186,12 @@ class DeviceBasis:
         numpy.add.at(T, (numpy.repeat(numpy.arange(self.nao), numpy.diff(f["sph_ptr"])), f["sph_idx"]), f["sph_coef"])
         return T
 
+    @property
+    def T_dev(self):
+        """The transform T on the device (None for a Cartesian basis)."""
+        import torch
+        return torch.from_numpy(self.T).to(self.device) if self.spherical else None
+
     def c_grad(self, grad):
         """Gradient with respect to C_eff (nmo, ncart) -> with respect to the MO coefficients (nmo, nao)."""
         import torch
