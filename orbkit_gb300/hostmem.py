@@ -58,11 +58,9 @@ def _take(size):
     """(address, size) of a block of at least `size` bytes, or None."""
     global _held
     with _lock:
-        fit = [b for b in _waiting if size <= b[1] <= 2 * size]
+        fit = [i for i, b in enumerate(_waiting) if size <= b[1] <= 2 * size]
         if fit:
-            best = min(fit, key=lambda b: b[1])
-            _waiting.remove(best)
-            return best
+            return _waiting.pop(min(fit, key=lambda i: (_waiting[i][1], -i)))  # (the last used of the smallest)
         step = 1 << max(16, size.bit_length() - 4)  # (sizes in steps of 1/16 .. 1/8: blocks fit similar results)
         size = -(-size // step) * step
         _free(_held + size - HELD_MAX)
