@@ -12,11 +12,23 @@
 //   * every AO value a (FP64) of a grid point is scaled by a power of two 2^-E above the
 //     largest AO of that point and rounded to a 55-bit integer, cut into 7 balanced
 //     base-256 digits (-128 .. 127); the coefficients likewise per MO;
-//   * digit products are integers below 2^14; sums over up to 160 columns stay below
-//     2^24, so the FP32 accumulators of tcgen05.mma hold them exactly;
-//   * the products d_i(a) d_j(c) with i + j = w have the weight 2^(-14 - 8 w); w = 0..6
-//     are kept, 7 accumulators per MO; what is left out is below 2^-52 of the largest
-//     product, less than the rounding of an FP64 accumulation of the same sum.
+//   * the products d_i(a) d_j(c) with i + j = w, integers up to 2^14, have the weight
+//     2^(-14 - 8 w); w = 0..6 are kept, 7 accumulators per MO;
+//   * an accumulator adds w + 1 products per column.  Up to 146 columns the FP32 accumulators of
+//     tcgen05.mma are exact (7 x 146 x 2^14 < 2^24); at the 160 columns of a group the last one
+//     (w = 6) could pass 2^24 with every digit at its end, and then rounds by one unit of
+//     2^-62, which the products left out exceed 6 times per column.
+//
+// Error.  A value is fixed-point relative to the largest AO of its point, a coefficient to the
+// largest of its MO: per column 2^-56 each of their product for the roundings, 6.1 x 2^-56 for
+// the products left out.  With n columns the error of an MO value is at most
+//     n 2^-53 2^E 2^F,  2^F < 2.1 max|C|,  2^E about the largest AO value (derivative of the
+//     class: first derivatives share a scale, and so do second) at the point.
+// Where the largest AO and the largest coefficient meet that is the rounding of an FP64 sum;
+// an MO that is small at a point where another's AOs are large (a localised orbital near
+// another nucleus) keeps as many digits less as it is smaller: it is accurate relative to
+// max|C| max|AO|, not to itself, where the DFMA kernel is accurate relative to sum |C| |AO|.
+// Densities are sums of squares and see it only where no occupied MO holds the largest AO.
 //
 // Screening.  A shell (and the steep primitives of a shell) whose bound over the tile's
 // points lies 2^-62 below a value that the scale 2^E of every point is known to reach
@@ -34,7 +46,8 @@
 //                       shells, digits written to the panel's operand slot (ring of slots);
 //   epilogue warps (8, second derivatives 4)  accumulators -> FP64 MO values (integer
 //                       arithmetic) -> outputs;
-//   1 MMA warp, 1 coefficient loader (bulk copies), 1 tile warp (screening, scales).
+//   1 MMA warp, 2 tile warps (screening, scales) that take turns with the tile buffers; the
+//                       copies of coefficient digits are requested by a generation lane.
 // Every wait is bounded: one that expires raises the redo word, and the block drains its copies
 // and MMAs in flight and leaves.
 //
@@ -77,6 +90,12 @@ constexpr float NOTHING = -3000.0f;
 // 1.443 alpha (2 sqrt(3) d x + 3 x^2); where alpha d^2 <= 735 (beyond ABS_FLOOR nothing counts)
 // that is 136 sqrt(alpha) x + 4.3 alpha x^2, here 0.05 at most, which the scales have to spare.
 constexpr float WIDE = 3.6e-4f;
+// Error of a coordinate that the bounds of the polynomials allow for (a tile of 40 bohr; larger
+// ones are wide too).  A constant: kept in a register through the loop over the shells, the tile's
+// own error took 7 % of the kernel's time (20 atoms, gradients).  At CLOSE and beyond it is 3 % of
+// the distance, a quarter of a bit of the steepest polynomial; tiles with points closer to an
+// atom are wide as well (at a nucleus the bound of a steep gradient would be all allowance).
+constexpr float NEAR = 8.0e-6f, CLOSE = 64.0f * NEAR;
 
 template <int NCH>
 struct Cfg {
@@ -819,10 +838,10 @@ __device__ __forceinline__ BoxRange box_range(const Args& A, int atom, double ox
 }
 
 // Raises top (log2, per channel class) to a shell's bound at squared distances dd (coordinates
-// within err): sum over the primitives relative to the largest.
-template <int NCLS, int NQ>
+// within NEAR, or EXACT): sum over the primitives relative to the largest.
+template <int NCLS, bool EXACT, int NQ>
 __device__ __forceinline__ void point_bounds(const float4* __restrict__ pl, int np, int L, const float (&dd)[NQ],
-                                             const float (&dq)[NQ], float err, float (&top)[NQ][NCLS])
+                                             const float (&dq)[NQ], float (&top)[NQ][NCLS])
 {
     float m[NQ], R0[NQ], R1[NQ], R2[NQ];
 #pragma unroll
@@ -848,7 +867,7 @@ __device__ __forceinline__ void point_bounds(const float4* __restrict__ pl, int 
 #pragma unroll
     for (int q = 0; q < NQ; ++q) {
         if (m[q] < NOTHING) continue;
-        const Poly f = poly(L, sqrtf(dd[q]) + 2.f * err, dq[q] + err);
+        const Poly f = EXACT ? poly(L, sqrtf(dd[q]), dq[q]) : poly(L, sqrtf(dd[q]) + 2.f * NEAR, dq[q] + NEAR);
         top[q][0] = fmaxf(top[q][0], m[q] + __log2f(f.p0 * R0[q]));
         if (NCLS > 1) top[q][1] = fmaxf(top[q][1], m[q] + __log2f(f.p1 * R0[q] + 2.f * f.q1 * R1[q]));
         if (NCLS > 2)
@@ -875,7 +894,8 @@ __device__ __forceinline__ int row_scale(int special, float top, int* redo)
     return special ? special : (int)ceilf(fminf(fmaxf(top + 0.15f, -950.f), 990.f));
 }
 
-// The points' scales of a tile beyond WIDE, with FP64 differences to the atoms: every kept shell,
+// The points' scales of a tile beyond WIDE or NEAR, or with points within CLOSE, with FP64
+// differences to the atoms: every kept shell,
 // point after point (a call of its own: few tiles need it).
 template <int NCH>
 __device__ __noinline__ void wide_scales(const Args& A, long long t, const unsigned char* nkeep, short* rowexp, float r0,
@@ -896,7 +916,7 @@ __device__ __noinline__ void wide_scales(const Args& A, long long t, const unsig
             const double* at = A.B.atoms + 4 * rec.x;
             const float dx = (float)(x - __ldg(at)), dy = (float)(y - __ldg(at + 1)), dz = (float)(z - __ldg(at + 2));
             const float dd[1] = {fmaf(dx, dx, fmaf(dy, dy, dz * dz))}, dq[1] = {fmaxf(fabsf(dx), fmaxf(fabsf(dy), fabsf(dz)))};
-            point_bounds<NCLS>(A.S.prim_lg + rec.z, nkeep[s], rec.y & 0xFF, dd, dq, 0.f, top);
+            point_bounds<NCLS, true>(A.S.prim_lg + rec.z, nkeep[s], rec.y & 0xFF, dd, dq, top);
         }
         for (int c = 0; c < NCLS; ++c) rowexp[c * 128 + q * 32 + lane] = (short)row_scale(special_point(x, y, z), top[0][c], A.redo);
     }
@@ -980,12 +1000,14 @@ __device__ __forceinline__ void tile_role(const Args& A, const State& S, int tw)
         float ext = 0.f;
 #pragma unroll
         for (int c = 0; c < 3; ++c) ext = have ? fmaxf(ext, fmaxf(fabsf(lo[c]), fabsf(hi[c]))) : 0.f;
-        float err = 2.0e-7f * ext, amax = 0.f;  // 2^-23 + 2^-24 (the widened edge's rounding) = 1.8e-7
+        const float err = 2.0e-7f * ext;  // 2^-23 + 2^-24 (the widened edge's rounding) = 1.8e-7
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
             lo[c] -= err;
             hi[c] += err;
         }
+        float amax = 0.f;
+        bool exact = err > NEAR;
         for (int i = lane; i < MAX_PANELS / 32; i += 32) pbits[i] = 0u;
         __syncwarp();
         unsigned char* nkeep = S.nkeep + b * MAX_SHELLS;
@@ -1022,6 +1044,7 @@ __device__ __forceinline__ void tile_role(const Args& A, const State& S, int tw)
                 const int s = sb + lane;
                 int nk = 0;
                 bool big = false;
+                int atom = -1;  // of a kept shell within CLOSE of the box
                 if (s < nshell) {
                     const int4 rec = __ldg(A.S.shell + s);
                     const int L = rec.y & 0xFF, np = rec.w, pan = rec.y >> 16;
@@ -1044,6 +1067,7 @@ __device__ __forceinline__ void tile_role(const Args& A, const State& S, int tw)
                         if (nk == q + 1) amax = fmaxf(amax, a);
                     }
                     big = big && nk > 0;
+                    if (nk > 0 && br.dmin < CLOSE * CLOSE) atom = rec.x;
                     nkeep[s] = (unsigned char)nk;
                     if (nk > 0) atomicOr(pbits + (pan >> 5), 1u << (pan & 31));
                 }
@@ -1051,6 +1075,15 @@ __device__ __forceinline__ void tile_role(const Args& A, const State& S, int tw)
                 const int at = nbig + __popc(mb & ((1u << lane) - 1u));
                 if (big && at < MAX_BIG) bigl[at] = (unsigned short)s;
                 nbig += __popc(mb);
+                for (unsigned mc = __ballot_sync(0xffffffffu, atom >= 0); mc; mc &= mc - 1) {
+                    const double* at = A.B.atoms + 4 * __shfl_sync(0xffffffffu, atom, __ffs(mc) - 1);
+                    const float ax = (float)(__ldg(at) - ox), ay = (float)(__ldg(at + 1) - oy), az = (float)(__ldg(at + 2) - oz);
+#pragma unroll
+                    for (int q = 0; q < NQ; ++q) {
+                        const float dx = fx[q] - ax, dy = fy[q] - ay, dz = fz[q] - az;
+                        if (q < nsub && special[q] == 0) exact |= fmaf(dx, dx, fmaf(dy, dy, dz * dz)) < CLOSE * CLOSE;
+                    }
+                }
             }
             __syncwarp();
             for (int pb = 0; pb < A.S.npanel; pb += 32) {
@@ -1063,7 +1096,7 @@ __device__ __forceinline__ void tile_role(const Args& A, const State& S, int tw)
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
         short* rowexp = S.rowexp + b * 3 * 128;
-        if (sqrtf(amax) * err > WIDE) {
+        if (__any_sync(0xffffffffu, exact || sqrtf(amax) * err > WIDE)) {
             wide_scales<NCH>(A, t, nkeep, rowexp, ref[0], NCLS > 1 ? ref[1] : 0.f, NCLS > 2 ? ref[2] : 0.f);
             if (lane == 0) S.npan[b] = npan;
             __syncwarp();
@@ -1090,7 +1123,7 @@ __device__ __forceinline__ void tile_role(const Args& A, const State& S, int tw)
                 dd[q] = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
                 dq[q] = fmaxf(fabsf(dx), fmaxf(fabsf(dy), fabsf(dz)));
             }
-            point_bounds<NCLS>(A.S.prim_lg + rec.z, nk, L, dd, dq, err, top);
+            point_bounds<NCLS, false>(A.S.prim_lg + rec.z, nk, L, dd, dq, top);
         }
 #pragma unroll
         for (int q = 0; q < NQ; ++q)
