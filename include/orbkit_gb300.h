@@ -137,7 +137,13 @@ int okg_fold_coeff(const okg_basis* basis, int nmo, const double* d_csph, double
 int okg_unfold_coeff(const okg_basis* basis, int nmo, const double* d_ccart, double* d_csph, okg_stream stream);
 
 /* Large okg_rho, okg_eval_mo, okg_rho_backward and okg_ci_*_matrix calls run on the tensor
- * cores with bounded waits between the warps of a block.  Where a wait expires the call's
+ * cores.  Accuracy there: an MO value is within n 2^-50 max|C| max|AO| of the exact sum (n AOs,
+ * its largest coefficient, the largest AO at the point; of a derivative, in any direction),
+ * where small calls are within n 2^-53 sum |C| |AO|: an orbital that is many orders of
+ * magnitude below the AOs at a point has that many digits less there.  Likewise the detCI forms
+ * relative to the largest MO of a point and the largest coefficient of a row, and the adjoint's
+ * sums relative to the largest values of 64 points.
+ * These calls have bounded waits between the warps of a block.  Where a wait expires the call's
  * general kernel computes the outputs on the device behind it, so that they are complete
  * in any case: okg_wait_status reports OKG_OK and 0, and need not be called.
  * okg_set_wait_limit sets the polls per wait (default 2^24, >= 0) in the calls that the
