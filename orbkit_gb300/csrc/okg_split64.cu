@@ -16,8 +16,8 @@
 //     2^(-14 - 8 w); w = 0..6 are kept, 7 accumulators per MO;
 //   * an accumulator adds w + 1 products per column.  Up to 146 columns the FP32 accumulators of
 //     tcgen05.mma are exact (7 x 146 x 2^14 < 2^24); at the 160 columns of a group the last one
-//     (w = 6) could pass 2^24 with every digit at its end, and then rounds by one unit of
-//     2^-62, which the products left out exceed 6 times per column.
+//     (w = 6) could pass 2^24 with every digit at its end, and then rounds by a unit of 2^-62
+//     (the products left out may come to 6.1 x 2^-56 per column).
 //
 // Error.  A value is fixed-point relative to the largest AO of its point, a coefficient to the
 // largest of its MO: per column 2^-56 each of their product for the roundings, 6.1 x 2^-56 for
@@ -37,7 +37,8 @@
 //
 // Range.  What the digits cannot hold (a basis whose flags are raised, see split_prim; MOs
 // whose largest coefficient is not finite or not between 2^-900 and 2^1000; points at
-// |coordinate| >= 2^170; AO values from 2^985 on), and a wait that expires, raises the call's redo word, and the DFMA kernel, launched after this one, computes the call.
+// |coordinate| >= 2^170; AO values from 2^985 on), and a wait that expires, raises the call's
+// redo word, and the DFMA kernel, launched after this one, computes the call.
 //
 // Tile: 128 operand rows (2 x 128 with second derivatives): 128 points x 1 channel, or
 // 32 points x (value, d/dx, d/dy, d/dz) [+ 32 x (xx, yy, zz, unused)].  Persistent CTAs,
@@ -51,12 +52,12 @@
 // Every wait is bounded: one that expires raises the redo word, and the block drains its copies
 // and MMAs in flight and leaves.
 //
-// What bounds it (20 atoms, 180 AOs, 40 MOs, 160^3 points, density and gradient): 15.2 to
-// 16.7 ms (four runs) against 254 ms of the DFMA kernel; per 32-point tile and SM the FP64
-// pipe needs 13 K and the tensor cores 4 K of about 39 K cycles, the rest is the latency of
-// the integer code (digits, exponentials, conversion of the accumulators) behind a chain:
-// with more than 32 MOs only one set of accumulators fits tensor memory, and the MMAs of a
-// tile wait until the epilogue has read the previous tile's.
+// What bounds it (20 atoms, 180 AOs, 40 MOs, 160^3 points, density and gradient): 14.2 ms against
+// 254 ms of the DFMA kernel.  FP64 pipe 37 %, tensor pipe 11 % of active cycles (ncu, 96^3
+// points); the rest is latency, of tensor-memory loads and of the integer code (digits,
+// exponentials, conversion of the accumulators), behind a chain: with more than 32 MOs only one
+// set of accumulators fits tensor memory, and the MMAs of a tile wait until the epilogue has
+// read the previous tile's.
 #include <math.h>
 
 #include <mutex>
@@ -71,7 +72,7 @@ namespace sp {
 
 using namespace mx;
 
-constexpr int GROUP = 10;               // panels per accumulation (exact FP32 sums: see the header)
+constexpr int GROUP = 10;               // panels per accumulation (FP32 sums: see the header)
 constexpr int MAX_SHELLS = 2048;
 constexpr int MAX_PANELS = 768;
 constexpr int NBUF = 4;                 // tile buffers
@@ -886,12 +887,12 @@ __device__ __forceinline__ int special_point(double x, double y, double z)
     const int h = max(__double2hiint(x) & 0x7FFFFFFF, max(__double2hiint(y) & 0x7FFFFFFF, __double2hiint(z) & 0x7FFFFFFF));
     return h >= 0x4A900000 ? ROW_OUT : h >= 0x41D00000 ? ROW_ZERO : 0;
 }
-// Row exponent of a point with the bound `top` (log2): 0.1 for the roundings of the bound, 0.05 for
-// those of the coordinates.
+// Row exponent of a point with the bound `top` (log2); 0.1 to spare: 0.0145 that digits7 asks for,
+// 0.05 for the roundings of the coordinates (WIDE), below 0.001 for those of the bound.
 __device__ __forceinline__ int row_scale(int special, float top, int* redo)
 {
     if (special == ROW_OUT || (!special && !(top <= 985.f))) *(volatile int*)redo = 1;
-    return special ? special : (int)ceilf(fminf(fmaxf(top + 0.15f, -950.f), 990.f));
+    return special ? special : (int)ceilf(fminf(fmaxf(top + 0.1f, -950.f), 990.f));
 }
 
 // The points' scales of a tile beyond WIDE or NEAR, or with points within CLOSE, with FP64
