@@ -7,6 +7,7 @@ bookkeeping.  The pool locks at most HELD_MAX bytes in all, in results that the 
 holds and in blocks that wait for a later result, of which there are at most WAIT_MAX bytes
 (release() frees them); beyond that, and where locking fails, a result is an ordinary array.
 """
+import collections
 import ctypes
 import os
 import threading
@@ -19,9 +20,10 @@ PINNED_MIN_BYTES = 256 << 10
 HELD_MAX = 4 << 30
 WAIT_MAX = 1 << 30
 
-_lock = threading.RLock()  # (a block may be given back by the collector inside the pool's own code)
-_waiting = []              # [(address, size)], oldest first
-_held = 0                  # bytes locked
+_lock = threading.Lock()
+_returned = collections.deque()  # blocks given back; the collector may do so inside the pool's own code
+_waiting = []                    # [(address, size)], oldest first
+_held = 0                        # bytes locked
 
 
 class _Block:
@@ -34,12 +36,12 @@ class _Block:
     def __del__(self):
         # (a forked child has the pages, but not the lock on them; at the interpreter's end the
         # pool may be gone first)
-        if _lock is not None and os is not None and self.pid == os.getpid():
+        if _returned is not None and os is not None and self.pid == os.getpid():
             _give(self.address, self.size)
 
 
 def _free(size):
-    """Waiting blocks freed, oldest first, at least `size` bytes if there are."""
+    """Waiting blocks freed, oldest first, at least `size` bytes if there are (with the lock)."""
     global _held
     while size > 0 and _waiting:
         address, n = _waiting.pop(0)
@@ -48,40 +50,63 @@ def _free(size):
         _lib.load().okg_host_free(ctypes.c_void_p(address))
 
 
+def _settle():
+    """Blocks given back join the waiting ones, unless the lock is taken: then its holder does it."""
+    while _returned and _lock.acquire(blocking=False):
+        try:
+            _drain()
+        finally:
+            _lock.release()
+
+
+def _drain():
+    while _returned:
+        _waiting.append(_returned.popleft())
+    _free(sum(n for _, n in _waiting) - WAIT_MAX)
+
+
 def _give(address, size):
+    _returned.append((address, size))
+    _settle()
+
+
+def _locked(f):
     with _lock:
-        _waiting.append((address, size))
-        _free(sum(n for _, n in _waiting) - WAIT_MAX)
+        _drain()
+        out = f()
+    _settle()
+    return out
 
 
 def _take(size):
     """(address, size) of a block of at least `size` bytes, or None."""
-    global _held
-    with _lock:
+    def take():
+        global _held
         fit = [i for i, b in enumerate(_waiting) if size <= b[1] <= 2 * size]
         if fit:
             return _waiting.pop(min(fit, key=lambda i: (_waiting[i][1], -i)))  # (the last used of the smallest)
         step = 1 << max(16, size.bit_length() - 4)  # (sizes in steps of 1/16 .. 1/8: blocks fit similar results)
-        size = -(-size // step) * step
-        _free(_held + size - HELD_MAX)
-        if _held + size > HELD_MAX:
+        n = -(-size // step) * step
+        _free(_held + n - HELD_MAX)
+        if _held + n > HELD_MAX:
             return None
         p = ctypes.c_void_p()
-        if _lib.load().okg_host_alloc(size, ctypes.byref(p)) != _lib.OKG_OK:
+        if _lib.load().okg_host_alloc(n, ctypes.byref(p)) != _lib.OKG_OK:
             return None
-        _held += size
-        return p.value, size
+        _held += n
+        return p.value, n
+
+    return _locked(take)
 
 
 def release():
     """Free the blocks that wait for a later result."""
-    with _lock:
-        _free(_held)
+    _locked(lambda: _free(_held))
 
 
 def held():
     """Bytes of page-locked memory in results and waiting."""
-    return _held
+    return _locked(lambda: _held)
 
 
 class Result:
