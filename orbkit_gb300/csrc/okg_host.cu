@@ -6,11 +6,13 @@ using namespace okg;
 extern "C" int okg_host_alloc(size_t bytes, void** out)
 {
     if (!bytes || !out) return set_error(OKG_ERR_ARG, "okg_host_alloc: bad argument");
+    const RelaxedCapture guard;
     return cuda_status(cudaHostAlloc(out, bytes, cudaHostAllocPortable), "okg_host_alloc");
 }
 
 extern "C" int okg_host_free(void* p)
 {
+    const RelaxedCapture guard;
     return p ? cuda_status(cudaFreeHost(p), "okg_host_free") : OKG_OK;
 }
 

@@ -330,6 +330,16 @@ SplitLayout split_layout(const std::vector<Shell>& shells, const std::vector<int
                          const std::vector<double>& comp_g, const int* order);
 const uint64_t* split_exp_table();                   // host, OKG_SPLIT_EXP entries
 
+// While it lives, this host thread may allocate and free although a stream is being captured, by
+// this thread or another: under the default capture mode such a call fails and ends that capture.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    RelaxedCapture(const RelaxedCapture&) = delete;
+    RelaxedCapture& operator=(const RelaxedCapture&) = delete;
+};
+
 // Polls of the bounded device waits of a call from this host thread.
 long long split_wait_limit();
 

@@ -1400,6 +1400,7 @@ cudaMemPool_t workspace_pool(int device)
         props.allocType = cudaMemAllocationTypePinned;
         props.location.type = cudaMemLocationTypeDevice;
         props.location.id = device;
+        const RelaxedCapture guard;
         cudaMemPool_t p = nullptr;
         if (cudaMemPoolCreate(&p, &props) != cudaSuccess) {
             (void)cudaGetLastError();

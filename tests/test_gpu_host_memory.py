@@ -141,3 +141,39 @@ def test_evaluation_that_raises(core, monkeypatch):
     monkeypatch.undo()
     gc.collect()
     assert numpy.array_equal(orbitals(core, qc, 128), want)
+
+
+@pytest.mark.parametrize("thread", [False, True])
+def test_while_a_graph_is_captured(core, thread):
+    """Blocks locked and freed while a stream is captured (a result made by another thread, results
+    that the collector drops): the capture holds, and the results stay page-locked."""
+    import torch
+    from orbkit_gb300 import hostmem
+    x = torch.arange(1024.0, device="cuda")
+    torch.cuda.synchronize()
+    addresses = []
+
+    def work():
+        r = hostmem.Result(1 << 17)
+        addresses.append(r.address)
+        r.array[:] = 1.0
+        del r
+        hostmem.release()
+
+    gc.collect()
+    hostmem.release()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = x * 2.0
+        if thread:
+            t = threading.Thread(target=work)
+            t.start()
+            t.join()
+        else:
+            work()
+        z = y + 1.0
+    assert addresses[0] is not None
+    x.fill_(3.0)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert bool((z == 7.0).all())
