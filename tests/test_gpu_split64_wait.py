@@ -179,3 +179,22 @@ def test_wait_limit_argument_checked(core):
     from orbkit_gb300 import _lib
     with pytest.raises(_lib.OkgError):
         _lib.check(_lib.load().okg_set_wait_limit(-1))
+
+
+@pytest.mark.parametrize("flux", [False, True])
+@pytest.mark.parametrize("nmo", [20, 42])
+@pytest.mark.parametrize("last", [False, True])
+def test_detci_points_beyond_the_digits(core, nmo, flux, last):
+    """Such points in any of a block's tiles, or in the last one alone: they have the general
+    kernel's bits, the others the usual ones."""
+    npts = 150007
+    at = numpy.array([npts - 1]) if last else numpy.concatenate([numpy.arange(0, npts, 997), numpy.arange(70000, 70128)])
+
+    def change(mo, drv, q):
+        mo[nmo // 2, at] = numpy.where(at % 2 == 0, numpy.inf, -1e305)
+
+    got, general, usual = (ci_run(nmo, npts, flux, change=c, pad=p) for c, p in ((change, 0), (change, 65 - nmo), (None, 0)))
+    beyond = numpy.zeros(npts, dtype=bool)
+    beyond[at] = True
+    assert numpy.array_equal(got[:, beyond], general[:, beyond], equal_nan=True)
+    assert numpy.array_equal(got[:, ~beyond], usual[:, ~beyond])
