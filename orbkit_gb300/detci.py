@@ -79,7 +79,7 @@ def _zero_terms(zero):
 
 
 def _sing_terms(sing):
-    # plain lists of numbers and of index pairs within 32 bits convert in one go; anything else
+    # plain lists of numbers and of index pairs in 0 .. 2^31 - 1 convert in one go; anything else
     # (ragged rows, objects, device tensors, indices that do not fit) entry by entry
     try:
         coef, pairs = numpy.asarray(sing[0]), numpy.asarray(sing[1])
@@ -88,7 +88,7 @@ def _sing_terms(sing):
     else:
         if coef.ndim == 1 and coef.dtype.kind in "fiu" and pairs.ndim == 2 and pairs.shape[1] >= 2 and \
                 pairs.dtype.kind in "iu" and 0 < len(coef) == len(pairs) and \
-                -2 ** 31 <= pairs[:, :2].min() and pairs[:, :2].max() < 2 ** 31:
+                0 <= numpy.bitwise_or.reduce(pairs[:, :2], axis=None) < 2 ** 31:  # (every one of them)
             return coef.astype(numpy.float64), numpy.ascontiguousarray(pairs[:, :2], dtype=numpy.int32)
     coef = numpy.asarray([float(c) for c in sing[0]], dtype=numpy.float64)
     pairs = numpy.asarray([[int(p[0]), int(p[1])] for p in sing[1]], dtype=numpy.int32).reshape(-1, 2)
